@@ -53,6 +53,35 @@ void check(cudaError_t err, const char* what) {
     if (err != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(err));
 }
 
+// A group of one rank has no reader for a payload: its collectives are one pass that quantizes and decodes in
+// registers (roundtrip_kernels.cu), half to a third of the phases' memory traffic and one launch.  The pass writes
+// while other blocks still read, so the output has to be the input itself or disjoint from it, and the residual
+// disjoint from both; the phases, which meet between reading and writing, keep every other call.
+bool one_pass_ok(int world, uintptr_t x, uintptr_t out, uintptr_t residual, int64_t nbytes) {
+    if (world != 1) return false;
+    const auto apart = [nbytes](uintptr_t a, uintptr_t b) {
+        return a + static_cast<uintptr_t>(nbytes) <= b || b + static_cast<uintptr_t>(nbytes) <= a;
+    };
+    return (x == out || apart(x, out)) && (residual == 0 || (apart(residual, x) && apart(residual, out)));
+}
+
+LbcRoundtrip one_pass(int dtype, int group, int bit, uintptr_t x, uintptr_t out, uintptr_t residual, int64_t numel,
+                      int stages, bool update_residual, bool own_error, int max_blocks) {
+    LbcRoundtrip p{};
+    p.dtype = dtype;
+    p.group_size = group;
+    p.bit = bit;
+    p.x = reinterpret_cast<const void*>(x);
+    p.residual = reinterpret_cast<const void*>(residual);
+    p.out = reinterpret_cast<void*>(out);
+    p.residual_out = update_residual ? reinterpret_cast<void*>(residual) : nullptr;
+    p.numel = numel;
+    p.passes = stages;
+    p.own_error = residual != 0 && update_residual && own_error ? 1 : 0;
+    p.max_blocks = max_blocks;
+    return p;
+}
+
 struct Regions {        // byte offsets inside every rank's arena, for one chunk
     int64_t rs, ag, gather;
     int64_t shard_stride, gather_stride;
@@ -114,6 +143,12 @@ class FusedAllReducePlan {
         if (numel == 0) return 0;
         if (stages == 1 && gather_off_.size() != 2) throw std::invalid_argument("this plan has no gather region");
         cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
+        if (one_pass_ok(world_, x, out, residual, numel * elem_bytes_)) {
+            const LbcRoundtrip p = one_pass(dtype_, group_, bit_, x, out, residual, numel, stages == 1 ? 1 : 2,
+                                            update_residual, ef_local, max_blocks_);
+            check(lbc_roundtrip(&p, stream), "roundtrip");
+            return 1;
+        }
         const int parity = static_cast<int>(epoch & 1u);
         // chunk boundaries keep every chunk's shards whole multiples of eight groups
         const int64_t unit = int64_t(group_) * kAlignGroups * world_;
@@ -167,6 +202,16 @@ class FusedAllReducePlan {
         return launches;
     }
 
+    // All-gather of one rank: out = decode(encode(x)), one pass.  False when the call is not one for it (more ranks,
+    // overlapping buffers): the caller then quantizes, waits and decodes.
+    bool gather_own(uintptr_t x, uintptr_t out, int64_t numel, uintptr_t stream_ptr) {
+        if (numel < 0 || numel > max_numel_) throw std::invalid_argument("numel exceeds the workspace capacity");
+        if (!one_pass_ok(world_, x, out, 0, numel * elem_bytes_)) return false;
+        const LbcRoundtrip p = one_pass(dtype_, group_, bit_, x, out, 0, numel, 1, false, false, max_blocks_);
+        check(lbc_roundtrip(&p, reinterpret_cast<cudaStream_t>(stream_ptr)), "roundtrip");
+        return true;
+    }
+
     // Reduce-scatter to a dense shard: rank r receives the reduced elements [r * shard_numel, (r + 1) * shard_numel)
     // in `out_shard` (shard_numel = shard_groups * group size; the caller has zeroed what lies past the tensor's
     // end).  With a residual, error feedback uses this rank's own quantization error, written back in place.
@@ -176,6 +221,12 @@ class FusedAllReducePlan {
         if (numel < 0 || numel > max_numel_) throw std::invalid_argument("numel exceeds the workspace capacity");
         if (numel == 0) return 0;
         cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
+        if (one_pass_ok(world_, x, out_shard, residual, numel * elem_bytes_)) {
+            const LbcRoundtrip p = one_pass(dtype_, group_, bit_, x, out_shard, residual, numel, 1, update_residual,
+                                            true, max_blocks_);
+            check(lbc_roundtrip(&p, stream), "roundtrip");
+            return 1;
+        }
         const int parity = static_cast<int>(epoch & 1u);
         const int64_t groups = ceil_div(numel, group_);
         const int64_t shard_groups = round_up(ceil_div(groups, world_), kAlignGroups);
@@ -430,6 +481,13 @@ class PipeAllReducePlan {
         if (numel == 0) return 0;
         if (stages != 1 && stages != 2) throw std::invalid_argument("stages must be 1 or 2");
         cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
+        if (phase_mask == LBC_PIPE_ALL && profile_ == 0 &&
+            one_pass_ok(world_, x, out, residual, numel * (dtype_ == LBC_FP32 ? 4 : 2))) {
+            const LbcRoundtrip p = one_pass(dtype_, group_, bit_, x, out, residual, numel, stages, update_residual,
+                                            ef_local, max_blocks_);
+            check(lbc_roundtrip(&p, stream), "roundtrip");
+            return 1;
+        }
         LbcPipe p{};
         p.dtype = dtype_;
         p.group_size = group_;
@@ -506,6 +564,8 @@ void bind_fused_plan(py::module_& m) {
         .def("all_reduce", &FusedAllReducePlan::all_reduce, py::arg("x"), py::arg("out"), py::arg("residual"),
              py::arg("numel"), py::arg("stages"), py::arg("scale"), py::arg("update_residual"), py::arg("ef_local"),
              py::arg("epoch"), py::arg("stream"))
+        .def("gather_own", &FusedAllReducePlan::gather_own, py::arg("x"), py::arg("out"), py::arg("numel"),
+             py::arg("stream"))
         .def("reduce_scatter", &FusedAllReducePlan::reduce_scatter, py::arg("x"), py::arg("out_shard"),
              py::arg("residual"), py::arg("numel"), py::arg("scale"), py::arg("update_residual"), py::arg("epoch"),
              py::arg("stream"));

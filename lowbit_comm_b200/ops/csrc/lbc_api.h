@@ -154,6 +154,21 @@ cudaError_t lbc_pipe_gate(uint8_t* const* arena, int world, int rank, int64_t ct
 int lbc_pipe_stage_bytes(int dtype, int group_size, int bit, int world, int stages, int with_residual,
                          int with_prepared);
 
+// ---- collectives of one rank: quantize and decode in registers, no payload (roundtrip_kernels.cu) -----------
+typedef struct {
+    int dtype, group_size, bit;
+    const void* x;             // T[numel]
+    const void* residual;      // optional T[numel]: prepared = T(x + residual)
+    void* out;                 // T[numel]: T(y), y = decode(encode(prepared)); x itself or disjoint from it
+    void* residual_out;        // optional T[numel] = T(prepared - y) (only with `residual`; may alias it)
+    int64_t numel;
+    int passes;                // 2: T(y) is encoded and decoded once more (the two-stage all-reduce)
+    int own_error;             // residual_out = T(prepared - code * step) of the first encoding, one rounding
+    int max_blocks;            // 0 = one block per tile
+} LbcRoundtrip;
+
+cudaError_t lbc_roundtrip(const LbcRoundtrip* p, cudaStream_t stream);
+
 // ---- general path: top-k, 4-bit code-books, stochastic rounding --------------
 typedef struct {
     int dtype, group_size, bit, topk, quant_type, stochastic, compact;

@@ -1,0 +1,201 @@
+// Collectives of a group of one rank (a one-GPU DDP job, the inter-node stage of a single node): the payload has no
+// reader but its writer, so quantize and decode meet in registers and the payload never exists in memory.
+//
+// Math is identical, bit for bit, to the sequences of quant_push_kernel / reduce_kernel (fast_kernels.cu) and to the
+// phases of pipe_allreduce_kernel (pipe_kernels.cu) on one rank:
+//   prepared = T(x + residual), s = T(max |prepared|), q = clamp(rint(prepared * (L / max(s, 1e-6)))),
+//   y32 = fma(q, s / L, 0), out = T(y32), residual = T(prepared - y32)          (passes == 1)
+// and with passes == 2 (the two-stage all-reduce) T(y32) is quantized and decoded once more.
+// Reference: quantization/quant_pack_kernel.cu:84-163, quantization/dequant_reduce_kernel.cu:38-69, 150-221.
+//
+// What bounds it: memory.  x is read and out written once (with error feedback the residual too), which is all that
+// the result needs; the phases also wrote and read the payload, read the input's row twice and met at a grid-wide
+// flag.  A block per tile and no loop over tiles: on a B200 a persistent grid of the same kernel moved 5.9 TB/s where
+// the full grid moves 6.7-6.9, because the blocks of one wave end at different times and the next ones fill in.
+// Measured (bf16, int8 groups of 64): 512 Mi elements 919 -> 314 us (6.8 TB/s), 13.1 M elements 41.1 -> 13.9 us,
+// 124 M elements in 11 buckets with error feedback 636 -> 320 us (the rest is the host).
+#include "codec_device.cuh"
+#include "common.cuh"
+#include "lbc_api.h"
+
+namespace lbc {
+
+// What a receiver of the codes of 16 rounded values decodes, in fp32 before the rounding to T.  With `own_error` the
+// values are replaced by this rank's quantization error, one rounding: fma(-code, step, value).
+template <typename T, int G, int BIT>
+__device__ __forceinline__ void roundtrip16(float (&v)[16], float (&y)[16], bool own_error) {
+    constexpr int lim = BIT == 8 ? 127 : 7;
+    float amax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
+    // the values are exact in T, so their largest magnitude is the stored scale without a rounding
+    const float stored = group_max<G>(amax);
+    const float mul = float(lim) / fmaxf(stored, 1.0e-6f);
+    const float step = stored / float(lim);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        // the clamped sum is kRoundMagic + code exactly, and so is the difference (+0 for code 0, as the decoder has it)
+        const float code = __uint_as_float(quant_bits<lim>(v[i], mul)) - kRoundMagic;
+        y[i] = __fmaf_rn(code, step, 0.0f);
+        if (own_error) v[i] = __fmaf_rn(-code, step, v[i]);
+    }
+}
+
+// 16 elements as loaded.  Plain (not read-only) loads: `out` and the residual may be the buffers that were read, and a
+// thread only ever writes the elements that it has read itself.
+template <typename T> struct Raw16 {
+    U8x32 part[sizeof(T) / 2];
+};
+__device__ __forceinline__ U8x32 ld32_once(const void* p) {
+    U8x32 v;
+    asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]),
+                   "=r"(v.w[6]), "=r"(v.w[7]) : "l"(p));
+    return v;
+}
+template <typename T>
+__device__ __forceinline__ Raw16<T> raw16(const T* p) {
+    Raw16<T> r;
+#pragma unroll
+    for (int h = 0; h < int(sizeof(T)) / 2; ++h) r.part[h] = ld32_once(p + 16 / (sizeof(T) / 2) * h);
+    return r;
+}
+template <typename T>
+__device__ __forceinline__ void up16(const Raw16<T>& r, float (&v)[16]) {
+    if constexpr (sizeof(T) == 2) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) Src<T>::up2(r.part[0].w[i], v[2 * i], v[2 * i + 1]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r.part[i / 8].w[i % 8]);
+    }
+}
+
+// kResidual: the input is T(x + residual).  U chunks of 16 elements per thread are loaded before the first is computed.
+template <typename T, int G, int BIT, bool kResidual, int U>
+__global__ void __launch_bounds__(kThreads) roundtrip_kernel(const LbcRoundtrip p) {
+    constexpr int lanes = G / kElemsPerThread;
+    constexpr int tile_chunks = kThreads * U;
+    const T* x = static_cast<const T*>(p.x);
+    const T* res = static_cast<const T*>(p.residual);
+    T* out = static_cast<T*>(p.out);
+    T* rout = static_cast<T*>(p.residual_out);
+    const int64_t n = p.numel;
+    const int64_t chunks = (n + G - 1) / G * lanes;
+    const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) |
+                       reinterpret_cast<uintptr_t>(res) | reinterpret_cast<uintptr_t>(rout)) & 31) == 0;
+
+    auto compensate = [](float (&v)[16], const float (&r)[16]) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] += r[i];
+        round16<T>(v);
+    };
+    auto finish = [&](float (&v)[16], int64_t first, bool live) {     // convergent: the group maximum shuffles
+        const bool own_error = kResidual && p.own_error != 0;
+        float y[16];
+        roundtrip16<T, G, BIT>(v, y, own_error);
+        if (p.passes == 2) {
+            float z[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) z[i] = y[i];
+            round16<T>(z);
+            roundtrip16<T, G, BIT>(z, y, false);
+        }
+        if (!live) return;
+        if (kResidual && rout != nullptr) {
+            if (!own_error) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] -= y[i];
+            }
+            store16<T>(rout, first, n, vec, v);
+        }
+        store16<T>(out, first, n, vec, y);
+    };
+
+    for (int64_t c0 = int64_t(blockIdx.x) * tile_chunks; c0 < chunks; c0 += int64_t(gridDim.x) * tile_chunks) {
+        const int64_t mine = (c0 + threadIdx.x) * kElemsPerThread;
+        if (vec && (c0 + tile_chunks) * kElemsPerThread <= n) {       // a whole tile
+            Raw16<T> rx[U], rr[kResidual ? U : 1];
+#pragma unroll
+            for (int j = 0; j < U; ++j) {
+                rx[j] = raw16(x + mine + j * (kThreads * kElemsPerThread));
+                if (kResidual) rr[j] = raw16(res + mine + j * (kThreads * kElemsPerThread));
+            }
+#pragma unroll
+            for (int j = 0; j < U; ++j) {
+                float v[16];
+                up16<T>(rx[j], v);
+                if (kResidual) {
+                    float r[16];
+                    up16<T>(rr[j], r);
+                    compensate(v, r);
+                }
+                finish(v, mine + j * (kThreads * kElemsPerThread), true);
+            }
+        } else {
+            for (int j = 0; j < U; ++j) {
+                const int64_t first = mine + j * (kThreads * kElemsPerThread);
+                const bool live = first / kElemsPerThread < chunks;
+                float v[16];
+                load16<T>(x, first, n, vec, v, false);                // zeros past the end
+                if (kResidual) {
+                    float r[16];
+                    load16<T>(res, first, n, vec, r, false);
+                    compensate(v, r);
+                }
+                finish(v, first, live);
+            }
+        }
+    }
+}
+
+template <typename T, int G, int BIT>
+static cudaError_t launch_roundtrip(const LbcRoundtrip* p, cudaStream_t stream) {
+    const int64_t chunks = (p->numel + G - 1) / G * (G / kElemsPerThread);
+    const int64_t one = (chunks + kThreads - 1) / kThreads;           // blocks of one chunk per thread
+    auto grid = [&](int64_t blocks) {
+        const int64_t cap = p->max_blocks > 0 ? p->max_blocks : int64_t(1) << 30;
+        return unsigned(blocks < cap ? blocks : cap);
+    };
+    if (p->residual != nullptr) {
+        roundtrip_kernel<T, G, BIT, true, 1><<<grid(one), kThreads, 0, stream>>>(*p);
+        return cudaGetLastError();
+    }
+    // Two chunks per thread (64 bytes in flight) once there are many waves of blocks: 512 Mi bf16 elements take 310 us
+    // against 322-342 with one chunk, 13 M take 12.5 us either way, and fewer leave SMs without a block.  fp32 chunks and
+    // chunks with a residual have 64 bytes in flight already.
+    if constexpr (sizeof(T) == 2) {
+        if (one > 8 * lbc_default_max_blocks()) {
+            roundtrip_kernel<T, G, BIT, false, 2><<<grid((one + 1) / 2), kThreads, 0, stream>>>(*p);
+            return cudaGetLastError();
+        }
+    }
+    roundtrip_kernel<T, G, BIT, false, 1><<<grid(one), kThreads, 0, stream>>>(*p);
+    return cudaGetLastError();
+}
+
+}  // namespace lbc
+
+extern "C" {
+
+cudaError_t lbc_roundtrip(const LbcRoundtrip* p, cudaStream_t stream) {
+    if (p == nullptr || p->numel < 0 || (p->passes != 1 && p->passes != 2)) return cudaErrorInvalidValue;
+    if (p->residual == nullptr && (p->residual_out != nullptr || p->own_error)) return cudaErrorInvalidValue;
+    if (p->numel == 0) return cudaSuccess;
+    if (p->x == nullptr || p->out == nullptr) return cudaErrorInvalidValue;
+#define LBC_CASE(TT, GG, BB) \
+    if (p->group_size == GG && p->bit == BB) return lbc::launch_roundtrip<TT, GG, BB>(p, stream);
+#define LBC_TYPE(TT) \
+    LBC_CASE(TT, 64, 8) LBC_CASE(TT, 32, 8) LBC_CASE(TT, 16, 8) LBC_CASE(TT, 64, 4) LBC_CASE(TT, 32, 4) LBC_CASE(TT, 16, 4)
+    switch (p->dtype) {
+        case LBC_BF16: LBC_TYPE(__nv_bfloat16) break;
+        case LBC_FP16: LBC_TYPE(__half) break;
+        case LBC_FP32: LBC_TYPE(float) break;
+        default: break;
+    }
+#undef LBC_TYPE
+#undef LBC_CASE
+    return cudaErrorInvalidValue;
+}
+
+}  // extern "C"

@@ -566,6 +566,12 @@ class FusedWorkspace:
         parity = epoch & 1
         if geo.numel == 0:
             return outs
+        if g.world_size == 1 and self._native is not None and outs[0].is_contiguous() and outs[0].dtype == x.dtype \
+                and outs[0].numel() == geo.numel and outs[0].device == x.device:
+            # nobody else reads this rank's payload: it is encoded and decoded in registers, one launch
+            if self._native.gather_own(x.data_ptr(), outs[0].data_ptr(), geo.numel, _current_stream_ptr(x.device)):
+                self.launches += 1
+                return outs
         self._k1_broadcast(x.reshape(-1), None, None, None, geo, epoch, parity)
         region = self.gather_off[parity]
         self.ext.wait_signal(g.wait_all(self.channel, PHASE_REDUCE_SCATTER, epoch), None)

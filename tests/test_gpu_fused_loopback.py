@@ -13,7 +13,7 @@ import torch
 
 from lowbit_comm_b200.config import CompressionConfig
 from lowbit_comm_b200.exceptions import AsyncCommunicationError
-from lowbit_comm_b200.ops import oracle
+from lowbit_comm_b200.ops import codec, oracle
 from lowbit_comm_b200.parallel.fused import FusedWorkspace, geometry, run_loopback
 from lowbit_comm_b200.parallel.peer_memory import PHASE_P2P_DATA, PeerGroup
 
@@ -559,3 +559,58 @@ def test_canaries_catch_a_write_past_a_region(ext):
         groups[1].check_canaries()
     finally:
         PeerGroup.close_loopback(groups, check=False)
+
+
+@pytest.mark.parametrize("dtype,bit,group,passes", [("bf16", 8, 64, 1), ("fp16", 4, 32, 2), ("fp32", 8, 16, 1)])
+@pytest.mark.parametrize("engine", ("pipe", "legacy"))
+def test_one_rank_pass_matches_the_codec(ext, engine, dtype, bit, group, passes):
+    """The one-pass form of a one-rank all-reduce against quantize + decode through a payload: unaligned views, the
+    edges of its tiles, the size from which a thread takes two chunks, both residual rules, special values, and
+    overlapping buffers (which the phases keep)."""
+
+    cfg = CompressionConfig(bit=bit, group_size=group, allow_experimental=True)
+    max_numel = 8 * int(ext.default_max_blocks()) * 4096 + 70_001 if dtype == "bf16" else 300_000
+    groups, wss = _make(1, dtype, cfg, max_numel, engine=engine)
+    try:
+        ws = wss[0]
+        if engine == "legacy":
+            groups[0].process_group = object()          # the native plan serves real process groups only
+            ws._build_native()
+        data = torch.empty(max_numel + 64, dtype=DT[dtype], device="cuda").normal_(std=1e-2)
+        special = torch.tensor([float("inf"), -float("inf"), float("nan"), 0.0, -0.0, 1e-7], dtype=DT[dtype])
+
+        def through_payloads(x, residual, local):
+            prep = torch.empty_like(x)
+            cur, err = x, None
+            for k in range(passes):
+                res = residual if k == 0 else None
+                payload = codec.quantize_tensor(cur, cfg, residual=res, prepared_out=prep if k == 0 else None)
+                y, rout = torch.empty_like(x), torch.empty_like(x)
+                codec.inplace_dequantize_reduce_mean_update_error_feedback([payload], prep, y, rout, cfg)
+                if k == 0 and local:
+                    ext.quant_push(x, residual, None, rout, [payload.data_ptr()],
+                                   ext.PUSH_BROADCAST, 0, -(-x.numel() // group), 0, group, bit, None, 0)
+                    err = rout
+                cur = y
+            return cur, err if local else rout
+
+        for n, skew in ((max_numel, 0), (1, 0), (4096 * 3 + 17, 0), (4095, 1), (70_001, 8), (group, 3)):
+            for residual, mode in ((False, "reference"), (True, "reference"), (True, "local")):
+                x = data[skew:skew + n].clone() if skew == 0 else data[skew:skew + n]
+                x = x if skew == 0 else torch.cat([data[:skew], x])[skew:]
+                if n > 600:
+                    x[500:506] = special.to(x.device)
+                r = torch.empty(n, dtype=x.dtype, device="cuda").normal_(std=1e-4) if residual else None
+                want, want_r = through_payloads(x, r, mode == "local")
+                ws.all_reduce(x, residual=r, stages=passes, ef_mode=mode)
+                assert torch.equal(x.view(torch.uint8), want.view(torch.uint8)), (n, skew, mode)
+                if residual:
+                    assert torch.equal(r.view(torch.uint8), want_r.view(torch.uint8)), (n, skew, mode)
+        base = data[:50_064].clone()
+        want, _ = through_payloads(base[64:].clone(), None, False)
+        ws.all_reduce(base[64:], out=base[:50_000], stages=passes)
+        assert torch.equal(base[:50_000].view(torch.uint8), want.view(torch.uint8))
+        groups[0].check_status()
+    finally:
+        groups[0].process_group = None
+        PeerGroup.close_loopback(groups)
