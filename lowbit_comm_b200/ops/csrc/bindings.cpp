@@ -271,6 +271,42 @@ void quant_general_push(const at::Tensor& x, const std::optional<at::Tensor>& re
     cuda_check(lbc_quant_general(&p, at::cuda::getCurrentCUDAStream()), "lbc_quant_general(push)");
 }
 
+// The general all-reduce of one rank in one pass.  False (nothing launched) when the output is not like the input or
+// the buffers overlap in a way the pass does not allow: it writes `out` and the residual while other blocks still read.
+bool roundtrip_general(const at::Tensor& x, const std::optional<at::Tensor>& residual, at::Tensor& out,
+                       const std::optional<at::Tensor>& residual_out, int group_size, int bit, int topk, int quant_type,
+                       bool stochastic, uint64_t seed, int passes, int max_blocks) {
+    check_dense(x, "input");
+    check_dense(out, "output");
+    if (out.scalar_type() != x.scalar_type() || out.numel() != x.numel() || out.device() != x.device()) return false;
+    c10::cuda::CUDAGuard guard(x.device());
+    LbcRoundtripGeneral p{};
+    p.dtype = dtype_code(x);
+    p.group_size = group_size;
+    p.bit = bit;
+    p.topk = topk;
+    p.quant_type = quant_type;
+    p.stochastic = stochastic ? 1 : 0;
+    p.x = x.data_ptr();
+    p.residual = opt_ptr(residual, x, "residual");
+    p.out = out.data_ptr();
+    p.residual_out = const_cast<void*>(opt_ptr(residual_out, x, "residual_out"));
+    p.numel = x.numel();
+    p.passes = passes;
+    p.seed = seed;
+    p.max_blocks = max_blocks;
+    const auto same_or_apart = [&](const void* a, const void* b, bool may_be_same) {
+        const uintptr_t u = reinterpret_cast<uintptr_t>(a), v = reinterpret_cast<uintptr_t>(b), bytes = x.nbytes();
+        return a == nullptr || b == nullptr || (may_be_same && u == v) || u + bytes <= v || v + bytes <= u;
+    };
+    if (!same_or_apart(p.x, p.out, true) || !same_or_apart(p.residual, p.residual_out, true) ||
+        !same_or_apart(p.residual, p.out, false) || !same_or_apart(p.residual_out, p.x, false) ||
+        !same_or_apart(p.residual_out, p.out, false) || !same_or_apart(p.residual, p.x, false))
+        return false;
+    cuda_check(lbc_roundtrip_general(&p, at::cuda::getCurrentCUDAStream()), "lbc_roundtrip_general");
+    return true;
+}
+
 // Bounded wait, then one pass that decodes and sums every source payload, scales, and updates the residual.
 void reduce_general(const Ptrs& src, at::Tensor& out, int group_size, int bit, int topk, int quant_type, bool compact,
                     double scale, const std::optional<at::Tensor>& prepared, const std::optional<at::Tensor>& residual_out,
@@ -377,6 +413,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           py::arg("dst"), py::arg("group_size"), py::arg("bit"), py::arg("topk"), py::arg("quant_type"),
           py::arg("stochastic"), py::arg("compact"), py::arg("seed"), py::arg("signal") = py::none(),
           py::arg("max_blocks") = 0, py::arg("shard_groups") = 0);
+    m.def("roundtrip_general", &roundtrip_general, py::arg("x"), py::arg("residual"), py::arg("out"),
+          py::arg("residual_out"), py::arg("group_size"), py::arg("bit"), py::arg("topk"), py::arg("quant_type"),
+          py::arg("stochastic"), py::arg("seed"), py::arg("passes") = 1, py::arg("max_blocks") = 0);
     m.def("reduce_general", &reduce_general, py::arg("src"), py::arg("out"), py::arg("group_size"), py::arg("bit"),
           py::arg("topk"), py::arg("quant_type"), py::arg("compact"), py::arg("scale"), py::arg("prepared") = py::none(),
           py::arg("residual_out") = py::none(), py::arg("wait") = py::none(), py::arg("max_blocks") = 0,

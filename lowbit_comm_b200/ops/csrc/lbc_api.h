@@ -187,6 +187,7 @@ typedef struct {
     // Scatter (shard_groups > 0, with destinations): group g goes to dst[g / shard_groups] only, as group
     // g % shard_groups of a self-contained payload of shard_groups groups (a reduce-scatter's first half).
     int64_t shard_groups;
+    float thresholds[14];      // filled in by the launcher (code-books)
 } LbcQuantGeneral;
 
 typedef struct {
@@ -218,6 +219,21 @@ typedef struct {
                                // g % src_shard_groups of a payload of src_shard_groups groups (layout_groups unused)
 } LbcReduceGeneral;
 
+// One rank: encode and decode in registers, `passes` times; out = T(decode), residual_out = T(prepared - out).
+typedef struct {
+    int dtype, group_size, bit, topk, quant_type, stochastic;
+    const void* x;             // T[numel]
+    const void* residual;      // optional T[numel]: prepared = T(x + residual)
+    void* out;                 // T[numel], x itself or disjoint from it
+    void* residual_out;        // optional T[numel] (only with `residual`; may alias it)
+    int64_t numel;
+    int passes;                // 1 or 2
+    unsigned long long seed;
+    int max_blocks;            // 0 = library default
+    float thresholds[14];      // filled in by the launcher (code-books)
+} LbcRoundtripGeneral;
+
+cudaError_t lbc_roundtrip_general(const LbcRoundtripGeneral* p, cudaStream_t stream);
 cudaError_t lbc_quant_general(const LbcQuantGeneral* p, cudaStream_t stream);
 cudaError_t lbc_dequant_general(const LbcDequantGeneral* p, cudaStream_t stream);
 cudaError_t lbc_reduce_general(const LbcReduceGeneral* p, cudaStream_t stream);

@@ -108,13 +108,18 @@ class GeneralPeerWorkspace:
             return target
         g, cfg, ext = self.group, self.config, self.ext
         W, me = g.world_size, g.rank
-        nbytes = estimate_quantized_size(n, dtype=self.dtype, config=cfg).quantized_bytes
         epoch = g.next_epoch(self.channel)
         region = self.recv_off[epoch & 1]
         flat = x.reshape(-1)
         res = None if residual is None else residual.reshape(-1)
         keep = res if (res is not None and update_residual) else None      # `prepared` is parked here
         out_flat = target.reshape(-1)
+        if W == 1 and self.fused and ext.roundtrip_general(
+                flat, res, out_flat, keep, cfg.group_size, cfg.bit, cfg.topk, _QUANT_CODE[cfg.quant_type], cfg.stochastic,
+                _seed() if cfg.stochastic else 0, stages, self.max_blocks):
+            self.launches += 1        # one rank: nobody else reads the payload, it is encoded and decoded in registers
+            return target
+        nbytes = estimate_quantized_size(n, dtype=self.dtype, config=cfg).quantized_bytes
         dst = [g.addr(d, region + me * self.slot_bytes) for d in range(W)]
         if stages == 2:
             return self._two_stage(flat, out_flat, res, keep, n, epoch, region, dst, op, target)

@@ -183,3 +183,89 @@ def test_payload_size_is_validated(ext):
         codec.quantize_tensor(x, cfg, output=torch.empty(10, dtype=torch.uint8, device="cuda"))
     with pytest.raises(ValueError):
         codec.dequantize_tensor(torch.empty(10, dtype=torch.uint8, device="cuda"), (640,), cfg, dtype="bf16")
+
+
+@pytest.mark.parametrize("quant_type", ("normal", "uniform", "e3m0", "e2m1"))
+def test_codebook_codes_at_their_thresholds(ext, quant_type):
+    """Values next to the middle of two entries (and on the entries), where a code changes: the kernel counts
+    thresholds, the oracle searches the table."""
+
+    table = oracle.codebook(quant_type)[:15]
+    near = [table]
+    for mid in (table[:-1] + (table[1:] - table[:-1]) / 2,):
+        for toward in (-2.0, 2.0):
+            step = mid
+            for _ in range(3):
+                near.append(step)
+                step = torch.nextafter(step, torch.full_like(step, toward))
+    values = torch.cat(near)
+    for scale in (1.0, 0.7310584, 3.0e-7, 1.7e37):
+        groups = torch.zeros(-(-values.numel() // 15), 16)
+        flat = torch.zeros(groups.shape[0] * 15)
+        flat[:values.numel()] = values
+        groups[:, 1:] = flat.reshape(-1, 15)
+        groups[:, 0] = 1.0
+        x = (groups * scale).reshape(-1)
+        cfg = _cfg(bit=4, group_size=16, quant_type=quant_type)
+        assert torch.equal(codec.quantize_tensor(x.cuda(), cfg).cpu(), oracle.encode(x, cfg)), scale
+
+
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("bit,group,topk", [(8, 64, 0), (8, 16, 2), (4, 32, 1), (4, 64, 0)])
+def test_compact_records_through_warp_spans(ext, dtype, bit, group, topk):
+    """Payloads that start on 16 bytes move as a warp's span, others word by word; whole warps, ragged last warps,
+    and ends in the middle of a vector."""
+
+    cfg = _cfg(bit=bit, group_size=group, topk=topk, compact=True, quant_type="e2m1" if bit == 4 else "linear")
+    for n in (512 * 9, 512 * 8 + group + 1, 3 * group, 1):
+        x = _data(n, DTYPES[dtype], seed=n)
+        want = oracle.encode(x, cfg)
+        back = oracle.decode(want, n, cfg, dtype)
+        for skew in (0, 4, 16):
+            raw = torch.full((want.numel() + 64,), 0xA5, dtype=torch.uint8, device="cuda")
+            payload = raw[skew:skew + want.numel()]
+            codec.quantize_tensor(x.cuda(), cfg, output=payload)
+            assert torch.equal(payload.cpu(), want), (n, skew)
+            assert (raw[:skew] == 0xA5).all() and (raw[skew + want.numel():] == 0xA5).all()
+            got = codec.dequantize_tensor(payload, (n,), cfg, dtype=dtype)
+            assert torch.equal(got.cpu().view(torch.uint8), back.view(torch.uint8)), (n, skew)
+
+
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("bit,quant_type,topk,group", [(8, "linear", 1, 64), (4, "linear", 2, 32), (4, "e3m0", 0, 16),
+                                                       (4, "normal", 1, 64), (8, "linear", 2, 16)])
+@pytest.mark.parametrize("passes", (1, 2))
+def test_general_one_rank_pass_matches_the_codec(ext, dtype, bit, quant_type, topk, group, passes):
+    """encode + decode in registers against a payload in memory: residual, unaligned views, special values (an
+    all-NaN group among them), and buffers the pass declines."""
+
+    cfg = _cfg(bit=bit, group_size=group, topk=topk, quant_type=quant_type)
+    code = {"linear": 0, "normal": 1, "e3m0": 3}[quant_type]
+    for n, skew in ((20_000, 0), (4096 + 5, 1), (1, 0), (3 * group, 8)):
+        base = torch.empty(n + skew, dtype=DTYPES[dtype], device="cuda").normal_(std=1e-2)
+        x = base[skew:]
+        if n > 8 * group:
+            x[group:group + 4] = x[group]
+            x[2 * group:2 * group + 3] = torch.tensor([float("inf"), -float("inf"), float("nan")]).to(x)
+            x[4 * group:5 * group] = float("nan")
+            x[6 * group:7 * group] = 0
+        r = torch.empty(n, dtype=x.dtype, device="cuda").normal_(std=1e-4)
+        for residual in (None, r):
+            prepared = torch.empty_like(x)
+            cur = x
+            for k in range(passes):
+                payload = codec.quantize_tensor(cur, cfg, residual=residual if k == 0 else None,
+                                                prepared_out=prepared if k == 0 else None)
+                cur = codec.dequantize_tensor(payload, (n,), cfg, dtype=dtype)
+            out = x.clone() if residual is None else torch.empty_like(x)
+            rout = None if residual is None else residual.clone()
+            src = out if residual is None else x
+            assert ext.roundtrip_general(src, rout, out, rout, group, bit, topk, code, False, 0, passes)
+            assert torch.equal(out.view(torch.uint8), cur.view(torch.uint8)), (n, residual is None)
+            if residual is not None:
+                want = torch.empty_like(x)
+                codec.update_error_feedback_residual(prepared, cur.contiguous(), want)
+                assert torch.equal(rout.view(torch.uint8), want.view(torch.uint8)), n
+    both = torch.zeros(1000, dtype=DTYPES[dtype], device="cuda")
+    assert not ext.roundtrip_general(both[:900], None, both[100:], None, group, bit, topk, code, False, 0, passes)
+    assert not ext.roundtrip_general(both[:900], both[50:950], both[:900], None, group, bit, topk, code, False, 0, passes)
