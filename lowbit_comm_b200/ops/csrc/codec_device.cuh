@@ -47,6 +47,55 @@ __device__ __forceinline__ uint4 load_codes(const uint8_t* p, int n) {
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+// A warp's records of the compact layout: 512 elements are a multiple of 16 bytes whatever the group size, k and code,
+// so a warp's span starts on a 16-byte boundary when the payload does, although its records do not.  The span is built
+// (or read) in shared memory and moves as vectors; 2- and 4-byte accesses to the records took one instruction per word.
+constexpr int kWarpSpan = 1024;      // at most: 512 code bytes and 32 groups of 16 metadata bytes
+constexpr int span_bytes(int group, int record) { return 32 * kElemsPerThread / group * record; }
+
+__device__ __forceinline__ void span_to_global(uint8_t* dst, const uint8_t* span, int bytes, int wlane) {
+    for (int o = wlane * 16; o + 16 <= bytes; o += 32 * 16) st16(dst + o, *reinterpret_cast<const uint4*>(span + o));
+    for (int o = (bytes & ~15) + wlane * 2; o < bytes; o += 64)
+        *reinterpret_cast<uint16_t*>(dst + o) = *reinterpret_cast<const uint16_t*>(span + o);
+}
+__device__ __forceinline__ void span_from_global(uint8_t* span, const uint8_t* src, int bytes, int wlane) {
+    for (int o = wlane * 16; o + 16 <= bytes; o += 32 * 16) *reinterpret_cast<uint4*>(span + o) = ld16(src + o);
+    for (int o = (bytes & ~15) + wlane * 2; o < bytes; o += 64)
+        *reinterpret_cast<uint16_t*>(span + o) = *reinterpret_cast<const uint16_t*>(src + o);
+}
+// Code words to and from records that start on any even address (shared memory).
+template <int CB>
+__device__ __forceinline__ void span_put_codes(uint8_t* p, const uint32_t (&w)[4]) {
+    constexpr int words = CB / 4;
+    if ((reinterpret_cast<uintptr_t>(p) & 3) == 0) {
+#pragma unroll
+        for (int i = 0; i < words; ++i) reinterpret_cast<uint32_t*>(p)[i] = w[i];
+    } else {
+        *reinterpret_cast<uint16_t*>(p) = uint16_t(w[0]);
+#pragma unroll
+        for (int i = 0; i + 1 < words; ++i)
+            *reinterpret_cast<uint32_t*>(p + 2 + 4 * i) = __funnelshift_r(w[i], w[i + 1], 16);
+        *reinterpret_cast<uint16_t*>(p + 4 * words - 2) = uint16_t(w[words - 1] >> 16);
+    }
+}
+template <int CB>
+__device__ __forceinline__ void span_get_codes(const uint8_t* p, uint32_t (&w)[4]) {
+    constexpr int words = CB / 4;
+    w[2] = w[3] = 0u;
+    if ((reinterpret_cast<uintptr_t>(p) & 3) == 0) {
+#pragma unroll
+        for (int i = 0; i < words; ++i) w[i] = reinterpret_cast<const uint32_t*>(p)[i];
+    } else {
+        uint32_t mid[words + 1];
+        mid[0] = uint32_t(*reinterpret_cast<const uint16_t*>(p)) << 16;
+#pragma unroll
+        for (int i = 0; i + 1 < words; ++i) mid[i + 1] = *reinterpret_cast<const uint32_t*>(p + 2 + 4 * i);
+        mid[words] = *reinterpret_cast<const uint16_t*>(p + 4 * words - 2);
+#pragma unroll
+        for (int i = 0; i < words; ++i) w[i] = __funnelshift_r(mid[i], mid[i + 1], 16);
+    }
+}
+
 template <typename T>
 __device__ __forceinline__ void store_scale(uint8_t* p, float stored) {
     if constexpr (sizeof(T) == 2)
@@ -106,10 +155,7 @@ __device__ __forceinline__ uint4 encode16(const float (&vals)[16], float stored_
     if constexpr (BIT == 8) {
         return pack16_low_bytes<sizeof(T)>(b);
     } else {
-        int q[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) q[i] = int(b[i]);
-        const uint2 h = pack16_i4<sizeof(T)>(q);
+        const uint2 h = pack16_low_nibbles<sizeof(T)>(b);
         return make_uint4(h.x, h.y, 0, 0);
     }
 }
@@ -120,11 +166,27 @@ __device__ __forceinline__ void codes16(uint4 codes, float (&out)[16]) {
     if constexpr (BIT == 8) {
         unpack16_i8_fast<sizeof(T)>(codes, out);
     } else {
-        int c[16];
-        unpack16_i4<sizeof(T)>(make_uint2(codes.x, codes.y), c);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) out[i] = int4_value(c[i]);
+        unpack16_i4_fast<sizeof(T)>(make_uint2(codes.x, codes.y), out);
     }
+}
+
+// Picks the instantiation of a launcher for a call's dtype, group size and code width.
+template <template <typename, int, int> class Launcher, typename P>
+static cudaError_t dispatch_profile(const P* p, cudaStream_t stream) {
+#define LBC_CASE(TT, GG, BB)                                                        \
+    if (p->group_size == GG && p->bit == BB) return Launcher<TT, GG, BB>::run(p, stream);
+#define LBC_TYPE(TT)                                                                \
+    LBC_CASE(TT, 64, 8) LBC_CASE(TT, 32, 8) LBC_CASE(TT, 16, 8)                     \
+    LBC_CASE(TT, 64, 4) LBC_CASE(TT, 32, 4) LBC_CASE(TT, 16, 4)
+    switch (p->dtype) {
+        case LBC_BF16: LBC_TYPE(__nv_bfloat16) break;
+        case LBC_FP16: LBC_TYPE(__half) break;
+        case LBC_FP32: LBC_TYPE(float) break;
+        default: break;
+    }
+#undef LBC_TYPE
+#undef LBC_CASE
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace lbc

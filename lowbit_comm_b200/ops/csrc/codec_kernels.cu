@@ -1,0 +1,359 @@
+// The codec on its own (encode a tensor, decode a payload, reduce the payloads a rank has gathered) for the production
+// profiles: linear, no top-k, nearest-even rounding.  One payload in or out lies in this GPU's memory, nobody waits and
+// nobody is signalled; what the collectives add to that (peer destinations, flags, shards) is in fast_kernels.cu.
+//
+// Math is identical, bit for bit, to quant_push_kernel / reduce_kernel there.
+// Reference: quantization/quant_pack_kernel.cu:84-163, quantization/dequant_reduce_kernel.cu:38-69, 150-221.
+//
+// What bounds these kernels: memory.  A block per tile instead of a grid-stride loop (a persistent grid moved 10-15 %
+// less), 32 bytes of input per thread in one load, payloads read and written as 16-byte vectors in both layouts, the
+// whole-tile path free of bounds and alignment tests (their registers cost occupancy).
+// Measured on a B200, int8 groups of 64, before (grid-stride kernels of fast_kernels.cu) and after: encode of 32 Mi bf16
+// elements with error feedback 47.0 -> 39.5 us (6.0 TB/s), decode of 128 Mi 94 -> 66 us (6.2 TB/s), mean of eight
+// payloads of 32 Mi with error feedback 107 -> 82 us (5.8 TB/s).
+#include <type_traits>
+
+#include "codec_device.cuh"
+#include "common.cuh"
+#include "lbc_api.h"
+
+namespace lbc {
+
+// ---------------------------------------------------------------------------
+// encode
+// ---------------------------------------------------------------------------
+template <typename T, bool kWhole>
+__device__ __forceinline__ void store_chunk(T* to, int64_t first, int64_t numel, const float (&values)[16]) {
+    if constexpr (kWhole)
+        store16<T>(to + first, 0, 16, true, values);
+    else
+        store16_any<T>(to, first, numel, (reinterpret_cast<uintptr_t>(to) & 31) == 0, values);
+}
+
+// Quantizes and stores the thread's 16 values.  kWhole: they all lie inside 32-byte aligned tensors.  Convergent (the
+// group maximum shuffles); `span` is the warp's staging area for compact records.
+template <typename T, int G, int BIT, bool kCompact, bool kWhole>
+__device__ __forceinline__ void encode_chunk(const LbcQuantPush& p, float (&v)[16], int64_t chunk, uint8_t* span) {
+    constexpr int lanes = G / kElemsPerThread;
+    constexpr int VB = G * BIT / 8, MB = sizeof(T), CB = kElemsPerThread * BIT / 8;
+    T* prep = static_cast<T*>(p.prepared_out);
+    T* lef = static_cast<T*>(p.local_ef_out);
+    uint8_t* dst = p.dst[0];
+    const int64_t num_groups = (p.numel + G - 1) / G;
+    const int64_t first = chunk * kElemsPerThread;
+    const bool live = kWhole || chunk < num_groups * lanes;
+    const int64_t g = chunk / lanes;
+    const int lane = int(chunk) & (lanes - 1);
+    const int wlane = threadIdx.x & 31;
+    float amax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
+    const float stored = group_max<G>(amax);                      // exact in T, like the values
+    if (prep != nullptr && live) store_chunk<T, kWhole>(prep, first, p.numel, v);
+    float err[16];
+    const uint4 codes = encode16<T, BIT>(v, stored, lef != nullptr ? &err : nullptr);
+    if (lef != nullptr && live) store_chunk<T, kWhole>(lef, first, p.numel, err);
+    if (kCompact && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+        uint8_t* rec = span + (wlane / lanes) * (VB + MB);
+        const uint32_t w[4] = {codes.x, codes.y, codes.z, codes.w};
+        span_put_codes<CB>(rec + lane * CB, w);
+        if (lane == 0) store_scale<T>(rec + VB, stored);
+        __syncwarp();
+        const int64_t g0 = (chunk - wlane) / lanes;
+        const int64_t groups = min(int64_t(32 / lanes), num_groups - g0);
+        if (groups > 0) span_to_global(dst + g0 * (VB + MB), span, int(groups) * (VB + MB), wlane);
+        __syncwarp();
+    } else if (live) {
+        uint8_t* vptr = kCompact ? dst + g * (VB + MB) : dst + g * VB;
+        store_codes(vptr + lane * CB, codes, CB);
+        if (lane == 0) store_scale<T>(kCompact ? vptr + VB : dst + p.layout_groups * VB + g * MB, stored);
+    }
+}
+
+// A tile with the tensor's end in it, or of unaligned tensors.
+template <typename T, int G, int BIT, bool kCompact>
+__device__ __forceinline__ void encode_edge(const LbcQuantPush& p, int64_t c0, int chunks_per_thread, uint8_t* span) {
+    const T* x = static_cast<const T*>(p.x);
+    const T* res = static_cast<const T*>(p.residual);
+    for (int j = 0; j < chunks_per_thread; ++j) {
+        const int64_t chunk = c0 + j * kThreads + threadIdx.x;
+        float v[16];
+        load16_any<T>(x, chunk * kElemsPerThread, p.numel, (reinterpret_cast<uintptr_t>(x) & 31) == 0, v);
+        if (res != nullptr) {
+            float r[16];
+            load16_any<T>(res, chunk * kElemsPerThread, p.numel, (reinterpret_cast<uintptr_t>(res) & 31) == 0, r);
+            compensate16<T>(v, r);
+        }
+        encode_chunk<T, G, BIT, kCompact, false>(p, v, chunk, span);
+    }
+}
+
+template <typename T, int G, int BIT, bool kCompact, bool kResidual, int U>
+__global__ void __launch_bounds__(kThreads, 4) encode_kernel(const __grid_constant__ LbcQuantPush p) {
+    constexpr int lanes = G / kElemsPerThread;
+    constexpr int tile_chunks = kThreads * U;
+    const T* x = static_cast<const T*>(p.x);
+    const T* res = static_cast<const T*>(p.residual);
+    const int64_t chunks = (p.numel + G - 1) / G * lanes;
+    const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(res) |
+                       reinterpret_cast<uintptr_t>(p.prepared_out) | reinterpret_cast<uintptr_t>(p.local_ef_out)) & 31) == 0;
+    __shared__ __align__(16) uint8_t spans[kThreads / 32][kCompact ? span_bytes(G, G * BIT / 8 + int(sizeof(T))) : 16];
+    uint8_t* span = spans[threadIdx.x >> 5];
+    for (int64_t c0 = int64_t(blockIdx.x) * tile_chunks; c0 < chunks; c0 += int64_t(gridDim.x) * tile_chunks) {
+        if (!vec || (c0 + tile_chunks) * kElemsPerThread > p.numel) {
+            encode_edge<T, G, BIT, kCompact>(p, c0, U, span);
+            continue;
+        }
+        const int64_t mine = c0 + threadIdx.x;
+        Raw16<T> rx[U], rr[kResidual ? U : 1];
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            rx[j] = raw16(x + (mine + j * kThreads) * kElemsPerThread);
+            if (kResidual) rr[j] = raw16(res + (mine + j * kThreads) * kElemsPerThread);
+        }
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            float v[16];
+            up16<T>(rx[j], v);
+            if (kResidual) {
+                float r[16];
+                up16<T>(rr[j], r);
+                compensate16<T>(v, r);
+            }
+            encode_chunk<T, G, BIT, kCompact, true>(p, v, mine + j * kThreads, span);
+        }
+    }
+    grid_signal(p.signal);
+}
+
+template <typename T, int G, int BIT>
+struct EncodeLauncher {
+    static cudaError_t run(const LbcQuantPush* p, cudaStream_t stream) {
+        const int64_t chunks = (p->numel + G - 1) / G * (G / kElemsPerThread);
+        if (chunks == 0 && p->signal.num_remote == 0) return cudaSuccess;
+        const int64_t one = chunks > 0 ? (chunks + kThreads - 1) / kThreads : 1;
+        auto grid = [&](int64_t blocks) {
+            const int64_t cap = p->max_blocks > 0 ? p->max_blocks : int64_t(1) << 30;
+            return unsigned(blocks < cap ? blocks : cap);
+        };
+        const auto go = [&](auto compact) {
+            constexpr bool kCompact = decltype(compact)::value;
+            if (p->residual != nullptr) {
+                encode_kernel<T, G, BIT, kCompact, true, 1><<<grid(one), kThreads, 0, stream>>>(*p);
+                return;
+            }
+            if constexpr (sizeof(T) == 2) {
+                if (one > lbc_default_max_blocks()) {
+                    encode_kernel<T, G, BIT, kCompact, false, 2><<<grid((one + 1) / 2), kThreads, 0, stream>>>(*p);
+                    return;
+                }
+            }
+            encode_kernel<T, G, BIT, kCompact, false, 1><<<grid(one), kThreads, 0, stream>>>(*p);
+        };
+        if (p->mode == LBC_PUSH_COMPACT_LOCAL)
+            go(std::true_type{});
+        else
+            go(std::false_type{});
+        return cudaGetLastError();
+    }
+};
+
+// ---------------------------------------------------------------------------
+// decode and reduce
+// ---------------------------------------------------------------------------
+// acc += one payload's 16 values: fma(code, scale / L, acc), one rounding per payload.
+template <typename T, int BIT>
+__device__ __forceinline__ void add_payload(float (&acc)[16], uint4 codes, float scale) {
+    const float step = scale / (BIT == 8 ? 127.0f : 7.0f);
+    float d[16];
+    codes16<T, BIT>(codes, d);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) acc[i] = __fmaf_rn(d[i], step, acc[i]);
+}
+
+// Adds payloads r0 .. r0 + K - 1 to a thread's chunk; all K loads are issued before the first is decoded.  Whole warps
+// of whole groups, vector-aligned payloads.  Compact: the warp's span comes in as vectors and turns through `span`.
+template <typename T, int G, int BIT, bool kCompact, int K>
+__device__ __forceinline__ void add_batch(const LbcReduce& p, int r0, int64_t chunk, uint8_t* span, float (&acc)[16]) {
+    constexpr int lanes = G / kElemsPerThread;
+    constexpr int VB = G * BIT / 8, MB = sizeof(T), CB = kElemsPerThread * BIT / 8;
+    const int lane = int(chunk) & (lanes - 1);
+    const int64_t g = chunk / lanes;
+    if constexpr (!kCompact) {
+        uint4 codes[K];
+        float scale[K];
+        const int64_t voff = g * VB + lane * CB, soff = p.layout_groups * VB + g * MB;
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            const uint8_t* src = p.src[r0 + j];
+            if constexpr (CB == 16) {
+                codes[j] = ld16_stream(src + voff);
+            } else {
+                const uint2 c = *reinterpret_cast<const uint2*>(src + voff);
+                codes[j] = make_uint4(c.x, c.y, 0u, 0u);
+            }
+            scale[j] = load_scale<T>(src + soff);
+        }
+#pragma unroll
+        for (int j = 0; j < K; ++j) add_payload<T, BIT>(acc, codes[j], scale[j]);
+    } else {
+        constexpr int full = span_bytes(G, VB + MB);            // 17 to 40 vectors
+        const int wlane = threadIdx.x & 31;
+        const int64_t at = (chunk - wlane) / lanes * (VB + MB) + wlane * 16;
+        uint4 lo[K], hi[K];
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            const uint8_t* src = p.src[r0 + j] + at;
+            if (full >= 512 || wlane * 16 < full) lo[j] = ld16_stream(src);
+            if (full > 512 && wlane * 16 < full - 512) hi[j] = ld16_stream(src + 512);
+        }
+        const uint8_t* rec = span + (wlane / lanes) * (VB + MB);
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            if (full >= 512 || wlane * 16 < full) *reinterpret_cast<uint4*>(span + wlane * 16) = lo[j];
+            if (full > 512 && wlane * 16 < full - 512) *reinterpret_cast<uint4*>(span + wlane * 16 + 512) = hi[j];
+            __syncwarp();
+            uint32_t w[4];
+            span_get_codes<CB>(rec + lane * CB, w);
+            const float scale = load_scale<T>(rec + VB);
+            __syncwarp();
+            add_payload<T, BIT>(acc, make_uint4(w[0], w[1], w[2], w[3]), scale);
+        }
+    }
+}
+
+// A chunk with the tensor's end in its tile, of unaligned tensors or of payloads that are not vector-aligned.
+template <typename T, int G, int BIT, bool kCompact>
+__device__ __forceinline__ void decode_edge(const LbcReduce& p, int64_t chunk) {
+    constexpr int lanes = G / kElemsPerThread;
+    constexpr int VB = G * BIT / 8, MB = sizeof(T), CB = kElemsPerThread * BIT / 8;
+    if (chunk >= (p.numel + G - 1) / G * lanes) return;
+    T* out = static_cast<T*>(p.out);
+    T* rout = static_cast<T*>(p.residual_out);
+    const T* prep = static_cast<const T*>(p.prepared);
+    const auto on32 = [](const void* t) { return (reinterpret_cast<uintptr_t>(t) & 31) == 0; };
+    const int64_t first = chunk * kElemsPerThread, g = chunk / lanes;
+    const int lane = int(chunk) & (lanes - 1);
+    const int64_t voff = (kCompact ? g * (VB + MB) : g * VB) + lane * CB;
+    const int64_t soff = kCompact ? g * (VB + MB) + VB : p.layout_groups * VB + g * MB;
+    float acc[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) acc[i] = 0.0f;
+#pragma unroll 2
+    for (int r = 0; r < p.num_src; ++r)
+        add_payload<T, BIT>(acc, load_codes(p.src[r] + voff, CB), load_scale<T>(p.src[r] + soff));
+#pragma unroll
+    for (int i = 0; i < 16; ++i) acc[i] *= p.scale;
+    if (rout != nullptr) {
+        float e[16];
+        load16_any<T>(prep, first, p.numel, on32(prep), e);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) e[i] -= acc[i];
+        store16_any<T>(rout, first, p.numel, on32(rout), e);
+    }
+    if (p.accumulate) {
+        float prev[16];
+        load16_any<T>(out, first, p.numel, on32(out), prev);
+        round16<T>(acc);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[i] += prev[i];
+    }
+    store16_any<T>(out, first, p.numel, on32(out), acc);        // rounds to T
+}
+
+// B payloads are in flight per thread.  B == 1: one payload, no error feedback (the launcher's rule).
+// Blocks per SM, measured at 128 Mi bf16 elements (decode) and 32 Mi (mean of 8, with error feedback): decode with 8 / 6 /
+// 5 / 4 blocks 66 / 71 / 76 / 84 us; mean with four payloads in flight and 5 / 4 / 3 / 2 blocks 82 / 81 / 89 / 90 us (of two
+// payloads 49 / 50 / 56 / 56), eight in flight 107 / 82 / 91 / 100.  Compact, two in flight: 105 / 101 / 113 / 144.
+template <typename T, int G, int BIT, bool kCompact, int B>
+__global__ void __launch_bounds__(kThreads, B == 1 ? (sizeof(T) == 2 ? 8 : 6) : (kCompact || sizeof(T) == 4 ? 4 : 5))
+decode_kernel(const __grid_constant__ LbcReduce p) {
+    constexpr int lanes = G / kElemsPerThread;
+    constexpr int VB = G * BIT / 8, MB = sizeof(T), CB = kElemsPerThread * BIT / 8;
+    T* out = static_cast<T*>(p.out);
+    const T* prep = static_cast<const T*>(p.prepared);
+    T* rout = static_cast<T*>(p.residual_out);
+    const int64_t chunks = (p.numel + G - 1) / G * lanes;
+    const int R = B == 1 ? 1 : p.num_src;
+    uintptr_t bits = 0;
+    for (int r = 0; r < R; ++r) bits |= reinterpret_cast<uintptr_t>(p.src[r]);
+    const bool vec = (bits & (kCompact ? 15 : CB - 1)) == 0 &&
+                     ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(prep) |
+                       reinterpret_cast<uintptr_t>(rout)) & 31) == 0;
+    __shared__ __align__(16) uint8_t spans[kThreads / 32][kCompact ? span_bytes(G, VB + MB) : 16];
+    uint8_t* span = spans[threadIdx.x >> 5];
+
+    for (int64_t c0 = int64_t(blockIdx.x) * kThreads; c0 < chunks; c0 += int64_t(gridDim.x) * kThreads) {
+        const int64_t chunk = c0 + threadIdx.x;
+        if (!vec || (c0 + kThreads) * kElemsPerThread > p.numel) {
+            decode_edge<T, G, BIT, kCompact>(p, chunk);
+            continue;
+        }
+        const int64_t first = chunk * kElemsPerThread;
+        float acc[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[i] = 0.0f;
+        Raw16<T> held;
+        if (B > 1 && rout != nullptr) held = raw16(prep + first);      // on its way while the payloads are summed
+        int r = 0;
+        for (; r + B <= R; r += B) add_batch<T, G, BIT, kCompact, B>(p, r, chunk, span, acc);
+        if constexpr (B > 2)
+            for (; r + 2 <= R; r += 2) add_batch<T, G, BIT, kCompact, 2>(p, r, chunk, span, acc);
+        if constexpr (B > 1)
+            for (; r < R; ++r) add_batch<T, G, BIT, kCompact, 1>(p, r, chunk, span, acc);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[i] *= p.scale;
+        if (B > 1 && rout != nullptr) {
+            float e[16];
+            up16<T>(held, e);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) e[i] -= acc[i];
+            store16<T>(rout + first, 0, 16, true, e);
+        }
+        if (p.accumulate) {
+            float prev[16];
+            up16<T>(raw16(static_cast<const T*>(out) + first), prev);
+            round16<T>(acc);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) acc[i] += prev[i];
+        }
+        store16<T>(out + first, 0, 16, true, acc);                     // rounds to T
+    }
+}
+
+template <typename T, int G, int BIT>
+struct DecodeLauncher {
+    static cudaError_t run(const LbcReduce* p, cudaStream_t stream) {
+        const int64_t chunks = (p->numel + G - 1) / G * (G / kElemsPerThread);
+        if (chunks == 0) return cudaSuccess;
+        const int64_t blocks = (chunks + kThreads - 1) / kThreads;
+        const unsigned grid = unsigned(p->max_blocks > 0 && blocks > p->max_blocks ? p->max_blocks : blocks);
+        const auto go = [&](auto compact) {
+            constexpr bool kCompact = decltype(compact)::value;
+            // a compact payload takes two vectors per lane, so half as many are in flight
+            if (p->num_src == 1 && p->residual_out == nullptr)
+                decode_kernel<T, G, BIT, kCompact, 1><<<grid, kThreads, 0, stream>>>(*p);
+            else
+                decode_kernel<T, G, BIT, kCompact, kCompact ? 2 : 4><<<grid, kThreads, 0, stream>>>(*p);
+        };
+        if (p->compact)
+            go(std::true_type{});
+        else
+            go(std::false_type{});
+        return cudaGetLastError();
+    }
+};
+
+}  // namespace lbc
+
+extern "C" {
+
+cudaError_t lbc_encode(const LbcQuantPush* p, cudaStream_t stream) {
+    return lbc::dispatch_profile<lbc::EncodeLauncher>(p, stream);
+}
+
+cudaError_t lbc_decode(const LbcReduce* p, cudaStream_t stream) {
+    return lbc::dispatch_profile<lbc::DecodeLauncher>(p, stream);
+}
+
+}  // extern "C"

@@ -187,33 +187,87 @@ __device__ __forceinline__ void store16(T* base, int64_t first, int64_t numel, b
     }
 }
 
+// 16 elements as loaded, for kernels that hold several loads in flight.  Plain (not read-only) loads: an output may be
+// the buffer that was read, a thread only ever writes the elements that it has read itself.
+template <typename T> struct Raw16 {
+    U8x32 part[sizeof(T) / 2];
+};
+__device__ __forceinline__ U8x32 ld32_once(const void* p) {
+    U8x32 v;
+    asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]),
+                   "=r"(v.w[6]), "=r"(v.w[7]) : "l"(p));
+    return v;
+}
+template <typename T>
+__device__ __forceinline__ Raw16<T> raw16(const T* p) {
+    Raw16<T> r;
+#pragma unroll
+    for (int h = 0; h < int(sizeof(T)) / 2; ++h) r.part[h] = ld32_once(p + 16 / (sizeof(T) / 2) * h);
+    return r;
+}
+template <typename T>
+__device__ __forceinline__ void up16(const Raw16<T>& r, float (&v)[16]) {
+    if constexpr (sizeof(T) == 2) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) Src<T>::up2(r.part[0].w[i], v[2 * i], v[2 * i + 1]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r.part[i / 8].w[i % 8]);
+    }
+}
+
+// Tensor ends and unaligned tensors, element by element.  Out of line on purpose: inlined, their sixteen addresses and
+// predicates cost the whole-tile path registers (spills at four blocks per SM).
+template <typename T>
+__device__ __noinline__ void load16_edge(const T* base, int64_t first, int64_t numel, float* out) {
+    float v[16];
+    load16<T>(base, first, numel, false, v, false);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) out[i] = v[i];
+}
+template <typename T>
+__device__ __noinline__ void store16_edge(T* base, int64_t first, int64_t numel, const float* vals) {
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = vals[i];
+    store16<T>(base, first, numel, false, v);
+}
+// 16 elements at `first`, zeros past the end; `vec`: the tensor starts on 32 bytes.
+template <typename T>
+__device__ __forceinline__ void load16_any(const T* base, int64_t first, int64_t numel, bool vec, float (&out)[16]) {
+    if (vec && first + 16 <= numel) {
+        up16<T>(raw16(base + first), out);
+    } else {
+        float v[16];
+        load16_edge<T>(base, first, numel, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) out[i] = v[i];
+    }
+}
+template <typename T>
+__device__ __forceinline__ void store16_any(T* base, int64_t first, int64_t numel, bool vec, const float (&vals)[16]) {
+    if (vec && first + 16 <= numel) {
+        store16<T>(base + first, 0, 16, true, vals);
+    } else {
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = vals[i];
+        store16_edge<T>(base, first, numel, v);
+    }
+}
+
+// prepared = T(x + residual)
+template <typename T>
+__device__ __forceinline__ void compensate16(float (&v)[16], const float (&r)[16]) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] += r[i];
+    round16<T>(v);
+}
+
 // ---------------------------------------------------------------------------
 // wire-order packing of 16 codes
 // ---------------------------------------------------------------------------
-// int8: natural little-endian bytes (e0 lowest) -> wire order inside each word.
-template <int WordBytes>
-__device__ __forceinline__ uint32_t wire_perm8(uint32_t natural) {
-    return __byte_perm(natural, 0, WordBytes == 2 ? 0x2301 : 0x0123);
-}
-
-__device__ __forceinline__ int quant_rn(float v, float mul, int lim) {
-    int q = __float2int_rn(v * mul);
-    return max(-lim, min(lim, q));
-}
-
-// Packs 16 int8 codes (as ints in [-127,127]) into 16 wire-ordered bytes.
-template <int WordBytes>
-__device__ __forceinline__ uint4 pack16_i8(const int (&q)[16]) {
-    uint32_t w[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        uint32_t nat = (uint32_t(q[4 * j]) & 0xffu) | ((uint32_t(q[4 * j + 1]) & 0xffu) << 8) |
-                       ((uint32_t(q[4 * j + 2]) & 0xffu) << 16) | ((uint32_t(q[4 * j + 3]) & 0xffu) << 24);
-        w[j] = wire_perm8<WordBytes>(nat);
-    }
-    return make_uint4(w[0], w[1], w[2], w[3]);
-}
-
 // Round-to-nearest-even quantization without a float->int conversion: adding
 // 1.5 * 2^23 to t = v * mul leaves rint(t) in the low mantissa bits, so the low
 // byte (nibble) of the result's bit pattern is the two's-complement code.  The
@@ -259,50 +313,40 @@ __device__ __forceinline__ void unpack16_i8_fast(uint4 v, float (&out)[16]) {
     }
 }
 
-// Packs 16 int4 codes into 8 wire-ordered bytes (two 32-bit halves).
+// Low nibbles of 16 bit patterns -> 8 wire-ordered bytes: even and odd elements are gathered as bytes, then interleaved.
 template <int WordBytes>
-__device__ __forceinline__ uint2 pack16_i4(const int (&q)[16]) {
+__device__ __forceinline__ uint2 pack16_low_nibbles(const uint32_t (&b)[16]) {
     uint32_t w[2];
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-        uint32_t nat = 0;  // byte b = (e[2b] << 4) | e[2b+1]  (big-endian byte sequence)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            uint32_t hi = uint32_t(q[8 * j + 2 * b]) & 0xfu, lo = uint32_t(q[8 * j + 2 * b + 1]) & 0xfu;
-            nat |= ((hi << 4) | lo) << (8 * b);
+        const uint32_t* e = b + 8 * j;
+        uint32_t hi, lo;
+        if constexpr (WordBytes == 2) {
+            hi = __byte_perm(__byte_perm(e[2], e[0], 0x0040), __byte_perm(e[6], e[4], 0x0040), 0x5410);
+            lo = __byte_perm(__byte_perm(e[3], e[1], 0x0040), __byte_perm(e[7], e[5], 0x0040), 0x5410);
+        } else {
+            hi = __byte_perm(__byte_perm(e[6], e[4], 0x0040), __byte_perm(e[2], e[0], 0x0040), 0x5410);
+            lo = __byte_perm(__byte_perm(e[7], e[5], 0x0040), __byte_perm(e[3], e[1], 0x0040), 0x5410);
         }
-        w[j] = wire_perm8<WordBytes>(nat);
+        w[j] = ((hi << 4) & 0xf0f0f0f0u) | (lo & 0x0f0f0f0fu);
     }
     return make_uint2(w[0], w[1]);
 }
 
+// 8 wire-ordered int4 bytes -> their values as floats: (c ^ 8) dropped into the mantissa of 2^23, minus 2^23 + 8 (exact).
 template <int WordBytes>
-__device__ __forceinline__ void unpack16_i8(uint4 v, float (&out)[16]) {
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const uint32_t nat = wire_perm8<WordBytes>(w[j]);  // the permutation is its own inverse
-#pragma unroll
-        for (int b = 0; b < 4; ++b) out[4 * j + b] = float(int(int8_t((nat >> (8 * b)) & 0xffu)));
-    }
-}
-
-template <int WordBytes>
-__device__ __forceinline__ void unpack16_i4(uint2 v, int (&codes)[16]) {
-    const uint32_t w[2] = {v.x, v.y};
+__device__ __forceinline__ void unpack16_i4_fast(uint2 v, float (&out)[16]) {
+    const uint32_t w[2] = {v.x ^ 0x88888888u, v.y ^ 0x88888888u};
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-        const uint32_t nat = wire_perm8<WordBytes>(w[j]);
+        const uint32_t hi = (w[j] >> 4) & 0x0f0f0f0fu, lo = w[j] & 0x0f0f0f0fu;
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const uint32_t by = (nat >> (8 * b)) & 0xffu;
-            codes[8 * j + 2 * b] = int(by >> 4);
-            codes[8 * j + 2 * b + 1] = int(by & 0xfu);
+        for (int e = 0; e < 8; ++e) {
+            const int pos = WordBytes == 2 ? ((e >> 1) ^ 1) : (3 - (e >> 1));
+            out[8 * j + e] = __uint_as_float(__byte_perm((e & 1) ? lo : hi, 0x4B000000u, 0x7540 | pos)) - 8388616.0f;
         }
     }
 }
-
-__device__ __forceinline__ float int4_value(int code) { return float((code ^ 8) - 8); }
 
 // ---------------------------------------------------------------------------
 // cross-GPU signalling: release stores, acquire loads, bounded waits

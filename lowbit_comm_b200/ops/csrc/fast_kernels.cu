@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(kThreads, 4) quant_push_kernel(const LbcQuantP
     const bool l_vec = lef == nullptr || (reinterpret_cast<uintptr_t>(lef) & 31) == 0;
 
     __shared__ __align__(16) ScaleStage stage;
-    const bool vec_scales = p.mode != LBC_PUSH_COMPACT_LOCAL && (p.layout_groups & 7) == 0 &&
+    const bool vec_scales = (p.layout_groups & 7) == 0 &&
                             (p.group_offset & 7) == 0 && (p.shard_groups & 7) == 0 && dsts_aligned16(p.dst, p.num_dst);
     const bool mcast = vec_scales && p.mode == LBC_PUSH_BROADCAST && p.mc_dst != nullptr;
 
@@ -82,11 +82,7 @@ __global__ void __launch_bounds__(kThreads, 4) quant_push_kernel(const LbcQuantP
             float dq[16];
             const uint4 codes = encode16<T, BIT>(v, stored, lef != nullptr ? &dq : nullptr);
             if (lef != nullptr) store16<T>(lef, first, n, l_vec, dq);
-            if (p.mode == LBC_PUSH_COMPACT_LOCAL) {
-                uint8_t* rec = p.dst[0] + g * (VB + MB);
-                store_codes(rec + lane * CB, codes, CB);
-                if (lane == 0) store_scale<T>(rec + VB, stored);
-            } else if (p.mode == LBC_PUSH_SCATTER) {
+            if (p.mode == LBC_PUSH_SCATTER) {
                 const int64_t d = g / p.shard_groups;
                 const int64_t gl = g - d * p.shard_groups;
                 uint8_t* base = p.dst[d];
@@ -716,24 +712,6 @@ static int grid_for(int64_t chunks, int max_blocks) {
     return int(want < cap ? want : cap);
 }
 
-template <template <typename, int, int> class Launcher, typename P>
-static cudaError_t dispatch(const P* p, cudaStream_t stream) {
-#define LBC_CASE(TT, GG, BB)                                                        \
-    if (p->group_size == GG && p->bit == BB) return Launcher<TT, GG, BB>::run(p, stream);
-#define LBC_TYPE(TT)                                                                \
-    LBC_CASE(TT, 64, 8) LBC_CASE(TT, 32, 8) LBC_CASE(TT, 16, 8)                     \
-    LBC_CASE(TT, 64, 4) LBC_CASE(TT, 32, 4) LBC_CASE(TT, 16, 4)
-    switch (p->dtype) {
-        case LBC_BF16: LBC_TYPE(__nv_bfloat16) break;
-        case LBC_FP16: LBC_TYPE(__half) break;
-        case LBC_FP32: LBC_TYPE(float) break;
-        default: break;
-    }
-#undef LBC_TYPE
-#undef LBC_CASE
-    return cudaErrorInvalidValue;
-}
-
 // The bulk-store kernel needs 16-byte aligned destinations and layouts padded to 8 groups;
 // the collectives guarantee both, the local codec entry points (arbitrary payload tensors) do not.
 // Push variants (identical payload layout, so ranks may even differ):
@@ -761,6 +739,12 @@ struct QuantPushLauncher {
     static cudaError_t run(const LbcQuantPush* p, cudaStream_t stream) {
         const int64_t groups = (p->numel + G - 1) / G;
         if (groups == 0 && p->signal.num_remote == 0) return cudaSuccess;
+        // one payload in this GPU's memory and nobody to signal: the codec on its own (codec_kernels.cu), and the compact
+        // layout always (no collective moves it)
+        if (p->mode == LBC_PUSH_COMPACT_LOCAL ||
+            (p->mode == LBC_PUSH_BROADCAST && p->num_dst == 1 && p->signal.num_remote == 0 && p->group_offset == 0 &&
+             p->mc_dst == nullptr))
+            return lbc_encode(p, stream);
         const int grid = grid_for(groups * (G / kElemsPerThread), p->max_blocks);
         const int variant = tiled_path_ok(p) ? g_push_variant : 0;
         if (variant == 2) {
@@ -779,6 +763,10 @@ struct ReduceLauncher {
     static cudaError_t run(const LbcReduce* p, cudaStream_t stream) {
         const int64_t groups = (p->numel + G - 1) / G;
         if (groups == 0 && p->signal.num_remote == 0 && p->wait.flags == nullptr) return cudaSuccess;
+        // payloads in, dense out, nobody to wait for or to tell: the codec on its own (codec_kernels.cu)
+        if (p->num_dst == 0 && p->signal.num_remote == 0 && p->wait.flags == nullptr && p->src_shard_groups == 0 &&
+            p->group_offset == 0 && p->out != nullptr)
+            return lbc_decode(p, stream);
         int cap = p->max_blocks;
         if (p->num_dst > 1 && g_reduce_push_blocks >= 0) {   // several destinations: peers are among them
             const int push_cap = g_reduce_push_blocks > 0 ? g_reduce_push_blocks : default_max_blocks() / 4;
@@ -828,7 +816,7 @@ cudaError_t lbc_quant_push(const LbcQuantPush* p, cudaStream_t stream) {
     if (p->mode == LBC_PUSH_SCATTER && p->shard_groups <= 0) return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(p->mc_dst) & 15) != 0) return cudaErrorInvalidValue;
     if (p->mc_dst != nullptr && p->mode != LBC_PUSH_BROADCAST) return cudaErrorInvalidValue;
-    return lbc::dispatch<lbc::QuantPushLauncher>(p, stream);
+    return lbc::dispatch_profile<lbc::QuantPushLauncher>(p, stream);
 }
 
 cudaError_t lbc_reduce(const LbcReduce* p, cudaStream_t stream) {
@@ -843,7 +831,7 @@ cudaError_t lbc_reduce(const LbcReduce* p, cudaStream_t stream) {
         const int64_t groups = (p->numel + p->group_size - 1) / p->group_size;
         if ((p->group_offset + groups - 1) / p->src_shard_groups >= p->num_src) return cudaErrorInvalidValue;
     }
-    return lbc::dispatch<lbc::ReduceLauncher>(p, stream);
+    return lbc::dispatch_profile<lbc::ReduceLauncher>(p, stream);
 }
 
 cudaError_t lbc_error_feedback_update(int dtype, const void* prepared, const void* restored, void* residual,

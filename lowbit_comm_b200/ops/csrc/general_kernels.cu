@@ -24,6 +24,7 @@
 #include <cmath>
 #include <type_traits>
 
+#include "codec_device.cuh"
 #include "common.cuh"
 #include "lbc_api.h"
 
@@ -323,26 +324,6 @@ __device__ __forceinline__ GroupMeta select_group(float (&v)[16], const Packed16
     return m;
 }
 
-// Low nibbles of 16 bit patterns -> 8 wire-ordered bytes: even and odd elements are gathered as bytes, then interleaved.
-template <int WordBytes>
-__device__ __forceinline__ uint2 pack16_low_nibbles(const uint32_t (&b)[16]) {
-    uint32_t w[2];
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-        const uint32_t* e = b + 8 * j;
-        uint32_t hi, lo;
-        if constexpr (WordBytes == 2) {
-            hi = __byte_perm(__byte_perm(e[2], e[0], 0x0040), __byte_perm(e[6], e[4], 0x0040), 0x5410);
-            lo = __byte_perm(__byte_perm(e[3], e[1], 0x0040), __byte_perm(e[7], e[5], 0x0040), 0x5410);
-        } else {
-            hi = __byte_perm(__byte_perm(e[6], e[4], 0x0040), __byte_perm(e[2], e[0], 0x0040), 0x5410);
-            lo = __byte_perm(__byte_perm(e[7], e[5], 0x0040), __byte_perm(e[3], e[1], 0x0040), 0x5410);
-        }
-        w[j] = ((hi << 4) & 0xf0f0f0f0u) | (lo & 0x0f0f0f0fu);
-    }
-    return make_uint2(w[0], w[1]);
-}
-
 // Rounding parameters of one call.
 struct CodeRule {
     const float* thresholds;   // kBook: thresholds[c] = the least t = value / scale whose code is above c (14 of them)
@@ -488,54 +469,6 @@ struct GroupShape {
     }
 };
 
-// A warp's records of the compact layout: 512 elements are a multiple of 16 bytes whatever the group size, k and code,
-// so a warp's span starts on a 16-byte boundary when the payload does, although its records do not.  The span is built
-// (or read) in shared memory and moves as vectors; 2- and 4-byte accesses to the records took one instruction per word.
-constexpr int kWarpSpan = 1024;      // 512 code bytes and at most 32 groups of 16 metadata bytes
-
-__device__ __forceinline__ void span_to_global(uint8_t* dst, const uint8_t* span, int bytes, int wlane) {
-    for (int o = wlane * 16; o + 16 <= bytes; o += 32 * 16) st16(dst + o, *reinterpret_cast<const uint4*>(span + o));
-    for (int o = (bytes & ~15) + wlane * 2; o < bytes; o += 64)
-        *reinterpret_cast<uint16_t*>(dst + o) = *reinterpret_cast<const uint16_t*>(span + o);
-}
-__device__ __forceinline__ void span_from_global(uint8_t* span, const uint8_t* src, int bytes, int wlane) {
-    for (int o = wlane * 16; o + 16 <= bytes; o += 32 * 16) *reinterpret_cast<uint4*>(span + o) = ld16(src + o);
-    for (int o = (bytes & ~15) + wlane * 2; o < bytes; o += 64)
-        *reinterpret_cast<uint16_t*>(span + o) = *reinterpret_cast<const uint16_t*>(src + o);
-}
-// Code words to and from records that start on any even address (shared memory).
-template <int KIND>
-__device__ __forceinline__ void span_put_codes(uint8_t* p, const uint32_t (&w)[4]) {
-    constexpr int words = Kind<KIND>::CB / 4;
-    if ((reinterpret_cast<uintptr_t>(p) & 3) == 0) {
-#pragma unroll
-        for (int i = 0; i < words; ++i) reinterpret_cast<uint32_t*>(p)[i] = w[i];
-    } else {
-        *reinterpret_cast<uint16_t*>(p) = uint16_t(w[0]);
-#pragma unroll
-        for (int i = 0; i + 1 < words; ++i)
-            *reinterpret_cast<uint32_t*>(p + 2 + 4 * i) = __funnelshift_r(w[i], w[i + 1], 16);
-        *reinterpret_cast<uint16_t*>(p + 4 * words - 2) = uint16_t(w[words - 1] >> 16);
-    }
-}
-template <int KIND>
-__device__ __forceinline__ void span_get_codes(const uint8_t* p, uint32_t (&w)[4]) {
-    constexpr int words = Kind<KIND>::CB / 4;
-    w[2] = w[3] = 0u;
-    if ((reinterpret_cast<uintptr_t>(p) & 3) == 0) {
-#pragma unroll
-        for (int i = 0; i < words; ++i) w[i] = reinterpret_cast<const uint32_t*>(p)[i];
-    } else {
-        uint32_t mid[words + 1];
-        mid[0] = uint32_t(*reinterpret_cast<const uint16_t*>(p)) << 16;
-#pragma unroll
-        for (int i = 0; i + 1 < words; ++i) mid[i + 1] = *reinterpret_cast<const uint32_t*>(p + 2 + 4 * i);
-        mid[words] = *reinterpret_cast<const uint16_t*>(p + 4 * words - 2);
-#pragma unroll
-        for (int i = 0; i < words; ++i) w[i] = __funnelshift_r(mid[i], mid[i + 1], 16);
-    }
-}
-
 // The words of a group's metadata, dealt to the threads of the group.
 template <typename T, int TOPK>
 __device__ __forceinline__ void put_meta(uint8_t* meta, const GroupMeta& m, int lane, int lanes) {
@@ -599,7 +532,7 @@ __global__ void __launch_bounds__(kThreads) quant_general_kernel(const __grid_co
         if (staged) {
             const int gw = wlane >> shape.shift;                        // my group inside the warp's span
             uint8_t* rec = span + gw * (VB + MB);
-            span_put_codes<KIND>(rec + lane * CB, w);
+            span_put_codes<CB>(rec + lane * CB, w);
             put_meta<T, TOPK>(rec + VB, m, lane, lanes);
             __syncwarp();
             const int64_t g0 = (chunk - wlane) >> shape.shift;
@@ -679,7 +612,7 @@ __global__ void __launch_bounds__(kThreads) dequant_general_kernel(const __grid_
             __syncwarp();
             const uint8_t* rec = span + (wlane >> shape.shift) * (VB + MB);
             if (!live) continue;
-            span_get_codes<KIND>(rec + lane * CB, w);
+            span_get_codes<CB>(rec + lane * CB, w);
             meta = rec + VB;
         } else {
             if (!live) continue;

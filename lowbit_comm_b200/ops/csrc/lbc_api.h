@@ -95,6 +95,10 @@ typedef struct {
 
 cudaError_t lbc_quant_push(const LbcQuantPush* p, cudaStream_t stream);
 cudaError_t lbc_reduce(const LbcReduce* p, cudaStream_t stream);
+// What the two launchers above hand over (codec_kernels.cu): one local payload, planar or compact, no group offset, no
+// multicast; and local payloads into a dense output, no destinations, no gather, no flags.
+cudaError_t lbc_encode(const LbcQuantPush* p, cudaStream_t stream);
+cudaError_t lbc_decode(const LbcReduce* p, cudaStream_t stream);
 
 // ---- single-launch all-reduce: one persistent kernel, every NVLink byte moved by bulk loads ----------
 // Every rank quantizes its tensor into its OWN arena (phase QUANT), the owner of a shard pulls that

@@ -41,36 +41,6 @@ __device__ __forceinline__ void roundtrip16(float (&v)[16], float (&y)[16], bool
     }
 }
 
-// 16 elements as loaded.  Plain (not read-only) loads: `out` and the residual may be the buffers that were read, and a
-// thread only ever writes the elements that it has read itself.
-template <typename T> struct Raw16 {
-    U8x32 part[sizeof(T) / 2];
-};
-__device__ __forceinline__ U8x32 ld32_once(const void* p) {
-    U8x32 v;
-    asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]),
-                   "=r"(v.w[6]), "=r"(v.w[7]) : "l"(p));
-    return v;
-}
-template <typename T>
-__device__ __forceinline__ Raw16<T> raw16(const T* p) {
-    Raw16<T> r;
-#pragma unroll
-    for (int h = 0; h < int(sizeof(T)) / 2; ++h) r.part[h] = ld32_once(p + 16 / (sizeof(T) / 2) * h);
-    return r;
-}
-template <typename T>
-__device__ __forceinline__ void up16(const Raw16<T>& r, float (&v)[16]) {
-    if constexpr (sizeof(T) == 2) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) Src<T>::up2(r.part[0].w[i], v[2 * i], v[2 * i + 1]);
-    } else {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r.part[i / 8].w[i % 8]);
-    }
-}
-
 // kResidual: the input is T(x + residual).  U chunks of 16 elements per thread are loaded before the first is computed.
 template <typename T, int G, int BIT, bool kResidual, int U>
 __global__ void __launch_bounds__(kThreads) roundtrip_kernel(const LbcRoundtrip p) {
@@ -85,11 +55,6 @@ __global__ void __launch_bounds__(kThreads) roundtrip_kernel(const LbcRoundtrip 
     const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) |
                        reinterpret_cast<uintptr_t>(res) | reinterpret_cast<uintptr_t>(rout)) & 31) == 0;
 
-    auto compensate = [](float (&v)[16], const float (&r)[16]) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] += r[i];
-        round16<T>(v);
-    };
     auto finish = [&](float (&v)[16], int64_t first, bool live) {     // convergent: the group maximum shuffles
         const bool own_error = kResidual && p.own_error != 0;
         float y[16];
@@ -107,9 +72,9 @@ __global__ void __launch_bounds__(kThreads) roundtrip_kernel(const LbcRoundtrip 
 #pragma unroll
                 for (int i = 0; i < 16; ++i) v[i] -= y[i];
             }
-            store16<T>(rout, first, n, vec, v);
+            store16_any<T>(rout, first, n, vec, v);
         }
-        store16<T>(out, first, n, vec, y);
+        store16_any<T>(out, first, n, vec, y);
     };
 
     for (int64_t c0 = int64_t(blockIdx.x) * tile_chunks; c0 < chunks; c0 += int64_t(gridDim.x) * tile_chunks) {
@@ -128,7 +93,7 @@ __global__ void __launch_bounds__(kThreads) roundtrip_kernel(const LbcRoundtrip 
                 if (kResidual) {
                     float r[16];
                     up16<T>(rr[j], r);
-                    compensate(v, r);
+                    compensate16<T>(v, r);
                 }
                 finish(v, mine + j * (kThreads * kElemsPerThread), true);
             }
@@ -137,11 +102,11 @@ __global__ void __launch_bounds__(kThreads) roundtrip_kernel(const LbcRoundtrip 
                 const int64_t first = mine + j * (kThreads * kElemsPerThread);
                 const bool live = first / kElemsPerThread < chunks;
                 float v[16];
-                load16<T>(x, first, n, vec, v, false);                // zeros past the end
+                load16_any<T>(x, first, n, vec, v);                // zeros past the end
                 if (kResidual) {
                     float r[16];
-                    load16<T>(res, first, n, vec, r, false);
-                    compensate(v, r);
+                    load16_any<T>(res, first, n, vec, r);
+                    compensate16<T>(v, r);
                 }
                 finish(v, first, live);
             }
@@ -150,29 +115,31 @@ __global__ void __launch_bounds__(kThreads) roundtrip_kernel(const LbcRoundtrip 
 }
 
 template <typename T, int G, int BIT>
-static cudaError_t launch_roundtrip(const LbcRoundtrip* p, cudaStream_t stream) {
-    const int64_t chunks = (p->numel + G - 1) / G * (G / kElemsPerThread);
-    const int64_t one = (chunks + kThreads - 1) / kThreads;           // blocks of one chunk per thread
-    auto grid = [&](int64_t blocks) {
-        const int64_t cap = p->max_blocks > 0 ? p->max_blocks : int64_t(1) << 30;
-        return unsigned(blocks < cap ? blocks : cap);
-    };
-    if (p->residual != nullptr) {
-        roundtrip_kernel<T, G, BIT, true, 1><<<grid(one), kThreads, 0, stream>>>(*p);
-        return cudaGetLastError();
-    }
-    // Two chunks per thread (64 bytes in flight) once there are many waves of blocks: 512 Mi bf16 elements take 310 us
-    // against 322-342 with one chunk, 13 M take 12.5 us either way, and fewer leave SMs without a block.  fp32 chunks and
-    // chunks with a residual have 64 bytes in flight already.
-    if constexpr (sizeof(T) == 2) {
-        if (one > 8 * lbc_default_max_blocks()) {
-            roundtrip_kernel<T, G, BIT, false, 2><<<grid((one + 1) / 2), kThreads, 0, stream>>>(*p);
+struct RoundtripLauncher {
+    static cudaError_t run(const LbcRoundtrip* p, cudaStream_t stream) {
+        const int64_t chunks = (p->numel + G - 1) / G * (G / kElemsPerThread);
+        const int64_t one = (chunks + kThreads - 1) / kThreads;           // blocks of one chunk per thread
+        auto grid = [&](int64_t blocks) {
+            const int64_t cap = p->max_blocks > 0 ? p->max_blocks : int64_t(1) << 30;
+            return unsigned(blocks < cap ? blocks : cap);
+        };
+        if (p->residual != nullptr) {
+            roundtrip_kernel<T, G, BIT, true, 1><<<grid(one), kThreads, 0, stream>>>(*p);
             return cudaGetLastError();
         }
+        // Two chunks per thread (64 bytes in flight) once there are many waves of blocks: 512 Mi bf16 elements take 310 us
+        // against 322-342 with one chunk, 13 M take 12.5 us either way, and fewer leave SMs without a block.  fp32 chunks and
+        // chunks with a residual have 64 bytes in flight already.
+        if constexpr (sizeof(T) == 2) {
+            if (one > 8 * lbc_default_max_blocks()) {
+                roundtrip_kernel<T, G, BIT, false, 2><<<grid((one + 1) / 2), kThreads, 0, stream>>>(*p);
+                return cudaGetLastError();
+            }
+        }
+        roundtrip_kernel<T, G, BIT, false, 1><<<grid(one), kThreads, 0, stream>>>(*p);
+        return cudaGetLastError();
     }
-    roundtrip_kernel<T, G, BIT, false, 1><<<grid(one), kThreads, 0, stream>>>(*p);
-    return cudaGetLastError();
-}
+};
 
 }  // namespace lbc
 
@@ -183,19 +150,7 @@ cudaError_t lbc_roundtrip(const LbcRoundtrip* p, cudaStream_t stream) {
     if (p->residual == nullptr && (p->residual_out != nullptr || p->own_error)) return cudaErrorInvalidValue;
     if (p->numel == 0) return cudaSuccess;
     if (p->x == nullptr || p->out == nullptr) return cudaErrorInvalidValue;
-#define LBC_CASE(TT, GG, BB) \
-    if (p->group_size == GG && p->bit == BB) return lbc::launch_roundtrip<TT, GG, BB>(p, stream);
-#define LBC_TYPE(TT) \
-    LBC_CASE(TT, 64, 8) LBC_CASE(TT, 32, 8) LBC_CASE(TT, 16, 8) LBC_CASE(TT, 64, 4) LBC_CASE(TT, 32, 4) LBC_CASE(TT, 16, 4)
-    switch (p->dtype) {
-        case LBC_BF16: LBC_TYPE(__nv_bfloat16) break;
-        case LBC_FP16: LBC_TYPE(__half) break;
-        case LBC_FP32: LBC_TYPE(float) break;
-        default: break;
-    }
-#undef LBC_TYPE
-#undef LBC_CASE
-    return cudaErrorInvalidValue;
+    return lbc::dispatch_profile<lbc::RoundtripLauncher>(p, stream);
 }
 
 }  // extern "C"

@@ -269,3 +269,39 @@ def test_general_one_rank_pass_matches_the_codec(ext, dtype, bit, quant_type, to
     both = torch.zeros(1000, dtype=DTYPES[dtype], device="cuda")
     assert not ext.roundtrip_general(both[:900], None, both[100:], None, group, bit, topk, code, False, 0, passes)
     assert not ext.roundtrip_general(both[:900], both[50:950], both[:900], None, group, bit, topk, code, False, 0, passes)
+
+
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("bit,group,compact", [(8, 64, False), (8, 32, True), (4, 16, False), (4, 64, True)])
+def test_codec_kernels_at_tile_edges(ext, dtype, bit, group, compact):
+    """Encode (one and two chunks per thread), decode and the reduction of 1, 3, 4, 5 and 9 payloads: whole and ragged
+    tiles, unaligned tensors, payloads that start on an odd vector, accumulation into the output."""
+
+    cfg = _cfg(bit=bit, group_size=group, compact=compact)
+    large = 4096 * int(ext.default_max_blocks()) + 4097
+    for n, skew in ((large, 0), (8192, 0), (8192 + 4096 + 1, 0), (4095, 3), (2 * group + 1, 8)):
+        base, rbase = _data(n + skew, DTYPES[dtype], seed=n).cuda(), _data(n + skew, DTYPES[dtype], seed=n + 1).cuda()
+        x, r = base[skew:], rbase[skew:]
+        for residual in (None, r):
+            want = oracle.encode(x.cpu(), cfg, residual=None if residual is None else residual.cpu())
+            raw = torch.full((want.numel() + 16,), 0xA5, dtype=torch.uint8, device="cuda")
+            payload = raw[skew // 2 * 2:][:want.numel()] if dtype != "fp32" else raw[skew // 4 * 4:][:want.numel()]
+            prepared = torch.empty_like(base)[skew:]
+            codec.quantize_tensor(x, cfg, output=payload, residual=residual, prepared_out=prepared)
+            assert torch.equal(payload.cpu(), want), (n, skew)
+            assert torch.equal(prepared, oracle.prepare(x.cpu(), None if residual is None else residual.cpu()).cuda())
+        if n == large:
+            got = codec.dequantize_tensor(payload, (n,), cfg, dtype=dtype)
+            assert torch.equal(got.cpu().view(torch.uint8), oracle.decode(want, n, cfg, dtype).view(torch.uint8))
+            continue
+        for count in (1, 3, 4, 5, 9):
+            payloads = [oracle.encode(_data(n, DTYPES[dtype], seed=40 + k), cfg) for k in range(count)]
+            dev = [p.cuda() for p in payloads[:-1]] + [payload.copy_(payloads[-1])]
+            y, y32 = oracle.reduce_mean(payloads, n, cfg, dtype)
+            out, rout = torch.empty_like(base)[skew:], torch.empty_like(base)[skew:]
+            codec.inplace_dequantize_reduce_mean_update_error_feedback(dev, x, out, rout, cfg, reduce="mean")
+            assert torch.equal(out.cpu().view(torch.uint8), y.view(torch.uint8)), (n, skew, count)
+            assert torch.equal(rout.cpu().view(torch.uint8), oracle.residual_update(x.cpu(), y32).view(torch.uint8))
+        total = x.clone()
+        codec.dequantize_tensor(payload, (n,), cfg, dtype=dtype, output=total, reduce_op="sum")
+        assert torch.equal(total.cpu(), oracle.decode_accumulate(payloads[-1], x.cpu(), cfg)), (n, skew)
