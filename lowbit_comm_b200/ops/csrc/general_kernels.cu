@@ -19,7 +19,9 @@
 // words move as vectors, through shared memory where the records of the compact layout break the alignment.
 // Measured on a B200: encode + decode of 5 M fp32 elements, e2m1 code-book, 81 -> 27 us (the search in a table in
 // constant memory took one pass per distinct entry in a warp); all-reduce of one rank, 32 Mi bf16 elements, one kept
-// value per group, 107 -> 72 us.
+// value per group, 107 -> 72 us.  Then, without the clamp and the NaN test where the selection has shown that no value
+// needs them, without a trip through packed bytes, and with a block per tile: 72 -> 36 us (the SM's issue slots are 72 %
+// busy, DRAM 41 %), and 81 -> 25 us for the code-book.
 
 #include <cmath>
 #include <type_traits>
@@ -158,51 +160,71 @@ __device__ __forceinline__ void unpack_elems(const Packed16<T>& p, float (&v)[16
     }
 }
 
+// Tensor ends and unaligned tensors; out of line so that the common path keeps its registers (see load16_edge).
 template <typename T>
-__device__ __forceinline__ Packed16<T> load_elems(const T* base, int64_t first, int64_t n, bool vec) {
-    Packed16<T> p;
-    if (vec && first + 16 <= n) {
-#pragma unroll
-        for (int h = 0; h < Packed16<T>::kWords / 8; ++h) {
-            const U8x32 v = ld32(reinterpret_cast<const uint8_t*>(base + first) + 32 * h);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) p.w[8 * h + i] = v.w[i];
-        }
-    } else if constexpr (sizeof(T) == 2) {
+__device__ __noinline__ void load_elems_edge(const T* base, int64_t first, int64_t n, uint32_t* w) {
+    if constexpr (sizeof(T) == 2) {
         const uint16_t* b = reinterpret_cast<const uint16_t*>(base);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int64_t at = first + 2 * i;
-            p.w[i] = (at < n ? uint32_t(b[at]) : 0u) | (at + 1 < n ? uint32_t(b[at + 1]) << 16 : 0u);
+            w[i] = (at < n ? uint32_t(b[at]) : 0u) | (at + 1 < n ? uint32_t(b[at + 1]) << 16 : 0u);
         }
     } else {
         const uint32_t* b = reinterpret_cast<const uint32_t*>(base);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) p.w[i] = first + i < n ? b[first + i] : 0u;
+        for (int i = 0; i < 16; ++i) w[i] = first + i < n ? b[first + i] : 0u;
+    }
+}
+template <typename T>
+__device__ __noinline__ void store_elems_edge(T* base, int64_t first, int64_t n, const uint32_t* w) {
+    if constexpr (sizeof(T) == 2) {
+        uint16_t* b = reinterpret_cast<uint16_t*>(base);
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (first + i < n) b[first + i] = uint16_t(w[i / 2] >> (16 * (i & 1)));
+    } else {
+        uint32_t* b = reinterpret_cast<uint32_t*>(base);
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (first + i < n) b[first + i] = w[i];
+    }
+}
+
+// 16 elements at `first`, zeros past the end; `vec`: the tensor starts on 32 bytes.
+template <typename T>
+__device__ __forceinline__ Packed16<T> load_elems(const T* base, int64_t first, int64_t n, bool vec) {
+    constexpr int kWords = Packed16<T>::kWords;
+    Packed16<T> p;
+    if (vec && first + 16 <= n) {
+        const Raw16<T> r = raw16(base + first);
+#pragma unroll
+        for (int i = 0; i < kWords; ++i) p.w[i] = r.part[i / 8].w[i % 8];
+    } else {
+        uint32_t w[kWords];
+        load_elems_edge<T>(base, first, n, w);
+#pragma unroll
+        for (int i = 0; i < kWords; ++i) p.w[i] = w[i];
     }
     return p;
 }
 
 template <typename T>
 __device__ __forceinline__ void store_elems(T* base, int64_t first, int64_t n, bool vec, const Packed16<T>& p) {
+    constexpr int kWords = Packed16<T>::kWords;
     if (vec && first + 16 <= n) {
 #pragma unroll
-        for (int h = 0; h < Packed16<T>::kWords / 8; ++h) {
+        for (int h = 0; h < kWords / 8; ++h) {
             U8x32 v;
 #pragma unroll
             for (int i = 0; i < 8; ++i) v.w[i] = p.w[8 * h + i];
             st32(reinterpret_cast<uint8_t*>(base + first) + 32 * h, v);
         }
-    } else if constexpr (sizeof(T) == 2) {
-        uint16_t* b = reinterpret_cast<uint16_t*>(base);
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-            if (first + i < n) b[first + i] = uint16_t(p.w[i / 2] >> (16 * (i & 1)));
     } else {
-        uint32_t* b = reinterpret_cast<uint32_t*>(base);
+        uint32_t w[kWords];
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-            if (first + i < n) b[first + i] = p.w[i];
+        for (int i = 0; i < kWords; ++i) w[i] = p.w[i];
+        store_elems_edge<T>(base, first, n, w);
     }
 }
 
@@ -216,6 +238,19 @@ __device__ __forceinline__ void patch_elem(Packed16<T>& p, int at, uint32_t bits
     } else {
 #pragma unroll
         for (int j = 0; j < 16; ++j) p.w[j] = __byte_perm(p.w[j], bits, j == at ? 0x7654u : 0x3210u);
+    }
+}
+
+// Puts the element at position `at` of `from` in the same place.
+template <typename T>
+__device__ __forceinline__ void copy_elem(Packed16<T>& p, const Packed16<T>& from, int at) {
+    if constexpr (sizeof(T) == 2) {
+        const uint32_t how = (at & 1) ? 0x7610u : 0x3254u;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) p.w[j] = __byte_perm(p.w[j], from.w[j], j == (at >> 1) ? how : 0x3210u);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) p.w[j] = __byte_perm(p.w[j], from.w[j], j == at ? 0x7654u : 0x3210u);
     }
 }
 
@@ -240,7 +275,14 @@ struct GroupMeta {
     float stored;             // the scale, exact in T
     int idx[2];               // positions of the kept elements inside the group
     uint32_t kept[2];         // their bits
+    bool tame;                // 16-bit sources: no infinity and no NaN in the group
 };
+
+// Magnitude bits of infinity.
+template <typename T>
+__device__ __forceinline__ constexpr uint32_t inf_bits() {
+    return std::is_same<T, __half>::value ? 0x7c00u : 0x7f80u;
+}
 
 // The k largest magnitudes of a group and the next one, the scale.  `v` are the thread's 16 values, `p` the same in T;
 // the `lanes` threads of a group call this together and all get the answer.  fp32: v of a kept element turns into NaN.
@@ -249,6 +291,7 @@ __device__ __forceinline__ GroupMeta select_group(float (&v)[16], const Packed16
     GroupMeta m;
     m.idx[0] = m.idx[1] = 0;
     m.kept[0] = m.kept[1] = 0u;
+    m.tame = false;
     if constexpr (sizeof(T) == 2 && TOPK == 0) {
         uint32_t best = 0u;                                              // magnitudes as integers, two at a time
 #pragma unroll
@@ -256,6 +299,7 @@ __device__ __forceinline__ GroupMeta select_group(float (&v)[16], const Packed16
         uint32_t top = max(best >> 16, best & 0xffffu);
         for (int off = lanes / 2; off > 0; off >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, off, lanes));
         m.stored = Src<T>::up(uint16_t(top));
+        m.tame = top < inf_bits<T>();
     } else if constexpr (sizeof(T) == 2) {
         // key = magnitude bits << 17 | (63 - index) << 1 | sign: integer order is the order of the format (larger
         // magnitude first, lower index on ties), and a key holds everything that is stored of a kept element
@@ -292,6 +336,7 @@ __device__ __forceinline__ GroupMeta select_group(float (&v)[16], const Packed16
             m.kept[1] = canonical<T>((k1 >> 17) | ((k1 & 1u) << 15));
         }
         m.stored = Src<T>::up(uint16_t((TOPK == 1 ? k1 : k2) >> 17));
+        m.tame = (k0 >> 17) < inf_bits<T>();
     } else {
         auto largest = [&]() {                                           // -1: nothing but NaN left
             float a = -1.0f;
@@ -325,17 +370,26 @@ __device__ __forceinline__ GroupMeta select_group(float (&v)[16], const Packed16
 }
 
 // Rounding parameters of one call.
+constexpr float kThresholdScale = 1152921504606846976.0f;      // 2^60
+__device__ __forceinline__ float fma_saturated(float a, float b, float c) {
+    float r;
+    asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
 struct CodeRule {
-    const float* thresholds;   // kBook: thresholds[c] = the least t = value / scale whose code is above c (14 of them)
+    // kBook: thresholds[c] = -2^60 * the largest float below the least t = value / scale whose code is above c
+    const float* thresholds;
     const float* table;        // kBook, stochastic: the code-book
     int stochastic;
     unsigned long long seed;
 };
 
-// Codes of 16 values against the group's scale, as bit patterns whose low byte (nibble) is the code.
+// Codes of 16 values against the group's scale, as bit patterns whose low byte (nibble) is the code.  With `tame` (no
+// infinity and no NaN in any group of the warp) no value that is not kept verbatim is larger than the scale, so
+// |value * mul| rounds to at most the limit and neither the clamp nor the test for NaN has anything to do.
 template <int KIND>
-__device__ __forceinline__ void encode_general(const float (&v)[16], float stored, const CodeRule& rule, int64_t first,
-                                               uint32_t (&b)[16]) {
+__device__ __forceinline__ void encode_general(const float (&v)[16], float stored, bool tame, const CodeRule& rule,
+                                               int64_t first, uint32_t (&b)[16]) {
     constexpr int lim = Kind<KIND>::lim;
 #pragma unroll
     for (int i = 0; i < 16; ++i) b[i] = 0u;
@@ -350,19 +404,39 @@ __device__ __forceinline__ void encode_general(const float (&v)[16], float store
             for (int i = 0; i < 16; ++i)
                 t[i] = __fmaf_rn(v[i], mul, uniform01(rule.seed, (unsigned long long)(first + i)) - 0.5f);
         }
+        if (tame && !rule.stochastic) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) b[i] = __float_as_uint(__fadd_rn(t[i], kRoundMagic));
+            return;
+        }
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const float r = __fadd_rn(t[i] == t[i] ? t[i] : 0.0f, kRoundMagic);   // rint(t) in the low bits; NaN: code 0
             b[i] = __float_as_uint(fminf(fmaxf(r, kRoundMagic - float(lim)), kRoundMagic + float(lim)));
         }
     } else if (!rule.stochastic) {
+        // value / safe, correctly rounded: two Newton corrections of value * (1 / safe) with the exact remainder
+        // (Markstein, "Computation of elementary functions on the IBM RISC System/6000", 1990).  Its conditions (no
+        // overflow, no underflow of what decides) hold for scales up to 1e30: a quotient that is next to a threshold
+        // is at least 2^-7 and its dividend at least 2^-7 * 1e-6.
+        const bool near = __all_sync(0xffffffffu, safe < 1.0e30f);
+        const float inverse = __frcp_rn(safe);
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-            const float t = v[i] / safe;
-            uint32_t q = 0u;
+            float t;
+            if (near) {
+                t = __fmul_rn(v[i], inverse);
+                t = __fmaf_rn(__fmaf_rn(-t, safe, v[i]), inverse, t);
+                t = __fmaf_rn(__fmaf_rn(-t, safe, v[i]), inverse, t);
+            } else {
+                t = v[i] / safe;
+            }
+            // one saturated multiply-add per threshold: 1 when t has reached it, else 0 (the exact difference times
+            // 2^60 is above 1 or not above 0); comparing and counting in integers takes twice the issue slots
+            float q = kRoundMagic;
 #pragma unroll
-            for (int c = 0; c < 14; ++c) q += t < rule.thresholds[c] ? 0u : 1u;     // NaN: 14, as the search has it
-            b[i] = q;
+            for (int c = 0; c < 14; ++c) q += fma_saturated(t, kThresholdScale, rule.thresholds[c]);
+            b[i] = __float_as_uint(t == t ? q : kRoundMagic + 14.0f);      // NaN: 14, as the search has it
         }
     } else {
 #pragma unroll 1
@@ -425,6 +499,17 @@ __device__ __forceinline__ Packed16<T> decode_codes(const uint32_t (&w)[4], floa
     return pack_elems<T>(d);
 }
 
+// The same from the patterns of encode_general, without a trip through packed bytes.
+template <typename T, int KIND>
+__device__ __forceinline__ Packed16<T> decode_bits(const uint32_t (&b)[16], float stored, const float* lut) {
+    const float step = KIND == kBook ? stored : stored / float(Kind<KIND>::lim);
+    float d[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+        d[i] = __fmul_rn(KIND == kBook ? lut[b[i] & 0xfu] : __uint_as_float(b[i]) - kRoundMagic, step);
+    return pack_elems<T>(d);
+}
+
 template <int KIND>
 __device__ __forceinline__ void load_code_words(const uint8_t* p, uint32_t (&w)[4], bool vec) {
     if (vec) {
@@ -483,7 +568,7 @@ __device__ __forceinline__ void put_meta(uint8_t* meta, const GroupMeta& m, int 
 }
 
 template <typename T, int TOPK, int KIND>
-__global__ void __launch_bounds__(kThreads) quant_general_kernel(const __grid_constant__ LbcQuantGeneral p) {
+__global__ void __launch_bounds__(kThreads, 4) quant_general_kernel(const __grid_constant__ LbcQuantGeneral p) {
     const GroupShape shape = GroupShape::of<T, TOPK, KIND>(p.group_size);
     const int lanes = shape.lanes, VB = shape.VB, MB = shape.MB;
     constexpr int CB = Kind<KIND>::CB;
@@ -525,7 +610,7 @@ __global__ void __launch_bounds__(kThreads) quant_general_kernel(const __grid_co
         if (prep != nullptr && live) store_elems<T>(prep, first, n, p_vec, res != nullptr ? elems : pack_elems<T>(v));
         const GroupMeta m = select_group<T, TOPK>(v, elems, lane, lanes);
         uint32_t b[16], w[4];
-        encode_general<KIND>(v, m.stored, rule, first, b);
+        encode_general<KIND>(v, m.stored, __all_sync(0xffffffffu, m.tame), rule, first, b);
         pack_codes<T, KIND>(b, w);
 #pragma unroll
         for (int j = 0; j < TOPK; ++j) patch_code<T, KIND>(w, m.idx[j] - lane * 16);
@@ -579,7 +664,7 @@ __device__ __forceinline__ void load_lut(float (&lut)[16], int quant_type) {
 }
 
 template <typename T, int TOPK, int KIND>
-__global__ void __launch_bounds__(kThreads) dequant_general_kernel(const __grid_constant__ LbcDequantGeneral p) {
+__global__ void __launch_bounds__(kThreads, 4) dequant_general_kernel(const __grid_constant__ LbcDequantGeneral p) {
     const GroupShape shape = GroupShape::of<T, TOPK, KIND>(p.group_size);
     const int lanes = shape.lanes, VB = shape.VB, MB = shape.MB;
     constexpr int CB = Kind<KIND>::CB;
@@ -698,7 +783,7 @@ __global__ void __launch_bounds__(kThreads) reduce_general_kernel(const __grid_c
 // The all-reduce of a group of one rank: encode and decode in registers, no payload (see roundtrip_kernels.cu; here
 // the decoded values are rounded to T before the residual is taken, the rule of these profiles).
 template <typename T, int TOPK, int KIND>
-__global__ void __launch_bounds__(kThreads) roundtrip_general_kernel(const __grid_constant__ LbcRoundtripGeneral p) {
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 4 : 3) roundtrip_general_kernel(const __grid_constant__ LbcRoundtripGeneral p) {
     const GroupShape shape = GroupShape::of<T, TOPK, KIND>(p.group_size);
     const int lanes = shape.lanes;
     __shared__ float lut[16];
@@ -732,14 +817,14 @@ __global__ void __launch_bounds__(kThreads) roundtrip_general_kernel(const __gri
             float v[16];
             unpack_elems<T>(y, v);
             const GroupMeta m = select_group<T, TOPK>(v, y, lane, lanes);
-            uint32_t b[16], w[4];
-            encode_general<KIND>(v, m.stored, rule, first, b);
-            pack_codes<T, KIND>(b, w);
+            const bool tame = __all_sync(0xffffffffu, m.tame);
+            uint32_t b[16];
+            encode_general<KIND>(v, m.stored, tame, rule, first, b);
+            if (sizeof(T) == 2 && !tame) y = pack_elems<T>(v);          // a NaN that is kept has one pattern
+            const Packed16<T> from = y;
+            y = decode_bits<T, KIND>(b, m.stored, lut);
 #pragma unroll
-            for (int j = 0; j < TOPK; ++j) patch_code<T, KIND>(w, m.idx[j] - lane * 16);
-            y = decode_codes<T, KIND>(w, m.stored, lut);
-#pragma unroll
-            for (int j = 0; j < TOPK; ++j) patch_elem<T>(y, int(uint32_t(m.idx[j]) & 0xffu) - lane * 16, m.kept[j]);
+            for (int j = 0; j < TOPK; ++j) copy_elem<T>(y, from, int(uint32_t(m.idx[j]) & 0xffu) - lane * 16);
         }
         if (!live) continue;
         if (rout != nullptr) {
@@ -754,14 +839,16 @@ __global__ void __launch_bounds__(kThreads) roundtrip_general_kernel(const __gri
     }
 }
 
-static int general_grid(int64_t groups, int group_size, int max_blocks = 0) {
+// A block per 4096 elements, unless the caller caps the grid or the blocks meet at a flag or a counter (`shared`: then
+// each block costs a system-scope fence or a look at the flags, and a resident grid pays them once).
+static int general_grid(int64_t groups, int group_size, int max_blocks, bool shared) {
     int64_t want = (groups * (group_size / kElemsPerThread) + kThreads - 1) / kThreads;
-    const int cap = max_blocks > 0 ? max_blocks : lbc_default_max_blocks();
+    const int64_t cap = max_blocks > 0 ? max_blocks : (shared ? lbc_default_max_blocks() : int64_t(1) << 30);
     if (want < 1) want = 1;
     return int(want < cap ? want : cap);
 }
 
-// thresholds[c]: the least float t for which the rule "the last entry that is not above t, and the one after it when
+// The least float t for which the rule "the last entry that is not above t, and the one after it when
 // t - entry > gap / 2" gives a code above c, searched on the bit patterns around the middle of the two entries.
 struct BookThresholds {
     float of[4][14];
@@ -778,10 +865,11 @@ struct BookThresholds {
                 float t = a + (b - a) * 0.5f;
                 for (int i = 0; i < 64 && !above(t); ++i) t = std::nextafterf(t, 2.0f);
                 for (int i = 0; i < 64 && above(std::nextafterf(t, -2.0f)); ++i) t = std::nextafterf(t, -2.0f);
-                of[q][c] = t;
+                of[q][c] = -kThresholdScale * std::nextafterf(t, -2.0f);
             }
     }
 };
+// (stored as the kernel wants it, see CodeRule)
 static void fill_thresholds(float (&out)[14], int quant_type) {
     static const BookThresholds book;
     for (int c = 0; c < 14; ++c) out[c] = quant_type == LBC_LINEAR ? 0.0f : book.of[quant_type - 1][c];
@@ -825,10 +913,10 @@ static cudaError_t launch_typed(const P& p, int grid, cudaStream_t s) {
 }
 
 template <template <typename, int, int> class Kernel, typename P>
-static cudaError_t launch_general(const P& p, int max_blocks, cudaStream_t s) {
+static cudaError_t launch_general(const P& p, int max_blocks, bool shared, cudaStream_t s) {
     if (p.numel == 0) return cudaSuccess;
     if (p.group_size != 64 && p.group_size != 32 && p.group_size != 16) return cudaErrorInvalidValue;
-    const int grid = general_grid((p.numel + p.group_size - 1) / p.group_size, p.group_size, max_blocks);
+    const int grid = general_grid((p.numel + p.group_size - 1) / p.group_size, p.group_size, max_blocks, shared);
     switch (p.dtype) {
         case LBC_BF16: return launch_typed<Kernel, __nv_bfloat16>(p, grid, s);
         case LBC_FP16: return launch_typed<Kernel, __half>(p, grid, s);
@@ -861,12 +949,12 @@ cudaError_t lbc_quant_general(const LbcQuantGeneral* p, cudaStream_t stream) {
         if (p->dst[d] == nullptr) return cudaErrorInvalidValue;
     LbcQuantGeneral launch = *p;
     lbc::fill_thresholds(launch.thresholds, p->quant_type);
-    return lbc::launch_general<lbc::QuantGeneral>(launch, p->max_blocks, stream);
+    return lbc::launch_general<lbc::QuantGeneral>(launch, p->max_blocks, p->signal.num_remote > 0, stream);
 }
 
 cudaError_t lbc_dequant_general(const LbcDequantGeneral* p, cudaStream_t stream) {
     if (p == nullptr || p->numel < 0 || !lbc::general_args_ok(p->bit, p->topk, p->quant_type)) return cudaErrorInvalidValue;
-    return lbc::launch_general<lbc::DequantGeneral>(*p, 0, stream);
+    return lbc::launch_general<lbc::DequantGeneral>(*p, 0, false, stream);
 }
 
 cudaError_t lbc_reduce_general(const LbcReduceGeneral* p, cudaStream_t stream) {
@@ -881,7 +969,7 @@ cudaError_t lbc_reduce_general(const LbcReduceGeneral* p, cudaStream_t stream) {
     }
     for (int r = 0; r < p->num_src; ++r)
         if (p->src[r] == nullptr) return cudaErrorInvalidValue;
-    return lbc::launch_general<lbc::ReduceGeneral>(*p, p->max_blocks, stream);
+    return lbc::launch_general<lbc::ReduceGeneral>(*p, p->max_blocks, p->wait.flags != nullptr, stream);
 }
 
 cudaError_t lbc_roundtrip_general(const LbcRoundtripGeneral* p, cudaStream_t stream) {
@@ -890,7 +978,7 @@ cudaError_t lbc_roundtrip_general(const LbcRoundtripGeneral* p, cudaStream_t str
     if (p->numel > 0 && (p->x == nullptr || p->out == nullptr)) return cudaErrorInvalidValue;
     LbcRoundtripGeneral launch = *p;
     lbc::fill_thresholds(launch.thresholds, p->quant_type);
-    return lbc::launch_general<lbc::RoundtripGeneral>(launch, p->max_blocks, stream);
+    return lbc::launch_general<lbc::RoundtripGeneral>(launch, p->max_blocks, false, stream);
 }
 
 }  // extern "C"
