@@ -839,12 +839,15 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 4 : 3) roundtrip_ge
     }
 }
 
-// A block per 4096 elements, unless the caller caps the grid or the blocks meet at a flag or a counter (`shared`: then
-// each block costs a system-scope fence or a look at the flags, and a resident grid pays them once).
+// A block per 4096 elements up to four times the default grid: a grid that loops leaves most of the chip idle in its last
+// round (5 M elements are 1221 blocks, the default grid has 1184).  Above that the rounds even out and a looping grid pays
+// a block's set-up less often: top-k 1 on 32 Mi bf16 elements 36 us against 39.  The default grid also serves blocks
+// that meet at a flag or a counter (`shared`): each costs a system-scope fence or a look at the flags.
 static int general_grid(int64_t groups, int group_size, int max_blocks, bool shared) {
     int64_t want = (groups * (group_size / kElemsPerThread) + kThreads - 1) / kThreads;
-    const int64_t cap = max_blocks > 0 ? max_blocks : (shared ? lbc_default_max_blocks() : int64_t(1) << 30);
     if (want < 1) want = 1;
+    int64_t cap = max_blocks;
+    if (cap <= 0) cap = shared || want > 4 * lbc_default_max_blocks() ? lbc_default_max_blocks() : want;
     return int(want < cap ? want : cap);
 }
 
