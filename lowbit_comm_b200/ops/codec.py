@@ -1,9 +1,10 @@
 """Codec facade: the functions transports call to (de)quantize tensors.
 
 Parity: ccdl_comm/quantization/codec.py:104-498 (same public names and
-argument order).  CUDA tensors go to the sm_100a extension — the fused
-`quant_push` / `reduce` kernels for the production profile (linear, top-k 0,
-deterministic), the general kernels otherwise.  CPU tensors go to the bit-exact
+argument order).  CUDA tensors go to the sm_100a extension — through
+`quant_push` / `reduce` to the kernels of `csrc/codec_kernels.cu` for the
+production profile (linear, top-k 0, deterministic), to the general kernels
+otherwise.  CPU tensors go to the bit-exact
 torch oracle, which makes every transport testable without a GPU.  A CUDA
 tensor without the extension is an error, never a silent fallback.
 """
@@ -43,6 +44,14 @@ def _numel_of(shape) -> int:
     for dim in tuple(shape):
         total *= int(dim)
     return total
+
+
+def _dense(tensor: torch.Tensor | None) -> torch.Tensor | None:
+    """The tensor as the kernels take it: its elements in order, whatever its shape (a copy when it is strided)."""
+
+    if tensor is None or tensor.is_contiguous():
+        return tensor
+    return tensor.detach().reshape(-1)
 
 
 def _seed() -> int:
@@ -96,25 +105,25 @@ def quantize_tensor(tensor: torch.Tensor, config: CompressionConfig, *,
     """
 
     name = oracle.dtype_name(tensor)
+    numel = tensor.numel()
+    est = estimate_quantized_size(numel, dtype=name, config=config)
+    if output is None:
+        output = torch.empty(est.quantized_bytes, dtype=torch.uint8, device=tensor.device)
+    else:
+        _check_payload(output, numel, name, config)
+    if metadata is not None:
+        metadata.update(original_numel=numel, padded_numel=est.padded_numel, num_groups=est.num_groups,
+                        dtype=name, compact=config.compact)
+    if numel == 0:
+        return output
+    if tensor.is_cuda:
+        ext = require_extension(extension_status)
+        _cuda_quantize(ext, _dense(tensor), output, _dense(residual), _dense(prepared_out), config)
+        return output
     flat = tensor.detach().reshape(-1)
     if not flat.is_contiguous():
         flat = flat.contiguous()
     res = None if residual is None else residual.detach().reshape(-1)
-    est = estimate_quantized_size(flat.numel(), dtype=name, config=config)
-    if output is None:
-        output = torch.empty(est.quantized_bytes, dtype=torch.uint8, device=tensor.device)
-    else:
-        _check_payload(output, flat.numel(), name, config)
-    if metadata is not None:
-        metadata.update(original_numel=flat.numel(), padded_numel=est.padded_numel, num_groups=est.num_groups,
-                        dtype=name, compact=config.compact)
-    if flat.numel() == 0:
-        return output
-    if tensor.is_cuda:
-        ext = require_extension(extension_status)
-        prep = None if prepared_out is None else prepared_out.detach().reshape(-1)
-        _cuda_quantize(ext, flat, output, res, prep, config)
-        return output
     prep = None if prepared_out is None else prepared_out.detach().reshape(-1)
     if (host_codec.serves(config) and output.is_contiguous() and (res is None or res.is_contiguous())
             and (prep is None or prep.is_contiguous())):
@@ -152,14 +161,20 @@ def inplace_quantize_pack(tensor: torch.Tensor, output: torch.Tensor, residual: 
 # ---------------------------------------------------------------------------
 def _prepare_output(output, shape, numel: int, torch_dtype, device) -> tuple[torch.Tensor, torch.Tensor]:
     if output is None:
-        output = torch.empty(numel, dtype=torch_dtype, device=device)
+        output = torch.empty(tuple(shape), dtype=torch_dtype, device=device)
+        return output, output
     if output.numel() != numel:
         raise ValueError("output has the wrong number of elements")
     if output.dtype != torch_dtype:
         raise TypeError("output has the wrong dtype")
     if not output.is_contiguous():
         raise ValueError("output must be contiguous")
-    return output, output.reshape(-1)
+    return output, output          # contiguous: the kernels take the elements in order, whatever the shape
+
+
+def _shaped(out: torch.Tensor, shape) -> torch.Tensor:
+    shape = tuple(shape)
+    return out if out.shape == shape else out.reshape(shape)
 
 
 def dequantize_tensor(buffer: torch.Tensor, shape, config: CompressionConfig, *, dtype: str,
@@ -176,8 +191,10 @@ def dequantize_tensor(buffer: torch.Tensor, shape, config: CompressionConfig, *,
         raise ValueError("reduce_op='sum' needs an output to accumulate into")
     out, flat = _prepare_output(output, shape, numel, oracle.TORCH_DTYPES[name], buffer.device)
     if numel == 0:
-        return out.reshape(tuple(shape))
+        return _shaped(out, shape)
     accumulate = reduce_op == "sum"
+    if not buffer.is_cuda:
+        flat = flat.reshape(-1)
     if buffer.is_cuda:
         ext = require_extension(extension_status)
         groups = -(-numel // config.group_size)
@@ -193,13 +210,14 @@ def dequantize_tensor(buffer: torch.Tensor, shape, config: CompressionConfig, *,
         flat.copy_(oracle.decode_accumulate(buffer, flat, config))
     else:
         flat.copy_(oracle.decode(buffer, numel, config, name))
-    return out.reshape(tuple(shape))
+    return _shaped(out, shape)
 
 
 def _reduce_into(buffers: Sequence[torch.Tensor], flat_out: torch.Tensor, config: CompressionConfig, name: str,
                  divisor: float, extension_status, prepared=None, residual=None) -> None:
     """Shared body of the fused multi-payload reducers."""
 
+    flat_out = _dense(flat_out) if flat_out.is_cuda else flat_out.reshape(-1)
     numel = flat_out.numel()
     for b in buffers:
         _check_payload(b, numel, name, config)
@@ -210,9 +228,8 @@ def _reduce_into(buffers: Sequence[torch.Tensor], flat_out: torch.Tensor, config
         groups = -(-numel // config.group_size)
         if is_fast_profile(config) and len(buffers) <= MAX_FUSED_PAYLOADS:
             ext.reduce([b.data_ptr() for b in buffers], groups, 0, config.compact, numel, _DTYPE_CODE[name],
-                       config.group_size, config.bit, 1.0 / divisor, flat_out, False,
-                       None if prepared is None else prepared.reshape(-1),
-                       None if residual is None else residual.reshape(-1), [], 0, 0, None, None, 0)
+                       config.group_size, config.bit, 1.0 / divisor, flat_out, False, _dense(prepared),
+                       _dense(residual), [], 0, 0, None, None, 0)
             return
         # general profiles: per-payload decode, accumulation in the source dtype
         for i, b in enumerate(buffers):
@@ -268,7 +285,7 @@ def dequantize_reduce_tensors(buffers: Sequence[torch.Tensor], shape, config: Co
     numel = _numel_of(shape)
     out, flat = _prepare_output(output, shape, numel, oracle.TORCH_DTYPES[name], buffers[0].device)
     _reduce_into(buffers, flat, config, name, _divisor(reduce, len(buffers)), extension_status)
-    return out.reshape(tuple(shape))
+    return _shaped(out, shape)
 
 
 def inplace_dequantize_reduce_mean(buffers: Sequence[torch.Tensor], output: torch.Tensor, config: CompressionConfig, *,
@@ -276,7 +293,7 @@ def inplace_dequantize_reduce_mean(buffers: Sequence[torch.Tensor], output: torc
     if not buffers or not is_fast_profile(config) or len(buffers) > MAX_FUSED_PAYLOADS:
         return False
     name = oracle.dtype_name(output)
-    _reduce_into(buffers, output.reshape(-1), config, name, _divisor(reduce, len(buffers)), extension_status)
+    _reduce_into(buffers, output, config, name, _divisor(reduce, len(buffers)), extension_status)
     return True
 
 
@@ -291,7 +308,7 @@ def inplace_dequantize_reduce_mean_update_error_feedback(
     if not (prepared.numel() == restored.numel() == residual.numel()):
         raise ValueError("prepared, restored and residual must have the same number of elements")
     name = oracle.dtype_name(restored)
-    _reduce_into(buffers, restored.reshape(-1), config, name, _divisor(reduce, len(buffers)), extension_status,
+    _reduce_into(buffers, restored, config, name, _divisor(reduce, len(buffers)), extension_status,
                  prepared=prepared, residual=residual)
     return True
 

@@ -376,6 +376,17 @@ void wait_signal(const WaitArg& wait, const SignalArg& signal) {
     cuda_check(lbc_wait_signal(&w, &s, at::cuda::getCurrentCUDAStream()), "lbc_wait_signal");
 }
 
+// What is enqueued on `then` from here on waits for what `first` holds now (both streams of one device).
+void order_streams(uintptr_t first, uintptr_t then, int device_index) {
+    c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device_index));
+    cudaEvent_t event = nullptr;
+    cuda_check(cudaEventCreateWithFlags(&event, cudaEventDisableTiming), "cudaEventCreateWithFlags");
+    cudaError_t err = cudaEventRecord(event, reinterpret_cast<cudaStream_t>(first));
+    if (err == cudaSuccess) err = cudaStreamWaitEvent(reinterpret_cast<cudaStream_t>(then), event, 0);
+    cudaEventDestroy(event);      // released when the device is through with it
+    cuda_check(err, "order_streams");
+}
+
 at::Tensor tensor_from_address(uintptr_t ptr, int64_t nbytes, int device_index) {
     TORCH_CHECK(ptr != 0 && nbytes >= 0, "bad address or size");
     auto options = at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device_index);
@@ -451,6 +462,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("status_clear", &lbc::status_clear);
     m.def("tensor_from_address", &tensor_from_address);
     m.def("memset_async", &memset_async);
+    m.def("order_streams", &order_streams, py::arg("first"), py::arg("then"), py::arg("device_index"));
 
     lbc::bind_work(m);
     lbc::bind_fused_plan(m);

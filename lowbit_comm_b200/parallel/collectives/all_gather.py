@@ -9,6 +9,7 @@ from ...config import CompressionConfig
 from ...core.work import CollectiveWork, ImmediateWork
 from ...ops import codec
 from ..payload import GatheredPayloads, coerce_payload, payload_buffer
+from ._routes import communicator_module
 
 
 def compressed_all_gather(
@@ -28,9 +29,7 @@ def compressed_all_gather(
 
     injected = any(v is not None for v in (quantize, dequantize, all_gather))
     if not injected:
-        from ..communicator import get_communicator
-
-        return get_communicator(group).all_gather(tensor, config=config, async_op=async_op, dtype=dtype)
+        return communicator_module().get_communicator(group).all_gather(tensor, config=config, async_op=async_op, dtype=dtype)
     name = dtype if dtype != "auto" else codec.resolve_dtype(dtype, tensor)
     shape = tuple(tensor.shape)
     raw = quantize(tensor, config) if quantize is not None else codec.quantize_tensor(

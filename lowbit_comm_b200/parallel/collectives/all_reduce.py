@@ -13,6 +13,7 @@ from ..payload import (CompressedAllGatherReduce, CompressedAllReduce, Compresse
                        coerce_payload, payload_buffer)
 from ..payload_packing import (DEFAULT_FUSED_PAYLOAD_MIN_NUMEL, make_fused_payload_all_gather,
                                make_payload_all_gather, should_fuse_payload)
+from ._routes import communicator_module
 
 _STRATEGIES = {"all_gather", "all_reduce", "topology", "reduce_scatter", "hierarchical", "auto", "native_nccl"}
 
@@ -62,10 +63,9 @@ def compressed_all_reduce(
         raise UnsupportedCollective(f"all_reduce:{op}", reason="only op='sum' and op='mean' are implemented")
     if compiled_plan is not None:
         return _finish(compiled_plan.run(tensor), async_op)
-    injected = any(v is not None for v in (quantize, dequantize, all_reduce, all_gather, topology_all_reduce))
-    if not injected:
-        from ..communicator import get_communicator
-
+    if quantize is None and dequantize is None and all_reduce is None and all_gather is None \
+            and topology_all_reduce is None:
+        get_communicator = communicator_module().get_communicator
         comm = get_communicator(group, extension_status=extension_status) if extension_status is not None \
             else get_communicator(group)
         chosen = topology_method if (strategy == "topology" and topology_method) else strategy

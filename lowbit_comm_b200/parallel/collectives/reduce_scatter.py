@@ -17,13 +17,11 @@ from typing import Any
 from ...config import CompressionConfig
 from ...core.shard import ReducedShard
 from ...core.work import CollectiveWork
-from ._routes import as_requested, check_reduction, first_that_serves, injected
+from ._routes import as_requested, check_reduction, communicator_module, first_that_serves, injected
 
 
 def _communicator(group: Any | None):
-    from ..communicator import get_communicator
-
-    return get_communicator(group)
+    return communicator_module().get_communicator(group)
 
 
 def compressed_reduce_scatter(tensor: Any, *, config: CompressionConfig, op: str = "mean", async_op: bool = False,

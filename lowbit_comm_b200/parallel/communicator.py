@@ -27,6 +27,8 @@ import threading
 from importlib import import_module
 from typing import Any
 
+import torch
+
 from ..config import CompressionConfig
 from ..core.chunking import GroupShardPlan
 from ..core.info import ExecutionInfo
@@ -236,11 +238,8 @@ class Communicator:
     def _stream_scope(self, tensor: Any, async_op: bool):
         """(context manager, completion factory) for running on the side stream when async."""
 
-        torch = import_module("torch")
         if not async_op:
-            import contextlib
-
-            return contextlib.nullcontext(), None
+            return _NO_RANGE, None
         from .completion import comm_stream
 
         side = comm_stream(tensor.device)
@@ -282,6 +281,11 @@ class Communicator:
                     raise
                 ws = None
             if ws is not None:
+                if not async_op and not tracing.ENABLED:
+                    result = ws.all_reduce(tensor, out, residual=residual, update_residual=update_residual, op=op,
+                                           stages=stages, ef_mode=ef_mode)
+                    self.stats["peer_ops"] += 1
+                    return result
                 scope, side = self._stream_scope(tensor, async_op)
                 with scope, tracing.nvtx_range("lbc.all_reduce") if tracing.ENABLED else _NO_RANGE:
                     result = ws.all_reduce(tensor, out, residual=residual, update_residual=update_residual, op=op,
@@ -353,7 +357,6 @@ class Communicator:
         raise UnsupportedCollective(f"all_reduce:{strategy}", reason="unknown strategy")
 
     def _torch_all_reduce(self, tensor, config, op, stages, name, out, residual, update_residual):
-        torch = import_module("torch")
         prepared = tensor if residual is None else (tensor.float() + residual.float()).to(tensor.dtype)
         from .fused import default_stages
 
@@ -380,7 +383,6 @@ class Communicator:
         return out
 
     def _torch_reduce_scatter(self, tensor, config, op, name):
-        torch = import_module("torch")
         flat = tensor.reshape(-1)
         plan = GroupShardPlan.build(flat.numel(), self.world_size, config.group_size, 8)  # same geometry as the fused path
         padded = torch.nn.functional.pad(flat, (0, plan.padded_numel - flat.numel()))
@@ -399,7 +401,6 @@ class Communicator:
 
         if op not in ("sum", "mean"):
             raise UnsupportedCollective(f"reduce_scatter:{op}", reason="only op='sum' and op='mean' are implemented")
-        torch = import_module("torch")
         name = codec.resolve_dtype(dtype, tensor)
         shape = tuple(tensor.shape)
         n = tensor.numel()
@@ -412,7 +413,7 @@ class Communicator:
             ws = self.workspace(tensor, config, name)
             scope, side = self._stream_scope(tensor, async_op)
             with scope:
-                ws.reduce_scatter(tensor.reshape(-1), shard, residual=residual, op=op)
+                ws.reduce_scatter(tensor if tensor.is_contiguous() else tensor.reshape(-1), shard, residual=residual, op=op)
             self.stats["peer_ops"] += 1
             result = ReducedShard(shard=shard, shard_index=self.rank, shard_numel=geo.shard_numel,
                                   original_shape=shape, original_numel=n, world_size=self.world_size, reduce=op,
@@ -437,7 +438,6 @@ class Communicator:
     def _validated_out(out: Any, tensor: Any, shard_numel: int) -> Any:
         """Caller-owned output checks (parity: reduce_scatter_transport.py:390-431)."""
 
-        torch = import_module("torch")
         if out is None:
             return torch.empty(shard_numel, dtype=tensor.dtype, device=tensor.device)
         if hasattr(out, "tensor") and hasattr(out, "mark_submitting"):  # an output lease
@@ -465,7 +465,6 @@ class Communicator:
     # -- all-gather -------------------------------------------------------------
     def all_gather(self, tensor: Any, *, config: CompressionConfig, async_op: bool = False,
                    dtype: str = "auto") -> Any:
-        torch = import_module("torch")
         name = codec.resolve_dtype(dtype, tensor)
         shape = tuple(tensor.shape)
         if self.peer_usable(tensor, config):
@@ -531,7 +530,6 @@ class Communicator:
         per stage, ccdl_comm/cuda/transports/hierarchical.py:184-265).
         """
 
-        torch = import_module("torch")
         L = local_group_size or self._default_local_group()
         local, inter = self.sub_communicators(L)
         name = codec.resolve_dtype(dtype, tensor)

@@ -424,6 +424,24 @@ class _PeerEngine:
         return self._retired_launches + sum(ws.launches for ws in self.workspaces.values())
 
 
+class _OnSideStream:
+    """`with torch.cuda.stream(side)` behind `side.wait_stream(current)`, for a tensor on the current device: the same
+    two stream switches and one event, without the device bookkeeping (a third of the host time of a bucket)."""
+
+    __slots__ = ("_torch", "_side", "_producer")
+
+    def __init__(self, torch: Any, ext: Any, side: Any, index: int) -> None:
+        self._torch, self._side = torch, side
+        self._producer = torch.cuda.current_stream(index)
+        ext.order_streams(self._producer.cuda_stream, side.cuda_stream, index)
+
+    def __enter__(self) -> None:
+        self._torch.cuda.set_stream(self._side)
+
+    def __exit__(self, *exc: Any) -> None:
+        self._torch.cuda.set_stream(self._producer)
+
+
 class DDPCommHook:
     """The callable handed to `DistributedDataParallel.register_comm_hook`."""
 
@@ -705,9 +723,13 @@ def create_ddp_comm_hook(
         decision = policy.decide(key, numel=tensor.numel())
         residual = feedback.residual_for(key, tensor) if (decision.apply or decision.update) else None
         stages = {"all_gather": 1, "reduce_scatter": 2, "topology": 2}.get(effective)
-        producer = torch.cuda.current_stream(tensor.device)
-        peer.stream.wait_stream(producer)
-        with torch.cuda.stream(peer.stream):
+        index = tensor.device.index
+        if index == torch.cuda.current_device():
+            scope = _OnSideStream(torch, ws.ext, peer.stream, index)
+        else:
+            peer.stream.wait_stream(torch.cuda.current_stream(tensor.device))
+            scope = torch.cuda.stream(peer.stream)
+        with scope:
             ws.all_reduce(tensor, residual=residual if decision.apply else None,
                           update_residual=decision.update, op=reduce, stages=stages, ef_mode=ef_mode)
             future = torch.futures.Future(devices=[tensor.device])

@@ -42,6 +42,9 @@ chunk c of collective t+1 only after every peer's QUANT flag of t+1, which a pee
 kernel of collective t (the one that read this rank's reduced shard) has ended.
 The "legacy" engine is the K1/K2/K3 sequence described above; reduce-scatter and all-gather use it.
 
+A group of one rank takes neither engine: nobody else reads its payload, so the native plans run one kernel that
+quantizes and decodes in registers (`ops/csrc/roundtrip_kernels.cu`) unless the buffers overlap.
+
 This replaces the reference's quantize -> NCCL all_to_all / all_gather ->
 dequantize chains (ccdl_comm/communication/reduce_scatter_transport.py:186-377,
 ccdl_comm/collectives/all_reduce.py:158-271).
@@ -51,6 +54,7 @@ from __future__ import annotations
 
 import os
 from dataclasses import dataclass
+from functools import lru_cache
 
 import torch
 
@@ -75,7 +79,12 @@ def _chunk_slack(world_size: int, config: CompressionConfig) -> int:
     return 2 * MAX_CHUNKS * world_size * ALIGN_GROUPS * config.group_size + MAX_CHUNKS * 256 * 8
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _current_stream_ptr(device) -> int:
+    if _raw_stream is not None and device.index is not None:
+        return _raw_stream(device.index)              # the handle, without a Stream object around it
     return torch.cuda.current_stream(device).cuda_stream
 
 
@@ -113,9 +122,14 @@ class FusedGeometry:
 
 
 def geometry(numel: int, world_size: int, dtype: str, config: CompressionConfig) -> FusedGeometry:
-    plan = GroupShardPlan.build(numel, world_size, config.group_size, ALIGN_GROUPS)
-    return FusedGeometry(numel, world_size, config.group_size, config.group_size * config.bit // 8,
-                         dtype_bytes(dtype), plan.shard_groups, plan.num_groups)
+    return _geometry(numel, world_size, dtype, config.group_size, config.bit)
+
+
+@lru_cache(maxsize=1024)      # integers of a size: 0.3 us instead of 5 on every reduced-shard and gather call
+def _geometry(numel: int, world_size: int, dtype: str, group_size: int, bit: int) -> FusedGeometry:
+    plan = GroupShardPlan.build(numel, world_size, group_size, ALIGN_GROUPS)
+    return FusedGeometry(numel, world_size, group_size, group_size * bit // 8, dtype_bytes(dtype), plan.shard_groups,
+                         plan.num_groups)
 
 
 def default_stages(world_size: int, nbytes: int, multicast: bool = False) -> int:
@@ -539,7 +553,7 @@ class FusedWorkspace:
         epoch = self.group.next_epoch(self.channel)
         parity = epoch & 1
         valid = geo.shard_valid_numel(self.group.rank)
-        flat_out = out_shard.reshape(-1)
+        flat_out = out_shard if out_shard.dim() == 1 else out_shard.reshape(-1)
         if valid < geo.shard_numel:
             flat_out[valid:].zero_()
         if self._native is not None and self.phase_timer is None and hasattr(self._native, "reduce_scatter"):

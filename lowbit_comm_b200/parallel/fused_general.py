@@ -14,6 +14,8 @@ such a profile takes two kernels that fuse the codec with the movement; no NCCL 
                         source dtype in rank order (the reference's unfused SUM rule), scale by 1/W for a
                         mean, write the result and residual = T(prepared - result)
 
+A group of one rank needs neither: `roundtrip_general` encodes and decodes in registers, one launch.
+
 Every rank reduces all W payloads (the one-stage exchange, the default).  The result is, bit for bit, what
 `codec.dequantize_reduce_tensors` gives for the same payloads, so the torch.distributed path and this one
 are interchangeable.

@@ -289,7 +289,10 @@ class PeerGroup:
 
         if getattr(self, "_closed", False):
             return                                   # the status word went with the arena
-        status = DeviceWaitStatus(*self._ext.status_read(self.status_host))
+        words = self._ext.status_read(self.status_host)
+        if words[0] == 0:
+            return
+        status = DeviceWaitStatus(*words)
         if status.timed_out:
             raise AsyncCommunicationError.from_wait(self.rank, status)
 

@@ -305,3 +305,24 @@ def test_codec_kernels_at_tile_edges(ext, dtype, bit, group, compact):
         total = x.clone()
         codec.dequantize_tensor(payload, (n,), cfg, dtype=dtype, output=total, reduce_op="sum")
         assert torch.equal(total.cpu(), oracle.decode_accumulate(payloads[-1], x.cpu(), cfg)), (n, skew)
+
+
+@pytest.mark.parametrize("kw", [{}, {"topk": 1}, {"compact": True}])
+def test_codec_takes_tensors_of_any_shape(ext, kw):
+    """Shapes and strides at the entry points: the kernels see the elements in order, results have the asked shape."""
+
+    cfg = _cfg(**kw)
+    base = _data(48 * 130, torch.bfloat16).cuda()
+    dense, strided = base.reshape(48, 130), base.reshape(130, 48).t()
+    for x in (dense, strided, dense.reshape(4, 12, 130)):
+        want = oracle.encode(x.cpu().contiguous(), cfg)
+        payload = codec.quantize_tensor(x, cfg, residual=torch.zeros_like(x))
+        assert torch.equal(payload.cpu(), want)
+        back = oracle.decode(want, x.numel(), cfg, "bf16").reshape(x.shape)
+        got = codec.dequantize_tensor(payload, x.shape, cfg, dtype="bf16")
+        assert got.shape == x.shape and torch.equal(got.cpu(), back)
+        into = torch.zeros(x.numel(), dtype=x.dtype, device="cuda")
+        got = codec.dequantize_tensor(payload, x.shape, cfg, dtype="bf16", output=into, reduce_op="sum")
+        assert got.shape == x.shape and got.data_ptr() == into.data_ptr() and torch.equal(got.cpu(), back)
+        got = codec.dequantize_reduce_tensors([payload], x.shape, cfg, dtype="bf16", reduce="mean")
+        assert got.shape == x.shape and torch.equal(got.cpu(), back)
