@@ -12,8 +12,8 @@
 // the result needs; the phases also wrote and read the payload, read the input's row twice and met at a grid-wide
 // flag.  A block per tile and no loop over tiles: on a B200 a persistent grid of the same kernel moved 5.9 TB/s where
 // the full grid moves 6.7-6.9, because the blocks of one wave end at different times and the next ones fill in.
-// Measured (bf16, int8 groups of 64): 512 Mi elements 919 -> 314 us (6.8 TB/s), 13.1 M elements 41.1 -> 13.9 us,
-// 124 M elements in 11 buckets with error feedback 636 -> 320 us (the rest is the host).
+// Measured through the public calls (bf16, int8 groups of 64): 512 Mi elements 919 -> 312 us (6.9 TB/s), 13.1 M elements
+// 41.0 -> 10.2 us, 124 M elements in 7 buckets with error feedback 637 -> 183 us.
 #include "codec_device.cuh"
 #include "common.cuh"
 #include "lbc_api.h"
