@@ -418,8 +418,10 @@ __device__ __forceinline__ void encode_general(const float (&v)[16], float store
         // value / safe, correctly rounded: two Newton corrections of value * (1 / safe) with the exact remainder
         // (Markstein, "Computation of elementary functions on the IBM RISC System/6000", 1990).  Its conditions (no
         // overflow, no underflow of what decides) hold for scales up to 1e30: a quotient that is next to a threshold
-        // is at least 2^-7 and its dividend at least 2^-7 * 1e-6.
-        const bool near = __all_sync(0xffffffffu, safe < 1.0e30f);
+        // is at least 2^-7 and its dividend at least 2^-7 * 1e-6, and no value that is not kept is above the scale.
+        // A 16-bit group with more NaN than it keeps has NaN for its scale, which bounds no value (the quotient by 1e-6
+        // may overflow, and its remainder is NaN then): the test is on the scale as stored, false for NaN.
+        const bool near = __all_sync(0xffffffffu, stored < 1.0e30f);
         const float inverse = __frcp_rn(safe);
 #pragma unroll
         for (int i = 0; i < 16; ++i) {

@@ -210,6 +210,52 @@ def test_codebook_codes_at_their_thresholds(ext, quant_type):
         assert torch.equal(codec.quantize_tensor(x.cuda(), cfg).cpu(), oracle.encode(x, cfg)), scale
 
 
+@pytest.mark.parametrize("quant_type", ("normal", "uniform", "e3m0", "e2m1"))
+def test_codebook_codes_around_the_division_limit(ext, quant_type):
+    """The corrected reciprocal serves scales below 1e30, a division the others: values at every threshold with scales
+    next to the limit, and 16-bit sources (whose quotients round apart from the fp32 ones) on both sides of it."""
+
+    table = oracle.codebook(quant_type)[:15]
+    mids = table[:-1] + (table[1:] - table[:-1]) / 2
+    around = torch.cat([mids, torch.nextafter(mids, mids - 1), torch.nextafter(mids, mids + 1), table])
+    around = around[:around.numel() // 15 * 15].reshape(-1, 15)
+    groups = torch.cat([torch.ones(around.shape[0], 1), around], dim=1)
+    limit = torch.tensor(1.0e30)
+    below, above = torch.nextafter(limit, torch.tensor(0.0)), torch.nextafter(limit, torch.tensor(2.0e30))
+    cfg = _cfg(bit=4, group_size=16, quant_type=quant_type)
+    for name, scales in (("fp32", (below, limit, above)), ("bf16", (0.9e30, 1.1e30, 1.7, 3e-7)), ("fp16", (1.7, 3e-7))):
+        for scale in scales:
+            x = (groups * scale).to(DTYPES[name]).reshape(-1)
+            assert torch.equal(codec.quantize_tensor(x.cuda(), cfg).cpu(), oracle.encode(x, cfg)), (name, scale)
+
+
+@pytest.mark.parametrize("dtype", ("bf16", "fp16"))
+@pytest.mark.parametrize("topk", (0, 1))
+def test_codebook_codes_in_a_group_whose_scale_is_nan(ext, dtype, topk):
+    """More NaN than the group keeps: the scale is NaN, the codes are those of value / 1e-6 (the floor of a scale), as
+    a division gives them, also where that overflows."""
+
+    cfg = _cfg(bit=4, group_size=16, topk=topk, quant_type="e2m1")
+    top = torch.finfo(DTYPES[dtype]).max
+    x = torch.zeros(6 * 16)
+    x[:64] = _data(64, torch.float32, seed=1)                        # finite groups in the same warp
+    nan = [float("nan")] * (topk + 1)
+    for g, body in ((4, [-float("inf"), float("inf"), -top, top, -0.25 * top, 0.0, -1e-7, 1e-7]), (5, [-1.0, 1.0, -5e-7])):
+        x[16 * g:16 * g + len(nan) + len(body)] = torch.tensor(nan + body)
+    x = x.to(DTYPES[dtype])
+    table = oracle.codebook("e2m1")
+    t = x.float() / torch.tensor(1e-6)
+    low = (torch.searchsorted(table[:15].contiguous(), t, right=True) - 1).clamp_(0, 14)
+    want = low + ((t - table[low]) > (table[low + 1] - table[low]) / 2).to(torch.int64)
+    for g in (4, 5):
+        want[16 * g:16 * g + topk] = 7                               # what is kept has the code of zero
+    payload = codec.quantize_tensor(x.cuda(), cfg).cpu()
+    codes = oracle._unpack_words(payload[:x.numel() // 2].reshape(-1, 8), 4, 2).reshape(-1)
+    assert codes[64:].tolist() == want[64:].tolist()
+    finite = oracle.encode(x[:64], cfg)
+    assert torch.equal(payload[:32], finite[:32])
+
+
 @pytest.mark.parametrize("dtype", list(DTYPES))
 @pytest.mark.parametrize("bit,group,topk", [(8, 64, 0), (8, 16, 2), (4, 32, 1), (4, 64, 0)])
 def test_compact_records_through_warp_spans(ext, dtype, bit, group, topk):
