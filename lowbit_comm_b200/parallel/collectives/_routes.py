@@ -11,8 +11,8 @@ arguments, which is the calling convention the reference's transports are writte
 from __future__ import annotations
 
 import sys
-
 from collections.abc import Callable, Iterable
+from importlib import import_module
 from typing import Any
 
 from ...core.shard import ReducedShard
@@ -22,19 +22,22 @@ from ...exceptions import UnsupportedCollective
 Route = Callable[[Any], Any]
 
 
+_COMMUNICATOR = __name__.rpartition(".collectives.")[0] + ".communicator"
+_imported: Any = None       # set once the import has returned
+
+
 def communicator_module() -> Any:
     """`parallel.communicator`, imported on first use (it needs torch, the package import does not); afterwards a look
-    in `sys.modules`, a tenth of the cost of an import statement."""
+    in `sys.modules`, a tenth of the cost of an import statement.  `sys.modules` alone would not do: it holds a module
+    from before its body has run, and the import is what waits for another thread that is at it."""
 
+    global _imported
     module = sys.modules.get(_COMMUNICATOR)
-    if module is None:
-        from importlib import import_module
-
-        module = import_module(_COMMUNICATOR)
+    if module is None or module is not _imported:
+        module = _imported = import_module(_COMMUNICATOR)
     return module
 
 
-_COMMUNICATOR = __name__.rpartition(".collectives.")[0] + ".communicator"
 REDUCTIONS = ("sum", "mean")
 
 

@@ -1,0 +1,59 @@
+"""State that calls share: modules imported on first use, memoized sizes and geometry."""
+
+import subprocess
+import sys
+
+FIRST_USE = r"""
+import importlib.machinery, sys, threading, time
+from lowbit_comm_b200.parallel.collectives._routes import communicator_module
+
+NAME = "lowbit_comm_b200.parallel.communicator"
+started, found, failed = threading.Event(), [], []
+
+
+class Slow:
+    # the module's own loader, with a pause between its entry in sys.modules and its body
+    def __init__(self, loader): self.loader = loader
+    def __getattr__(self, name): return getattr(self.loader, name)
+    def create_module(self, spec): return self.loader.create_module(spec)
+    def exec_module(self, module):
+        started.set()
+        time.sleep(0.5)
+        self.loader.exec_module(module)
+
+
+class Finder:
+    @staticmethod
+    def find_spec(name, path, target=None):
+        if name != NAME:
+            return None
+        spec = importlib.machinery.PathFinder.find_spec(name, path)
+        spec.loader = Slow(spec.loader)
+        return spec
+
+
+def first_call():
+    try:
+        found.append(communicator_module().get_communicator)
+    except Exception as exc:
+        failed.append(repr(exc))
+
+
+assert NAME not in sys.modules
+sys.meta_path.insert(0, Finder)
+threads = [threading.Thread(target=first_call) for _ in range(8)]
+threads[0].start()
+assert started.wait(60)
+for t in threads[1:]: t.start()
+for t in threads: t.join()
+assert not failed, failed
+assert len(found) == 8 and len(set(found)) == 1
+replaced = type(sys)(NAME)
+sys.modules[NAME] = replaced            # as an import statement, a later look sees what is in sys.modules
+assert communicator_module() is replaced
+"""
+
+
+def test_threads_that_make_their_first_collective_wait_for_the_import():
+    done = subprocess.run([sys.executable, "-c", FIRST_USE], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
