@@ -122,14 +122,17 @@ class FusedGeometry:
 
 
 def geometry(numel: int, world_size: int, dtype: str, config: CompressionConfig) -> FusedGeometry:
-    return _geometry(numel, world_size, dtype, config.group_size, config.bit)
+    ask = _memoized if type(numel) is int else _geometry
+    return ask(numel, world_size, dtype, config.group_size, config.bit)
 
 
-@lru_cache(maxsize=1024)      # integers of a size: 0.3 us instead of 5 on every reduced-shard and gather call
 def _geometry(numel: int, world_size: int, dtype: str, group_size: int, bit: int) -> FusedGeometry:
     plan = GroupShardPlan.build(numel, world_size, group_size, ALIGN_GROUPS)
     return FusedGeometry(numel, world_size, group_size, group_size * bit // 8, dtype_bytes(dtype), plan.shard_groups,
                          plan.num_groups)
+
+
+_memoized = lru_cache(maxsize=1024, typed=True)(_geometry)     # plain integers only, as in ops/sizing.py; 0.3 us instead of 5
 
 
 def default_stages(world_size: int, nbytes: int, multicast: bool = False) -> int:

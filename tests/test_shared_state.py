@@ -1,7 +1,15 @@
 """State that calls share: modules imported on first use, memoized sizes and geometry."""
 
+import dataclasses
 import subprocess
 import sys
+
+import numpy as np
+import pytest
+import torch
+
+from lowbit_comm_b200 import CompressionConfig, estimate_quantized_size, quantize_tensor
+from lowbit_comm_b200.parallel.fused import geometry
 
 FIRST_USE = r"""
 import importlib.machinery, sys, threading, time
@@ -57,3 +65,19 @@ assert communicator_module() is replaced
 def test_threads_that_make_their_first_collective_wait_for_the_import():
     done = subprocess.run([sys.executable, "-c", FIRST_USE], capture_output=True, text=True, timeout=300)
     assert done.returncode == 0, done.stderr[-2000:]
+
+
+@pytest.mark.parametrize("first", (float, np.int64, np.int32, np.array, bool))
+def test_memoized_sizes_keep_the_types_of_each_caller(first):
+    """Sizes that are equal but of another type are other keys: what one caller asks for changes nothing for the next."""
+
+    numel = 1 if first is bool else 640 + len(first.__name__)
+    config = CompressionConfig()
+    estimate_quantized_size(first(numel), dtype="bf16", config=config)
+    geometry(first(numel), 2, "bf16", config)
+    estimate, shape = estimate_quantized_size(numel, dtype="bf16", config=config), geometry(numel, 2, "bf16", config)
+    for value in (*dataclasses.asdict(estimate).values(), *dataclasses.asdict(shape).values()):
+        assert type(value) in (int, float, str), value
+    assert type(estimate.quantized_bytes) is int and type(estimate.numel) is int and type(shape.shard_groups) is int
+    payload = quantize_tensor(torch.randn(numel, dtype=torch.bfloat16), config)
+    assert payload.numel() == estimate.quantized_bytes
