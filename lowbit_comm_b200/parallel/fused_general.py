@@ -116,9 +116,10 @@ class GeneralPeerWorkspace:
         res = None if residual is None else residual.reshape(-1)
         keep = res if (res is not None and update_residual) else None      # `prepared` is parked here
         out_flat = target.reshape(-1)
+        seed = _seed() if cfg.stochastic else 0        # one draw a call, whichever kernels serve it
         if W == 1 and self.fused and ext.roundtrip_general(
                 flat, res, out_flat, keep, cfg.group_size, cfg.bit, cfg.topk, _QUANT_CODE[cfg.quant_type], cfg.stochastic,
-                _seed() if cfg.stochastic else 0, stages, self.max_blocks):
+                seed, stages, self.max_blocks):
             self.launches += 1        # one rank: nobody else reads the payload, it is encoded and decoded in registers
             return target
         nbytes = estimate_quantized_size(n, dtype=self.dtype, config=cfg).quantized_bytes
@@ -127,7 +128,7 @@ class GeneralPeerWorkspace:
             return self._two_stage(flat, out_flat, res, keep, n, epoch, region, dst, op, target)
         if self.fused:
             ext.quant_general_push(flat, res, keep, dst, cfg.group_size, cfg.bit, cfg.topk, _QUANT_CODE[cfg.quant_type],
-                                   cfg.stochastic, cfg.compact, _seed() if cfg.stochastic else 0,
+                                   cfg.stochastic, cfg.compact, seed,
                                    g.signal_all(self.channel, PHASE_REDUCE_SCATTER, epoch), self.max_blocks)
             ext.reduce_general([g.local_ptr + region + r * self.slot_bytes for r in range(W)], out_flat, cfg.group_size,
                                cfg.bit, cfg.topk, _QUANT_CODE[cfg.quant_type], cfg.compact,
@@ -137,7 +138,7 @@ class GeneralPeerWorkspace:
             return target
         payload = g.local_view(self.stage_off, nbytes)
         ext.quant_general(flat, res, keep, payload, cfg.group_size, cfg.bit, cfg.topk, _QUANT_CODE[cfg.quant_type],
-                          cfg.stochastic, cfg.compact, _seed() if cfg.stochastic else 0)
+                          cfg.stochastic, cfg.compact, seed)
         ext.push_bytes(g.local_ptr + self.stage_off, _round_up(nbytes, 16), dst, None,
                        g.signal_all(self.channel, PHASE_REDUCE_SCATTER, epoch), self.max_blocks)
         ext.wait_signal(g.wait_all(self.channel, PHASE_REDUCE_SCATTER, epoch), None)

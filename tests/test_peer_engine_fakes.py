@@ -443,3 +443,54 @@ def test_communicator_arena_grows_collectively_and_refuses_when_it_cannot(monkey
     boxed.mailbox = object()
     with pytest.raises(CCDLUnavailableError, match="mailbox"):
         boxed.workspace(T(16_000_000), cfg, "bf16")
+
+
+@pytest.mark.parametrize("world,fused,serves", [(1, True, True), (1, True, False), (1, False, False), (2, True, False),
+                                                (2, False, False)])
+def test_a_stochastic_all_reduce_draws_one_seed(world, fused, serves):
+    """Whichever kernels serve the call (the one-pass form may decline it), the generator moves by one draw and the
+    kernels get that number."""
+
+    from lowbit_comm_b200.ops import codec
+    from lowbit_comm_b200.parallel.fused_general import GeneralPeerWorkspace
+
+    seeds = []
+
+    class Ext:
+        def roundtrip_general(self, x, residual, out, keep, group, bit, topk, code, stochastic, seed, passes, blocks):
+            seeds.append(seed)
+            return serves
+
+        def quant_general(self, *args):
+            seeds.append(args[-1])
+
+        def quant_general_push(self, *args):
+            seeds.append(args[10])
+
+        def __getattr__(self, name):
+            return lambda *args: None
+
+    class Group:
+        world_size, rank, local_ptr, _ext = world, 0, 0, Ext()
+
+        def alloc(self, nbytes):
+            return 0
+
+        def next_epoch(self, channel):
+            return 1
+
+        def local_view(self, offset, nbytes):
+            return torch.empty(nbytes, dtype=torch.uint8)
+
+        def __getattr__(self, name):
+            return lambda *args: 0
+
+    config = CompressionConfig(stochastic=True, allow_experimental=True)
+    ws = GeneralPeerWorkspace(Group(), dtype="bf16", config=config, max_numel=640, fused=fused)
+    torch.manual_seed(5)
+    want = codec._seed()
+    after = codec._seed()
+    torch.manual_seed(5)
+    ws.all_reduce(torch.zeros(640, dtype=torch.bfloat16))
+    assert seeds and set(seeds) == {want}
+    assert codec._seed() == after
