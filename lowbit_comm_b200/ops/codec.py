@@ -118,7 +118,8 @@ def quantize_tensor(tensor: torch.Tensor, config: CompressionConfig, *,
         return output
     if tensor.is_cuda:
         ext = require_extension(extension_status)
-        _cuda_quantize(ext, _dense(tensor), output, _dense(residual), _dense(prepared_out), config)
+        # (of a view with one stride, base[::2] say, reshape(-1) is that view and no copy)
+        _cuda_quantize(ext, _dense(tensor).contiguous(), output, _dense(residual), _dense(prepared_out), config)
         return output
     flat = tensor.detach().reshape(-1)
     if not flat.is_contiguous():

@@ -372,3 +372,16 @@ def test_codec_takes_tensors_of_any_shape(ext, kw):
         assert got.shape == x.shape and got.data_ptr() == into.data_ptr() and torch.equal(got.cpu(), back)
         got = codec.dequantize_reduce_tensors([payload], x.shape, cfg, dtype="bf16", reduce="mean")
         assert got.shape == x.shape and torch.equal(got.cpu(), back)
+
+
+@pytest.mark.parametrize("kw", [{}, {"topk": 1}, {"compact": True}, {"bit": 4, "quant_type": "normal"}])
+def test_codec_takes_views_with_one_stride(ext, kw):
+    """Every other element, one element repeated, a column: views whose flattened form is a view again."""
+
+    cfg = _cfg(**kw)
+    base = _data(6000, torch.bfloat16).cuda()
+    for x in (base[::2], base[3::7], base[:1].expand(200), base.reshape(60, 100)[:, :1]):
+        want = oracle.encode(x.cpu().contiguous(), cfg)
+        assert torch.equal(codec.quantize_tensor(x, cfg).cpu(), want)
+        assert torch.equal(codec.quantize_tensor(x, cfg, residual=torch.zeros(x.shape, dtype=x.dtype, device="cuda")).cpu(),
+                           want)
