@@ -54,6 +54,13 @@ def _dense(tensor: torch.Tensor | None) -> torch.Tensor | None:
     return tensor.detach().reshape(-1)
 
 
+def _write_back(target: torch.Tensor | None, dense: torch.Tensor | None) -> None:
+    """After the kernels: what `_dense` copied for an output goes back to the tensor the caller holds."""
+
+    if dense is not target:
+        target.detach().copy_(dense.view(target.shape))
+
+
 def _seed() -> int:
     return int(torch.randint(0, 2**62, (1,), dtype=torch.int64).item())
 
@@ -118,25 +125,30 @@ def quantize_tensor(tensor: torch.Tensor, config: CompressionConfig, *,
         return output
     if tensor.is_cuda:
         ext = require_extension(extension_status)
+        prep = _dense(prepared_out)
         # (of a view with one stride, base[::2] say, reshape(-1) is that view and no copy)
-        _cuda_quantize(ext, _dense(tensor).contiguous(), output, _dense(residual), _dense(prepared_out), config)
+        _cuda_quantize(ext, _dense(tensor).contiguous(), output, _dense(residual), prep, config)
+        _write_back(prepared_out, prep)
         return output
     flat = tensor.detach().reshape(-1)
     if not flat.is_contiguous():
         flat = flat.contiguous()
     res = None if residual is None else residual.detach().reshape(-1)
-    prep = None if prepared_out is None else prepared_out.detach().reshape(-1)
+    dense = _dense(prepared_out)
+    prep = None if dense is None else dense.detach().reshape(-1)
     if (host_codec.serves(config) and output.is_contiguous() and (res is None or res.is_contiguous())
             and (prep is None or prep.is_contiguous())):
         host_codec.quantize(flat, config, name, output, res, prep)   # C++ twin of the oracle, bit-identical
+        _write_back(prepared_out, dense)
         return output
     noise = None
     if config.stochastic:
         noise = torch.rand(est.padded_numel) - 0.5
     encoded = oracle.encode(flat, config, residual=res, noise=noise)
     output.copy_(encoded)
-    if prepared_out is not None:
-        prepared_out.reshape(-1).copy_(oracle.prepare(flat, res))
+    if prep is not None:
+        prep.copy_(oracle.prepare(flat, res))
+        _write_back(prepared_out, dense)
     return output
 
 
@@ -214,11 +226,19 @@ def dequantize_tensor(buffer: torch.Tensor, shape, config: CompressionConfig, *,
     return _shaped(out, shape)
 
 
-def _reduce_into(buffers: Sequence[torch.Tensor], flat_out: torch.Tensor, config: CompressionConfig, name: str,
+def _reduce_into(buffers: Sequence[torch.Tensor], out: torch.Tensor, config: CompressionConfig, name: str,
                  divisor: float, extension_status, prepared=None, residual=None) -> None:
-    """Shared body of the fused multi-payload reducers."""
+    """Shared body of the fused multi-payload reducers: `out` and `residual` of any strides."""
 
-    flat_out = _dense(flat_out) if flat_out.is_cuda else flat_out.reshape(-1)
+    dense_out, dense_residual = _dense(out), _dense(residual)
+    _reduce_dense(buffers, dense_out, config, name, divisor, extension_status, _dense(prepared), dense_residual)
+    _write_back(out, dense_out)
+    _write_back(residual, dense_residual)
+
+
+def _reduce_dense(buffers, flat_out, config, name, divisor, extension_status, prepared, residual) -> None:
+    if not flat_out.is_cuda:
+        flat_out = flat_out.reshape(-1)
     numel = flat_out.numel()
     for b in buffers:
         _check_payload(b, numel, name, config)
@@ -229,8 +249,8 @@ def _reduce_into(buffers: Sequence[torch.Tensor], flat_out: torch.Tensor, config
         groups = -(-numel // config.group_size)
         if is_fast_profile(config) and len(buffers) <= MAX_FUSED_PAYLOADS:
             ext.reduce([b.data_ptr() for b in buffers], groups, 0, config.compact, numel, _DTYPE_CODE[name],
-                       config.group_size, config.bit, 1.0 / divisor, flat_out, False, _dense(prepared),
-                       _dense(residual), [], 0, 0, None, None, 0)
+                       config.group_size, config.bit, 1.0 / divisor, flat_out, False, prepared, residual,
+                       [], 0, 0, None, None, 0)
             return
         # general profiles: per-payload decode, accumulation in the source dtype
         for i, b in enumerate(buffers):
@@ -330,9 +350,11 @@ def update_error_feedback_residual(prepared: torch.Tensor, restored: torch.Tenso
                                    extension_status: CudaExtensionStatus | None = None) -> torch.Tensor:
     """residual = T(float(prepared) - float(restored)), written in place."""
 
+    dense = _dense(residual)
     if prepared.is_cuda:
         require_extension(extension_status).error_feedback_update(
-            prepared.reshape(-1), restored.reshape(-1), residual.reshape(-1))
+            prepared.reshape(-1), restored.reshape(-1), dense.reshape(-1))
     else:
-        residual.reshape(-1).copy_(oracle.residual_update_from_restored(prepared, restored))
+        dense.reshape(-1).copy_(oracle.residual_update_from_restored(prepared, restored))
+    _write_back(residual, dense)
     return residual
