@@ -54,11 +54,10 @@ def _dense(tensor: torch.Tensor | None) -> torch.Tensor | None:
     return tensor.detach().reshape(-1)
 
 
-def _write_back(target: torch.Tensor | None, dense: torch.Tensor | None) -> None:
+def _write_back(target: torch.Tensor, dense: torch.Tensor) -> None:
     """After the kernels: what `_dense` copied for an output goes back to the tensor the caller holds."""
 
-    if dense is not target:
-        target.detach().copy_(dense.view(target.shape))
+    target.detach().copy_(dense.view(target.shape))
 
 
 def _seed() -> int:
@@ -125,10 +124,12 @@ def quantize_tensor(tensor: torch.Tensor, config: CompressionConfig, *,
         return output
     if tensor.is_cuda:
         ext = require_extension(extension_status)
-        prep = _dense(prepared_out)
         # (of a view with one stride, base[::2] say, reshape(-1) is that view and no copy)
-        _cuda_quantize(ext, _dense(tensor).contiguous(), output, _dense(residual), prep, config)
-        _write_back(prepared_out, prep)
+        x = tensor if tensor.is_contiguous() else tensor.detach().contiguous()
+        prep = _dense(prepared_out)
+        _cuda_quantize(ext, x, output, _dense(residual), prep, config)
+        if prep is not prepared_out:
+            _write_back(prepared_out, prep)
         return output
     flat = tensor.detach().reshape(-1)
     if not flat.is_contiguous():
@@ -139,7 +140,8 @@ def quantize_tensor(tensor: torch.Tensor, config: CompressionConfig, *,
     if (host_codec.serves(config) and output.is_contiguous() and (res is None or res.is_contiguous())
             and (prep is None or prep.is_contiguous())):
         host_codec.quantize(flat, config, name, output, res, prep)   # C++ twin of the oracle, bit-identical
-        _write_back(prepared_out, dense)
+        if dense is not prepared_out:
+            _write_back(prepared_out, dense)
         return output
     noise = None
     if config.stochastic:
@@ -148,7 +150,8 @@ def quantize_tensor(tensor: torch.Tensor, config: CompressionConfig, *,
     output.copy_(encoded)
     if prep is not None:
         prep.copy_(oracle.prepare(flat, res))
-        _write_back(prepared_out, dense)
+        if dense is not prepared_out:
+            _write_back(prepared_out, dense)
     return output
 
 
@@ -232,8 +235,10 @@ def _reduce_into(buffers: Sequence[torch.Tensor], out: torch.Tensor, config: Com
 
     dense_out, dense_residual = _dense(out), _dense(residual)
     _reduce_dense(buffers, dense_out, config, name, divisor, extension_status, _dense(prepared), dense_residual)
-    _write_back(out, dense_out)
-    _write_back(residual, dense_residual)
+    if dense_out is not out:
+        _write_back(out, dense_out)
+    if dense_residual is not residual:
+        _write_back(residual, dense_residual)
 
 
 def _reduce_dense(buffers, flat_out, config, name, divisor, extension_status, prepared, residual) -> None:
@@ -356,5 +361,6 @@ def update_error_feedback_residual(prepared: torch.Tensor, restored: torch.Tenso
             prepared.reshape(-1), restored.reshape(-1), dense.reshape(-1))
     else:
         dense.reshape(-1).copy_(oracle.residual_update_from_restored(prepared, restored))
-    _write_back(residual, dense)
+    if dense is not residual:
+        _write_back(residual, dense)
     return residual
