@@ -22,17 +22,9 @@ namespace lbc {
 // ---------------------------------------------------------------------------
 // encode
 // ---------------------------------------------------------------------------
-template <typename T, bool kWhole>
-__device__ __forceinline__ void store_chunk(T* to, int64_t first, int64_t numel, const float (&values)[16]) {
-    if constexpr (kWhole)
-        store16<T>(to + first, 0, 16, true, values);
-    else
-        store16_any<T>(to, first, numel, (reinterpret_cast<uintptr_t>(to) & 31) == 0, values);
-}
-
-// Quantizes and stores the thread's 16 values.  kWhole: they all lie inside 32-byte aligned tensors.  Convergent (the
-// group maximum shuffles); `span` is the warp's staging area for compact records.
-template <typename T, int G, int BIT, bool kCompact, bool kWhole>
+// Quantizes and stores the thread's 16 values.  Convergent (the group maximum shuffles); `span` is the warp's staging area
+// for compact records.
+template <typename T, int G, int BIT, bool kCompact, int kFit>
 __device__ __forceinline__ void encode_chunk(const LbcQuantPush& p, float (&v)[16], int64_t chunk, uint8_t* span) {
     constexpr int lanes = G / kElemsPerThread;
     constexpr int VB = G * BIT / 8, MB = sizeof(T), CB = kElemsPerThread * BIT / 8;
@@ -41,7 +33,7 @@ __device__ __forceinline__ void encode_chunk(const LbcQuantPush& p, float (&v)[1
     uint8_t* dst = p.dst[0];
     const int64_t num_groups = (p.numel + G - 1) / G;
     const int64_t first = chunk * kElemsPerThread;
-    const bool live = kWhole || chunk < num_groups * lanes;
+    const bool live = kFit == kFitWhole || chunk < num_groups * lanes;
     const int64_t g = chunk / lanes;
     const int lane = int(chunk) & (lanes - 1);
     const int wlane = threadIdx.x & 31;
@@ -49,10 +41,10 @@ __device__ __forceinline__ void encode_chunk(const LbcQuantPush& p, float (&v)[1
 #pragma unroll
     for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
     const float stored = group_max<G>(amax);                      // exact in T, like the values
-    if (prep != nullptr && live) store_chunk<T, kWhole>(prep, first, p.numel, v);
+    if (prep != nullptr && live) store16_fit<T, kFit>(prep, first, p.numel, v);
     float err[16];
     const uint4 codes = encode16<T, BIT>(v, stored, lef != nullptr ? &err : nullptr);
-    if (lef != nullptr && live) store_chunk<T, kWhole>(lef, first, p.numel, err);
+    if (lef != nullptr && live) store16_fit<T, kFit>(lef, first, p.numel, err);
     if (kCompact && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
         uint8_t* rec = span + (wlane / lanes) * (VB + MB);
         const uint32_t w[4] = {codes.x, codes.y, codes.z, codes.w};
@@ -70,24 +62,28 @@ __device__ __forceinline__ void encode_chunk(const LbcQuantPush& p, float (&v)[1
     }
 }
 
-// A tile with the tensor's end in it, or of unaligned tensors.
-template <typename T, int G, int BIT, bool kCompact>
+// A tile with the tensor's end in it (kFitTail), or of unaligned tensors.
+template <typename T, int G, int BIT, bool kCompact, int kFit>
 __device__ __forceinline__ void encode_edge(const LbcQuantPush& p, int64_t c0, int chunks_per_thread, uint8_t* span) {
     const T* x = static_cast<const T*>(p.x);
     const T* res = static_cast<const T*>(p.residual);
     for (int j = 0; j < chunks_per_thread; ++j) {
         const int64_t chunk = c0 + j * kThreads + threadIdx.x;
         float v[16];
-        load16_any<T>(x, chunk * kElemsPerThread, p.numel, (reinterpret_cast<uintptr_t>(x) & 31) == 0, v);
+        load16_fit<T, kFit>(x, chunk * kElemsPerThread, p.numel, v);
         if (res != nullptr) {
             float r[16];
-            load16_any<T>(res, chunk * kElemsPerThread, p.numel, (reinterpret_cast<uintptr_t>(res) & 31) == 0, r);
+            load16_fit<T, kFit>(res, chunk * kElemsPerThread, p.numel, r);
             compensate16<T>(v, r);
         }
-        encode_chunk<T, G, BIT, kCompact, false>(p, v, chunk, span);
+        encode_chunk<T, G, BIT, kCompact, kFit>(p, v, chunk, span);
     }
 }
 
+template <int G, int BIT, typename T>
+constexpr int encode_span(bool compact) { return compact ? span_bytes(G, G * BIT / 8 + int(sizeof(T))) : 16; }
+
+// All tensors on 32 bytes (the payload may start anywhere).
 template <typename T, int G, int BIT, bool kCompact, bool kResidual, int U>
 __global__ void __launch_bounds__(kThreads, 4) encode_kernel(const __grid_constant__ LbcQuantPush p) {
     constexpr int lanes = G / kElemsPerThread;
@@ -95,13 +91,11 @@ __global__ void __launch_bounds__(kThreads, 4) encode_kernel(const __grid_consta
     const T* x = static_cast<const T*>(p.x);
     const T* res = static_cast<const T*>(p.residual);
     const int64_t chunks = (p.numel + G - 1) / G * lanes;
-    const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(res) |
-                       reinterpret_cast<uintptr_t>(p.prepared_out) | reinterpret_cast<uintptr_t>(p.local_ef_out)) & 31) == 0;
-    __shared__ __align__(16) uint8_t spans[kThreads / 32][kCompact ? span_bytes(G, G * BIT / 8 + int(sizeof(T))) : 16];
+    __shared__ __align__(16) uint8_t spans[kThreads / 32][encode_span<G, BIT, T>(kCompact)];
     uint8_t* span = spans[threadIdx.x >> 5];
     for (int64_t c0 = int64_t(blockIdx.x) * tile_chunks; c0 < chunks; c0 += int64_t(gridDim.x) * tile_chunks) {
-        if (!vec || (c0 + tile_chunks) * kElemsPerThread > p.numel) {
-            encode_edge<T, G, BIT, kCompact>(p, c0, U, span);
+        if ((c0 + tile_chunks) * kElemsPerThread > p.numel) {
+            encode_edge<T, G, BIT, kCompact, kFitTail>(p, c0, U, span);
             continue;
         }
         const int64_t mine = c0 + threadIdx.x;
@@ -120,9 +114,22 @@ __global__ void __launch_bounds__(kThreads, 4) encode_kernel(const __grid_consta
                 up16<T>(rr[j], r);
                 compensate16<T>(v, r);
             }
-            encode_chunk<T, G, BIT, kCompact, true>(p, v, mine + j * kThreads, span);
+            encode_chunk<T, G, BIT, kCompact, kFitWhole>(p, v, mine + j * kThreads, span);
         }
     }
+    grid_signal(p.signal);
+}
+
+// A tensor on another boundary (a view into a larger one), in a kernel of its own: as a branch of encode_kernel this ran
+// out of line, element by element.  16 Mi elements, the input one element in, with error feedback (grid-stride kernel of
+// fast_kernels.cu / that branch / here): bf16 45.8 / 41.1 / 27.1 us, fp32 45.6 / 61.7 / 43.5.  Blocks per SM, fp32, 4 / 3:
+// 46.3 / 43.1 us.
+template <typename T, int G, int BIT, bool kCompact>
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 4) encode_ragged_kernel(const __grid_constant__ LbcQuantPush p) {
+    const int64_t chunks = (p.numel + G - 1) / G * (G / kElemsPerThread);
+    __shared__ __align__(16) uint8_t spans[kThreads / 32][encode_span<G, BIT, T>(kCompact)];
+    for (int64_t c0 = int64_t(blockIdx.x) * kThreads; c0 < chunks; c0 += int64_t(gridDim.x) * kThreads)
+        encode_edge<T, G, BIT, kCompact, kFitRagged>(p, c0, 1, spans[threadIdx.x >> 5]);
     grid_signal(p.signal);
 }
 
@@ -138,6 +145,10 @@ struct EncodeLauncher {
         };
         const auto go = [&](auto compact) {
             constexpr bool kCompact = decltype(compact)::value;
+            if (!on_boundary(32, p->x, p->residual, p->prepared_out, p->local_ef_out)) {
+                encode_ragged_kernel<T, G, BIT, kCompact><<<grid(one), kThreads, 0, stream>>>(*p);
+                return;
+            }
             if (p->residual != nullptr) {
                 encode_kernel<T, G, BIT, kCompact, true, 1><<<grid(one), kThreads, 0, stream>>>(*p);
                 return;
@@ -222,8 +233,8 @@ __device__ __forceinline__ void add_batch(const LbcReduce& p, int r0, int64_t ch
     }
 }
 
-// A chunk with the tensor's end in its tile, of unaligned tensors or of payloads that are not vector-aligned.
-template <typename T, int G, int BIT, bool kCompact>
+// A chunk with the tensor's end in its tile (kFitTail), or of tensors or payloads on any boundary.
+template <typename T, int G, int BIT, bool kCompact, int kFit>
 __device__ __forceinline__ void decode_edge(const LbcReduce& p, int64_t chunk) {
     constexpr int lanes = G / kElemsPerThread;
     constexpr int VB = G * BIT / 8, MB = sizeof(T), CB = kElemsPerThread * BIT / 8;
@@ -231,7 +242,6 @@ __device__ __forceinline__ void decode_edge(const LbcReduce& p, int64_t chunk) {
     T* out = static_cast<T*>(p.out);
     T* rout = static_cast<T*>(p.residual_out);
     const T* prep = static_cast<const T*>(p.prepared);
-    const auto on32 = [](const void* t) { return (reinterpret_cast<uintptr_t>(t) & 31) == 0; };
     const int64_t first = chunk * kElemsPerThread, g = chunk / lanes;
     const int lane = int(chunk) & (lanes - 1);
     const int64_t voff = (kCompact ? g * (VB + MB) : g * VB) + lane * CB;
@@ -246,22 +256,22 @@ __device__ __forceinline__ void decode_edge(const LbcReduce& p, int64_t chunk) {
     for (int i = 0; i < 16; ++i) acc[i] *= p.scale;
     if (rout != nullptr) {
         float e[16];
-        load16_any<T>(prep, first, p.numel, on32(prep), e);
+        load16_fit<T, kFit>(prep, first, p.numel, e);
 #pragma unroll
         for (int i = 0; i < 16; ++i) e[i] -= acc[i];
-        store16_any<T>(rout, first, p.numel, on32(rout), e);
+        store16_fit<T, kFit>(rout, first, p.numel, e);
     }
     if (p.accumulate) {
         float prev[16];
-        load16_any<T>(out, first, p.numel, on32(out), prev);
+        load16_fit<T, kFit>(static_cast<const T*>(out), first, p.numel, prev);
         round16<T>(acc);
 #pragma unroll
         for (int i = 0; i < 16; ++i) acc[i] += prev[i];
     }
-    store16_any<T>(out, first, p.numel, on32(out), acc);        // rounds to T
+    store16_fit<T, kFit>(out, first, p.numel, acc);             // rounds to T
 }
 
-// B payloads are in flight per thread.  B == 1: one payload, no error feedback (the launcher's rule).
+// Tensors on 32 bytes, payloads on their vectors.  B payloads are in flight per thread.  B == 1: one payload, no error feedback (the launcher's rule).
 // Blocks per SM, measured at 128 Mi bf16 elements (decode) and 32 Mi (mean of 8, with error feedback): decode with 8 / 6 /
 // 5 / 4 blocks 66 / 71 / 76 / 84 us; mean with four payloads in flight and 5 / 4 / 3 / 2 blocks 82 / 81 / 89 / 90 us (of two
 // payloads 49 / 50 / 56 / 56), eight in flight 107 / 82 / 91 / 100.  Compact, two in flight: 105 / 101 / 113 / 144.
@@ -269,24 +279,19 @@ template <typename T, int G, int BIT, bool kCompact, int B>
 __global__ void __launch_bounds__(kThreads, B == 1 ? (sizeof(T) == 2 ? 8 : 6) : (kCompact || sizeof(T) == 4 ? 4 : 5))
 decode_kernel(const __grid_constant__ LbcReduce p) {
     constexpr int lanes = G / kElemsPerThread;
-    constexpr int VB = G * BIT / 8, MB = sizeof(T), CB = kElemsPerThread * BIT / 8;
+    constexpr int VB = G * BIT / 8, MB = sizeof(T);
     T* out = static_cast<T*>(p.out);
     const T* prep = static_cast<const T*>(p.prepared);
     T* rout = static_cast<T*>(p.residual_out);
     const int64_t chunks = (p.numel + G - 1) / G * lanes;
     const int R = B == 1 ? 1 : p.num_src;
-    uintptr_t bits = 0;
-    for (int r = 0; r < R; ++r) bits |= reinterpret_cast<uintptr_t>(p.src[r]);
-    const bool vec = (bits & (kCompact ? 15 : CB - 1)) == 0 &&
-                     ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(prep) |
-                       reinterpret_cast<uintptr_t>(rout)) & 31) == 0;
     __shared__ __align__(16) uint8_t spans[kThreads / 32][kCompact ? span_bytes(G, VB + MB) : 16];
     uint8_t* span = spans[threadIdx.x >> 5];
 
     for (int64_t c0 = int64_t(blockIdx.x) * kThreads; c0 < chunks; c0 += int64_t(gridDim.x) * kThreads) {
         const int64_t chunk = c0 + threadIdx.x;
-        if (!vec || (c0 + kThreads) * kElemsPerThread > p.numel) {
-            decode_edge<T, G, BIT, kCompact>(p, chunk);
+        if ((c0 + kThreads) * kElemsPerThread > p.numel) {
+            decode_edge<T, G, BIT, kCompact, kFitTail>(p, chunk);
             continue;
         }
         const int64_t first = chunk * kElemsPerThread;
@@ -321,6 +326,22 @@ decode_kernel(const __grid_constant__ LbcReduce p) {
     }
 }
 
+// A tensor or a payload on another boundary (a view into a larger one; a row of a gather buffer whose payloads are no
+// multiple of 16 bytes).  kSeveral: more than one payload, or error feedback.
+// Blocks per SM, 16 Mi bf16 elements, planar 8-bit payloads of which one starts on 4 bytes, inputs beyond L2, 4 / 5 / 6
+// blocks: one payload 17.6 / 16.5 / 18.5 us, mean of two with error feedback 35.2 / 32.9 / 28.8, of eight 73.8 / 67.8 /
+// 61.6; 8-bit records, mean of eight 82.6 / 76.2 / 84.9.
+// As a branch of decode_kernel this ran out of line, element by element.  16 Mi bf16 elements, buffers in L2 (grid-stride
+// kernel of fast_kernels.cu / that branch / here): a payload on 8 bytes 14.8 / 18.8 / 11.5 us, an output one element in
+// 99.7 / 107.7 / 37.2.
+template <typename T, int G, int BIT, bool kCompact, bool kSeveral>
+__global__ void __launch_bounds__(kThreads, kSeveral && !(kCompact && BIT == 8 && sizeof(T) == 2) ? 6 : 5)
+decode_ragged_kernel(const __grid_constant__ LbcReduce p) {
+    const int64_t chunks = (p.numel + G - 1) / G * (G / kElemsPerThread);
+    for (int64_t c0 = int64_t(blockIdx.x) * kThreads; c0 < chunks; c0 += int64_t(gridDim.x) * kThreads)
+        decode_edge<T, G, BIT, kCompact, kFitRagged>(p, c0 + threadIdx.x);
+}
+
 template <typename T, int G, int BIT>
 struct DecodeLauncher {
     static cudaError_t run(const LbcReduce* p, cudaStream_t stream) {
@@ -330,6 +351,16 @@ struct DecodeLauncher {
         const unsigned grid = unsigned(p->max_blocks > 0 && blocks > p->max_blocks ? p->max_blocks : blocks);
         const auto go = [&](auto compact) {
             constexpr bool kCompact = decltype(compact)::value;
+            bool vectors = on_boundary(32, p->out, p->prepared, p->residual_out);
+            for (int r = 0; r < p->num_src; ++r)
+                vectors = vectors && on_boundary(kCompact ? 16 : kElemsPerThread * BIT / 8, p->src[r]);
+            if (!vectors) {
+                if (p->num_src == 1 && p->residual_out == nullptr)
+                    decode_ragged_kernel<T, G, BIT, kCompact, false><<<grid, kThreads, 0, stream>>>(*p);
+                else
+                    decode_ragged_kernel<T, G, BIT, kCompact, true><<<grid, kThreads, 0, stream>>>(*p);
+                return;
+            }
             // a compact payload takes two vectors per lane, so half as many are in flight
             if (p->num_src == 1 && p->residual_out == nullptr)
                 decode_kernel<T, G, BIT, kCompact, 1><<<grid, kThreads, 0, stream>>>(*p);

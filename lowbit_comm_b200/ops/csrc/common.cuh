@@ -217,8 +217,8 @@ __device__ __forceinline__ void up16(const Raw16<T>& r, float (&v)[16]) {
     }
 }
 
-// Tensor ends and unaligned tensors, element by element.  Out of line on purpose: inlined, their sixteen addresses and
-// predicates cost the whole-tile path registers (spills at four blocks per SM).
+// Tensor ends, element by element.  Out of line on purpose: inlined, their sixteen addresses and predicates cost the
+// whole-tile path registers (spills at four blocks per SM).
 template <typename T>
 __device__ __noinline__ void load16_edge(const T* base, int64_t first, int64_t numel, float* out) {
     float v[16];
@@ -255,6 +255,119 @@ __device__ __forceinline__ void store16_any(T* base, int64_t first, int64_t nume
         for (int i = 0; i < 16; ++i) v[i] = vals[i];
         store16_edge<T>(base, first, numel, v);
     }
+}
+
+// The same for tensors of any element alignment, inline: kernels of unaligned calls are instantiated apart from those of
+// aligned ones, so what this takes in registers costs the others nothing.  The widest accesses that the address allows
+// (it is a tensor's, alike for every chunk); only the chunk with the tensor's end goes element by element.
+template <typename T>
+__device__ __forceinline__ void load16_ragged(const T* base, int64_t first, int64_t numel, float (&out)[16]) {
+    if (first + 16 > numel) {
+        float v[16];
+        load16_edge<T>(base, first, numel, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) out[i] = v[i];
+        return;
+    }
+    const T* p = base + first;
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    Raw16<T> r;
+    constexpr int kWords = 4 * int(sizeof(T));
+    uint32_t w[kWords];
+    if ((a & 31) == 0) {
+        r = raw16(p);
+        up16<T>(r, out);
+        return;
+    }
+    if ((a & 15) == 0) {
+#pragma unroll
+        for (int i = 0; i < kWords / 4; ++i) {
+            const uint4 v = ld16(reinterpret_cast<const uint4*>(p) + i);
+            w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
+        }
+    } else if (sizeof(T) == 4 || (a & 3) == 0) {
+#pragma unroll
+        for (int i = 0; i < kWords; ++i) w[i] = reinterpret_cast<const uint32_t*>(p)[i];
+    } else {                                            // 16-bit elements from an odd one on: the words between lie on 4 bytes
+        const uint16_t* h = reinterpret_cast<const uint16_t*>(p);
+        uint32_t before = uint32_t(h[0]) << 16;
+#pragma unroll
+        for (int i = 0; i < kWords; ++i) {
+            const uint32_t next = i + 1 < kWords ? *reinterpret_cast<const uint32_t*>(h + 1 + 2 * i) : uint32_t(h[15]);
+            w[i] = __funnelshift_r(before, next, 16);
+            before = next;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) r.part[i / 8].w[i % 8] = w[i];
+    up16<T>(r, out);
+}
+template <typename T>
+__device__ __forceinline__ void store16_ragged(T* base, int64_t first, int64_t numel, const float (&vals)[16]) {
+    if (first + 16 > numel) {
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = vals[i];
+        store16_edge<T>(base, first, numel, v);
+        return;
+    }
+    T* p = base + first;
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    constexpr int kWords = 4 * int(sizeof(T));
+    if ((a & 31) == 0) {
+        store16<T>(p, 0, 16, true, vals);
+        return;
+    }
+    uint32_t w[kWords];
+    if constexpr (sizeof(T) == 2) {
+#pragma unroll
+        for (int i = 0; i < kWords; ++i) w[i] = Src<T>::down2(vals[2 * i], vals[2 * i + 1]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < kWords; ++i) w[i] = __float_as_uint(vals[i]);
+    }
+    if ((a & 15) == 0) {
+#pragma unroll
+        for (int i = 0; i < kWords / 4; ++i)
+            st16(reinterpret_cast<uint4*>(p) + i, make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]));
+    } else if (sizeof(T) == 4 || (a & 3) == 0) {
+#pragma unroll
+        for (int i = 0; i < kWords; ++i) reinterpret_cast<uint32_t*>(p)[i] = w[i];
+    } else {
+        uint16_t* h = reinterpret_cast<uint16_t*>(p);
+        h[0] = uint16_t(w[0]);
+#pragma unroll
+        for (int i = 0; i + 1 < kWords; ++i)
+            *reinterpret_cast<uint32_t*>(h + 1 + 2 * i) = __funnelshift_r(w[i], w[i + 1], 16);
+        h[15] = uint16_t(w[kWords - 1] >> 16);
+    }
+}
+
+// How a chunk lies in its tensors: inside, all of them on 32 bytes; perhaps with their end in it; on any element.
+enum : int { kFitWhole = 0, kFitTail = 1, kFitRagged = 2 };
+template <typename T, int kFit>
+__device__ __forceinline__ void load16_fit(const T* base, int64_t first, int64_t numel, float (&out)[16]) {
+    if constexpr (kFit == kFitWhole)
+        up16<T>(raw16(base + first), out);
+    else if constexpr (kFit == kFitTail)
+        load16_any<T>(base, first, numel, true, out);
+    else
+        load16_ragged<T>(base, first, numel, out);
+}
+template <typename T, int kFit>
+__device__ __forceinline__ void store16_fit(T* base, int64_t first, int64_t numel, const float (&vals)[16]) {
+    if constexpr (kFit == kFitWhole)
+        store16<T>(base + first, 0, 16, true, vals);
+    else if constexpr (kFit == kFitTail)
+        store16_any<T>(base, first, numel, true, vals);
+    else
+        store16_ragged<T>(base, first, numel, vals);
+}
+// Host: do all of these (null included) start on `bytes`?
+inline bool on_boundary(uintptr_t bytes, const void* a, const void* b = nullptr, const void* c = nullptr,
+                        const void* d = nullptr) {
+    return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) |
+             reinterpret_cast<uintptr_t>(d)) & (bytes - 1)) == 0;
 }
 
 // prepared = T(x + residual)

@@ -41,45 +41,60 @@ __device__ __forceinline__ void roundtrip16(float (&v)[16], float (&y)[16], bool
     }
 }
 
-// kResidual: the input is T(x + residual).  U chunks of 16 elements per thread are loaded before the first is computed.
+// From the prepared values to the outputs.  Convergent: the group maximum shuffles.
+template <typename T, int G, int BIT, bool kResidual, int kFit>
+__device__ __forceinline__ void roundtrip_chunk(const LbcRoundtrip& p, float (&v)[16], int64_t first, bool live) {
+    T* out = static_cast<T*>(p.out);
+    T* rout = static_cast<T*>(p.residual_out);
+    const bool own_error = kResidual && p.own_error != 0;
+    float y[16];
+    roundtrip16<T, G, BIT>(v, y, own_error);
+    if (p.passes == 2) {
+        float z[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) z[i] = y[i];
+        round16<T>(z);
+        roundtrip16<T, G, BIT>(z, y, false);
+    }
+    if (!live) return;
+    if (kResidual && rout != nullptr) {
+        if (!own_error) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] -= y[i];
+        }
+        store16_fit<T, kFit>(rout, first, p.numel, v);
+    }
+    store16_fit<T, kFit>(out, first, p.numel, y);
+}
+
+// A chunk with the tensor's end in its tile (kFitTail), or of unaligned tensors.
+template <typename T, int G, int BIT, bool kResidual, int kFit>
+__device__ __forceinline__ void roundtrip_edge(const LbcRoundtrip& p, int64_t chunk, int64_t chunks) {
+    const int64_t first = chunk * kElemsPerThread;
+    float v[16];
+    load16_fit<T, kFit>(static_cast<const T*>(p.x), first, p.numel, v);      // zeros past the end
+    if (kResidual) {
+        float r[16];
+        load16_fit<T, kFit>(static_cast<const T*>(p.residual), first, p.numel, r);
+        compensate16<T>(v, r);
+    }
+    roundtrip_chunk<T, G, BIT, kResidual, kFit>(p, v, first, chunk < chunks);
+}
+
+// All tensors on 32 bytes.  kResidual: the input is T(x + residual).  U chunks of 16 elements per thread are loaded before
+// the first is computed.
 template <typename T, int G, int BIT, bool kResidual, int U>
 __global__ void __launch_bounds__(kThreads) roundtrip_kernel(const LbcRoundtrip p) {
     constexpr int lanes = G / kElemsPerThread;
     constexpr int tile_chunks = kThreads * U;
     const T* x = static_cast<const T*>(p.x);
     const T* res = static_cast<const T*>(p.residual);
-    T* out = static_cast<T*>(p.out);
-    T* rout = static_cast<T*>(p.residual_out);
     const int64_t n = p.numel;
     const int64_t chunks = (n + G - 1) / G * lanes;
-    const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) |
-                       reinterpret_cast<uintptr_t>(res) | reinterpret_cast<uintptr_t>(rout)) & 31) == 0;
-
-    auto finish = [&](float (&v)[16], int64_t first, bool live) {     // convergent: the group maximum shuffles
-        const bool own_error = kResidual && p.own_error != 0;
-        float y[16];
-        roundtrip16<T, G, BIT>(v, y, own_error);
-        if (p.passes == 2) {
-            float z[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) z[i] = y[i];
-            round16<T>(z);
-            roundtrip16<T, G, BIT>(z, y, false);
-        }
-        if (!live) return;
-        if (kResidual && rout != nullptr) {
-            if (!own_error) {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) v[i] -= y[i];
-            }
-            store16_any<T>(rout, first, n, vec, v);
-        }
-        store16_any<T>(out, first, n, vec, y);
-    };
 
     for (int64_t c0 = int64_t(blockIdx.x) * tile_chunks; c0 < chunks; c0 += int64_t(gridDim.x) * tile_chunks) {
         const int64_t mine = (c0 + threadIdx.x) * kElemsPerThread;
-        if (vec && (c0 + tile_chunks) * kElemsPerThread <= n) {       // a whole tile
+        if ((c0 + tile_chunks) * kElemsPerThread <= n) {              // a whole tile
             Raw16<T> rx[U], rr[kResidual ? U : 1];
 #pragma unroll
             for (int j = 0; j < U; ++j) {
@@ -95,23 +110,23 @@ __global__ void __launch_bounds__(kThreads) roundtrip_kernel(const LbcRoundtrip 
                     up16<T>(rr[j], r);
                     compensate16<T>(v, r);
                 }
-                finish(v, mine + j * (kThreads * kElemsPerThread), true);
+                roundtrip_chunk<T, G, BIT, kResidual, kFitWhole>(p, v, mine + j * (kThreads * kElemsPerThread), true);
             }
         } else {
-            for (int j = 0; j < U; ++j) {
-                const int64_t first = mine + j * (kThreads * kElemsPerThread);
-                const bool live = first / kElemsPerThread < chunks;
-                float v[16];
-                load16_any<T>(x, first, n, vec, v);                // zeros past the end
-                if (kResidual) {
-                    float r[16];
-                    load16_any<T>(res, first, n, vec, r);
-                    compensate16<T>(v, r);
-                }
-                finish(v, first, live);
-            }
+            for (int j = 0; j < U; ++j)
+                roundtrip_edge<T, G, BIT, kResidual, kFitTail>(p, c0 + threadIdx.x + j * kThreads, chunks);
         }
     }
+}
+
+// A tensor on another boundary (a view into a larger one), in a kernel of its own: as a branch of roundtrip_kernel this ran
+// out of line, element by element, on all four tensors.  16 Mi elements with error feedback through the public call, the
+// input one element in (phases / that branch / here): bf16 176.7 / 182.0 / 42.6 us, fp32 156.4 / 190.9 / 95.0.
+template <typename T, int G, int BIT, bool kResidual>
+__global__ void __launch_bounds__(kThreads) roundtrip_ragged_kernel(const LbcRoundtrip p) {
+    const int64_t chunks = (p.numel + G - 1) / G * (G / kElemsPerThread);
+    for (int64_t c0 = int64_t(blockIdx.x) * kThreads; c0 < chunks; c0 += int64_t(gridDim.x) * kThreads)
+        roundtrip_edge<T, G, BIT, kResidual, kFitRagged>(p, c0 + threadIdx.x, chunks);
 }
 
 template <typename T, int G, int BIT>
@@ -123,6 +138,13 @@ struct RoundtripLauncher {
             const int64_t cap = p->max_blocks > 0 ? p->max_blocks : int64_t(1) << 30;
             return unsigned(blocks < cap ? blocks : cap);
         };
+        if (!on_boundary(32, p->x, p->residual, p->out, p->residual_out)) {
+            if (p->residual != nullptr)
+                roundtrip_ragged_kernel<T, G, BIT, true><<<grid(one), kThreads, 0, stream>>>(*p);
+            else
+                roundtrip_ragged_kernel<T, G, BIT, false><<<grid(one), kThreads, 0, stream>>>(*p);
+            return cudaGetLastError();
+        }
         if (p->residual != nullptr) {
             roundtrip_kernel<T, G, BIT, true, 1><<<grid(one), kThreads, 0, stream>>>(*p);
             return cudaGetLastError();

@@ -13,6 +13,8 @@ import torch
 
 from lowbit_comm_b200.config import CompressionConfig
 from lowbit_comm_b200.ops import codec, oracle
+from lowbit_comm_b200.parallel.fused import FusedWorkspace
+from lowbit_comm_b200.parallel.peer_memory import PeerGroup
 
 pytestmark = pytest.mark.gpu
 
@@ -385,3 +387,68 @@ def test_codec_takes_views_with_one_stride(ext, kw):
         assert torch.equal(codec.quantize_tensor(x, cfg).cpu(), want)
         assert torch.equal(codec.quantize_tensor(x, cfg, residual=torch.zeros(x.shape, dtype=x.dtype, device="cuda")).cpu(),
                            want)
+
+
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("bit,group,compact", [(8, 64, False), (8, 16, True), (4, 32, False)])
+@pytest.mark.parametrize("which", ("input", "residual", "prepared", "payload", "output", "all"))
+def test_each_tensor_on_its_own_boundary(ext, dtype, bit, group, compact, which):
+    """Encode, decode, reduction and the one-rank pass where one tensor starts 1 element, 4, 8 or 16 bytes past a
+    32-byte boundary and the others on it: same results, and nothing written beside the outputs."""
+
+    cfg = _cfg(bit=bit, group_size=group, compact=compact)
+    T = DTYPES[dtype]
+    width, edge = T.itemsize, 32 // T.itemsize
+    sizes = (2 * 4096 + group + 5, 4096, 15)
+    ranks = PeerGroup.loopback(1, FusedWorkspace.required_bytes(1, dtype, cfg, sizes[0], True) + (1 << 20))
+    ws = FusedWorkspace(ranks[0], dtype=dtype, config=cfg, max_numel=sizes[0], engine="pipe")
+    for n in sizes:
+        x, r = _data(n, T, seed=n), _data(n, T, seed=n + 1, outliers=False)
+        payload = oracle.encode(x, cfg, residual=r)
+        prepared = oracle.prepare(x, r)
+        y, y32 = oracle.reduce_mean([payload, payload, payload], n, cfg, dtype)
+        once, once32 = oracle.reduce_mean([payload], n, cfg, dtype)
+        left = oracle.residual_update(prepared, y32)
+        for off in sorted({1, 4 // width, 8 // width, 16 // width}):
+            held = []
+
+            def place(values, name):
+                at = edge + (off if which in (name, "all") else 0)
+                raw = torch.full((n + 3 * edge,), 7.0, dtype=T, device="cuda")
+                view = raw[at:at + n]
+                if values is not None:
+                    view.copy_(values)
+                held.append((raw, at))
+                return view
+
+            def wire(values):
+                at = 32 + (max(off * width, width) if which in ("payload", "all") else 0)
+                raw = torch.full((payload.numel() + 96,), 0xA5, dtype=torch.uint8, device="cuda")
+                if values is not None:
+                    raw[at:at + payload.numel()] = values.cuda()
+                return raw, raw[at:at + payload.numel()], at
+
+            raw, to, at = wire(None)
+            keep = place(None, "prepared")
+            codec.quantize_tensor(place(x, "input"), cfg, output=to, residual=place(r, "residual"), prepared_out=keep)
+            assert torch.equal(to.cpu(), payload) and torch.equal(keep.cpu(), prepared), (n, off)
+            assert (raw[:at] == 0xA5).all() and (raw[at + payload.numel():] == 0xA5).all()
+            out, res = place(None, "output"), place(None, "residual")
+            codec.inplace_dequantize_reduce_mean_update_error_feedback(
+                [wire(payload)[1], payload.cuda(), wire(payload)[1]], place(prepared, "prepared"), out, res, cfg,
+                reduce="mean")
+            assert torch.equal(out.cpu(), y) and torch.equal(res.cpu(), left), (n, off)
+            out = place(None, "output")
+            codec.dequantize_tensor(wire(payload)[1], (n,), cfg, dtype=dtype, output=out)
+            assert torch.equal(out.cpu(), once), (n, off)
+            if which != "payload":
+                out, res = place(None, "output"), place(r, "residual")
+                ws.all_reduce(place(x, "input"), out, residual=res)
+                assert torch.equal(out.cpu(), once), (n, off)
+                assert torch.equal(res.cpu(), oracle.residual_update(prepared, once32)), (n, off)
+                same = place(x, "input")
+                ws.all_reduce(same)
+                assert torch.equal(same.cpu(), oracle.decode(oracle.encode(x, cfg), n, cfg, dtype)), (n, off)
+            for raw, at in held:
+                assert (raw[:at] == 7.0).all() and (raw[at + n:] == 7.0).all(), (n, off)
+    PeerGroup.close_loopback(ranks)
