@@ -84,8 +84,10 @@ template <int G, int BIT, typename T>
 constexpr int encode_span(bool compact) { return compact ? span_bytes(G, G * BIT / 8 + int(sizeof(T))) : 16; }
 
 // All tensors on 32 bytes (the payload may start anywhere).
+// Blocks per SM: fp32 values alone take half of the 64 registers that four blocks leave; without a residual and records
+// to turn, three blocks are as fast or faster (4 Mi elements into a payload on 8 bytes 8.3 -> 6.3 us).
 template <typename T, int G, int BIT, bool kCompact, bool kResidual, int U>
-__global__ void __launch_bounds__(kThreads, 4) encode_kernel(const __grid_constant__ LbcQuantPush p) {
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 && !kCompact && !kResidual ? 3 : 4) encode_kernel(const __grid_constant__ LbcQuantPush p) {
     constexpr int lanes = G / kElemsPerThread;
     constexpr int tile_chunks = kThreads * U;
     const T* x = static_cast<const T*>(p.x);
@@ -153,9 +155,17 @@ struct EncodeLauncher {
                 encode_kernel<T, G, BIT, kCompact, true, 1><<<grid(one), kThreads, 0, stream>>>(*p);
                 return;
             }
-            if constexpr (sizeof(T) == 2) {
-                if (one > lbc_default_max_blocks()) {
+            // Above one default grid.  Two chunks per thread, but for fp32 records, which gain nothing from them: those
+            // loop over the default grid.  fp32, planar payload on 16 bytes / on 8, one chunk against two: 16 Mi elements
+            // 18.5 / 18.7 -> 16.5 / 18.0 us, 32 Mi 33.3 / 34.9 -> 29.1 / 30.8; records, full against looping grid: 16 Mi
+            // 18.5 -> 18.3 us, 20 M 20.8 -> 20.6, 32 Mi 34.0 -> 30.9 (all with inputs beyond L2).
+            if (one > lbc_default_max_blocks()) {
+                if constexpr (sizeof(T) == 2 || !kCompact) {
                     encode_kernel<T, G, BIT, kCompact, false, 2><<<grid((one + 1) / 2), kThreads, 0, stream>>>(*p);
+                    return;
+                }
+                if (p->max_blocks <= 0) {
+                    encode_kernel<T, G, BIT, kCompact, false, 1><<<lbc_default_max_blocks(), kThreads, 0, stream>>>(*p);
                     return;
                 }
             }
