@@ -8,6 +8,7 @@ allocation.
 
 import itertools
 
+import numpy as np
 import pytest
 import torch
 
@@ -452,3 +453,172 @@ def test_each_tensor_on_its_own_boundary(ext, dtype, bit, group, compact, which)
             for raw, at in held:
                 assert (raw[:at] == 7.0).all() and (raw[at + n:] == 7.0).all(), (n, off)
     PeerGroup.close_loopback(ranks)
+
+
+def _repeated(base, n):
+    """`base` over and over, n elements: a tensor of any size whose payload is the oracle's payload of `base`, repeated."""
+
+    return base.repeat(-(-n // base.numel()))[:n]
+
+
+def _repeated_payload(base, n, cfg, dtype):
+    """The oracle's payload of `_repeated(base, n)`; `base` is whole groups."""
+
+    groups, tail = n // cfg.group_size, n % cfg.group_size
+    values, metas = oracle._split(oracle.encode(base, cfg), base.numel(), cfg, dtype)
+    times = -(-groups // values.shape[0])
+    values, metas = values.repeat(times, 1)[:groups], metas.repeat(times, 1)[:groups]
+    if tail:
+        at = groups * cfg.group_size % base.numel()
+        last = oracle._split(oracle.encode(base[at:at + tail], cfg), tail, cfg, dtype)
+        values, metas = torch.cat([values, last[0]]), torch.cat([metas, last[1]])
+    if cfg.compact:
+        return torch.cat([values, metas], dim=1).reshape(-1)
+    return torch.cat([values.reshape(-1), metas.reshape(-1)])
+
+
+@pytest.mark.parametrize("dtype", ("bf16", "fp32"))
+@pytest.mark.parametrize("bit,quant_type,topk,group,compact", [
+    (8, "linear", 1, 64, True), (8, "linear", 2, 16, False), (4, "linear", 2, 32, True), (4, "e2m1", 0, 64, True),
+    (4, "normal", 1, 32, False)])
+def test_general_kernels_on_a_grid_that_loops(ext, dtype, bit, quant_type, topk, group, compact):
+    """Above four default grids the general kernels loop over one: the warp's staging area is used again and offsets grow.
+    Whole result against the oracle, for the default grid and for three blocks; the last tile is ragged."""
+
+    cfg = _cfg(bit=bit, group_size=group, topk=topk, quant_type=quant_type, compact=compact)
+    code = codec._QUANT_CODE[quant_type]
+    base = _data(group * 997, DTYPES[dtype], seed=11)
+    base_dev = base.cuda()
+    full = 4 * 4096 * int(ext.default_max_blocks())
+    n = full + 5 * 4096 * 37 + group + 3
+    x = _repeated(base_dev, n)
+    want = _repeated_payload(base, n, cfg, dtype).cuda()
+    once = oracle.decode(oracle.encode(base, cfg), base.numel(), cfg, dtype)
+    decoded = _repeated(once.cuda(), n)
+    # the last group is ragged: its scale is that of the elements it has
+    tail = n % group
+    at = (n - tail) % base.numel()
+    ends = oracle.decode(oracle.encode(base[at:at + tail], cfg), tail, cfg, dtype)
+    decoded[n - tail:] = ends.cuda()
+    assert torch.equal(codec.quantize_tensor(x, cfg), want)
+    back = codec.dequantize_tensor(want, (n,), cfg, dtype=dtype)
+    assert torch.equal(back.view(torch.uint8), decoded.view(torch.uint8))
+    total = codec.dequantize_tensor(want, (n,), cfg, dtype=dtype, output=back, reduce_op="sum")
+    assert torch.equal(total, (decoded.float() * 2).to(decoded.dtype))
+    small = 3 * 4096 * 5 + group + 3
+    for numel, blocks in ((n, 0), (small, 3)):
+        expect = decoded[:numel].clone()
+        ragged = numel % group
+        at = (numel - ragged) % base.numel()
+        expect[numel - ragged:] = oracle.decode(oracle.encode(base[at:at + ragged], cfg), ragged, cfg, dtype).cuda()
+        out = torch.empty_like(x[:numel])
+        assert ext.roundtrip_general(x[:numel].clone(), None, out, None, group, bit, topk, code, False, 0, 1, blocks)
+        assert torch.equal(out.view(torch.uint8), expect.view(torch.uint8))
+        payload = codec.quantize_tensor(x[:numel], cfg)
+        ext.reduce_general([payload.data_ptr()] * 2, out, group, bit, topk, code, compact, 0.5, None, None, None, blocks)
+        half = ((expect.float() * 2).to(out.dtype).float() * 0.5).to(out.dtype)
+        assert torch.equal(out, half)
+
+
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("bit,quant_type,topk,group", [(8, "linear", 0, 64), (8, "linear", 1, 32), (4, "linear", 2, 16),
+                                                       (4, "normal", 0, 64), (4, "e3m0", 1, 32)])
+def test_stochastic_one_rank_pass_matches_the_codec(ext, dtype, bit, quant_type, topk, group):
+    """The same seed gives the same numbers in registers and through a payload; another seed gives others; and the codes
+    are the oracle's for the counter-based numbers of `uniform01`, but for values that a rounding puts on the edge."""
+
+    cfg = _cfg(bit=bit, group_size=group, topk=topk, quant_type=quant_type, stochastic=True)
+    code = codec._QUANT_CODE[quant_type]
+    for n, skew in ((20_000 // group * group, 0), (4096 + 5, 1), (group, 8)):
+        x = torch.empty(n + skew, dtype=DTYPES[dtype], device="cuda").normal_(std=1e-2)[skew:]
+        r = torch.empty(n, dtype=x.dtype, device="cuda").normal_(std=1e-4)
+        results = []
+        for seed in (12345, 2**61 + 7):
+            payload, prepared = codec.allocate_quantized_buffer(x, cfg), torch.empty_like(x)
+            ext.quant_general(x, r, prepared, payload, group, bit, topk, code, True, False, seed)
+            want = codec.dequantize_tensor(payload, (n,), cfg, dtype=dtype)
+            out, rout = torch.empty_like(x), r.clone()
+            assert ext.roundtrip_general(x, rout, out, rout, group, bit, topk, code, True, seed, 1)
+            assert torch.equal(out.view(torch.uint8), want.view(torch.uint8))
+            left = torch.empty_like(x)
+            codec.update_error_feedback_residual(prepared, want, left)
+            assert torch.equal(rout.view(torch.uint8), left.view(torch.uint8))
+            results.append(out)
+            if n % group == 0:
+                noise = torch.from_numpy(_uniform01(seed, n)) - 0.5
+                expect = oracle.encode(x.cpu(), cfg, residual=r.cpu(), noise=noise)
+                codes = [oracle._unpack_words(oracle._split(p, n, cfg, dtype)[0], bit, x.element_size())
+                         for p in (payload, expect)]
+                # one rounding of value * mul + noise in the kernel, two in the oracle: up to 2^-17 apart (an ulp of 127),
+                # so another code for at most one value in 2^16, 0.3 of the 20 000
+                assert int((codes[0] != codes[1]).sum()) <= 6
+        assert n < 1000 or not torch.equal(*results)
+
+
+def _uniform01(seed, n):
+    """The kernels' uniform numbers in (0, 1] by element index."""
+
+    z = np.uint64(seed) + np.uint64(0x9E3779B97F4A7C15) * np.arange(1, n + 1, dtype=np.uint64)
+    z = (z ^ (z >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
+    z = (z ^ (z >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
+    z ^= z >> np.uint64(31)
+    return ((z >> np.uint64(40)).astype(np.float32) + np.float32(1)) * np.float32(2.0**-24)
+
+
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("bit,quant_type,topk,group", [(8, "linear", 1, 64), (4, "linear", 2, 32), (4, "e3m0", 0, 16),
+                                                       (4, "uniform", 1, 64), (8, "linear", 2, 16)])
+def test_general_one_rank_pass_matches_the_oracle(ext, dtype, bit, quant_type, topk, group):
+    """Both pass counts and the residual against the oracle, beside groups with infinities and NaN (which the oracle does
+    not define; the finite groups of the same warp are compared)."""
+
+    cfg = _cfg(bit=bit, group_size=group, topk=topk, quant_type=quant_type)
+    code = codec._QUANT_CODE[quant_type]
+    n = 40 * group + 7
+    x, r = _data(n, DTYPES[dtype], seed=2), _data(n, DTYPES[dtype], seed=3, outliers=False)
+    finite = torch.ones(n, dtype=torch.bool)
+    special = x.clone()
+    special[2 * group:2 * group + 3] = torch.tensor([float("inf"), -float("inf"), float("nan")]).to(x)
+    special[4 * group:5 * group] = float("nan")
+    finite[2 * group:3 * group] = finite[4 * group:5 * group] = False
+    for passes in (1, 2):
+        y = prepared = oracle.prepare(x, r)
+        for _ in range(passes):
+            y = oracle.decode(oracle.encode(y, cfg), n, cfg, dtype)
+        left = oracle.residual_update_from_restored(prepared, y)
+        for source, mask in ((x, torch.ones_like(finite)), (special, finite)):
+            out, rout = torch.empty_like(x).cuda(), r.cuda()
+            assert ext.roundtrip_general(source.cuda(), rout, out, rout, group, bit, topk, code, False, 0, passes)
+            assert torch.equal(out.cpu()[mask].view(torch.uint8), y[mask].view(torch.uint8)), passes
+            assert torch.equal(rout.cpu()[mask].view(torch.uint8), left[mask].view(torch.uint8)), passes
+
+
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("bit,group,compact", [(8, 64, False), (8, 32, True), (4, 16, True)])
+@pytest.mark.parametrize("skew", (0, 1))
+def test_codec_kernels_on_a_capped_grid(ext, dtype, bit, group, compact, skew):
+    """`max_blocks` below the tiles: every block goes round several times, aligned and unaligned, whole and ragged ends."""
+
+    cfg = _cfg(bit=bit, group_size=group, compact=compact)
+    code = codec._DTYPE_CODE[dtype]
+    for n in (7 * 4096 + group + 3, 6 * 4096):
+        base, rbase = _data(n + skew, DTYPES[dtype], seed=n), _data(n + skew, DTYPES[dtype], seed=n + 1, outliers=False)
+        x, r = base.cuda()[skew:], rbase.cuda()[skew:]
+        groups = -(-n // group)
+        want = oracle.encode(base[skew:], cfg, residual=rbase[skew:])
+        plain = oracle.encode(base[skew:], cfg)
+        for residual, expect in ((r, want), (None, plain)):
+            payload = torch.zeros(want.numel(), dtype=torch.uint8, device="cuda")
+            ext.quant_push(x, residual, None, None, [payload.data_ptr()],
+                           ext.PUSH_COMPACT_LOCAL if compact else ext.PUSH_BROADCAST, 0, groups, 0, group, bit, None, 2)
+            assert torch.equal(payload.cpu(), expect)
+        for count in (1, 5):
+            dev = [want.cuda() if k % 2 else plain.cuda() for k in range(count)]
+            y, y32 = oracle.reduce_mean([d.cpu() for d in dev], n, cfg, dtype)
+            out, res = torch.empty_like(rbase).cuda()[skew:], torch.empty_like(rbase).cuda()[skew:]
+            ext.reduce([d.data_ptr() for d in dev], groups, 0, compact, n, code, group, bit, 1.0 / count, out, False, x, res,
+                       [], 0, 0, None, None, 2)
+            assert torch.equal(out.cpu(), y) and torch.equal(res.cpu(), oracle.residual_update(base[skew:], y32))
+        ext.reduce([payload.data_ptr()], groups, 0, compact, n, code, group, bit, 1.0, out, False, None, None, [], 0, 0, None,
+                   None, 2)
+        assert torch.equal(out.cpu(), oracle.decode(plain, n, cfg, dtype))
