@@ -66,6 +66,13 @@ void fill_ptrs(uint8_t** dst, int* count, const Ptrs& ptrs, const char* name) {
     }
 }
 
+// The kernels access a payload in words as wide as the source elements; a view into a byte tensor may start anywhere.
+void check_words(const void* payload, int dtype, const char* name) {
+    const uintptr_t width = dtype == LBC_FP32 ? 4 : 2;
+    TORCH_CHECK((reinterpret_cast<uintptr_t>(payload) & (width - 1)) == 0, name, " must start on a multiple of ", width,
+                " bytes");
+}
+
 LbcSignal make_signal(const SignalArg& arg) {
     LbcSignal s{};
     if (!arg.has_value()) return s;
@@ -114,6 +121,7 @@ void quant_push(const at::Tensor& x, const std::optional<at::Tensor>& residual,
     p.numel = x.numel();
     p.mode = mode;
     fill_ptrs(p.dst, &p.num_dst, dst, "dst");
+    for (int d = 0; d < p.num_dst; ++d) check_words(p.dst[d], p.dtype, "payload");
     const int64_t groups = ceil_div(p.numel, group_size);
     if (mode == LBC_PUSH_SCATTER) {
         TORCH_CHECK(shard_groups > 0, "scatter needs shard_groups > 0");
@@ -150,6 +158,7 @@ void reduce(const Ptrs& src, int64_t layout_groups, int64_t group_offset, bool c
     for (size_t i = 0; i < src.size(); ++i) {
         TORCH_CHECK(src[i] != 0, "src: null address");
         p.src[i] = reinterpret_cast<const uint8_t*>(src[i]);
+        check_words(p.src[i], dtype, "payload");
     }
     const int64_t groups = ceil_div(numel, group_size);
     if (src_shard_groups > 0) {
@@ -216,6 +225,7 @@ void quant_general(const at::Tensor& x, const std::optional<at::Tensor>& residua
     const int64_t need = ceil_div(p.numel, group_size) * (group_size * bit / 8 + meta_words * x.element_size());
     TORCH_CHECK(out.numel() == need, "output has an invalid quantized payload size: ", out.numel(), " != ", need);
     p.out = out.data_ptr<uint8_t>();
+    check_words(p.out, p.dtype, "payload");
     p.seed = seed;
     cuda_check(lbc_quant_general(&p, at::cuda::getCurrentCUDAStream()), "lbc_quant_general");
 }
@@ -238,6 +248,7 @@ void dequant_general(const at::Tensor& src, at::Tensor& out, int group_size, int
     const int64_t need = ceil_div(p.numel, group_size) * (group_size * bit / 8 + meta_words * out.element_size());
     TORCH_CHECK(src.numel() == need, "payload has an invalid size: ", src.numel(), " != ", need);
     p.src = src.data_ptr<uint8_t>();
+    check_words(p.src, p.dtype, "payload");
     p.out = out.data_ptr();
     p.accumulate = accumulate ? 1 : 0;
     cuda_check(lbc_dequant_general(&p, at::cuda::getCurrentCUDAStream()), "lbc_dequant_general");
@@ -265,6 +276,7 @@ void quant_general_push(const at::Tensor& x, const std::optional<at::Tensor>& re
     p.numel = x.numel();
     p.seed = seed;
     fill_ptrs(p.dst, &p.num_dst, dst, "dst");
+    for (int d = 0; d < p.num_dst; ++d) check_words(p.dst[d], p.dtype, "payload");
     p.signal = make_signal(signal);
     p.max_blocks = max_blocks;
     p.shard_groups = shard_groups;
@@ -323,7 +335,10 @@ void reduce_general(const Ptrs& src, at::Tensor& out, int group_size, int bit, i
     p.compact = compact ? 1 : 0;
     uint8_t* ptrs[LBC_MAX_RANKS];
     fill_ptrs(ptrs, &p.num_src, src, "src");
-    for (int r = 0; r < p.num_src; ++r) p.src[r] = ptrs[r];
+    for (int r = 0; r < p.num_src; ++r) {
+        p.src[r] = ptrs[r];
+        check_words(p.src[r], p.dtype, "payload");
+    }
     p.numel = out.numel();
     p.out = out.data_ptr();
     p.scale = static_cast<float>(scale);

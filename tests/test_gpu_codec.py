@@ -622,3 +622,27 @@ def test_codec_kernels_on_a_capped_grid(ext, dtype, bit, group, compact, skew):
         ext.reduce([payload.data_ptr()], groups, 0, compact, n, code, group, bit, 1.0, out, False, None, None, [], 0, 0, None,
                    None, 2)
         assert torch.equal(out.cpu(), oracle.decode(plain, n, cfg, dtype))
+
+
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("kw", [{}, {"compact": True}, {"topk": 1}, {"bit": 4, "quant_type": "e2m1", "compact": True}])
+def test_payloads_off_their_words_are_refused(ext, dtype, kw):
+    """A payload view that starts between two words of the source's width: an error before any launch."""
+
+    cfg = _cfg(**kw)
+    x = _data(640, DTYPES[dtype]).cuda()
+    need = codec.allocate_quantized_buffer(x, cfg).numel()
+    raw = torch.zeros(need + 8, dtype=torch.uint8, device="cuda")
+    for off in (1, 3) if dtype != "fp32" else (1, 2, 3):
+        view, out, res = raw[off:off + need], torch.zeros_like(x), torch.zeros_like(x)
+        with pytest.raises(RuntimeError, match="multiple of"):
+            codec.quantize_tensor(x, cfg, output=view)
+        with pytest.raises(RuntimeError, match="multiple of"):
+            codec.dequantize_tensor(view, x.shape, cfg, dtype=dtype, output=out)
+        with pytest.raises(RuntimeError, match="multiple of"):
+            codec.dequantize_reduce_update_error_feedback([view], x, res, x.shape, cfg, dtype=dtype)
+        torch.cuda.synchronize()
+        assert not out.any() and not res.any() and not raw.any()
+    view = raw[4:4 + need]
+    codec.quantize_tensor(x, cfg, output=view)
+    assert torch.equal(view.cpu(), oracle.encode(x.cpu(), cfg))
