@@ -119,7 +119,6 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 && !kCompact && !kRes
             encode_chunk<T, G, BIT, kCompact, kFitWhole>(p, v, mine + j * kThreads, span);
         }
     }
-    grid_signal(p.signal);
 }
 
 // A tensor on another boundary (a view into a larger one), in a kernel of its own: as a branch of encode_kernel this ran
@@ -132,15 +131,14 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 4) encode_ragge
     __shared__ __align__(16) uint8_t spans[kThreads / 32][encode_span<G, BIT, T>(kCompact)];
     for (int64_t c0 = int64_t(blockIdx.x) * kThreads; c0 < chunks; c0 += int64_t(gridDim.x) * kThreads)
         encode_edge<T, G, BIT, kCompact, kFitRagged>(p, c0, 1, spans[threadIdx.x >> 5]);
-    grid_signal(p.signal);
 }
 
 template <typename T, int G, int BIT>
 struct EncodeLauncher {
     static cudaError_t run(const LbcQuantPush* p, cudaStream_t stream) {
         const int64_t chunks = (p->numel + G - 1) / G * (G / kElemsPerThread);
-        if (chunks == 0 && p->signal.num_remote == 0) return cudaSuccess;
-        const int64_t one = chunks > 0 ? (chunks + kThreads - 1) / kThreads : 1;
+        if (chunks == 0) return cudaSuccess;
+        const int64_t one = (chunks + kThreads - 1) / kThreads;
         auto grid = [&](int64_t blocks) {
             const int64_t cap = p->max_blocks > 0 ? p->max_blocks : int64_t(1) << 30;
             return unsigned(blocks < cap ? blocks : cap);

@@ -367,7 +367,6 @@ __global__ void __launch_bounds__(kThreads, 4) reduce_kernel(const LbcReduce p) 
     const bool p_vec = prep == nullptr || (reinterpret_cast<uintptr_t>(prep) & 31) == 0;
     const bool r_vec = rout == nullptr || (reinterpret_cast<uintptr_t>(rout) & 31) == 0;
     const int R = p.num_src;
-    const int64_t rec = p.compact ? (VB + MB) : VB;
     __shared__ __align__(16) ScaleStage stage;
     const bool vec_scales = p.num_dst > 0 && (p.dst_layout_groups & 7) == 0 && (p.dst_group_offset & 7) == 0 &&
                             dsts_aligned16(p.dst, p.num_dst);
@@ -417,8 +416,8 @@ __global__ void __launch_bounds__(kThreads, 4) reduce_kernel(const LbcReduce p) 
 #pragma unroll
         for (int i = 0; i < 16; ++i) acc[i] = 0.0f;
         if (live) {
-            int64_t voff = gs * rec + lane * CB;
-            int64_t soff = p.compact ? gs * rec + VB : p.layout_groups * VB + gs * MB;
+            int64_t voff = gs * VB + lane * CB;
+            int64_t soff = p.layout_groups * VB + gs * MB;
             int first_src = 0, last_src = R;
             if (p.src_shard_groups > 0) {
                 // gather mode: the group lives in exactly one source, the owner's reduced shard,
@@ -767,6 +766,7 @@ struct ReduceLauncher {
         if (p->num_dst == 0 && p->signal.num_remote == 0 && p->wait.flags == nullptr && p->src_shard_groups == 0 &&
             p->group_offset == 0 && p->out != nullptr)
             return lbc_decode(p, stream);
+        if (p->compact) return cudaErrorInvalidValue;      // only the codec reads compact payloads
         int cap = p->max_blocks;
         if (p->num_dst > 1 && g_reduce_push_blocks >= 0) {   // several destinations: peers are among them
             const int push_cap = g_reduce_push_blocks > 0 ? g_reduce_push_blocks : default_max_blocks() / 4;
@@ -776,7 +776,7 @@ struct ReduceLauncher {
         LbcReduce launch = *p;
         if constexpr (BIT == 8) {
             const bool plain_gather = p->src_shard_groups > 0 && p->num_dst == 0 && p->group_offset == 0 &&
-                                      p->accumulate == 0 && p->compact == 0;
+                                      p->accumulate == 0;
             if (plain_gather && g_gather_prefetch >= 2) {
                 if (g_gather_prefetch >= 4)
                     gather_decode_kernel<T, G, BIT, 4><<<grid, kThreads, 0, stream>>>(launch);
@@ -816,6 +816,7 @@ cudaError_t lbc_quant_push(const LbcQuantPush* p, cudaStream_t stream) {
     if (p->mode == LBC_PUSH_SCATTER && p->shard_groups <= 0) return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(p->mc_dst) & 15) != 0) return cudaErrorInvalidValue;
     if (p->mc_dst != nullptr && p->mode != LBC_PUSH_BROADCAST) return cudaErrorInvalidValue;
+    if (p->mode == LBC_PUSH_COMPACT_LOCAL && p->signal.num_remote > 0) return cudaErrorInvalidValue;   // a local payload
     return lbc::dispatch_profile<lbc::QuantPushLauncher>(p, stream);
 }
 
