@@ -9,6 +9,8 @@ built for sm_100 under baseline/_ref, loaded into the same process) on the same
 tensors: `inplace_quantize_pack`, `inplace_dequantize_reduce_mean` and
 `inplace_dequantize_reduce_mean_update_error_feedback`
 (ccdl_comm/quantization/codec.py:161-217, 355-466).
+The codec's rows run the kernels of `csrc/codec_kernels.cu` (one local payload); the kernels that push to and reduce
+from peers run in the all-reduce on emulated ranks.
 `--topk K` also times the general-profile all-reduce (K outliers per group kept verbatim) on the emulated ranks,
 in its one-stage and its two-stage form.
 """
@@ -88,21 +90,21 @@ def main() -> None:
         pb = out.numel()
         if not args.skip_codec:
             t = time_cuda(lambda: codec.quantize_tensor(x, cfg, output=out), iters=args.iters, flush=flush, warmup=warm)
-            record("quant_push(local)", mib, 2 * n + pb, t)
+            record("quantize_tensor", mib, 2 * n + pb, t)
             t = time_cuda(lambda: codec.quantize_tensor(x, cfg, output=out, residual=res, prepared_out=res),
                           iters=args.iters, flush=flush, warmup=warm)
-            record("quant_push(local,+EF in place)", mib, 6 * n + pb, t)
+            record("quantize_tensor(+EF in place)", mib, 6 * n + pb, t)
             y = torch.empty_like(x)
             t = time_cuda(lambda: codec.dequantize_tensor(out, x.shape, cfg, dtype="bf16", output=y),
                           iters=args.iters, flush=flush, warmup=warm)
-            record("reduce(1 payload)", mib, 2 * n + pb, t)
+            record("dequantize_tensor", mib, 2 * n + pb, t)
             t = time_cuda(lambda: codec.inplace_dequantize_reduce_mean_update_error_feedback(
                 [out], res, y, res, cfg, reduce="mean"), iters=args.iters, flush=flush, warmup=warm)
-            record("reduce(1 payload,+EF in place)", mib, 6 * n + pb, t)
+            record("mean of 1 payload(+EF in place)", mib, 6 * n + pb, t)
             bufs = [out] + [out.clone() for _ in range(7)]
             t = time_cuda(lambda: codec.inplace_dequantize_reduce_mean(bufs, y, cfg, reduce="mean"),
                           iters=args.iters, flush=flush, warmup=warm)
-            record("reduce(8 payloads)", mib, 2 * n + 8 * pb, t)
+            record("mean of 8 payloads", mib, 2 * n + 8 * pb, t)
             z = torch.empty_like(x)
             t = time_cuda(lambda: z.copy_(x), iters=args.iters, flush=flush, warmup=warm)
             record("torch copy_ (reference point)", mib, 4 * n, t)
@@ -127,7 +129,7 @@ def main() -> None:
                     record("reference inplace_quantize_pack(compact,+residual)", mib, 4 * n + pb, t, fused=bool(ok))
                     t = time_cuda(lambda: codec.quantize_tensor(x, ccompact, output=out, residual=res),
                                   iters=args.iters, flush=flush, warmup=warm)
-                    record("quant_push(local,compact,+residual)", mib, 4 * n + pb, t)
+                    record("quantize_tensor(compact,+residual)", mib, 4 * n + pb, t)
                     rbufs = [rout] + [rout.clone() for _ in range(7)]
                     t = time_cuda(lambda: rc.inplace_dequantize_reduce_mean(rbufs[:1], y, rcfg, extension_status=rstatus,
                                                                             reduce="mean"),

@@ -5,12 +5,15 @@
 // Math is identical, bit for bit, to quant_push_kernel / reduce_kernel there.
 // Reference: quantization/quant_pack_kernel.cu:84-163, quantization/dequant_reduce_kernel.cu:38-69, 150-221.
 //
-// What bounds these kernels: memory.  A block per tile instead of a grid-stride loop (a persistent grid moved 10-15 %
-// less), 32 bytes of input per thread in one load, payloads read and written as 16-byte vectors in both layouts, the
-// whole-tile path free of bounds and alignment tests (their registers cost occupancy).
-// Measured on a B200, int8 groups of 64, before (grid-stride kernels of fast_kernels.cu) and after: encode of 32 Mi bf16
-// elements with error feedback 47.0 -> 39.5 us (6.0 TB/s), decode of 128 Mi 94 -> 66 us (6.2 TB/s), mean of eight
-// payloads of 32 Mi with error feedback 107 -> 82 us (5.8 TB/s).
+// What bounds these kernels: memory.  A block per tile (a persistent grid moved 10-15 % less; the loops over tiles serve
+// grids that a caller caps, and fp32 records), 32 bytes of input per thread in one load, payloads read and written as
+// 16-byte vectors in both layouts, the whole-tile path free of bounds and alignment tests (their registers cost
+// occupancy); tensors and payloads off those boundaries have kernels of their own.
+// Measured on a B200 through the public calls, int8 groups of 64, before (grid-stride kernels of fast_kernels.cu) and
+// after: encode of 32 Mi bf16 elements with error feedback 47.0 -> 39.3 us (6.0 TB/s), decode of 128 Mi 94 -> 67.6 us
+// (6.0 TB/s), mean of eight payloads of 32 Mi with error feedback 107 -> 89.6 us (5.3 TB/s).  Those are passes repeated for
+// a second; in bursts of a few milliseconds the same calls take 38.9, 65.7 and 81 us: the mean of eight draws the card's
+// 1000 W, and its clock falls to 1.7 GHz.
 #include <type_traits>
 
 #include "codec_device.cuh"
@@ -154,7 +157,9 @@ struct EncodeLauncher {
                 return;
             }
             // Above one default grid.  Two chunks per thread, but for fp32 records, which gain nothing from them: those
-            // loop over the default grid.  fp32, planar payload on 16 bytes / on 8, one chunk against two: 16 Mi elements
+            // loop over the default grid.  bf16, one chunk against two, planar: 4 M elements (0.8 grids) 6.6 / 7.1 us, 6 M
+            // 8.2 / 8.2, 8 M 10.3 / 8.3, 16 M 14.4 / 12.4, 64 M 47.2 / 36.9; records: 4 M 8.1 / 8.3, 6 M 9.0 / 9.9,
+            // 10 M 12.3 / 12.3, 16 M 16.4 / 14.5, 64 M 53.4 / 45.0.  fp32, planar payload on 16 bytes / on 8, one chunk against two: 16 Mi elements
             // 18.5 / 18.7 -> 16.5 / 18.0 us, 32 Mi 33.3 / 34.9 -> 29.1 / 30.8; records, full against looping grid: 16 Mi
             // 18.5 -> 18.3 us, 20 M 20.8 -> 20.6, 32 Mi 34.0 -> 30.9 (all with inputs beyond L2).
             if (one > lbc_default_max_blocks()) {

@@ -149,9 +149,10 @@ struct RoundtripLauncher {
             roundtrip_kernel<T, G, BIT, true, 1><<<grid(one), kThreads, 0, stream>>>(*p);
             return cudaGetLastError();
         }
-        // Two chunks per thread (64 bytes in flight) once there are many waves of blocks: 512 Mi bf16 elements take 310 us
-        // against 322-342 with one chunk, 13 M take 12.5 us either way, and fewer leave SMs without a block.  fp32 chunks and
-        // chunks with a residual have 64 bytes in flight already.
+        // Two chunks per thread (64 bytes in flight) once there are many waves of blocks.  One chunk against two, bf16: 2 M
+        // elements 5.2 / 6.2 us (two leave SMs without a block), 4 M 6.2 / 7.0, 8 M (1.6 default grids) 9.4 / 9.2, 13 M
+        // 12.3 / 12.3, 16 M 14.4 / 13.9, 24 M 18.5 / 18.5, 32 M (6.6) 23.8 / 22.5, 40 M (8.2) 28.6 / 27.5, 64 M 43.1 / 41.6,
+        // 256 M 158 / 152.  fp32 chunks and chunks with a residual have 64 bytes in flight already.
         if constexpr (sizeof(T) == 2) {
             if (one > 8 * lbc_default_max_blocks()) {
                 roundtrip_kernel<T, G, BIT, false, 2><<<grid((one + 1) / 2), kThreads, 0, stream>>>(*p);
