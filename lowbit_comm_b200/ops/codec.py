@@ -79,13 +79,23 @@ def allocate_dequantized_buffer(tensor: torch.Tensor, shape, config: Compression
 # quantize
 # ---------------------------------------------------------------------------
 def _check_payload(buffer: torch.Tensor, numel: int, dtype: str, config: CompressionConfig) -> None:
-    need = estimate_quantized_size(numel, dtype=dtype, config=config).quantized_bytes
+    _check_bytes(buffer, estimate_quantized_size(numel, dtype=dtype, config=config).quantized_bytes)
+
+
+def _check_bytes(buffer: torch.Tensor, need: int) -> None:
     if buffer.dtype != torch.uint8:
         raise TypeError("payload must be a uint8 tensor")
     if buffer.numel() != need:
         raise ValueError(f"payload has {buffer.numel()} bytes, expected {need}")
     if not buffer.is_contiguous():
         raise ValueError("payload must be contiguous")
+
+
+def _check_reachable(buffer: torch.Tensor) -> None:
+    """A payload goes to the kernels by its address: memory of the GPU, or pinned memory of the host."""
+
+    if not buffer.is_pinned():
+        raise ValueError("payload must be on the GPU like the tensor")
 
 
 def _cuda_quantize(ext, flat: torch.Tensor, out: torch.Tensor, residual, prepared_out, config: CompressionConfig) -> None:
@@ -116,7 +126,9 @@ def quantize_tensor(tensor: torch.Tensor, config: CompressionConfig, *,
     if output is None:
         output = torch.empty(est.quantized_bytes, dtype=torch.uint8, device=tensor.device)
     else:
-        _check_payload(output, numel, name, config)
+        _check_bytes(output, est.quantized_bytes)
+        if tensor.is_cuda and not output.is_cuda:
+            _check_reachable(output)
     if metadata is not None:
         metadata.update(original_numel=numel, padded_numel=est.padded_numel, num_groups=est.num_groups,
                         dtype=name, compact=config.compact)
@@ -251,6 +263,9 @@ def _reduce_dense(buffers, flat_out, config, name, divisor, extension_status, pr
         return
     if flat_out.is_cuda:
         ext = require_extension(extension_status)
+        for b in buffers:
+            if not b.is_cuda:
+                _check_reachable(b)
         groups = -(-numel // config.group_size)
         if is_fast_profile(config) and len(buffers) <= MAX_FUSED_PAYLOADS:
             ext.reduce([b.data_ptr() for b in buffers], groups, 0, config.compact, numel, _DTYPE_CODE[name],

@@ -281,6 +281,8 @@ class Communicator:
                     raise
                 ws = None
             if ws is not None:
+                if out is not None or residual is not None:
+                    self._check_alike(tensor, out=out, residual=residual)
                 if not async_op and not tracing.ENABLED:
                     result = ws.all_reduce(tensor, out, residual=residual, update_residual=update_residual, op=op,
                                            stages=stages, ef_mode=ef_mode)
@@ -300,18 +302,32 @@ class Communicator:
                     raise
                 gws = None
             if gws is not None:
+                # a strided residual goes in as a copy, which is written back
+                dense = residual if residual is None or residual.is_contiguous() else residual.contiguous()
+                self._check_alike(tensor, out=out, residual=dense)
                 scope, side = self._stream_scope(tensor, async_op)
                 # a strategy that names the two-stage algorithm gets it (reduce-scatter, requantize, gather); "auto"
                 # and "all_gather" keep the one-stage exchange, and so does stochastic rounding
                 two = stages == 2 and not config.stochastic
                 with scope:
-                    result = gws.all_reduce(tensor, out, residual=residual, update_residual=update_residual, op=op,
+                    result = gws.all_reduce(tensor, out, residual=dense, update_residual=update_residual, op=op,
                                             stages=2 if two else 1)
+                    if dense is not residual and update_residual:
+                        residual.copy_(dense)
                 self.stats["peer_ops"] += 1
-                return self._finish(result, side, resources=(tensor, out, residual))
+                return self._finish(result, side, resources=(tensor, out, residual, dense))
         result = self._torch_all_reduce(tensor, config, op, stages, name, out, residual, update_residual)
         self.stats["torch_ops"] += 1
         return ImmediateWork(result) if async_op else result
+
+    @staticmethod
+    def _check_alike(tensor: Any, **others: Any) -> None:
+        """The kernels take addresses: what goes with `tensor` has its dtype, size and device, and its elements in order."""
+
+        for name, other in others.items():
+            if other is not None and (other.dtype != tensor.dtype or other.numel() != tensor.numel()
+                                      or other.device != tensor.device or not other.is_contiguous()):
+                raise ValueError(f"{name} must be contiguous, with the dtype, the device and the number of elements of the tensor")
 
     def bind_all_reduce(self, *, config: CompressionConfig, op: str = "mean", strategy: str = "auto",
                         dtype: str = "auto"):

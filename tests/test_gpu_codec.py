@@ -646,3 +646,60 @@ def test_payloads_off_their_words_are_refused(ext, dtype, kw):
     view = raw[4:4 + need]
     codec.quantize_tensor(x, cfg, output=view)
     assert torch.equal(view.cpu(), oracle.encode(x.cpu(), cfg))
+
+
+@pytest.mark.parametrize("kw", [{}, {"topk": 1}])
+def test_tensors_that_the_kernels_cannot_address_are_refused(ext, kw):
+    """Payloads in pageable host memory, and outputs or residuals of a collective that are not like its tensor: errors
+    before any launch; pinned payloads stay served where the kernels take an address."""
+
+    import torch.distributed as dist
+
+    from lowbit_comm_b200.parallel.communicator import Communicator
+
+    cfg = _cfg(**kw)
+    x = _data(640, torch.bfloat16).cuda()
+    payload = codec.quantize_tensor(x, cfg)
+    with pytest.raises(ValueError, match="on the GPU"):
+        codec.quantize_tensor(x, cfg, output=torch.empty(payload.numel(), dtype=torch.uint8))
+    out, res = torch.zeros_like(x), torch.zeros_like(x)
+    with pytest.raises(ValueError, match="on the GPU"):
+        codec.inplace_dequantize_reduce_mean([payload.cpu(), payload], out, cfg) or codec.dequantize_reduce_update_error_feedback(
+            [payload, payload.cpu()], x, res, x.shape, cfg, dtype="bf16")
+    if not kw:
+        pinned = torch.empty(payload.numel(), dtype=torch.uint8).pin_memory()
+        codec.quantize_tensor(x, cfg, output=pinned)
+        assert codec.inplace_dequantize_reduce_mean([pinned], out, cfg)
+        torch.cuda.synchronize()
+        assert torch.equal(pinned, payload.cpu())
+        assert torch.equal(out, codec.dequantize_tensor(payload, x.shape, cfg, dtype="bf16"))
+    created = not dist.is_initialized()
+    if created:
+        dist.init_process_group("nccl", store=dist.HashStore(), rank=0, world_size=1, device_id=torch.device("cuda", 0))
+    comm = Communicator(None)
+    try:
+        before = x.clone()
+        for wrong in (torch.zeros(640), torch.zeros(640, device="cuda"), torch.zeros(639, dtype=x.dtype, device="cuda"),
+                      torch.zeros(640, 2, dtype=x.dtype, device="cuda")[:, 0]):
+            if wrong.is_contiguous() or not kw:      # (general profiles: a strided out takes the torch path)
+                with pytest.raises(ValueError, match="out must be"):
+                    comm.all_reduce(x, config=cfg, out=wrong)
+            if wrong.is_contiguous() or not kw:      # (there a strided residual is copied in and out)
+                with pytest.raises(ValueError, match="residual must be"):
+                    comm.all_reduce(x, config=cfg, residual=wrong)
+        assert torch.equal(x, before)
+        if kw:
+            strided, dense = torch.zeros(640, 2, dtype=x.dtype, device="cuda")[:, 0], torch.zeros_like(x)
+            strided.fill_(1e-4)
+            dense.fill_(1e-4)
+            out2 = torch.zeros_like(x)
+            comm.all_reduce(x, config=cfg, out=out, residual=dense)
+            comm.all_reduce(x, config=cfg, out=out2, residual=strided)
+            assert torch.equal(out, out2) and torch.equal(strided, dense) and not torch.equal(dense, torch.full_like(dense, 1e-4))
+        good = torch.zeros(32, 20, dtype=x.dtype, device="cuda")
+        comm.all_reduce(x, config=cfg, out=good, residual=res)
+        assert torch.equal(good.reshape(-1), codec.dequantize_tensor(payload, x.shape, cfg, dtype="bf16"))
+    finally:
+        comm.close()
+        if created:
+            dist.destroy_process_group()
