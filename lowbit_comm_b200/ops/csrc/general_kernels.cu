@@ -399,10 +399,10 @@ __device__ __forceinline__ void encode_general(const float (&v)[16], float store
         float t[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) t[i] = __fmul_rn(v[i], mul);
-        if (rule.stochastic) {
+        if (rule.stochastic) {      // two roundings, the product's and the sum's, as the oracle has it
 #pragma unroll
             for (int i = 0; i < 16; ++i)
-                t[i] = __fmaf_rn(v[i], mul, uniform01(rule.seed, (unsigned long long)(first + i)) - 0.5f);
+                t[i] = __fadd_rn(t[i], uniform01(rule.seed, (unsigned long long)(first + i)) - 0.5f);
         }
         if (tame && !rule.stochastic) {
 #pragma unroll

@@ -524,12 +524,13 @@ def test_general_kernels_on_a_grid_that_loops(ext, dtype, bit, quant_type, topk,
 @pytest.mark.parametrize("bit,quant_type,topk,group", [(8, "linear", 0, 64), (8, "linear", 1, 32), (4, "linear", 2, 16),
                                                        (4, "normal", 0, 64), (4, "e3m0", 1, 32)])
 def test_stochastic_one_rank_pass_matches_the_codec(ext, dtype, bit, quant_type, topk, group):
-    """The same seed gives the same numbers in registers and through a payload; another seed gives others; and the codes
-    are the oracle's for the counter-based numbers of `uniform01`, but for values that a rounding puts on the edge."""
+    """The same seed gives the same numbers in registers and through a payload; another seed gives others; and the payload
+    is the oracle's, bit for bit, for the counter-based numbers of `uniform01`."""
 
     cfg = _cfg(bit=bit, group_size=group, topk=topk, quant_type=quant_type, stochastic=True)
     code = codec._QUANT_CODE[quant_type]
-    for n, skew in ((20_000 // group * group, 0), (4096 + 5, 1), (group, 8)):
+    # (a fused product and sum would give another code for one value in 2^17: the first size has several of those)
+    for n, skew in ((2_000_000 // group * group, 0), (4096 + 5, 1), (group, 8)):
         x = torch.empty(n + skew, dtype=DTYPES[dtype], device="cuda").normal_(std=1e-2)[skew:]
         r = torch.empty(n, dtype=x.dtype, device="cuda").normal_(std=1e-4)
         results = []
@@ -547,11 +548,7 @@ def test_stochastic_one_rank_pass_matches_the_codec(ext, dtype, bit, quant_type,
             if n % group == 0:
                 noise = torch.from_numpy(_uniform01(seed, n)) - 0.5
                 expect = oracle.encode(x.cpu(), cfg, residual=r.cpu(), noise=noise)
-                codes = [oracle._unpack_words(oracle._split(p, n, cfg, dtype)[0], bit, x.element_size())
-                         for p in (payload, expect)]
-                # one rounding of value * mul + noise in the kernel, two in the oracle: up to 2^-17 apart (an ulp of 127),
-                # so another code for at most one value in 2^16, 0.3 of the 20 000
-                assert int((codes[0] != codes[1]).sum()) <= 6
+                assert torch.equal(payload.cpu(), expect)
         assert n < 1000 or not torch.equal(*results)
 
 
