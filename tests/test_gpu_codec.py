@@ -522,7 +522,7 @@ def test_general_kernels_on_a_grid_that_loops(ext, dtype, bit, quant_type, topk,
 
 @pytest.mark.parametrize("dtype", list(DTYPES))
 @pytest.mark.parametrize("bit,quant_type,topk,group", [(8, "linear", 0, 64), (8, "linear", 1, 32), (4, "linear", 2, 16),
-                                                       (4, "normal", 0, 64), (4, "e3m0", 1, 32)])
+                                                       (4, "normal", 0, 64), (4, "e3m0", 1, 32), (4, "uniform", 2, 16)])
 def test_stochastic_one_rank_pass_matches_the_codec(ext, dtype, bit, quant_type, topk, group):
     """The same seed gives the same numbers in registers and through a payload; another seed gives others; and the payload
     is the oracle's, bit for bit, for the counter-based numbers of `uniform01`."""
