@@ -58,11 +58,6 @@ __device__ __forceinline__ void span_to_global(uint8_t* dst, const uint8_t* span
     for (int o = (bytes & ~15) + wlane * 2; o < bytes; o += 64)
         *reinterpret_cast<uint16_t*>(dst + o) = *reinterpret_cast<const uint16_t*>(span + o);
 }
-__device__ __forceinline__ void span_from_global(uint8_t* span, const uint8_t* src, int bytes, int wlane) {
-    for (int o = wlane * 16; o + 16 <= bytes; o += 32 * 16) *reinterpret_cast<uint4*>(span + o) = ld16(src + o);
-    for (int o = (bytes & ~15) + wlane * 2; o < bytes; o += 64)
-        *reinterpret_cast<uint16_t*>(span + o) = *reinterpret_cast<const uint16_t*>(src + o);
-}
 // Code words to and from records that start on any even address (shared memory).
 template <int CB>
 __device__ __forceinline__ void span_put_codes(uint8_t* p, const uint32_t (&w)[4]) {

@@ -682,37 +682,20 @@ __global__ void __launch_bounds__(kThreads, 4) dequant_general_kernel(const __gr
     const int64_t n = p.numel;
     const int64_t num_groups = (n + p.group_size - 1) / p.group_size;
     const int64_t num_chunks = num_groups << shape.shift;
-    const int64_t chunk_span = (num_chunks + 31) / 32 * 32;
     const bool o_vec = (reinterpret_cast<uintptr_t>(out) & 31) == 0;
-    const bool staged = p.compact && (reinterpret_cast<uintptr_t>(p.src) & 15) == 0;
-    const bool c_vec = (reinterpret_cast<uintptr_t>(p.src) & (CB - 1)) == 0;      // planar
-    __shared__ __align__(16) uint8_t spans[kThreads / 32][kWarpSpan];
-    const int wlane = threadIdx.x & 31;
-    uint8_t* span = spans[threadIdx.x >> 5];
-    for (int64_t chunk = int64_t(blockIdx.x) * kThreads + threadIdx.x; chunk < chunk_span;
+    const bool c_vec = !p.compact && (reinterpret_cast<uintptr_t>(p.src) & (CB - 1)) == 0;
+    for (int64_t chunk = int64_t(blockIdx.x) * kThreads + threadIdx.x; chunk < num_chunks;
          chunk += int64_t(gridDim.x) * kThreads) {
-        const bool live = chunk < num_chunks;
         const int64_t first = chunk * kElemsPerThread;
         const int64_t g = chunk >> shape.shift;
         const int lane = int(chunk) & (lanes - 1);
+        // Records are read where they lie.  Turning a warp's span of them through shared memory, as the encoder does, was as
+        // fast or slower in every profile (16 Mi elements, records of 64 / k = 1, 16 / k = 2, int8: bf16 18.9 against 17.2 us,
+        // 22.9 against 18.8; fp32 20.9 against 20.1, 26.9 against 23.0).
+        const uint8_t* vptr = p.compact ? p.src + g * (VB + MB) : p.src + g * VB;
+        const uint8_t* meta = p.compact ? vptr + VB : p.src + num_groups * VB + g * MB;
         uint32_t w[4];
-        const uint8_t* meta;
-        if (staged) {
-            const int64_t g0 = (chunk - wlane) >> shape.shift;
-            const int groups = int(min(int64_t(32 >> shape.shift), num_groups - g0));
-            __syncwarp();
-            span_from_global(span, p.src + g0 * (VB + MB), groups * (VB + MB), wlane);
-            __syncwarp();
-            const uint8_t* rec = span + (wlane >> shape.shift) * (VB + MB);
-            if (!live) continue;
-            span_get_codes<CB>(rec + lane * CB, w);
-            meta = rec + VB;
-        } else {
-            if (!live) continue;
-            const uint8_t* vptr = p.compact ? p.src + g * (VB + MB) : p.src + g * VB;
-            meta = p.compact ? vptr + VB : p.src + num_groups * VB + g * MB;
-            load_code_words<KIND>(vptr + lane * CB, w, c_vec && !p.compact);
-        }
+        load_code_words<KIND>(vptr + lane * CB, w, c_vec);
         Packed16<T> d = decode_group<T, TOPK, KIND>(w, meta, lane, lut);
         if (p.accumulate) {
             float a[16], b[16];
