@@ -402,6 +402,16 @@ void order_streams(uintptr_t first, uintptr_t then, int device_index) {
     cuda_check(err, "order_streams");
 }
 
+// The name of the first of the two that is not like `x` (dtype, elements, device, in order), or an empty string: one crossing
+// for what a collective takes by address.
+const char* unlike(const at::Tensor& x, const std::optional<at::Tensor>& out, const std::optional<at::Tensor>& residual) {
+    const auto differs = [&](const std::optional<at::Tensor>& t) {
+        return t.has_value() && (t->scalar_type() != x.scalar_type() || t->numel() != x.numel() ||
+                                 t->device() != x.device() || !t->is_contiguous());
+    };
+    return differs(out) ? "out" : (differs(residual) ? "residual" : "");
+}
+
 at::Tensor tensor_from_address(uintptr_t ptr, int64_t nbytes, int device_index) {
     TORCH_CHECK(ptr != 0 && nbytes >= 0, "bad address or size");
     auto options = at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device_index);
@@ -477,6 +487,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("status_clear", &lbc::status_clear);
     m.def("tensor_from_address", &tensor_from_address);
     m.def("memset_async", &memset_async);
+    m.def("unlike", &unlike, py::arg("x"), py::arg("out"), py::arg("residual"));
     m.def("order_streams", &order_streams, py::arg("first"), py::arg("then"), py::arg("device_index"));
 
     lbc::bind_work(m);

@@ -282,7 +282,7 @@ class Communicator:
                 ws = None
             if ws is not None:
                 if out is not None or residual is not None:
-                    self._check_alike(tensor, out=out, residual=residual)
+                    self._check_alike(ws.ext, tensor, out, residual)
                 if not async_op and not tracing.ENABLED:
                     result = ws.all_reduce(tensor, out, residual=residual, update_residual=update_residual, op=op,
                                            stages=stages, ef_mode=ef_mode)
@@ -304,7 +304,8 @@ class Communicator:
             if gws is not None:
                 # a strided residual goes in as a copy, which is written back
                 dense = residual if residual is None or residual.is_contiguous() else residual.contiguous()
-                self._check_alike(tensor, out=out, residual=dense)
+                if out is not None or residual is not None:
+                    self._check_alike(gws.ext, tensor, out, dense)
                 scope, side = self._stream_scope(tensor, async_op)
                 # a strategy that names the two-stage algorithm gets it (reduce-scatter, requantize, gather); "auto"
                 # and "all_gather" keep the one-stage exchange, and so does stochastic rounding
@@ -321,13 +322,12 @@ class Communicator:
         return ImmediateWork(result) if async_op else result
 
     @staticmethod
-    def _check_alike(tensor: Any, **others: Any) -> None:
+    def _check_alike(ext: Any, tensor: Any, out: Any, residual: Any) -> None:
         """The kernels take addresses: what goes with `tensor` has its dtype, size and device, and its elements in order."""
 
-        for name, other in others.items():
-            if other is not None and (other.dtype != tensor.dtype or other.numel() != tensor.numel()
-                                      or other.device != tensor.device or not other.is_contiguous()):
-                raise ValueError(f"{name} must be contiguous, with the dtype, the device and the number of elements of the tensor")
+        name = ext.unlike(tensor, out, residual)
+        if name:
+            raise ValueError(f"{name} must be contiguous, with the dtype, the device and the number of elements of the tensor")
 
     def bind_all_reduce(self, *, config: CompressionConfig, op: str = "mean", strategy: str = "auto",
                         dtype: str = "auto"):
