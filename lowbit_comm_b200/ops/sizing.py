@@ -49,8 +49,9 @@ class QuantizationSizeEstimate:
 def estimate_quantized_size(numel: int, *, dtype: str, config: CompressionConfig) -> QuantizationSizeEstimate:
     """Bytes a tensor of `numel` elements occupies once quantized."""
 
-    ask = _memoized if type(numel) is int else _estimate
-    return ask(numel, dtype, config.group_size, config.bit, config.topk)
+    if type(numel) is int:
+        return _memoized(numel, dtype, config.group_size, config.bit, config.topk)
+    return _estimate(numel, dtype, config.group_size, config.bit, config.topk)
 
 
 def _estimate(numel: int, dtype: str, group_size: int, bit: int, topk: int) -> QuantizationSizeEstimate:
@@ -67,9 +68,12 @@ def _estimate(numel: int, dtype: str, group_size: int, bit: int, topk: int) -> Q
         compression_ratio=(raw / packed) if packed else 0.0)
 
 
-# Every codec call asks, a job asks for few sizes: 0.3 us instead of 4.  Only for plain integers: 640.0 and 640 would be
-# one key, but an estimate's fields have the type of the size it was asked for.
-_memoized = lru_cache(maxsize=1024, typed=True)(_estimate)
+# Every codec call asks, a job asks for few sizes: 0.2 us instead of 4.  Only for sizes that are plain integers: 640.0 and
+# 640 would be one key, but an estimate's fields have the type of the size it was asked for.  A policy's 64.0 and 64 are
+# one key too, and one value.
+@lru_cache(maxsize=1024)
+def _memoized(numel: int, dtype: str, group_size: int, bit: int, topk: int) -> QuantizationSizeEstimate:
+    return _estimate(numel, dtype, int(group_size), int(bit), int(topk))
 
 
 @dataclass(frozen=True)

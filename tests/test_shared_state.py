@@ -75,6 +75,8 @@ def test_memoized_sizes_keep_the_types_of_each_caller(first):
     config = CompressionConfig()
     estimate_quantized_size(first(numel), dtype="bf16", config=config)
     geometry(first(numel), 2, "bf16", config)
+    estimate_quantized_size(numel, dtype="bf16", config=CompressionConfig(bit=8.0, group_size=np.float64(64)))
+    geometry(numel, np.int64(2), "bf16", CompressionConfig(group_size=64.0))
     estimate, shape = estimate_quantized_size(numel, dtype="bf16", config=config), geometry(numel, 2, "bf16", config)
     for value in (*dataclasses.asdict(estimate).values(), *dataclasses.asdict(shape).values()):
         assert type(value) in (int, float, str), value
