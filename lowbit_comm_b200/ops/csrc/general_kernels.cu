@@ -3,7 +3,7 @@
 // per group), 4-bit code-books (normal, uniform, e3m0, e2m1), stochastic
 // rounding — for fp16/bf16/fp32 sources, group sizes 16/32/64, both payload
 // layouts.  One kernel per (dtype, k, kind of code); group size, layout, code-book
-// and rounding rule are runtime parameters.
+// and the rounding of linear codes are runtime parameters.
 //
 // Parity: quantization/quant_kernel.cuh:25-153 (top-k selection, scale = the
 // (k+1)-th largest magnitude, selected elements zeroed), inner.cuh:9-96
@@ -16,12 +16,12 @@
 // more cycles per element than its bytes cost DRAM.  Hence: k and the kind of code are template parameters (nothing is
 // selected that the profile does not keep); kept elements are patched into the packed words (8 predicated permutes
 // instead of 32 selects on the values); a code is a count of thresholds that sit in the kernel's parameters; payload
-// words move as vectors, through shared memory where the records of the compact layout break the alignment.
+// words move as vectors; records of the compact layout, which break the alignment, are built in shared memory.
 // Measured on a B200: encode + decode of 5 M fp32 elements, e2m1 code-book, 81 -> 27 us (the search in a table in
 // constant memory took one pass per distinct entry in a warp); all-reduce of one rank, 32 Mi bf16 elements, one kept
 // value per group, 107 -> 72 us.  Then, without the clamp and the NaN test where the selection has shown that no value
 // needs them, without a trip through packed bytes, and with a block per tile: 72 -> 36 us (the SM's issue slots are 68-72 %
-// busy, DRAM 41 %), and 81 -> 25 us for the code-book (encode 16.7, decode 8.7; SM 71 % and 28 % busy, DRAM 21 % and 33 %).
+// busy, DRAM 41 %), and 81 -> 25 us for the code-book (encode 16.7, decode 8.5; SM 72 % and 26 % busy, DRAM 21 % and 34 %).
 
 #include <cmath>
 #include <type_traits>
@@ -833,9 +833,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 4 : 3) roundtrip_ge
 // A block per 4096 elements up to four times the default grid, a grid that loops above: it pays a block's set-up less
 // often.  One-rank pass, full grid against a looping one: bf16 top-k 1, 8 M elements (1.6 default grids) 12.5 / 12.5 us,
 // 16 M 20.7 / 20.6, 20 M (4.1) 24.8 / 24.2, 24 M 28.9 / 27.5, 32 M 37.1 / 35.0, 64 M 69.8 / 64.0; fp32 top-k 1, 10 M
-// 20.6 / 20.6, 20 M 36.1 / 35.0, 64 M 102.5 / 96.6; fp32 code-book, 10 M 30.9 / 29.5, 20 M 55.0 / 55.2, 64 M 159 / 152.  The
-// 16-bit code-book is the exception (20 M 47.3 / 49.3, 64 M 140 / 144).  The default grid also serves blocks that meet
-// at a flag or a counter (`shared`): each costs a system-scope fence or a look at the flags.
+// 20.6 / 20.6, 20 M 36.1 / 35.0, 64 M 102.5 / 96.6.  A code-book does not care: fp32, 10 M 28.8 / 28.9, 20 M 49.4 / 49.8, 64 M
+// 146 / 147; bf16, 20 M 48.0 / 49.3, 64 M 143.6 / 144.3.  The default grid also serves blocks that meet at a flag or a
+// counter (`shared`): each costs a system-scope fence or a look at the flags.
 static int general_grid(int64_t groups, int group_size, int max_blocks, bool shared) {
     int64_t want = (groups * (group_size / kElemsPerThread) + kThreads - 1) / kThreads;
     if (want < 1) want = 1;
