@@ -15,15 +15,17 @@
 // What bounds these kernels is the instruction issue, not memory: selecting, searching a code-book and packing cost
 // more cycles per element than its bytes cost DRAM.  Hence: k and the kind of code are template parameters (nothing is
 // selected that the profile does not keep); kept elements are patched into the packed words (8 predicated permutes
-// instead of 32 selects on the values); a code is a count of thresholds that sit in the kernel's parameters; payload
+// instead of 32 selects on the values); a code of a code-book is one look-up and one addition; payload
 // words move as vectors; records of the compact layout, which break the alignment, are built in shared memory.
 // Measured on a B200: encode + decode of 5 M fp32 elements, e2m1 code-book, 81 -> 27 us (the search in a table in
 // constant memory took one pass per distinct entry in a warp); all-reduce of one rank, 32 Mi bf16 elements, one kept
 // value per group, 107 -> 72 us.  Then, without the clamp and the NaN test where the selection has shown that no value
 // needs them, without a trip through packed bytes, and with a block per tile: 72 -> 36 us (the SM's issue slots are 68-72 %
-// busy, DRAM 41 %), and 81 -> 25 us for the code-book (encode 16.7, decode 8.5; SM 72 % and 26 % busy, DRAM 21 % and 34 %).
+// busy, DRAM 41 %), and 81 -> 25 us for the code-book.  Then, with a look-up instead of fourteen thresholds: 24.5 -> 18.4 us for
+// the code-book; encode of 16 MiB, beyond L2, bf16 22.5 -> 14.5 us, fp32 14.0 -> 8.6, one-rank pass bf16 22.7 -> 14.5.
 
 #include <cmath>
+#include <cstring>
 #include <type_traits>
 
 #include "codec_device.cuh"
@@ -379,13 +381,86 @@ __device__ __forceinline__ float fma_saturated(float a, float b, float c) {
     asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
 }
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t how) {      // with the sign mode, which __byte_perm lacks
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(how));
+    return r;
+}
 struct CodeRule {
+    uint32_t step;             // kBook: the entry of LbcBook::steps that this lane of the warp holds
+    float nudge;
     // kBook: thresholds[c] = -2^60 * the largest float below the least t = value / scale whose code is above c
     const float* thresholds;
     const float* table;        // kBookNoise: the code-book
     int stochastic;            // linear
     unsigned long long seed;
+    template <int KIND>
+    __device__ __forceinline__ static CodeRule of(const LbcBook& book, int quant_type, int stochastic, unsigned long long seed) {
+        CodeRule r{0u, 0.0f, book.thresholds, KIND == kBookNoise ? kCodebooks[quant_type - 1] : nullptr, stochastic, seed};
+        if (KIND == kBook) {
+            r.step = book.steps[threadIdx.x & 31];
+            r.nudge = book.nudge;
+        }
+        return r;
+    }
 };
+
+// ---- deterministic code-books -----------------------------------------------------------------------------------
+// A code is 7 plus or minus the number of thresholds that |t|, t = value / scale, has reached.  The bits of |t| down to its
+// second mantissa bit name one of 32 buckets (2^-7 to 2, four to an octave), none of which holds two thresholds in any of the
+// four tables; the entry of a bucket, added to the bits below, carries into the count when they reach its threshold.  Each lane
+// of the warp holds one entry, and a shuffle, whose index is its five low bits, looks it up.  Counting the fourteen
+// thresholds one by one took 28 issue slots per element, this takes six.
+// A tie goes to the lower entry, so the two signs differ by the last bit of |t|: the sign is appended to it.  Two thresholds
+// at powers of two (the lowest of e3m0 and of e2m1) differ by more, because the rule's t - entry rounds there; `nudge`, half
+// a bit of the octave below them, takes both signs to the same side.
+// t, correctly rounded where that decides: value * (1 / scale) with one Newton correction by its exact remainder (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000", 1990).  Before its rounding the corrected quotient is off
+// by 3 * 2^-24 ulp at most; quotients of two floats that lie nearer than ten times that to a rounding boundary beside a threshold
+// solve v * 2^k = m * s + d for a small d, and none of them rounds wrongly; quotients of 16-bit operands lie 2^-11 ulp away.
+// It holds for scales up to 1e30 (nothing that decides overflows or underflows) with no value above the scale but kept ones.
+struct BookCode {
+    uint32_t bits;             // the count in the top byte
+    uint32_t t;                // the sign on top
+};
+__device__ __forceinline__ BookCode book_code(float v, float safe, float inverse, const CodeRule& rule) {
+    float t = __fmul_rn(v, inverse);
+    t = __fmaf_rn(__fmaf_rn(-t, safe, v), inverse, t);
+    BookCode c;
+    c.t = __float_as_uint(__fsub_rn(t, rule.nudge));
+    const uint32_t key = max(__funnelshift_l(c.t, c.t, 1), 0x78000000u);      // no threshold below 2^-7.  NaN: the last bucket, 7
+    c.bits = key * 4u + __shfl_sync(0xffffffffu, rule.step, int(key >> 22));
+    return c;
+}
+// Eight of them -> one word of wire-ordered codes (see pack16_low_nibbles): 7 + count, or 7 - count = 7 ^ count.
+template <int WordBytes>
+__device__ __forceinline__ uint32_t pack_book(const BookCode (&c)[8]) {
+    uint32_t k[2], s[2];
+#pragma unroll
+    for (int odd = 0; odd < 2; ++odd) {
+        const BookCode &a = c[odd], &b = c[2 + odd], &d = c[4 + odd], &e = c[6 + odd];
+        const uint32_t k0 = prmt(b.bits, a.bits, 0x0073), k1 = prmt(e.bits, d.bits, 0x0073);
+        const uint32_t s0 = prmt(b.t, a.t, 0x00fb), s1 = prmt(e.t, d.t, 0x00fb);      // 0xff where the sign is set
+        k[odd] = WordBytes == 2 ? prmt(k0, k1, 0x5410) : prmt(k1, k0, 0x5410);
+        s[odd] = WordBytes == 2 ? prmt(s0, s1, 0x5410) : prmt(s1, s0, 0x5410);
+    }
+    const uint32_t counts = ((k[0] << 4) & 0xf0f0f0f0u) | (k[1] & 0x0f0f0f0fu);
+    const uint32_t signs = (s[0] & 0xf0f0f0f0u) | (s[1] & 0x0f0f0f0fu);
+    return ((counts ^ signs) & 0x77777777u) + (~signs & 0x77777777u);
+}
+// A scale that is infinite, NaN or above 1e30: the machine's division and one saturated multiply-add per threshold (1 when
+// t has reached it, else 0: the exact difference times 2^60 is above 1 or not above 0).  NaN: 14, as the search has it.
+__device__ __noinline__ void book_codes_far(const float* v, float safe, const float* thresholds, uint32_t* b) {
+    for (int i = 0; i < 16; ++i) {
+        const float t = v[i] / safe;
+        float q = kRoundMagic;
+        for (int c = 0; c < 14; ++c) q += fma_saturated(t, kThresholdScale, thresholds[c]);
+        b[i] = __float_as_uint(t == t ? q : kRoundMagic + 14.0f);
+    }
+}
+// Is the scale of every group of the warp one that book_code takes?  (A 16-bit group with more NaN than it keeps has NaN for
+// its scale, which bounds no value: the test is on the scale as stored, false for NaN.)
+__device__ __forceinline__ bool book_near(float stored) { return __all_sync(0xffffffffu, stored < 1.0e30f); }
 
 // Codes of 16 values against the group's scale, as bit patterns whose low byte (nibble) is the code.  With `tame` (no
 // infinity and no NaN in any group of the warp) no value that is not kept verbatim is larger than the scale, so
@@ -393,6 +468,7 @@ struct CodeRule {
 template <int KIND>
 __device__ __forceinline__ void encode_general(const float (&v)[16], float stored, bool tame, const CodeRule& rule,
                                                int64_t first, uint32_t (&b)[16]) {
+    static_assert(KIND != kBook, "book_code");
     constexpr int lim = Kind<KIND>::lim;
 #pragma unroll
     for (int i = 0; i < 16; ++i) b[i] = 0u;
@@ -416,32 +492,6 @@ __device__ __forceinline__ void encode_general(const float (&v)[16], float store
         for (int i = 0; i < 16; ++i) {
             const float r = __fadd_rn(t[i] == t[i] ? t[i] : 0.0f, kRoundMagic);   // rint(t) in the low bits; NaN: code 0
             b[i] = __float_as_uint(fminf(fmaxf(r, kRoundMagic - float(lim)), kRoundMagic + float(lim)));
-        }
-    } else if constexpr (KIND == kBook) {
-        // value / safe, correctly rounded: two Newton corrections of value * (1 / safe) with the exact remainder
-        // (Markstein, "Computation of elementary functions on the IBM RISC System/6000", 1990).  Its conditions (no
-        // overflow, no underflow of what decides) hold for scales up to 1e30: a quotient that is next to a threshold
-        // is at least 2^-7 and its dividend at least 2^-7 * 1e-6, and no value that is not kept is above the scale.
-        // A 16-bit group with more NaN than it keeps has NaN for its scale, which bounds no value (the quotient by 1e-6
-        // may overflow, and its remainder is NaN then): the test is on the scale as stored, false for NaN.
-        const bool near = __all_sync(0xffffffffu, stored < 1.0e30f);
-        const float inverse = __frcp_rn(safe);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            float t;
-            if (near) {
-                t = __fmul_rn(v[i], inverse);
-                t = __fmaf_rn(__fmaf_rn(-t, safe, v[i]), inverse, t);
-                t = __fmaf_rn(__fmaf_rn(-t, safe, v[i]), inverse, t);
-            } else {
-                t = v[i] / safe;
-            }
-            // one saturated multiply-add per threshold: 1 when t has reached it, else 0 (the exact difference times
-            // 2^60 is above 1 or not above 0); comparing and counting in integers takes twice the issue slots
-            float q = kRoundMagic;
-#pragma unroll
-            for (int c = 0; c < 14; ++c) q += fma_saturated(t, kThresholdScale, rule.thresholds[c]);
-            b[i] = __float_as_uint(t == t ? q : kRoundMagic + 14.0f);      // NaN: 14, as the search has it
         }
     } else {
         // The last entry that is not above t, by looking at all of them in order: their addresses are the same for every
@@ -475,6 +525,35 @@ __device__ __forceinline__ void pack_codes(const uint32_t (&b)[16], uint32_t (&w
         const uint2 c = pack16_low_nibbles<sizeof(T)>(b);
         w[0] = c.x; w[1] = c.y; w[2] = w[3] = 0u;
     }
+}
+
+// Values to packed codes.  Convergent.
+template <typename T, int KIND>
+__device__ __forceinline__ void encode_words(const float (&v)[16], float stored, bool tame, const CodeRule& rule,
+                                             int64_t first, uint32_t (&w)[4]) {
+    uint32_t b[16];
+    if constexpr (KIND == kBook) {
+        const float safe = fmaxf(stored, 1.0e-6f);
+        if (book_near(stored)) {
+            const float inverse = __frcp_rn(safe);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                BookCode c[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) c[e] = book_code(v[8 * j + e], safe, inverse, rule);
+                w[j] = pack_book<sizeof(T)>(c);
+            }
+            w[2] = w[3] = 0u;
+            return;
+        }
+        float far[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) far[i] = v[i];
+        book_codes_far(far, safe, rule.thresholds, b);
+    } else {
+        encode_general<KIND>(v, stored, tame, rule, first, b);
+    }
+    pack_codes<T, KIND>(b, w);
 }
 
 // 16 codes -> T(value), scale applied; `lut` is the code-book in shared memory.
@@ -516,6 +595,36 @@ __device__ __forceinline__ Packed16<T> decode_bits(const uint32_t (&b)[16], floa
     for (int i = 0; i < 16; ++i)
         d[i] = __fmul_rn(Kind<KIND>::book ? lut[b[i] & 0xfu] : __uint_as_float(b[i]) - kRoundMagic, step);
     return pack_elems<T>(d);
+}
+
+// Values -> T(decode(encode(value))).  Convergent.
+template <typename T, int KIND>
+__device__ __forceinline__ Packed16<T> requantize(const float (&v)[16], float stored, bool tame, const CodeRule& rule,
+                                                  int64_t first, const float* lut) {
+    uint32_t b[16];
+    if constexpr (KIND == kBook) {
+        const float safe = fmaxf(stored, 1.0e-6f);
+        if (book_near(stored)) {
+            const float inverse = __frcp_rn(safe);
+            const float entry = lut[7 + (threadIdx.x & 7)];             // the entries from zero on, one per lane
+            float d[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const BookCode c = book_code(v[i], safe, inverse, rule);
+                const float size = __shfl_sync(0xffffffffu, entry, int(c.bits >> 24), 8);
+                // (adding zero makes the zero of code 7 positive, as the decoder's product is)
+                d[i] = __fmaf_rn(size, __uint_as_float(__float_as_uint(stored) ^ (c.t & 0x80000000u)), 0.0f);
+            }
+            return pack_elems<T>(d);
+        }
+        float far[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) far[i] = v[i];
+        book_codes_far(far, safe, rule.thresholds, b);
+    } else {
+        encode_general<KIND>(v, stored, tame, rule, first, b);
+    }
+    return decode_bits<T, KIND>(b, stored, lut);
 }
 
 template <int KIND>
@@ -594,7 +703,7 @@ __global__ void __launch_bounds__(kThreads, 4) quant_general_kernel(const __grid
     const int copies = (p.num_dst > 0 && !scatter) ? p.num_dst : 1;
     const bool staged = p.compact && p.num_dst == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
     __shared__ __align__(16) uint8_t spans[kThreads / 32][kWarpSpan];
-    const CodeRule rule{p.thresholds, KIND == kBookNoise ? kCodebooks[p.quant_type - 1] : nullptr, p.stochastic, p.seed};
+    const CodeRule rule = CodeRule::of<KIND>(p.book, p.quant_type, p.stochastic, p.seed);
     const int wlane = threadIdx.x & 31;
     uint8_t* span = spans[threadIdx.x >> 5];
 
@@ -617,9 +726,8 @@ __global__ void __launch_bounds__(kThreads, 4) quant_general_kernel(const __grid
         }
         if (prep != nullptr && live) store_elems<T>(prep, first, n, p_vec, res != nullptr ? elems : pack_elems<T>(v));
         const GroupMeta m = select_group<T, TOPK>(v, elems, lane, lanes);
-        uint32_t b[16], w[4];
-        encode_general<KIND>(v, m.stored, __all_sync(0xffffffffu, m.tame), rule, first, b);
-        pack_codes<T, KIND>(b, w);
+        uint32_t w[4];
+        encode_words<T, KIND>(v, m.stored, __all_sync(0xffffffffu, m.tame), rule, first, w);
 #pragma unroll
         for (int j = 0; j < TOPK; ++j) patch_code<T, KIND>(w, m.idx[j] - lane * 16);
         if (staged) {
@@ -788,7 +896,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 4 : 3) roundtrip_ge
     const int64_t chunk_span = (num_chunks + 31) / 32 * 32;
     const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(res) |
                        reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(rout)) & 31) == 0;
-    const CodeRule rule{p.thresholds, KIND == kBookNoise ? kCodebooks[p.quant_type - 1] : nullptr, p.stochastic, p.seed};
+    const CodeRule rule = CodeRule::of<KIND>(p.book, p.quant_type, p.stochastic, p.seed);
     for (int64_t chunk = int64_t(blockIdx.x) * kThreads + threadIdx.x; chunk < chunk_span;
          chunk += int64_t(gridDim.x) * kThreads) {
         const bool live = chunk < num_chunks;
@@ -809,11 +917,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 4 : 3) roundtrip_ge
             unpack_elems<T>(y, v);
             const GroupMeta m = select_group<T, TOPK>(v, y, lane, lanes);
             const bool tame = __all_sync(0xffffffffu, m.tame);
-            uint32_t b[16];
-            encode_general<KIND>(v, m.stored, tame, rule, first, b);
             if (sizeof(T) == 2 && !tame) y = pack_elems<T>(v);          // a NaN that is kept has one pattern
             const Packed16<T> from = y;
-            y = decode_bits<T, KIND>(b, m.stored, lut);
+            y = requantize<T, KIND>(v, m.stored, tame, rule, first, lut);
 #pragma unroll
             for (int j = 0; j < TOPK; ++j) copy_elem<T>(y, from, int(uint32_t(m.idx[j]) & 0xffu) - lane * 16);
         }
@@ -844,13 +950,17 @@ static int general_grid(int64_t groups, int group_size, int max_blocks, bool sha
     return int(want < cap ? want : cap);
 }
 
-// The least float t for which the rule "the last entry that is not above t, and the one after it when
-// t - entry > gap / 2" gives a code above c, searched on the bit patterns around the middle of the two entries.
-struct BookThresholds {
-    float of[4][14];
-    BookThresholds() {
+// The thresholds of the rule "the last entry that is not above t, and the one after it when t - entry > gap / 2", searched on
+// the bit patterns around the middle of two entries, and what the kernels make of them (see book_code and book_codes_far).
+struct BookTable {
+    LbcBook of[4];
+    BookTable() {
         static const float tables[4][15] = LBC_CODEBOOKS;
-        for (int q = 0; q < 4; ++q)
+        static const float nudges[4] = {0.0f, 0.0f, 2.3283064365386963e-10f, 1.862645149230957e-09f};      // 2^-32, 2^-29
+        for (int q = 0; q < 4; ++q) {
+            LbcBook& book = of[q];
+            book.nudge = nudges[q];
+            float least[14];                           // the least t whose code is above c
             for (int c = 0; c < 14; ++c) {
                 const float a = tables[q][c], b = tables[q][c + 1];
                 const auto above = [&](float t) {
@@ -861,14 +971,33 @@ struct BookThresholds {
                 float t = a + (b - a) * 0.5f;
                 for (int i = 0; i < 64 && !above(t); ++i) t = std::nextafterf(t, 2.0f);
                 for (int i = 0; i < 64 && above(std::nextafterf(t, -2.0f)); ++i) t = std::nextafterf(t, -2.0f);
-                of[q][c] = -kThresholdScale * std::nextafterf(t, -2.0f);
+                least[c] = t;
+                book.thresholds[c] = -kThresholdScale * std::nextafterf(t, -2.0f);
             }
+            const auto key = [&](float t) {            // as book_code forms it
+                volatile float nudged = t - book.nudge;
+                const float f = nudged;
+                uint32_t bits;
+                std::memcpy(&bits, &f, sizeof(bits));
+                return bits << 1 | bits >> 31;
+            };
+            for (uint32_t i = 0; i < 32; ++i) {
+                const uint32_t upper = (0x78000000u >> 22) + i;           // the bits of a key that name the bucket
+                uint32_t below = 0u, inside = 0u;
+                for (int c = 7; c < 14; ++c) {         // a threshold above zero and its mirror image
+                    const uint32_t plus = key(least[c]), minus = key(std::nextafterf(least[13 - c], -2.0f));
+                    const uint32_t at = plus < minus ? plus : minus;
+                    if (at >> 22 < upper) ++below;
+                    if (at >> 22 == upper) inside = (1u << 24) - ((at * 4u) & 0xffffffu);
+                }
+                book.steps[i] = (below << 24) - (upper << 24) + inside;
+            }
+        }
     }
 };
-// (stored as the kernel wants it, see CodeRule)
-static void fill_thresholds(float (&out)[14], int quant_type) {
-    static const BookThresholds book;
-    for (int c = 0; c < 14; ++c) out[c] = quant_type == LBC_LINEAR ? 0.0f : book.of[quant_type - 1][c];
+static LbcBook book_of(int quant_type) {
+    static const BookTable table;
+    return quant_type == LBC_LINEAR ? LbcBook{} : table.of[quant_type - 1];
 }
 
 template <typename T, int TOPK, int KIND>
@@ -956,7 +1085,7 @@ cudaError_t lbc_quant_general(const LbcQuantGeneral* p, cudaStream_t stream) {
     for (int d = 0; d < p->num_dst; ++d)
         if (p->dst[d] == nullptr) return cudaErrorInvalidValue;
     LbcQuantGeneral launch = *p;
-    lbc::fill_thresholds(launch.thresholds, p->quant_type);
+    launch.book = lbc::book_of(p->quant_type);
     return lbc::launch_general<lbc::QuantGeneral>(launch, p->max_blocks, p->signal.num_remote > 0, stream);
 }
 
@@ -985,7 +1114,7 @@ cudaError_t lbc_roundtrip_general(const LbcRoundtripGeneral* p, cudaStream_t str
     if (p->passes < 1 || p->passes > 2 || (p->residual == nullptr && p->residual_out != nullptr)) return cudaErrorInvalidValue;
     if (p->numel > 0 && (p->x == nullptr || p->out == nullptr)) return cudaErrorInvalidValue;
     LbcRoundtripGeneral launch = *p;
-    lbc::fill_thresholds(launch.thresholds, p->quant_type);
+    launch.book = lbc::book_of(p->quant_type);
     return lbc::launch_general<lbc::RoundtripGeneral>(launch, p->max_blocks, false, stream);
 }
 

@@ -174,6 +174,13 @@ typedef struct {
 cudaError_t lbc_roundtrip(const LbcRoundtrip* p, cudaStream_t stream);
 
 // ---- general path: top-k, 4-bit code-books, stochastic rounding --------------
+// How the kernels find a code (filled in by the launchers, see BookTable in general_kernels.cu).
+typedef struct {
+    uint32_t steps[32];        // per bucket of a quotient's bits: the code below its threshold, and the way to it
+    float nudge;               // taken off every quotient first
+    float thresholds[14];      // for the scales whose quotients the buckets do not hold
+} LbcBook;
+
 typedef struct {
     int dtype, group_size, bit, topk, quant_type, stochastic, compact;
     const void* x;
@@ -191,7 +198,7 @@ typedef struct {
     // Scatter (shard_groups > 0, with destinations): group g goes to dst[g / shard_groups] only, as group
     // g % shard_groups of a self-contained payload of shard_groups groups (a reduce-scatter's first half).
     int64_t shard_groups;
-    float thresholds[14];      // filled in by the launcher (code-books)
+    LbcBook book;              // filled in by the launcher (code-books)
 } LbcQuantGeneral;
 
 typedef struct {
@@ -234,7 +241,7 @@ typedef struct {
     int passes;                // 1 or 2
     unsigned long long seed;
     int max_blocks;            // 0 = library default
-    float thresholds[14];      // filled in by the launcher (code-books)
+    LbcBook book;              // filled in by the launcher (code-books)
 } LbcRoundtripGeneral;
 
 cudaError_t lbc_roundtrip_general(const LbcRoundtripGeneral* p, cudaStream_t stream);

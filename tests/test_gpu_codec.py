@@ -214,6 +214,34 @@ def test_codebook_codes_at_their_thresholds(ext, quant_type):
 
 
 @pytest.mark.parametrize("quant_type", ("normal", "uniform", "e3m0", "e2m1"))
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("topk", (0, 2))
+def test_codebook_look_up_in_every_bucket(ext, quant_type, dtype, topk):
+    """Encode and the one-rank pass where the look-up changes its entry: the powers of two and their quarters, the middles of the
+    entries, each with its neighbours in the type, both signs, beside what is too small for any bucket."""
+
+    table = oracle.codebook(quant_type)[:15]
+    edges = torch.cat([torch.tensor([2.0 ** -e * (1 + q / 4) for e in range(1, 10) for q in range(4)]),
+                       table[:-1] + (table[1:] - table[:-1]) / 2, torch.tensor([0.0, 1e-7, 2.0 ** -20])]).to(DTYPES[dtype])
+    way = torch.full_like(edges, 2.0)
+    values = torch.cat([edges, torch.nextafter(edges, way), torch.nextafter(edges, -way)]).clamp(-1, 1)
+    values = torch.cat([values, -values])
+    for scale in (1.0, 0.7310584, 3.0e-7):
+        groups = torch.zeros(-(-values.numel() // 12), 16)
+        flat = torch.zeros(groups.shape[0] * 12)
+        flat[:values.numel()] = values
+        groups[:, 4:] = flat.reshape(-1, 12)
+        groups[:, :3] = torch.tensor([1.0, 4.0, -3.0]) if topk else torch.tensor([1.0, -1.0, 0.0])
+        x = (groups * scale).reshape(-1).to(DTYPES[dtype])
+        cfg = _cfg(bit=4, group_size=16, topk=topk, quant_type=quant_type)
+        payload = oracle.encode(x, cfg)
+        assert torch.equal(codec.quantize_tensor(x.cuda(), cfg).cpu(), payload), scale
+        out = torch.empty_like(x).cuda()
+        assert ext.roundtrip_general(x.cuda(), None, out, None, 16, 4, topk, codec._QUANT_CODE[quant_type], False, 0, 1)
+        assert torch.equal(out.cpu().view(torch.uint8), oracle.decode(payload, x.numel(), cfg, dtype).view(torch.uint8)), scale
+
+
+@pytest.mark.parametrize("quant_type", ("normal", "uniform", "e3m0", "e2m1"))
 def test_codebook_codes_around_the_division_limit(ext, quant_type):
     """The corrected reciprocal serves scales below 1e30, a division the others: values at every threshold with scales
     next to the limit, and 16-bit sources (whose quotients round apart from the fp32 ones) on both sides of it."""
