@@ -23,6 +23,8 @@
 // needs them, without a trip through packed bytes, and with a block per tile: 72 -> 36 us (the SM's issue slots are 68-72 %
 // busy, DRAM 41 %), and 81 -> 25 us for the code-book.  Then, with a look-up instead of fourteen thresholds: 24.5 -> 18.4 us for
 // the code-book; encode of 16 MiB, beyond L2, bf16 22.5 -> 14.5 us, fp32 14.0 -> 8.6, one-rank pass bf16 22.7 -> 14.5.
+// The one-rank pass without the places of the kept elements: 35.9 -> 30.8 us (32 Mi bf16 elements, one kept value); of 16 MiB
+// beyond L2, two kept values, bf16 14.4 -> 12.4 us, fp32 12.4 -> 10.3.
 
 #include <cmath>
 #include <cstring>
@@ -372,6 +374,139 @@ __device__ __forceinline__ GroupMeta select_group(float (&v)[16], const Packed16
         }
     }
     return m;
+}
+
+// ---- the scale of a group without the places of what it keeps ------------------------------------------------------
+// Magnitudes of two 16-bit elements per word (the signs that come out mean nothing; NaN wins).
+template <typename T>
+__device__ __forceinline__ uint32_t abs_max2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    if constexpr (std::is_same<T, __half>::value)
+        asm("max.NaN.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    else
+        asm("max.NaN.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+template <typename T>
+__device__ __forceinline__ uint32_t abs_min2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    if constexpr (std::is_same<T, __half>::value)
+        asm("min.NaN.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    else
+        asm("min.NaN.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+// All ones in the halves of `a` whose magnitude is above that of `b`, which has no signs.
+template <typename T>
+__device__ __forceinline__ uint32_t abs_above2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    if constexpr (std::is_same<T, __half>::value)
+        asm("{.reg .b32 m; abs.f16x2 m, %1; set.gt.u32.f16x2 %0, m, %2;}" : "=r"(r) : "r"(a), "r"(b));
+    else
+        asm("{.reg .b32 m; abs.bf16x2 m, %1; set.gt.u32.bf16x2 %0, m, %2;}" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b) {      // NaN wins
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// The (TOPK + 1)-th largest magnitude of a group and the one before it; all `lanes` threads of the group get the answer.
+struct GroupTop {
+    float stored, last_kept;
+    bool finite;               // no infinity and no NaN in the group
+};
+template <typename T, int TOPK>
+__device__ __forceinline__ GroupTop top_of_group(const Packed16<T>& p, int lanes) {
+    static_assert(TOPK == 1 || TOPK == 2, "two or three magnitudes");
+    GroupTop g;
+    if constexpr (sizeof(T) == 2) {
+        uint32_t k0 = p.w[0], k1 = 0u, k2 = 0u;                  // per half word, |k0| >= |k1| >= |k2|
+#pragma unroll
+        for (int i = 1; i < 8; ++i) {
+            const uint32_t a = abs_min2<T>(k0, p.w[i]);
+            k0 = abs_max2<T>(k0, p.w[i]);
+            if (TOPK == 2) k2 = abs_max2<T>(k2, abs_min2<T>(k1, a));
+            k1 = abs_max2<T>(k1, a);
+        }
+        uint32_t t0 = k0 & 0x7fffu, t1 = k1 & 0x7fffu, t2 = k2 & 0x7fffu;
+        auto merge = [&](uint32_t o0, uint32_t o1, uint32_t o2) {
+            if (TOPK == 2) t2 = max(max(t2, o2), max(min(t0, o1), min(t1, o0)));
+            t1 = max(max(t1, o1), min(t0, o0));
+            t0 = max(t0, o0);
+        };
+        merge(k0 >> 16 & 0x7fffu, k1 >> 16 & 0x7fffu, k2 >> 16 & 0x7fffu);
+        for (int off = lanes / 2; off > 0; off >>= 1) {
+            const uint32_t o = __shfl_xor_sync(0xffffffffu, t0 << 16 | t1, off, lanes);
+            merge(o >> 16, o & 0xffffu, TOPK == 2 ? __shfl_xor_sync(0xffffffffu, t2, off, lanes) : 0u);
+        }
+        g.stored = Src<T>::up(uint16_t(TOPK == 1 ? t1 : t2));
+        g.last_kept = Src<T>::up(uint16_t(TOPK == 1 ? t0 : t1));
+        g.finite = t0 < inf_bits<T>();
+    } else {
+        float t0 = 0.0f, t1 = 0.0f, t2 = 0.0f;
+        auto merge = [&](float o0, float o1, float o2) {
+            if (TOPK == 2) t2 = max3(t2, o2, fmaxf(fminf(t0, o1), fminf(t1, o0)));
+            t1 = max3(t1, o1, fminf(t0, o0));
+            t0 = max_nan(t0, o0);
+        };
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+            const float a = fabsf(__uint_as_float(p.w[i])), b = fabsf(__uint_as_float(p.w[i + 1]));
+            merge(max_nan(a, b), fminf(a, b), 0.0f);
+        }
+        for (int off = lanes / 2; off > 0; off >>= 1)
+            merge(__shfl_xor_sync(0xffffffffu, t0, off, lanes), __shfl_xor_sync(0xffffffffu, t1, off, lanes),
+                  TOPK == 2 ? __shfl_xor_sync(0xffffffffu, t2, off, lanes) : 0.0f);
+        g.stored = TOPK == 1 ? t1 : t2;
+        g.last_kept = TOPK == 1 ? t0 : t1;
+        g.finite = t0 < INFINITY;                                // false for NaN
+    }
+    return g;
+}
+
+// Is what a receiver has, the k kept elements verbatim and the others decoded, the same whichever of several equal magnitudes
+// are kept?  Everything above the scale is kept in any case, and
+//  - nothing else is, if the last kept magnitude is above the scale; or
+//  - what else is kept equals the scale, and its own code gives it back (16-bit types: T(L * (scale / L)) = scale for every
+//    scale that is not clamped); or
+//  - the scale is zero, and what else is kept is +0, like its decoded value.
+// Then the places need not be found, which took a key with index and sign through every comparison.
+template <typename T, int TOPK>
+__device__ __forceinline__ bool kept_by_magnitude(const GroupTop& g, const Packed16<T>& p, bool noise) {
+    bool ok = g.finite && (g.last_kept > g.stored || (sizeof(T) == 2 && !noise && g.stored >= 1.0e-6f));
+    if (__all_sync(0xffffffffu, ok)) return true;
+    if (!ok && g.finite && !noise && g.stored == 0.0f) {
+        bool minus = false;
+#pragma unroll
+        for (int i = 0; i < Packed16<T>::kWords; ++i) {
+            if (sizeof(T) == 2) minus = minus || (p.w[i] & 0xffffu) == 0x8000u || p.w[i] >> 16 == 0x8000u;
+            else minus = minus || p.w[i] == 0x80000000u;
+        }
+        ok = !minus;
+    }
+    return __all_sync(0xffffffffu, ok);
+}
+template <typename T>
+__device__ __forceinline__ void keep_above(Packed16<T>& y, const Packed16<T>& from, float stored) {
+    if constexpr (sizeof(T) == 2) {
+        const uint32_t scale = Src<T>::down2(stored, stored);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t m = abs_above2<T>(from.w[i], scale);
+            y.w[i] = (from.w[i] & m) | (y.w[i] & ~m);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (fabsf(__uint_as_float(from.w[i])) > stored) y.w[i] = from.w[i];
+    }
 }
 
 // Rounding parameters of one call.
@@ -915,6 +1050,15 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 4 : 3) roundtrip_ge
         for (int pass = 0; pass < p.passes; ++pass) {
             float v[16];
             unpack_elems<T>(y, v);
+            if constexpr (TOPK >= 1 && KIND != kBookNoise) {
+                const GroupTop top = top_of_group<T, TOPK>(y, lanes);
+                if (kept_by_magnitude<T, TOPK>(top, y, p.stochastic)) {
+                    const Packed16<T> from = y;
+                    y = requantize<T, KIND>(v, top.stored, true, rule, first, lut);
+                    keep_above<T>(y, from, top.stored);
+                    continue;
+                }
+            }
             const GroupMeta m = select_group<T, TOPK>(v, y, lane, lanes);
             const bool tame = __all_sync(0xffffffffu, m.tame);
             if (sizeof(T) == 2 && !tame) y = pack_elems<T>(v);          // a NaN that is kept has one pattern

@@ -728,3 +728,42 @@ def test_tensors_that_the_kernels_cannot_address_are_refused(ext, kw):
         comm.close()
         if created:
             dist.destroy_process_group()
+
+
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("bit,quant_type,topk,group", [(8, "linear", 1, 64), (8, "linear", 2, 16), (4, "linear", 1, 32),
+                                                       (4, "e2m1", 1, 64), (4, "normal", 2, 32)])
+@pytest.mark.parametrize("case", ("ties", "sparse", "minus zero", "tiny", "all"))
+def test_one_rank_pass_whichever_of_equal_magnitudes_is_kept(ext, dtype, bit, quant_type, topk, group, case):
+    """The pass keeps what is above the scale and looks for the places only where that could matter: equal magnitudes around the
+    last kept one, groups with fewer non-zero elements than are kept, zeros of both signs, scales below the clamp."""
+
+    cfg = _cfg(bit=bit, group_size=group, topk=topk, quant_type=quant_type)
+    n = 96 * group + 5
+    x = _data(n, torch.float32, seed=9)
+    for g in range(0, 96, 3):                                        # groups of every kind side by side in a warp
+        part = x[g * group:(g + 1) * group]
+        if case in ("ties", "all"):
+            top = part.abs().max()
+            part[1] = top
+            part[group // 2] = -top
+            if g % 2:
+                part[group - 1] = top
+                part[3] = top
+        if case == "sparse" or (case == "all" and g % 2):
+            part[:] = 0
+            part[g % group] = 0.25 if g % 4 else 0.0
+        if case == "minus zero" or (case == "all" and g % 5 == 0):
+            part[:] = 0
+            part[2 + g % 7] = -0.0
+            part[9] = 1e-3 if g % 2 else -0.0
+        if case == "tiny" or (case == "all" and g % 7 == 0):
+            part[:] = 0
+            part[4:8] = torch.tensor([2e-7, -2e-7, 1e-7, 3e-7 if g % 2 else 2e-7])
+    x = x.to(DTYPES[dtype])
+    y = x
+    for passes in (1, 2):
+        y = oracle.decode(oracle.encode(y, cfg), n, cfg, dtype)
+        out = torch.empty_like(x).cuda()
+        assert ext.roundtrip_general(x.cuda(), None, out, None, group, bit, topk, codec._QUANT_CODE[quant_type], False, 0, passes)
+        assert torch.equal(out.cpu().view(torch.uint8), y.view(torch.uint8)), passes
