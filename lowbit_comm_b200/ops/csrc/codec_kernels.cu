@@ -10,10 +10,10 @@
 // 16-byte vectors in both layouts, the whole-tile path free of bounds and alignment tests (their registers cost
 // occupancy); tensors and payloads off those boundaries have kernels of their own.
 // Measured on a B200 through the public calls, int8 groups of 64, before (grid-stride kernels of fast_kernels.cu) and
-// after: encode of 32 Mi bf16 elements with error feedback 47.0 -> 39.3 us (6.0 TB/s), decode of 128 Mi 94 -> 67.6 us
-// (6.0 TB/s), mean of eight payloads of 32 Mi with error feedback 107 -> 89.6 us (5.3 TB/s).  Those are passes repeated for
-// a second; in bursts of a few milliseconds the same calls take 38.9, 65.7 and 81 us: the mean of eight draws the card's
-// 1000 W, and its clock falls to 1.7 GHz.
+// after: encode of 32 Mi bf16 elements with error feedback 47.0 -> 39.2 us, decode of 128 Mi 94 -> 67.6 us, mean of eight payloads
+// of 32 Mi with error feedback 107 -> 89.8 us; then, each kernel started before the one ahead of it ends: 37.6 us (6.3 TB/s),
+// 65.7 us (6.2 TB/s) and 87.9 us (5.4 TB/s).  Those are passes repeated for a second; in bursts of a few milliseconds the mean of
+// eight takes 81 us: it draws the card's 1000 W, and its clock falls to 1.7 GHz.
 #include <type_traits>
 
 #include "codec_device.cuh"
@@ -91,6 +91,7 @@ constexpr int encode_span(bool compact) { return compact ? span_bytes(G, G * BIT
 // to turn, three blocks are as fast or faster (4 Mi elements into a payload on 8 bytes 8.3 -> 6.3 us).
 template <typename T, int G, int BIT, bool kCompact, bool kResidual, int U>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 && !kCompact && !kResidual ? 3 : 4) encode_kernel(const __grid_constant__ LbcQuantPush p) {
+    chain_wait();
     constexpr int lanes = G / kElemsPerThread;
     constexpr int tile_chunks = kThreads * U;
     const T* x = static_cast<const T*>(p.x);
@@ -130,6 +131,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 && !kCompact && !kRes
 // 46.3 / 43.1 us.
 template <typename T, int G, int BIT, bool kCompact>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 4) encode_ragged_kernel(const __grid_constant__ LbcQuantPush p) {
+    chain_wait();
     const int64_t chunks = (p.numel + G - 1) / G * (G / kElemsPerThread);
     __shared__ __align__(16) uint8_t spans[kThreads / 32][encode_span<G, BIT, T>(kCompact)];
     for (int64_t c0 = int64_t(blockIdx.x) * kThreads; c0 < chunks; c0 += int64_t(gridDim.x) * kThreads)
@@ -149,11 +151,11 @@ struct EncodeLauncher {
         const auto go = [&](auto compact) {
             constexpr bool kCompact = decltype(compact)::value;
             if (!on_boundary(32, p->x, p->residual, p->prepared_out, p->local_ef_out)) {
-                encode_ragged_kernel<T, G, BIT, kCompact><<<grid(one), kThreads, 0, stream>>>(*p);
+                launch_chained(encode_ragged_kernel<T, G, BIT, kCompact>, grid(one), stream, *p);
                 return;
             }
             if (p->residual != nullptr) {
-                encode_kernel<T, G, BIT, kCompact, true, 1><<<grid(one), kThreads, 0, stream>>>(*p);
+                launch_chained(encode_kernel<T, G, BIT, kCompact, true, 1>, grid(one), stream, *p);
                 return;
             }
             // Above one default grid.  Two chunks per thread, but for fp32 records, which gain nothing from them: those
@@ -164,15 +166,15 @@ struct EncodeLauncher {
             // 18.5 -> 18.3 us, 20 M 20.8 -> 20.6, 32 Mi 34.0 -> 30.9 (all with inputs beyond L2).
             if (one > lbc_default_max_blocks()) {
                 if constexpr (sizeof(T) == 2 || !kCompact) {
-                    encode_kernel<T, G, BIT, kCompact, false, 2><<<grid((one + 1) / 2), kThreads, 0, stream>>>(*p);
+                    launch_chained(encode_kernel<T, G, BIT, kCompact, false, 2>, grid((one + 1) / 2), stream, *p);
                     return;
                 }
                 if (p->max_blocks <= 0) {
-                    encode_kernel<T, G, BIT, kCompact, false, 1><<<lbc_default_max_blocks(), kThreads, 0, stream>>>(*p);
+                    launch_chained(encode_kernel<T, G, BIT, kCompact, false, 1>, lbc_default_max_blocks(), stream, *p);
                     return;
                 }
             }
-            encode_kernel<T, G, BIT, kCompact, false, 1><<<grid(one), kThreads, 0, stream>>>(*p);
+            launch_chained(encode_kernel<T, G, BIT, kCompact, false, 1>, grid(one), stream, *p);
         };
         if (p->mode == LBC_PUSH_COMPACT_LOCAL)
             go(std::true_type{});
@@ -291,6 +293,7 @@ __device__ __forceinline__ void decode_edge(const LbcReduce& p, int64_t chunk) {
 template <typename T, int G, int BIT, bool kCompact, int B>
 __global__ void __launch_bounds__(kThreads, B == 1 ? (sizeof(T) == 2 ? 8 : 6) : (kCompact || sizeof(T) == 4 ? 4 : 5))
 decode_kernel(const __grid_constant__ LbcReduce p) {
+    chain_wait();
     constexpr int lanes = G / kElemsPerThread;
     constexpr int VB = G * BIT / 8, MB = sizeof(T);
     T* out = static_cast<T*>(p.out);
@@ -350,6 +353,7 @@ decode_kernel(const __grid_constant__ LbcReduce p) {
 template <typename T, int G, int BIT, bool kCompact, bool kSeveral>
 __global__ void __launch_bounds__(kThreads, kSeveral && !(kCompact && BIT == 8 && sizeof(T) == 2) ? 6 : 5)
 decode_ragged_kernel(const __grid_constant__ LbcReduce p) {
+    chain_wait();
     const int64_t chunks = (p.numel + G - 1) / G * (G / kElemsPerThread);
     for (int64_t c0 = int64_t(blockIdx.x) * kThreads; c0 < chunks; c0 += int64_t(gridDim.x) * kThreads)
         decode_edge<T, G, BIT, kCompact, kFitRagged>(p, c0 + threadIdx.x);
@@ -369,16 +373,16 @@ struct DecodeLauncher {
                 vectors = vectors && on_boundary(kCompact ? 16 : kElemsPerThread * BIT / 8, p->src[r]);
             if (!vectors) {
                 if (p->num_src == 1 && p->residual_out == nullptr)
-                    decode_ragged_kernel<T, G, BIT, kCompact, false><<<grid, kThreads, 0, stream>>>(*p);
+                    launch_chained(decode_ragged_kernel<T, G, BIT, kCompact, false>, grid, stream, *p);
                 else
-                    decode_ragged_kernel<T, G, BIT, kCompact, true><<<grid, kThreads, 0, stream>>>(*p);
+                    launch_chained(decode_ragged_kernel<T, G, BIT, kCompact, true>, grid, stream, *p);
                 return;
             }
             // a compact payload takes two vectors per lane, so half as many are in flight
             if (p->num_src == 1 && p->residual_out == nullptr)
-                decode_kernel<T, G, BIT, kCompact, 1><<<grid, kThreads, 0, stream>>>(*p);
+                launch_chained(decode_kernel<T, G, BIT, kCompact, 1>, grid, stream, *p);
             else
-                decode_kernel<T, G, BIT, kCompact, kCompact ? 2 : 4><<<grid, kThreads, 0, stream>>>(*p);
+                launch_chained(decode_kernel<T, G, BIT, kCompact, kCompact ? 2 : 4>, grid, stream, *p);
         };
         if (p->compact)
             go(std::true_type{});

@@ -35,6 +35,33 @@ struct DeviceStatus {
 };
 
 // ---------------------------------------------------------------------------
+// kernels in a row
+// ---------------------------------------------------------------------------
+// A kernel launched with launch_chained starts while the last blocks of the one before it in the stream still run, and
+// waits in chain_wait() until that one is through and its stores are visible: its launch and the start of its blocks
+// are off the path (2 to 2.7 us per kernel: 13.1 M bf16 elements through the one-rank pass 10.2 -> 7.8 us, encode of 16 MiB
+// 8.3 -> 6.7, decode 8.0 -> 5.7).  All blocks of the first have started by then, so the early ones take no place
+// from it.  Only for kernels that wait for nobody else.  chain_wait comes before the first access to memory (constants and parameters aside), in every thread;
+// without the attribute it returns at once.
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename P>
+static cudaError_t launch_chained(void (*kernel)(const P), unsigned grid, cudaStream_t stream, const P& p) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(grid);
+    config.blockDim = dim3(kThreads);
+    config.stream = stream;
+    config.attrs = &attr;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernel, p);
+}
+
+// ---------------------------------------------------------------------------
 // dtype traits
 // ---------------------------------------------------------------------------
 template <typename T> struct Src;

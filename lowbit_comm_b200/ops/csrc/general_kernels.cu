@@ -24,7 +24,8 @@
 // busy, DRAM 41 %), and 81 -> 25 us for the code-book.  Then, with a look-up instead of fourteen thresholds: 24.5 -> 18.4 us for
 // the code-book; encode of 16 MiB, beyond L2, bf16 22.5 -> 14.5 us, fp32 14.0 -> 8.6, one-rank pass bf16 22.7 -> 14.5.
 // The one-rank pass without the places of the kept elements: 35.9 -> 30.8 us (32 Mi bf16 elements, one kept value); of 16 MiB
-// beyond L2, two kept values, bf16 14.4 -> 12.4 us, fp32 12.4 -> 10.3.
+// beyond L2, two kept values, bf16 14.4 -> 12.4 us, fp32 12.4 -> 10.3.  Each kernel started before the one ahead of it ends: 29.2 us, and
+// 15.4 us for the code-book.
 
 #include <cmath>
 #include <cstring>
@@ -821,6 +822,7 @@ __device__ __forceinline__ void put_meta(uint8_t* meta, const GroupMeta& m, int 
 
 template <typename T, int TOPK, int KIND>
 __global__ void __launch_bounds__(kThreads, 4) quant_general_kernel(const __grid_constant__ LbcQuantGeneral p) {
+    chain_wait();
     const GroupShape shape = GroupShape::of<T, TOPK, KIND>(p.group_size);
     const int lanes = shape.lanes, VB = shape.VB, MB = shape.MB;
     constexpr int CB = Kind<KIND>::CB;
@@ -916,6 +918,7 @@ __device__ __forceinline__ void load_lut(float (&lut)[16], int quant_type) {
 
 template <typename T, int TOPK, int KIND>
 __global__ void __launch_bounds__(kThreads, 4) dequant_general_kernel(const __grid_constant__ LbcDequantGeneral p) {
+    chain_wait();
     const GroupShape shape = GroupShape::of<T, TOPK, KIND>(p.group_size);
     const int lanes = shape.lanes, VB = shape.VB, MB = shape.MB;
     constexpr int CB = Kind<KIND>::CB;
@@ -1018,6 +1021,7 @@ __global__ void __launch_bounds__(kThreads) reduce_general_kernel(const __grid_c
 // the decoded values are rounded to T before the residual is taken, the rule of these profiles).
 template <typename T, int TOPK, int KIND>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 4 : 3) roundtrip_general_kernel(const __grid_constant__ LbcRoundtripGeneral p) {
+    chain_wait();
     const GroupShape shape = GroupShape::of<T, TOPK, KIND>(p.group_size);
     const int lanes = shape.lanes;
     __shared__ float lut[16];
@@ -1148,14 +1152,17 @@ template <typename T, int TOPK, int KIND>
 struct QuantGeneral {
     static constexpr bool noise = true;
     static void run(const LbcQuantGeneral& p, int grid, cudaStream_t s) {
-        quant_general_kernel<T, TOPK, KIND><<<grid, kThreads, 0, s>>>(p);
+        if (p.num_dst > 0)      // for other ranks, who are waited for
+            quant_general_kernel<T, TOPK, KIND><<<grid, kThreads, 0, s>>>(p);
+        else
+            launch_chained(quant_general_kernel<T, TOPK, KIND>, unsigned(grid), s, p);
     }
 };
 template <typename T, int TOPK, int KIND>
 struct DequantGeneral {
     static constexpr bool noise = false;
     static void run(const LbcDequantGeneral& p, int grid, cudaStream_t s) {
-        dequant_general_kernel<T, TOPK, KIND><<<grid, kThreads, 0, s>>>(p);
+        launch_chained(dequant_general_kernel<T, TOPK, KIND>, unsigned(grid), s, p);
     }
 };
 template <typename T, int TOPK, int KIND>
@@ -1169,7 +1176,7 @@ template <typename T, int TOPK, int KIND>
 struct RoundtripGeneral {
     static constexpr bool noise = true;
     static void run(const LbcRoundtripGeneral& p, int grid, cudaStream_t s) {
-        roundtrip_general_kernel<T, TOPK, KIND><<<grid, kThreads, 0, s>>>(p);
+        launch_chained(roundtrip_general_kernel<T, TOPK, KIND>, unsigned(grid), s, p);
     }
 };
 

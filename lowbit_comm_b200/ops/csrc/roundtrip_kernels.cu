@@ -13,7 +13,8 @@
 // flag.  A block per tile and no loop over tiles: on a B200 a persistent grid of the same kernel moved 5.9 TB/s where
 // the full grid moves 6.7-6.9, because the blocks of one wave end at different times and the next ones fill in.
 // Measured through the public calls (bf16, int8 groups of 64): 512 Mi elements 919 -> 312 us (6.9 TB/s), 13.1 M elements
-// 41.0 -> 10.2 us, 124 M elements in 7 buckets with error feedback 637 -> 183 us.
+// 41.0 -> 10.2 us, 124 M elements in 7 buckets with error feedback 637 -> 186 us; then, each kernel started before the one ahead
+// of it ends: 7.8 and 178 us.
 #include "codec_device.cuh"
 #include "common.cuh"
 #include "lbc_api.h"
@@ -85,6 +86,7 @@ __device__ __forceinline__ void roundtrip_edge(const LbcRoundtrip& p, int64_t ch
 // the first is computed.
 template <typename T, int G, int BIT, bool kResidual, int U>
 __global__ void __launch_bounds__(kThreads) roundtrip_kernel(const LbcRoundtrip p) {
+    chain_wait();
     constexpr int lanes = G / kElemsPerThread;
     constexpr int tile_chunks = kThreads * U;
     const T* x = static_cast<const T*>(p.x);
@@ -124,6 +126,7 @@ __global__ void __launch_bounds__(kThreads) roundtrip_kernel(const LbcRoundtrip 
 // input one element in (phases / that branch / here): bf16 176.7 / 182.0 / 42.6 us, fp32 156.4 / 190.9 / 95.0.
 template <typename T, int G, int BIT, bool kResidual>
 __global__ void __launch_bounds__(kThreads) roundtrip_ragged_kernel(const LbcRoundtrip p) {
+    chain_wait();
     const int64_t chunks = (p.numel + G - 1) / G * (G / kElemsPerThread);
     for (int64_t c0 = int64_t(blockIdx.x) * kThreads; c0 < chunks; c0 += int64_t(gridDim.x) * kThreads)
         roundtrip_edge<T, G, BIT, kResidual, kFitRagged>(p, c0 + threadIdx.x, chunks);
@@ -140,13 +143,13 @@ struct RoundtripLauncher {
         };
         if (!on_boundary(32, p->x, p->residual, p->out, p->residual_out)) {
             if (p->residual != nullptr)
-                roundtrip_ragged_kernel<T, G, BIT, true><<<grid(one), kThreads, 0, stream>>>(*p);
+                launch_chained(roundtrip_ragged_kernel<T, G, BIT, true>, grid(one), stream, *p);
             else
-                roundtrip_ragged_kernel<T, G, BIT, false><<<grid(one), kThreads, 0, stream>>>(*p);
+                launch_chained(roundtrip_ragged_kernel<T, G, BIT, false>, grid(one), stream, *p);
             return cudaGetLastError();
         }
         if (p->residual != nullptr) {
-            roundtrip_kernel<T, G, BIT, true, 1><<<grid(one), kThreads, 0, stream>>>(*p);
+            launch_chained(roundtrip_kernel<T, G, BIT, true, 1>, grid(one), stream, *p);
             return cudaGetLastError();
         }
         // Two chunks per thread (64 bytes in flight) once there are many waves of blocks.  One chunk against two, bf16: 2 M
@@ -155,11 +158,11 @@ struct RoundtripLauncher {
         // 256 M 158 / 152.  fp32 chunks and chunks with a residual have 64 bytes in flight already.
         if constexpr (sizeof(T) == 2) {
             if (one > 8 * lbc_default_max_blocks()) {
-                roundtrip_kernel<T, G, BIT, false, 2><<<grid((one + 1) / 2), kThreads, 0, stream>>>(*p);
+                launch_chained(roundtrip_kernel<T, G, BIT, false, 2>, grid((one + 1) / 2), stream, *p);
                 return cudaGetLastError();
             }
         }
-        roundtrip_kernel<T, G, BIT, false, 1><<<grid(one), kThreads, 0, stream>>>(*p);
+        launch_chained(roundtrip_kernel<T, G, BIT, false, 1>, grid(one), stream, *p);
         return cudaGetLastError();
     }
 };

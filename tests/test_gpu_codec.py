@@ -767,3 +767,49 @@ def test_one_rank_pass_whichever_of_equal_magnitudes_is_kept(ext, dtype, bit, qu
         out = torch.empty_like(x).cuda()
         assert ext.roundtrip_general(x.cuda(), None, out, None, group, bit, topk, codec._QUANT_CODE[quant_type], False, 0, passes)
         assert torch.equal(out.cpu().view(torch.uint8), y.view(torch.uint8)), passes
+
+
+@pytest.mark.parametrize("kw", [{}, {"compact": True}, {"topk": 1}, {"bit": 4, "quant_type": "e2m1"}])
+@pytest.mark.parametrize("n,skew", [(4099, 0), (300_001, 1), (3 << 20, 0)])
+def test_kernels_in_a_row_wait_for_each_other(ext, kw, n, skew):
+    """Kernels start while the one ahead of them still runs: calls that read what the call before wrote, in place and through
+    other buffers, beside kernels of torch, alone and captured in a graph, against the same calls one at a time."""
+
+    cfg = _cfg(**kw)
+    first = _data(n + skew, torch.bfloat16, seed=7).cuda()
+    state = {"x": first.clone()[skew:], "r": torch.zeros(n, dtype=torch.bfloat16, device="cuda"),
+             "y": torch.empty(n, dtype=torch.bfloat16, device="cuda")}
+    state["p"] = codec.quantize_tensor(state["x"], cfg)
+
+    def chain(pause):
+        for _ in range(3):
+            for call in (lambda: codec.quantize_tensor(state["x"], cfg, output=state["p"], residual=state["r"], prepared_out=state["r"]),
+                         lambda: codec.dequantize_tensor(state["p"], (n,), cfg, dtype="bf16", output=state["y"]),
+                         lambda: state["x"].add_(state["y"], alpha=0.25),
+                         lambda: codec.quantize_tensor(state["x"], cfg, output=state["p"]),
+                         lambda: codec.dequantize_tensor(state["p"], (n,), cfg, dtype="bf16", output=state["y"], reduce_op="sum"),
+                         lambda: state["x"].copy_(state["y"])):
+                call()
+                if pause:
+                    torch.cuda.synchronize()
+
+    def restart():
+        state["x"].copy_(first[skew:])
+        state["r"].zero_()
+        state["y"].zero_()
+
+    restart()
+    chain(pause=True)
+    want = {name: t.clone() for name, t in state.items()}
+    for _ in range(5):
+        restart()
+        chain(pause=False)
+        assert all(torch.equal(t, want[name]) for name, t in state.items())
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.graph(graph, stream=stream):
+        restart()
+        chain(pause=False)
+    for _ in range(5):
+        graph.replay()
+        assert all(torch.equal(t, want[name]) for name, t in state.items())
