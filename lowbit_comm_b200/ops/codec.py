@@ -46,6 +46,12 @@ def _numel_of(shape) -> int:
     return total
 
 
+def _whole(shape) -> bool:
+    """Is it a shape as the native call takes it?  (The general way converts what it is given, iterables and floats too.)"""
+
+    return type(shape) is torch.Size or (type(shape) in (tuple, list) and all(type(dim) is int for dim in shape))
+
+
 def _dense(tensor: torch.Tensor | None) -> torch.Tensor | None:
     """The tensor as the kernels take it: its elements in order, whatever its shape (a copy when it is strided)."""
 
@@ -120,6 +126,11 @@ def quantize_tensor(tensor: torch.Tensor, config: CompressionConfig, *,
     `residual`.  `metadata`, when a dict, is filled with the payload geometry.
     """
 
+    if metadata is None and extension_status is None and tensor.is_cuda and not config.stochastic:
+        done = require_extension().codec_encode(tensor, output, residual, prepared_out, config.group_size, config.bit,
+                                                config.topk, _QUANT_CODE[config.quant_type], config.compact)
+        if done is not None:
+            return done
     name = oracle.dtype_name(tensor)
     numel = tensor.numel()
     est = estimate_quantized_size(numel, dtype=name, config=config)
@@ -210,6 +221,11 @@ def dequantize_tensor(buffer: torch.Tensor, shape, config: CompressionConfig, *,
                       reduce_op: str = "none") -> torch.Tensor:
     """Decode one payload; `reduce_op="sum"` adds into `output` in the source dtype."""
 
+    if reduce_op == "none" and extension_status is None and buffer.is_cuda and dtype in _DTYPE_CODE and _whole(shape):
+        done = require_extension().codec_decode(buffer, shape, _DTYPE_CODE[dtype], output, config.group_size, config.bit,
+                                                config.topk, _QUANT_CODE[config.quant_type], config.compact)
+        if done is not None:
+            return done
     if reduce_op not in ("none", "sum"):
         raise ValueError(f"unsupported reduce_op {reduce_op!r}")
     name = resolve_dtype(dtype)

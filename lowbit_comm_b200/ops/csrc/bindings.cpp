@@ -351,6 +351,118 @@ void reduce_general(const Ptrs& src, at::Tensor& out, int group_size, int bit, i
     cuda_check(lbc_reduce_general(&p, at::cuda::getCurrentCUDAStream()), "lbc_reduce_general");
 }
 
+// ---- whole codec calls: sizes, checks, allocation and the launch in one crossing --------------------------------
+// The forms that jobs use all the time: dense tensors of one GPU, deterministic rounding.  Anything else (and everything
+// that is an error) gives None and launches nothing; the caller then goes the general way, which says what is wrong.
+bool plain(const at::Tensor& t, const at::Device& device) {
+    return t.is_cuda() && t.device() == device && t.layout() == at::kStrided && t.is_contiguous();
+}
+bool on_words(const at::Tensor& payload, int dtype) {
+    return (reinterpret_cast<uintptr_t>(payload.data_ptr()) & (dtype == LBC_FP32 ? 3 : 1)) == 0;
+}
+int64_t payload_bytes(int64_t numel, int64_t width, int group_size, int bit, int topk) {
+    return ceil_div(numel, group_size) * (group_size * bit / 8 + (topk == 0 ? 1 : topk + 2) * width);
+}
+
+std::optional<at::Tensor> codec_encode(const at::Tensor& x, const std::optional<at::Tensor>& output,
+                                       const std::optional<at::Tensor>& residual,
+                                       const std::optional<at::Tensor>& prepared_out, int group_size, int bit, int topk,
+                                       int quant_type, bool compact) {
+    const int64_t n = x.numel();
+    const at::ScalarType type = x.scalar_type();
+    if (n == 0 || (type != at::kBFloat16 && type != at::kHalf && type != at::kFloat) || !plain(x, x.device()))
+        return std::nullopt;
+    const auto like_x = [&](const std::optional<at::Tensor>& t) {
+        return !t.has_value() || (plain(*t, x.device()) && t->scalar_type() == type && t->numel() == n);
+    };
+    const int dtype = dtype_code(x);
+    const int64_t need = payload_bytes(n, x.element_size(), group_size, bit, topk);
+    if (!like_x(residual) || !like_x(prepared_out)) return std::nullopt;
+    if (output.has_value() && !(plain(*output, x.device()) && output->scalar_type() == at::kByte &&
+                                output->numel() == need && on_words(*output, dtype)))
+        return std::nullopt;
+    c10::cuda::CUDAGuard guard(x.device());
+    at::Tensor out = output.has_value() ? *output : at::empty({need}, at::TensorOptions().dtype(at::kByte).device(x.device()));
+    const void* res = residual.has_value() ? residual->data_ptr() : nullptr;
+    void* prep = prepared_out.has_value() ? prepared_out->data_ptr() : nullptr;
+    if (quant_type == LBC_LINEAR && topk == 0) {
+        LbcQuantPush p{};
+        p.dtype = dtype;
+        p.group_size = group_size;
+        p.bit = bit;
+        p.x = x.data_ptr();
+        p.residual = res;
+        p.prepared_out = prep;
+        p.numel = n;
+        p.mode = compact ? LBC_PUSH_COMPACT_LOCAL : LBC_PUSH_BROADCAST;
+        p.dst[0] = static_cast<uint8_t*>(out.data_ptr());
+        p.num_dst = 1;
+        p.layout_groups = ceil_div(n, group_size);
+        cuda_check(lbc_quant_push(&p, at::cuda::getCurrentCUDAStream()), "lbc_quant_push");
+    } else {
+        LbcQuantGeneral p{};
+        p.dtype = dtype;
+        p.group_size = group_size;
+        p.bit = bit;
+        p.topk = topk;
+        p.quant_type = quant_type;
+        p.compact = compact ? 1 : 0;
+        p.x = x.data_ptr();
+        p.residual = res;
+        p.prepared_out = prep;
+        p.numel = n;
+        p.out = static_cast<uint8_t*>(out.data_ptr());
+        cuda_check(lbc_quant_general(&p, at::cuda::getCurrentCUDAStream()), "lbc_quant_general");
+    }
+    return out;
+}
+
+std::optional<at::Tensor> codec_decode(const at::Tensor& payload, const std::vector<int64_t>& shape, int dtype,
+                                       const std::optional<at::Tensor>& output, int group_size, int bit, int topk,
+                                       int quant_type, bool compact) {
+    int64_t n = 1;
+    for (const int64_t d : shape) {
+        if (d <= 0 || n > (int64_t(1) << 40) / d) return std::nullopt;
+        n *= d;
+    }
+    const at::ScalarType type = dtype == LBC_FP16 ? at::kHalf : (dtype == LBC_BF16 ? at::kBFloat16 : at::kFloat);
+    if (!plain(payload, payload.device()) || payload.scalar_type() != at::kByte ||
+        payload.numel() != payload_bytes(n, dtype == LBC_FP32 ? 4 : 2, group_size, bit, topk) || !on_words(payload, dtype))
+        return std::nullopt;
+    if (output.has_value() && !(plain(*output, payload.device()) && output->scalar_type() == type &&
+                                output->sizes() == c10::IntArrayRef(shape)))
+        return std::nullopt;
+    c10::cuda::CUDAGuard guard(payload.device());
+    at::Tensor out = output.has_value() ? *output : at::empty(shape, at::TensorOptions().dtype(type).device(payload.device()));
+    if (quant_type == LBC_LINEAR && topk == 0) {
+        LbcReduce p{};
+        p.dtype = dtype;
+        p.group_size = group_size;
+        p.bit = bit;
+        p.num_src = 1;
+        p.src[0] = static_cast<const uint8_t*>(payload.data_ptr());
+        p.layout_groups = ceil_div(n, group_size);
+        p.compact = compact ? 1 : 0;
+        p.numel = n;
+        p.scale = 1.0f;
+        p.out = out.data_ptr();
+        cuda_check(lbc_reduce(&p, at::cuda::getCurrentCUDAStream()), "lbc_reduce");
+    } else {
+        LbcDequantGeneral p{};
+        p.dtype = dtype;
+        p.group_size = group_size;
+        p.bit = bit;
+        p.topk = topk;
+        p.quant_type = quant_type;
+        p.compact = compact ? 1 : 0;
+        p.numel = n;
+        p.src = static_cast<const uint8_t*>(payload.data_ptr());
+        p.out = out.data_ptr();
+        cuda_check(lbc_dequant_general(&p, at::cuda::getCurrentCUDAStream()), "lbc_dequant_general");
+    }
+    return out;
+}
+
 void error_feedback_update(const at::Tensor& prepared, const at::Tensor& restored, at::Tensor& residual) {
     check_dense(prepared, "prepared");
     check_dense(restored, "restored");
@@ -456,6 +568,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           py::arg("topk"), py::arg("quant_type"), py::arg("compact"), py::arg("scale"), py::arg("prepared") = py::none(),
           py::arg("residual_out") = py::none(), py::arg("wait") = py::none(), py::arg("max_blocks") = 0,
           py::arg("layout_groups") = 0, py::arg("src_shard_groups") = 0);
+    m.def("codec_encode", &codec_encode);
+    m.def("codec_decode", &codec_decode);
     m.def("error_feedback_update", &error_feedback_update);
     m.def("scale_inplace", &scale_inplace);
     m.def("push_bytes", &push_bytes, py::arg("src"), py::arg("nbytes"), py::arg("dst"), py::arg("wait") = py::none(),

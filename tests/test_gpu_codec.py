@@ -813,3 +813,82 @@ def test_kernels_in_a_row_wait_for_each_other(ext, kw, n, skew):
     for _ in range(5):
         graph.replay()
         assert all(torch.equal(t, want[name]) for name, t in state.items())
+
+
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("kw", [{}, {"compact": True}, {"topk": 2}, {"bit": 4, "quant_type": "e3m0", "compact": True}])
+def test_native_codec_calls_and_the_general_way(ext, dtype, kw, monkeypatch):
+    """The calls that settle everything natively give what the general way gives, for every form of argument that they take, and
+    leave the others to it: the same calls with the native ones taken away."""
+
+    from lowbit_comm_b200.ops.loader import load_cuda_extension
+
+    cfg, torch_dtype, other = _cfg(**kw), DTYPES[dtype], "fp16" if dtype == "fp32" else "fp32"
+    size = lambda n: codec.estimate_quantized_size(n, dtype=dtype, config=cfg).quantized_bytes
+    base = _data(3 * 4160, torch_dtype, seed=4).cuda()
+    bytes_ = torch.zeros(2 * size(4160) + 8, dtype=torch.uint8, device="cuda")
+    x, r = base[:4099], base[4160:8259] * 0.01
+    whole = codec.quantize_tensor(x, cfg)
+    encodes = {
+        "plain": lambda: codec.quantize_tensor(x, cfg),
+        "shaped": lambda: codec.quantize_tensor(base[:4096].view(16, 256), cfg),
+        "view off its vectors": lambda: codec.quantize_tensor(base[1:4100], cfg),
+        "transposed": lambda: codec.quantize_tensor(base[:4096].view(64, 64).t(), cfg),
+        "one stride": lambda: codec.quantize_tensor(base[:8198:2], cfg),
+        "empty": lambda: codec.quantize_tensor(base[:0], cfg),
+        "residual": lambda: codec.quantize_tensor(x, cfg, residual=r),
+        "strided residual": lambda: codec.quantize_tensor(x, cfg, residual=base[:8198:2]),
+        "output": lambda: codec.quantize_tensor(x, cfg, output=bytes_[4:4 + size(4099)]),
+        "output off its words": lambda: codec.quantize_tensor(x, cfg, output=bytes_[1:1 + size(4099)]),
+        "output too small": lambda: codec.quantize_tensor(x, cfg, output=bytes_[:8]),
+        "output of floats": lambda: codec.quantize_tensor(x, cfg, output=r),
+        "residual of another type": lambda: codec.quantize_tensor(x, cfg, residual=r.to(DTYPES[other])),
+        "residual too short": lambda: codec.quantize_tensor(x, cfg, residual=r[:-1]),
+        "residual on the host": lambda: codec.quantize_tensor(x, cfg, residual=r.cpu()),
+        "whole numbers": lambda: codec.quantize_tensor(torch.ones(64, dtype=torch.int32, device="cuda"), cfg),
+        "prepared": lambda: torch.cat([codec.quantize_tensor(x, cfg, residual=r, prepared_out=(p := torch.empty_like(x))).float(), p.float()]),
+    }
+    decodes = {
+        "plain": lambda: codec.dequantize_tensor(whole, (4099,), cfg, dtype=dtype),
+        "a list": lambda: codec.dequantize_tensor(whole, [4099, 1], cfg, dtype=dtype),
+        "a size": lambda: codec.dequantize_tensor(whole, x.shape, cfg, dtype=dtype),
+        "floats": lambda: codec.dequantize_tensor(whole, (4099.0,), cfg, dtype=dtype),
+        "an iterator": lambda: codec.dequantize_tensor(whole, np.array([4099]), cfg, dtype=dtype),
+        "negative": lambda: codec.dequantize_tensor(whole, (-4099, -1), cfg, dtype=dtype),
+        "empty": lambda: codec.dequantize_tensor(bytes_[:0], (0, 3), cfg, dtype=dtype),
+        "output": lambda: codec.dequantize_tensor(whole, (4099,), cfg, dtype=dtype, output=torch.empty_like(x)),
+        "output of another shape": lambda: codec.dequantize_tensor(whole, (1, 4099), cfg, dtype=dtype, output=torch.empty_like(x)),
+        "output of another type": lambda: codec.dequantize_tensor(whole, (4099,), cfg, dtype=dtype, output=torch.empty_like(x, dtype=DTYPES[other])),
+        "strided output": lambda: codec.dequantize_tensor(whole, (4099,), cfg, dtype=dtype, output=base[:8198:2].clone().as_strided((4099,), (1,))),
+        "sum": lambda: codec.dequantize_tensor(whole, (4099,), cfg, dtype=dtype, output=r.clone(), reduce_op="sum"),
+        "payload too short": lambda: codec.dequantize_tensor(whole[:-2], (4099,), cfg, dtype=dtype),
+        "unknown type": lambda: codec.dequantize_tensor(whole, (4099,), cfg, dtype="int8"),
+        "unknown reduction": lambda: codec.dequantize_tensor(whole, (4099,), cfg, dtype=dtype, reduce_op="max"),
+        "type of its own": lambda: codec.dequantize_tensor(whole, (4099,), cfg, dtype="auto"),
+    }
+
+    def outcome(call):
+        try:
+            result = call()
+        except Exception as error:  # noqa: BLE001
+            return type(error)
+        return result.shape, result.dtype, result.contiguous().view(torch.uint8).cpu().numpy().tobytes()
+
+    native = {name: outcome(call) for calls in (encodes, decodes) for name, call in calls.items()}
+    taken = {"encode": 0, "decode": 0}
+
+    class General:
+        def __getattr__(self, name):
+            return getattr(ext, name)
+
+        def codec_encode(self, *args):
+            taken["encode"] += ext.codec_encode(*args) is not None
+
+        def codec_decode(self, *args):
+            taken["decode"] += ext.codec_decode(*args) is not None
+
+    monkeypatch.setattr(codec, "require_extension", lambda status=None: General())
+    assert load_cuda_extension().available
+    general = {name: outcome(call) for calls in (encodes, decodes) for name, call in calls.items()}
+    assert {name for name in native if native[name] != general[name]} == set()
+    assert taken["encode"] >= 5 and taken["decode"] >= 4
