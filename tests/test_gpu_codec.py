@@ -892,3 +892,26 @@ def test_native_codec_calls_and_the_general_way(ext, dtype, kw, monkeypatch):
     general = {name: outcome(call) for calls in (encodes, decodes) for name, call in calls.items()}
     assert {name for name in native if native[name] != general[name]} == set()
     assert taken["encode"] >= 5 and taken["decode"] >= 4
+
+
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("bit,quant_type,topk,group,compact", [
+    (8, "linear", 1, 64, False), (8, "linear", 2, 16, True), (4, "linear", 1, 32, True), (4, "normal", 0, 16, False),
+    (4, "e2m1", 2, 64, True), (4, "uniform", 1, 32, False)])
+def test_general_encode_at_tile_edges(ext, dtype, bit, quant_type, topk, group, compact):
+    """Sizes around a block's 4096 elements, each tensor on and off its vectors, payloads on 16, 8 and 4 bytes: the kernel of whole
+    tiles, its last tile and the kernel of payloads off their vectors."""
+
+    cfg = _cfg(bit=bit, group_size=group, topk=topk, quant_type=quant_type, compact=compact)
+    for n in (4096 - 1, 4096, 4096 + 1, 3 * 4096 + group + 5, 2 * 4096 - group, 7):
+        x, r = _data(n, DTYPES[dtype], seed=n), _data(n, DTYPES[dtype], seed=n + 1, outliers=False)
+        want, prepared = oracle.encode(x, cfg, residual=r), oracle.prepare(x, r)
+        for where, skew in ((0, (0, 0, 0)), (16, (16, 0, 0)), (8, (1, 0, 0)), (4, (0, 3, 0)), (0, (0, 0, 8)), (16, (5, 1, 2))):
+            at = [torch.zeros(n + 16, dtype=DTYPES[dtype], device="cuda")[s:s + n] for s in skew]
+            at[0].copy_(x)
+            at[1].copy_(r)
+            raw = torch.full((want.numel() + 48,), 0xAB, dtype=torch.uint8, device="cuda")
+            codec.quantize_tensor(at[0], cfg, output=raw[where:where + want.numel()], residual=at[1], prepared_out=at[2])
+            assert torch.equal(raw[where:where + want.numel()].cpu(), want), (n, where, skew)
+            assert bool((raw[:where] == 0xAB).all()) and bool((raw[where + want.numel():] == 0xAB).all())
+            assert torch.equal(at[2].cpu().view(torch.uint8), prepared.view(torch.uint8)), (n, where, skew)
