@@ -12,7 +12,7 @@
 // Measured on a B200 through the public calls, int8 groups of 64, before (grid-stride kernels of fast_kernels.cu) and
 // after: encode of 32 Mi bf16 elements with error feedback 47.0 -> 39.2 us, decode of 128 Mi 94 -> 67.6 us, mean of eight payloads
 // of 32 Mi with error feedback 107 -> 89.8 us; then, each kernel started before the one ahead of it ends: 37.6 us (6.3 TB/s),
-// 65.7 us (6.2 TB/s) and 87.9 us (5.4 TB/s).  Those are passes repeated for a second; in bursts of a few milliseconds the mean of
+// 65.7 us (6.2 TB/s) and 84.2 us (5.7 TB/s).  Those are passes repeated for a second; in bursts of a few milliseconds the mean of
 // eight takes 81 us: it draws the card's 1000 W, and its clock falls to 1.7 GHz.
 #include <type_traits>
 
@@ -187,19 +187,29 @@ struct EncodeLauncher {
 // ---------------------------------------------------------------------------
 // decode and reduce
 // ---------------------------------------------------------------------------
-// acc += one payload's 16 values: fma(code, scale / L, acc), one rounding per payload.
-template <typename T, int BIT>
+// acc += one payload's 16 values: fma(code, scale / L, acc), one rounding per payload.  kPairs: two of them to an instruction
+// (sm_100+) and the quotient without a branch.  Several payloads draw the card's power limit, so instructions are time; one
+// payload alone is 3 % slower with it (128 Mi bf16 elements 63.6 -> 65.7 us); the mean of eight of 32 Mi 86.5 -> 84.2.
+template <typename T, int BIT, bool kPairs>
 __device__ __forceinline__ void add_payload(float (&acc)[16], uint4 codes, float scale) {
-    const float step = scale / (BIT == 8 ? 127.0f : 7.0f);
     float d[16];
     codes16<T, BIT>(codes, d);
+    if constexpr (kPairs) {
+        const float step = over_limit<BIT == 8 ? 127 : 7>(scale);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) acc[i] = __fmaf_rn(d[i], step, acc[i]);
+        for (int i = 0; i < 16; i += 2)
+            asm("{.reg .b64 a, b, c; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %4}; mov.b64 c, {%0, %1}; fma.rn.f32x2 c, a, b, c; mov.b64 {%0, %1}, c;}"
+                : "+f"(acc[i]), "+f"(acc[i + 1]) : "f"(d[i]), "f"(d[i + 1]), "f"(step));
+    } else {
+        const float step = scale / (BIT == 8 ? 127.0f : 7.0f);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[i] = __fmaf_rn(d[i], step, acc[i]);
+    }
 }
 
 // Adds payloads r0 .. r0 + K - 1 to a thread's chunk; all K loads are issued before the first is decoded.  Whole warps
 // of whole groups, vector-aligned payloads.  Compact: the warp's span comes in as vectors and turns through `span`.
-template <typename T, int G, int BIT, bool kCompact, int K>
+template <typename T, int G, int BIT, bool kCompact, int K, bool kPairs>
 __device__ __forceinline__ void add_batch(const LbcReduce& p, int r0, int64_t chunk, uint8_t* span, float (&acc)[16]) {
     constexpr int lanes = G / kElemsPerThread;
     constexpr int VB = G * BIT / 8, MB = sizeof(T), CB = kElemsPerThread * BIT / 8;
@@ -221,7 +231,7 @@ __device__ __forceinline__ void add_batch(const LbcReduce& p, int r0, int64_t ch
             scale[j] = load_scale<T>(src + soff);
         }
 #pragma unroll
-        for (int j = 0; j < K; ++j) add_payload<T, BIT>(acc, codes[j], scale[j]);
+        for (int j = 0; j < K; ++j) add_payload<T, BIT, kPairs>(acc, codes[j], scale[j]);
     } else {
         constexpr int full = span_bytes(G, VB + MB);            // 17 to 40 vectors
         const int wlane = threadIdx.x & 31;
@@ -243,7 +253,7 @@ __device__ __forceinline__ void add_batch(const LbcReduce& p, int r0, int64_t ch
             span_get_codes<CB>(rec + lane * CB, w);
             const float scale = load_scale<T>(rec + VB);
             __syncwarp();
-            add_payload<T, BIT>(acc, make_uint4(w[0], w[1], w[2], w[3]), scale);
+            add_payload<T, BIT, kPairs>(acc, make_uint4(w[0], w[1], w[2], w[3]), scale);
         }
     }
 }
@@ -266,7 +276,7 @@ __device__ __forceinline__ void decode_edge(const LbcReduce& p, int64_t chunk) {
     for (int i = 0; i < 16; ++i) acc[i] = 0.0f;
 #pragma unroll 2
     for (int r = 0; r < p.num_src; ++r)
-        add_payload<T, BIT>(acc, load_codes(p.src[r] + voff, CB), load_scale<T>(p.src[r] + soff));
+        add_payload<T, BIT, false>(acc, load_codes(p.src[r] + voff, CB), load_scale<T>(p.src[r] + soff));
 #pragma unroll
     for (int i = 0; i < 16; ++i) acc[i] *= p.scale;
     if (rout != nullptr) {
@@ -317,11 +327,11 @@ decode_kernel(const __grid_constant__ LbcReduce p) {
         Raw16<T> held;
         if (B > 1 && rout != nullptr) held = raw16(prep + first);      // on its way while the payloads are summed
         int r = 0;
-        for (; r + B <= R; r += B) add_batch<T, G, BIT, kCompact, B>(p, r, chunk, span, acc);
+        for (; r + B <= R; r += B) add_batch<T, G, BIT, kCompact, B, (B > 1)>(p, r, chunk, span, acc);
         if constexpr (B > 2)
-            for (; r + 2 <= R; r += 2) add_batch<T, G, BIT, kCompact, 2>(p, r, chunk, span, acc);
+            for (; r + 2 <= R; r += 2) add_batch<T, G, BIT, kCompact, 2, true>(p, r, chunk, span, acc);
         if constexpr (B > 1)
-            for (; r < R; ++r) add_batch<T, G, BIT, kCompact, 1>(p, r, chunk, span, acc);
+            for (; r < R; ++r) add_batch<T, G, BIT, kCompact, 1, true>(p, r, chunk, span, acc);
 #pragma unroll
         for (int i = 0; i < 16; ++i) acc[i] *= p.scale;
         if (B > 1 && rout != nullptr) {

@@ -12,6 +12,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 
 #include "lbc_api.h"
@@ -419,6 +420,15 @@ __device__ __forceinline__ uint32_t quant_bits(float v, float mul) {
     float r = __fadd_rn(__fmul_rn(v, mul), kRoundMagic);
     r = fminf(fmaxf(r, kRoundMagic - float(LIM)), kRoundMagic + float(LIM));
     return __float_as_uint(r);
+}
+// s / LIM, correctly rounded (every finite s was tried): the product with 1 / LIM and one Newton correction by its exact
+// remainder, five instructions and no branch.
+template <int LIM>
+__device__ __forceinline__ float over_limit(float s) {
+    constexpr float inverse = 1.0f / float(LIM);
+    const float q = __fmul_rn(s, inverse);
+    const float t = __fmaf_rn(__fmaf_rn(-q, float(LIM), s), inverse, q);
+    return fabsf(s) < INFINITY ? t : q;
 }
 __device__ __forceinline__ int code_of_bits(uint32_t bits) { return int(bits) - 0x4B400000; }
 
