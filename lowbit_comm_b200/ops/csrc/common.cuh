@@ -398,6 +398,21 @@ inline bool on_boundary(uintptr_t bytes, const void* a, const void* b = nullptr,
              reinterpret_cast<uintptr_t>(d)) & (bytes - 1)) == 0;
 }
 
+// 16 floats, two to an instruction (sm_100+), with the roundings of the scalar forms.  Never a packed product before a packed sum: the
+// assembler contracts the two, although both ask for a rounding of their own.
+__device__ __forceinline__ void mul16(float (&v)[16], float s) {
+#pragma unroll
+    for (int i = 0; i < 16; i += 2)
+        asm("{.reg .b64 a, b; mov.b64 a, {%0, %1}; mov.b64 b, {%2, %2}; mul.rn.f32x2 a, a, b; mov.b64 {%0, %1}, a;}"
+            : "+f"(v[i]), "+f"(v[i + 1]) : "f"(s));
+}
+__device__ __forceinline__ void add16(float (&v)[16], float s) {
+#pragma unroll
+    for (int i = 0; i < 16; i += 2)
+        asm("{.reg .b64 a, b; mov.b64 a, {%0, %1}; mov.b64 b, {%2, %2}; add.rn.f32x2 a, a, b; mov.b64 {%0, %1}, a;}"
+            : "+f"(v[i]), "+f"(v[i + 1]) : "f"(s));
+}
+
 // prepared = T(x + residual)
 template <typename T>
 __device__ __forceinline__ void compensate16(float (&v)[16], const float (&r)[16]) {

@@ -25,7 +25,8 @@
 // the code-book; encode of 16 MiB, beyond L2, bf16 22.5 -> 14.5 us, fp32 14.0 -> 8.6, one-rank pass bf16 22.7 -> 14.5.
 // The one-rank pass without the places of the kept elements: 35.9 -> 30.8 us (32 Mi bf16 elements, one kept value); of 16 MiB
 // beyond L2, two kept values, bf16 14.4 -> 12.4 us, fp32 12.4 -> 10.3.  Each kernel started before the one ahead of it ends: 29.2 us, and
-// 15.4 us for the code-book.
+// 15.4 us for the code-book.  The rare warps of the one-rank pass out of line, its group steps without loops, its sums and products two
+// to an instruction, 32 Mi elements beyond L2: bf16 29.6 -> 26.6 us, two kept values 30.6 -> 28.2, fp16 in 4 bits 29.1 -> 26.4.
 
 #include <cmath>
 #include <cstring>
@@ -423,6 +424,13 @@ struct GroupTop {
     float stored, last_kept;
     bool finite;               // no infinity and no NaN in the group
 };
+// Calls `step` with the distances of a butterfly over a group's `lanes` threads (no loop, no width: the partner of a thread
+// of an aligned group is in it anyway).
+template <typename Step>
+__device__ __forceinline__ void over_group(int lanes, const Step& step) {
+    if (lanes >= 4) step(2);
+    if (lanes >= 2) step(1);
+}
 template <typename T, int TOPK>
 __device__ __forceinline__ GroupTop top_of_group(const Packed16<T>& p, int lanes) {
     static_assert(TOPK == 1 || TOPK == 2, "two or three magnitudes");
@@ -443,10 +451,10 @@ __device__ __forceinline__ GroupTop top_of_group(const Packed16<T>& p, int lanes
             t0 = max(t0, o0);
         };
         merge(k0 >> 16 & 0x7fffu, k1 >> 16 & 0x7fffu, k2 >> 16 & 0x7fffu);
-        for (int off = lanes / 2; off > 0; off >>= 1) {
-            const uint32_t o = __shfl_xor_sync(0xffffffffu, t0 << 16 | t1, off, lanes);
-            merge(o >> 16, o & 0xffffu, TOPK == 2 ? __shfl_xor_sync(0xffffffffu, t2, off, lanes) : 0u);
-        }
+        over_group(lanes, [&](int off) {
+            const uint32_t o = __shfl_xor_sync(0xffffffffu, t0 << 16 | t1, off);
+            merge(o >> 16, o & 0xffffu, TOPK == 2 ? __shfl_xor_sync(0xffffffffu, t2, off) : 0u);
+        });
         g.stored = Src<T>::up(uint16_t(TOPK == 1 ? t1 : t2));
         g.last_kept = Src<T>::up(uint16_t(TOPK == 1 ? t0 : t1));
         g.finite = t0 < inf_bits<T>();
@@ -462,9 +470,10 @@ __device__ __forceinline__ GroupTop top_of_group(const Packed16<T>& p, int lanes
             const float a = fabsf(__uint_as_float(p.w[i])), b = fabsf(__uint_as_float(p.w[i + 1]));
             merge(max_nan(a, b), fminf(a, b), 0.0f);
         }
-        for (int off = lanes / 2; off > 0; off >>= 1)
-            merge(__shfl_xor_sync(0xffffffffu, t0, off, lanes), __shfl_xor_sync(0xffffffffu, t1, off, lanes),
-                  TOPK == 2 ? __shfl_xor_sync(0xffffffffu, t2, off, lanes) : 0.0f);
+        over_group(lanes, [&](int off) {
+            merge(__shfl_xor_sync(0xffffffffu, t0, off), __shfl_xor_sync(0xffffffffu, t1, off),
+                  TOPK == 2 ? __shfl_xor_sync(0xffffffffu, t2, off) : 0.0f);
+        });
         g.stored = TOPK == 1 ? t1 : t2;
         g.last_kept = TOPK == 1 ? t0 : t1;
         g.finite = t0 < INFINITY;                                // false for NaN
@@ -614,15 +623,16 @@ __device__ __forceinline__ void encode_general(const float (&v)[16], float store
         float t[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) t[i] = __fmul_rn(v[i], mul);
+        if (tame && !rule.stochastic) {
+            add16(t, kRoundMagic);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) b[i] = __float_as_uint(t[i]);
+            return;
+        }
         if (rule.stochastic) {      // two roundings, the product's and the sum's, as the oracle has it
 #pragma unroll
             for (int i = 0; i < 16; ++i)
                 t[i] = __fadd_rn(t[i], uniform01(rule.seed, (unsigned long long)(first + i)) - 0.5f);
-        }
-        if (tame && !rule.stochastic) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) b[i] = __float_as_uint(__fadd_rn(t[i], kRoundMagic));
-            return;
         }
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
@@ -725,11 +735,15 @@ __device__ __forceinline__ Packed16<T> decode_codes(const uint32_t (&w)[4], floa
 // The same from the patterns of encode_general, without a trip through packed bytes.
 template <typename T, int KIND>
 __device__ __forceinline__ Packed16<T> decode_bits(const uint32_t (&b)[16], float stored, const float* lut) {
-    const float step = Kind<KIND>::book ? stored : stored / float(Kind<KIND>::lim);
     float d[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i)
-        d[i] = __fmul_rn(Kind<KIND>::book ? lut[b[i] & 0xfu] : __uint_as_float(b[i]) - kRoundMagic, step);
+    for (int i = 0; i < 16; ++i) d[i] = Kind<KIND>::book ? lut[b[i] & 0xfu] : __uint_as_float(b[i]);
+    if constexpr (Kind<KIND>::book) {
+        mul16(d, stored);
+    } else {
+        add16(d, -kRoundMagic);
+        mul16(d, over_limit<Kind<KIND>::lim>(stored));
+    }
     return pack_elems<T>(d);
 }
 
@@ -1066,10 +1080,39 @@ __global__ void __launch_bounds__(kThreads) reduce_general_kernel(const __grid_c
     }
 }
 
+// 16 elements -> what a receiver has of them, with the places of the kept ones.  Convergent.
+template <typename T, int TOPK, int KIND>
+__device__ __forceinline__ Packed16<T> place_and_requantize(Packed16<T> y, int lane, int lanes, const CodeRule& rule,
+                                                            int64_t first, const float* lut) {
+    float v[16];
+    unpack_elems<T>(y, v);
+    const GroupMeta m = select_group<T, TOPK>(v, y, lane, lanes);
+    const bool tame = __all_sync(0xffffffffu, m.tame);
+    if (sizeof(T) == 2 && !tame) y = pack_elems<T>(v);          // a NaN that is kept has one pattern
+    const Packed16<T> from = y;
+    y = requantize<T, KIND>(v, m.stored, tame, rule, first, lut);
+#pragma unroll
+    for (int j = 0; j < TOPK; ++j) copy_elem<T>(y, from, int(uint32_t(m.idx[j]) & 0xffu) - lane * 16);
+    return y;
+}
+// The same out of line, for the few warps of a 16-bit pass that need it: inline it cost every warp of them its registers.
+template <typename T, int TOPK, int KIND>
+__device__ __noinline__ void requantize_by_place(uint32_t* words, int lane, int lanes, const LbcRoundtripGeneral& p,
+                                                 int64_t first, const float* lut) {
+    const CodeRule rule = CodeRule::of<KIND>(p.book, p.quant_type, p.stochastic, p.seed);
+    Packed16<T> y;
+#pragma unroll
+    for (int i = 0; i < Packed16<T>::kWords; ++i) y.w[i] = words[i];
+    y = place_and_requantize<T, TOPK, KIND>(y, lane, lanes, rule, first, lut);
+#pragma unroll
+    for (int i = 0; i < Packed16<T>::kWords; ++i) words[i] = y.w[i];
+}
+
 // The all-reduce of a group of one rank: encode and decode in registers, no payload (see roundtrip_kernels.cu; here
 // the decoded values are rounded to T before the residual is taken, the rule of these profiles).
 template <typename T, int TOPK, int KIND>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 4 : 3) roundtrip_general_kernel(const __grid_constant__ LbcRoundtripGeneral p) {
+    constexpr bool by_magnitude = TOPK >= 1 && KIND != kBookNoise;
     chain_wait();
     const GroupShape shape = GroupShape::of<T, TOPK, KIND>(p.group_size);
     const int lanes = shape.lanes;
@@ -1101,24 +1144,27 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? 4 : 3) roundtrip_ge
         }
         Packed16<T> y = elems;
         for (int pass = 0; pass < p.passes; ++pass) {
-            float v[16];
-            unpack_elems<T>(y, v);
-            if constexpr (TOPK >= 1 && KIND != kBookNoise) {
+            if constexpr (by_magnitude) {
                 const GroupTop top = top_of_group<T, TOPK>(y, lanes);
                 if (kept_by_magnitude<T, TOPK>(top, y, p.stochastic)) {
+                    float v[16];
+                    unpack_elems<T>(y, v);
                     const Packed16<T> from = y;
                     y = requantize<T, KIND>(v, top.stored, true, rule, first, lut);
                     keep_above<T>(y, from, top.stored);
-                    continue;
-                }
-            }
-            const GroupMeta m = select_group<T, TOPK>(v, y, lane, lanes);
-            const bool tame = __all_sync(0xffffffffu, m.tame);
-            if (sizeof(T) == 2 && !tame) y = pack_elems<T>(v);          // a NaN that is kept has one pattern
-            const Packed16<T> from = y;
-            y = requantize<T, KIND>(v, m.stored, tame, rule, first, lut);
+                } else if constexpr (sizeof(T) == 4) {
+                    y = place_and_requantize<T, TOPK, KIND>(y, lane, lanes, rule, first, lut);
+                } else {
+                    uint32_t words[Packed16<T>::kWords];
 #pragma unroll
-            for (int j = 0; j < TOPK; ++j) copy_elem<T>(y, from, int(uint32_t(m.idx[j]) & 0xffu) - lane * 16);
+                    for (int i = 0; i < Packed16<T>::kWords; ++i) words[i] = y.w[i];
+                    requantize_by_place<T, TOPK, KIND>(words, lane, lanes, p, first, lut);
+#pragma unroll
+                    for (int i = 0; i < Packed16<T>::kWords; ++i) y.w[i] = words[i];
+                }
+            } else {
+                y = place_and_requantize<T, TOPK, KIND>(y, lane, lanes, rule, first, lut);
+            }
         }
         if (!live) continue;
         if (rout != nullptr) {
