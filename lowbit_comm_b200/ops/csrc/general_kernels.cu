@@ -979,8 +979,9 @@ __device__ __forceinline__ void load_lut(float (&lut)[16], int quant_type) {
     }
 }
 
-template <typename T, int TOPK, int KIND>
-__global__ void __launch_bounds__(kThreads, 4) dequant_general_kernel(const __grid_constant__ LbcDequantGeneral p) {
+// kMayAdd: with p.accumulate, out = T(out + decode).
+template <typename T, int TOPK, int KIND, bool kMayAdd, int kBlocks>
+__global__ void __launch_bounds__(kThreads, kBlocks) dequant_general_kernel(const __grid_constant__ LbcDequantGeneral p) {
     chain_wait();
     const GroupShape shape = GroupShape::of<T, TOPK, KIND>(p.group_size);
     const int lanes = shape.lanes, VB = shape.VB, MB = shape.MB;
@@ -1006,7 +1007,7 @@ __global__ void __launch_bounds__(kThreads, 4) dequant_general_kernel(const __gr
         uint32_t w[4];
         load_code_words<KIND>(vptr + lane * CB, w, c_vec);
         Packed16<T> d = decode_group<T, TOPK, KIND>(w, meta, lane, lut);
-        if (p.accumulate) {
+        if (kMayAdd && p.accumulate) {
             float a[16], b[16];
             unpack_elems<T>(d, a);
             unpack_elems<T>(load_elems<T>(out, first, n, o_vec), b);
@@ -1262,7 +1263,17 @@ template <typename T, int TOPK, int KIND>
 struct DequantGeneral {
     static constexpr bool noise = false;
     static void run(const LbcDequantGeneral& p, int grid, cudaStream_t s) {
-        launch_chained(dequant_general_kernel<T, TOPK, KIND>, unsigned(grid), s, p);
+        // Blocks per SM.  A decode waits for its loads: as many as the registers leave without the sum into `out`, but for 16-bit
+        // records with kept values, whose words are read one by one (64 MiB beyond L2 24.5 us with four, 25.2 with eight), and
+        // for fp32 up to two default grids, where six blocks per SM leave a short last wave (16 MiB, e2m1, 5.58 / 5.89 us).  64 MiB, 4 blocks
+        // against 8 (fp32: 6): bf16, one kept value 21.9 / 20.1, two 23.1 / 22.4, e2m1 19.4 / 17.1, its records 20.6 / 17.8; fp32 16.6 / 15.2,
+        // 18.1 / 16.4, 16.6 / 14.7, 17.1 / 15.2; 16 MiB bf16 7.94 / 7.01, 8.45 / 7.73, 7.63 / 6.42, 8.14 / 6.50.
+        const int64_t tiles = (p.numel + kThreads * kElemsPerThread - 1) / (kThreads * kElemsPerThread);
+        const bool many = sizeof(T) == 2 ? !(p.compact && TOPK >= 1) : tiles > 2 * lbc_default_max_blocks();
+        if (many && !p.accumulate)
+            launch_chained(dequant_general_kernel<T, TOPK, KIND, false, sizeof(T) == 2 ? 8 : 6>, unsigned(grid), s, p);
+        else
+            launch_chained(dequant_general_kernel<T, TOPK, KIND, true, 4>, unsigned(grid), s, p);
     }
 };
 template <typename T, int TOPK, int KIND>
