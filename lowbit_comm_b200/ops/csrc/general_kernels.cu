@@ -908,8 +908,16 @@ __global__ void __launch_bounds__(kThreads, 4) quant_general_kernel(const __grid
 // What bounds it: instruction issue.  Before (quant_general_kernel, which asks every chunk where it goes) and here, beyond L2: 64 MiB,
 // bf16, planar, one kept value 34.8 -> 32.7 us, e2m1 36.8 -> 31.7, with one kept value 46.0 -> 41.9, records of e2m1 38.2 -> 34.4;
 // fp32 25.6 -> 23.0, 22.0 -> 18.9, 28.0 -> 23.5, 22.6 -> 19.9; 1 MiB bf16 3.24 -> 2.73, 3.48 -> 2.88.
+// Blocks per SM, 4 against 5 (no spills at either), 64 MiB: bf16, one kept value 32.1 / 30.6 us, two 39.8 / 40.3, e2m1 31.9 / 33.8, its
+// records 34.6 / 36.1; fp32 23.0 / 21.7, 29.3 / 27.5, 19.0 / 18.9, 20.1 / 18.3, e2m1 with one kept value 23.8 / 25.1; 16 MiB bf16, one
+// kept value 10.4 / 9.5, fp32 7.8 / 7.5.
+template <typename T, int TOPK, int KIND>
+constexpr int encode_blocks() {
+    if (KIND == kBook) return sizeof(T) == 4 && TOPK == 0 ? 5 : 4;
+    return KIND != kBookNoise && (TOPK == 1 || (TOPK == 2 && sizeof(T) == 4)) ? 5 : 4;
+}
 template <typename T, int TOPK, int KIND, bool kCompact>
-__global__ void __launch_bounds__(kThreads, 4) encode_general_kernel(const __grid_constant__ LbcQuantGeneral p) {
+__global__ void __launch_bounds__(kThreads, encode_blocks<T, TOPK, KIND>()) encode_general_kernel(const __grid_constant__ LbcQuantGeneral p) {
     chain_wait();
     const GroupShape shape = GroupShape::of<T, TOPK, KIND>(p.group_size);
     const int lanes = shape.lanes, VB = shape.VB, MB = shape.MB;
