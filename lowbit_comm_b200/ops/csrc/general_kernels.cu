@@ -25,7 +25,7 @@
 // the code-book; encode of 16 MiB, beyond L2, bf16 22.5 -> 14.5 us, fp32 14.0 -> 8.6, one-rank pass bf16 22.7 -> 14.5.
 // The one-rank pass without the places of the kept elements: 35.9 -> 30.8 us (32 Mi bf16 elements, one kept value); of 16 MiB
 // beyond L2, two kept values, bf16 14.4 -> 12.4 us, fp32 12.4 -> 10.3.  Each kernel started before the one ahead of it ends: 29.2 us, and
-// 15.4 us for the code-book.  The rare warps of the one-rank pass out of line, its group steps without loops, its sums and products two
+// 15.4 us for the code-book; 12.8 us with the encoder for local payloads and native calls around both.  The rare warps of the one-rank pass out of line, its group steps without loops, its sums and products two
 // to an instruction, 32 Mi elements beyond L2: bf16 29.6 -> 26.6 us, two kept values 30.6 -> 28.2, fp16 in 4 bits 29.1 -> 26.4.
 
 #include <cmath>
@@ -916,8 +916,8 @@ __global__ void __launch_bounds__(kThreads, 4) quant_general_kernel(const __grid
 // Encode of a payload of this GPU alone, on its vectors: no destinations, shards or signal, whole tiles without a test per chunk.
 // kCompact: records, built in shared memory.
 // What bounds it: instruction issue.  Before (quant_general_kernel, which asks every chunk where it goes) and here, beyond L2: 64 MiB,
-// bf16, planar, one kept value 34.8 -> 32.7 us, e2m1 36.8 -> 31.7, with one kept value 46.0 -> 41.9, records of e2m1 38.2 -> 34.4;
-// fp32 25.6 -> 23.0, 22.0 -> 18.9, 28.0 -> 23.5, 22.6 -> 19.9; 1 MiB bf16 3.24 -> 2.73, 3.48 -> 2.88.
+// bf16, planar, one kept value 34.8 -> 30.6 us, two 42.0 -> 38.5, e2m1 36.8 -> 31.1, with one kept value 46.0 -> 42.1, records of e2m1
+// 38.2 -> 34.2; fp32 25.6 -> 20.7, 31.1 -> 27.5, 22.0 -> 17.4, 28.0 -> 23.2, 22.6 -> 18.0; 1 MiB bf16 3.24 -> 2.54, 3.48 -> 2.87.
 // Blocks per SM, 4 against 5 (no spills at either), 64 MiB: bf16, one kept value 32.1 / 30.6 us, two 39.8 / 40.3, e2m1 31.9 / 33.8, its
 // records 34.6 / 36.1; fp32 23.0 / 21.7, 29.3 / 27.5, 19.0 / 18.9, 20.1 / 18.3, e2m1 with one kept value 23.8 / 25.1; 16 MiB bf16, one
 // kept value 10.4 / 9.5, fp32 7.8 / 7.5.
