@@ -1146,21 +1146,26 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 || TOPK == 1 ? 4 : 3)
     T* out = static_cast<T*>(p.out);
     T* rout = static_cast<T*>(p.residual_out);
     const int64_t n = p.numel;
-    const int64_t num_chunks = (n + p.group_size - 1) / p.group_size << shape.shift;
+    const int64_t num_chunks = (n + p.group_size - 1) >> (shape.shift + 4) << shape.shift;
     const int64_t chunk_span = (num_chunks + 31) / 32 * 32;
     const bool vec = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(res) |
                        reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(rout)) & 31) == 0;
     const CodeRule rule = CodeRule::of<KIND>(p.book, p.quant_type, p.stochastic, p.seed);
-    for (int64_t chunk = int64_t(blockIdx.x) * kThreads + threadIdx.x; chunk < chunk_span;
-         chunk += int64_t(gridDim.x) * kThreads) {
-        const bool live = chunk < num_chunks;
-        const int64_t first = chunk * kElemsPerThread;
-        const int lane = int(chunk) & (lanes - 1);
-        Packed16<T> elems = load_elems<T>(x, first, n, vec);            // zeros past the end
+    // 16-bit tensors: tile by tile, whole ones without a test per chunk (32 Mi bf16 elements, e2m1 40.7 -> 38.0 us; 8 Mi, one kept value
+    // 9.6 -> 9.3).  fp32: chunk by chunk (by tiles it spills: 16 Mi elements, one kept value, 22.6 -> 30.4 us).
+    constexpr bool tiles = sizeof(T) == 2;
+    for (int64_t at = int64_t(blockIdx.x) * kThreads + (tiles ? 0 : threadIdx.x); at < (tiles ? num_chunks : chunk_span);
+         at += int64_t(gridDim.x) * kThreads) {
+        const int64_t chunk = tiles ? at + threadIdx.x : at;
+        const bool whole = tiles && vec && (at + kThreads) * kElemsPerThread <= n;
+        const bool live = whole || chunk < num_chunks;
+        const int64_t first = chunk * kElemsPerThread, end = whole ? first + 16 : n;
+        const int lane = tiles ? int(threadIdx.x) & (lanes - 1) : int(chunk) & (lanes - 1);
+        Packed16<T> elems = load_elems<T>(x, first, end, vec);          // zeros past the end
         if (res != nullptr) {
             float v[16], r[16];
             unpack_elems<T>(elems, v);
-            unpack_elems<T>(load_elems<T>(res, first, n, vec), r);
+            unpack_elems<T>(load_elems<T>(res, first, end, vec), r);
 #pragma unroll
             for (int i = 0; i < 16; ++i) v[i] += r[i];
             elems = pack_elems<T>(v);
@@ -1196,9 +1201,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 || TOPK == 1 ? 4 : 3)
             unpack_elems<T>(elems, e);
 #pragma unroll
             for (int i = 0; i < 16; ++i) e[i] -= a[i];
-            store_elems<T>(rout, first, n, vec, pack_elems<T>(e));
+            store_elems<T>(rout, first, end, vec, pack_elems<T>(e));
         }
-        store_elems<T>(out, first, n, vec, y);
+        store_elems<T>(out, first, end, vec, y);
     }
 }
 
