@@ -25,7 +25,7 @@
 // the code-book; encode of 16 MiB, beyond L2, bf16 22.5 -> 14.5 us, fp32 14.0 -> 8.6, one-rank pass bf16 22.7 -> 14.5.
 // The one-rank pass without the places of the kept elements: 35.9 -> 30.8 us (32 Mi bf16 elements, one kept value); of 16 MiB
 // beyond L2, two kept values, bf16 14.4 -> 12.4 us, fp32 12.4 -> 10.3.  Each kernel started before the one ahead of it ends: 29.2 us, and
-// 15.4 us for the code-book; 12.8 us with the encoder for local payloads and native calls around both.  The rare warps of the one-rank pass out of line, its group steps without loops, its sums and products two
+// 15.4 us for the code-book; 12.2 us with the encoder for local payloads and native calls around both.  The rare warps of the one-rank pass out of line, its group steps without loops, its sums and products two
 // to an instruction, 32 Mi elements beyond L2: bf16 29.6 -> 26.6 us, two kept values 30.6 -> 28.2, fp16 in 4 bits 29.1 -> 26.4.
 
 #include <cmath>
