@@ -223,7 +223,7 @@ __device__ __forceinline__ void add_batch(const LbcReduce& p, int r0, int64_t ch
         for (int j = 0; j < K; ++j) {
             const uint8_t* src = p.src[r0 + j];
             if constexpr (CB == 16) {
-                codes[j] = ld16_stream(src + voff);
+                codes[j] = ld16_once(src + voff);
             } else {
                 const uint2 c = *reinterpret_cast<const uint2*>(src + voff);
                 codes[j] = make_uint4(c.x, c.y, 0u, 0u);
@@ -240,8 +240,8 @@ __device__ __forceinline__ void add_batch(const LbcReduce& p, int r0, int64_t ch
 #pragma unroll
         for (int j = 0; j < K; ++j) {
             const uint8_t* src = p.src[r0 + j] + at;
-            if (full >= 512 || wlane * 16 < full) lo[j] = ld16_stream(src);
-            if (full > 512 && wlane * 16 < full - 512) hi[j] = ld16_stream(src + 512);
+            if (full >= 512 || wlane * 16 < full) lo[j] = ld16_once(src);
+            if (full > 512 && wlane * 16 < full - 512) hi[j] = ld16_once(src + 512);
         }
         const uint8_t* rec = span + (wlane / lanes) * (VB + MB);
 #pragma unroll

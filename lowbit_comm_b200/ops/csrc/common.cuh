@@ -227,6 +227,12 @@ __device__ __forceinline__ U8x32 ld32_once(const void* p) {
                    "=r"(v.w[6]), "=r"(v.w[7]) : "l"(p));
     return v;
 }
+__device__ __forceinline__ uint4 ld16_once(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
 template <typename T>
 __device__ __forceinline__ Raw16<T> raw16(const T* p) {
     Raw16<T> r;

@@ -915,3 +915,82 @@ def test_general_encode_at_tile_edges(ext, dtype, bit, quant_type, topk, group, 
             assert torch.equal(raw[where:where + want.numel()].cpu(), want), (n, where, skew)
             assert bool((raw[:where] == 0xAB).all()) and bool((raw[where + want.numel():] == 0xAB).all())
             assert torch.equal(at[2].cpu().view(torch.uint8), prepared.view(torch.uint8)), (n, where, skew)
+
+
+@pytest.mark.parametrize("dtype", ("bf16", "fp32"))
+@pytest.mark.parametrize("kw", [{}, {"compact": True}, {"bit": 4, "group_size": 16}, {"topk": 1}, {"topk": 2, "compact": True},
+                                {"bit": 4, "quant_type": "e2m1"}])
+@pytest.mark.parametrize("n,skew", [(2 * 4096, 0), (4099, 1), (150_001, 0)])
+def test_only_codec_and_one_rank_calls_in_a_row(ext, dtype, kw, n, skew):
+    """Rows of calls with no kernel of another library between them, small enough that three and more are on the GPU at once: a
+    payload decoded, written anew and decoded again, one-rank passes in place, a mean of several payloads; every call
+    reads what the one before it wrote.  Alone and captured in a graph, against the same calls one at a time."""
+
+    cfg, T, rounds = _cfg(**kw), DTYPES[dtype], 4
+    fast = codec.is_fast_profile(cfg)
+    grads = [_data(n, T, seed=i).cuda() for i in range(rounds)]
+    size = codec.estimate_quantized_size(n, dtype=dtype, config=cfg).quantized_bytes
+    held = lambda: torch.empty(n + skew, dtype=T, device="cuda")[skew:]
+    x, a, b, c = ([held() for _ in range(rounds)] for _ in range(4))
+    residual, prepared = held(), held()
+    p, q = (torch.empty(size, dtype=torch.uint8, device="cuda") for _ in range(2))
+    ranks = PeerGroup.loopback(1, FusedWorkspace.required_bytes(1, dtype, cfg, n, True) + (1 << 20)) if fast else []
+    ws = FusedWorkspace(ranks[0], dtype=dtype, config=cfg, max_numel=n, engine="pipe") if fast else None
+
+    def one_rank(t):
+        if fast:
+            ws.all_reduce(t, t, residual=residual)
+        else:
+            assert ext.roundtrip_general(t, residual, t, residual, cfg.group_size, cfg.bit, cfg.topk,
+                                         codec._QUANT_CODE[cfg.quant_type], False, 0, 1)
+
+    def row(pause):
+        for i in range(rounds):
+            for call in (lambda: codec.quantize_tensor(x[i], cfg, output=p),
+                         lambda: codec.dequantize_tensor(p, (n,), cfg, dtype=dtype, output=a[i]),
+                         lambda: codec.quantize_tensor(a[i], cfg, output=p, residual=residual, prepared_out=residual),
+                         lambda: codec.dequantize_tensor(p, (n,), cfg, dtype=dtype, output=b[i]),
+                         lambda: one_rank(b[i]),
+                         lambda: one_rank(b[i]),
+                         lambda: codec.quantize_tensor(b[i], cfg, output=q, residual=residual, prepared_out=prepared),
+                         lambda: codec.dequantize_tensor(q, (n,), cfg, dtype=dtype, output=x[i]),
+                         lambda: codec.dequantize_tensor(p, (n,), cfg, dtype=dtype, output=c[i]),
+                         lambda: codec.inplace_dequantize_reduce_mean_update_error_feedback([p, q, p], prepared, c[i], residual,
+                                                                                            cfg, reduce="mean"),
+                         lambda: codec.dequantize_tensor(q, (n,), cfg, dtype=dtype, output=c[i], reduce_op="sum")):
+                call()
+                if pause:
+                    torch.cuda.synchronize()
+
+    def restart():
+        for i in range(rounds):
+            x[i].copy_(grads[i])
+            for t in (a[i], b[i], c[i]):
+                t.zero_()
+        residual.zero_()
+        prepared.zero_()
+
+    def everything():
+        return [t.clone() for t in (*x, *a, *b, *c, residual, prepared, p, q)]
+
+    restart()
+    row(pause=True)
+    want = everything()
+    for _ in range(5):
+        restart()
+        row(pause=False)
+        assert all(torch.equal(t, w) for t, w in zip(everything(), want))
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.graph(graph, stream=stream):
+        restart()
+        row(pause=False)
+    for _ in range(5):
+        graph.replay()
+        assert all(torch.equal(t, w) for t, w in zip(everything(), want))
+    # payloads and results that are allocated by the calls: the allocator gives the same addresses again and again
+    alone = [codec.dequantize_tensor(codec.quantize_tensor(g, cfg), (n,), cfg, dtype=dtype).cpu() for g in grads]
+    for _ in range(5):
+        results = [codec.dequantize_tensor(codec.quantize_tensor(g, cfg), (n,), cfg, dtype=dtype) for g in grads * 3]
+        assert all(torch.equal(r.cpu(), w) for r, w in zip(results, alone * 3))
+    PeerGroup.close_loopback(ranks)
