@@ -26,7 +26,8 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 EXT_NAME = "_lbc_cuda"
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
-NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
+NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
+              "-Xptxas", "-v"]
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-Wno-attributes"]
 
 
@@ -83,7 +84,7 @@ def _fingerprint(files: list[Path], flags: list[str]) -> str:
     return h.hexdigest()
 
 
-def _run(cmd: list[str], verbose: bool) -> None:
+def _run(cmd: list[str], verbose: bool) -> str:
     if verbose:
         print(" ".join(cmd), flush=True)
     proc = subprocess.run(cmd, capture_output=True, text=True)
@@ -91,6 +92,13 @@ def _run(cmd: list[str], verbose: bool) -> None:
         raise RuntimeError(f"command failed ({proc.returncode}): {' '.join(cmd)}\n{proc.stdout}\n{proc.stderr}")
     if verbose and proc.stderr.strip():
         print(proc.stderr, file=sys.stderr)
+    return proc.stderr
+
+
+def ptxas_report(source: str) -> Path:
+    """Registers, stack and spills of every kernel of one `.cu` file, as ptxas printed them when it was last compiled."""
+
+    return HERE / "build" / f"{Path(source).stem}.ptxas.txt"
 
 
 def build_extension(*, force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> Path:
@@ -114,10 +122,7 @@ def build_extension(*, force: bool = False, verbose: bool = False, ptxas_info: b
     jobs = []
     for src in cuda_sources():
         obj = obj_dir / (src.stem + ".cu.o")
-        cmd = [nvcc, *ARCH_FLAGS, *NVCC_FLAGS, f"-I{CSRC}", "-c", str(src), "-o", str(obj)]
-        if ptxas_info:
-            cmd += ["-Xptxas", "-v"]
-        jobs.append((cmd, obj))
+        jobs.append(([nvcc, *ARCH_FLAGS, *NVCC_FLAGS, f"-I{CSRC}", "-c", str(src), "-o", str(obj)], obj))
     for src in cxx_sources():
         obj = obj_dir / (src.stem + ".cpp.o")
         cmd = ["g++", *CXX_FLAGS, f"-DTORCH_EXTENSION_NAME={EXT_NAME}", "-DTORCH_API_INCLUDE_EXTENSION_H",
@@ -125,7 +130,11 @@ def build_extension(*, force: bool = False, verbose: bool = False, ptxas_info: b
                "-c", str(src), "-o", str(obj)]
         jobs.append((cmd, obj))
     with ThreadPoolExecutor(max_workers=min(8, len(jobs))) as pool:
-        list(pool.map(lambda job: _run(job[0], verbose or ptxas_info), jobs))
+        printed = list(pool.map(lambda job: _run(job[0], verbose), jobs))
+    for src, text in zip(cuda_sources(), printed):
+        ptxas_report(src.name).write_text(text)
+        if ptxas_info:
+            print(text, file=sys.stderr)
     lib_dirs = cpp_extension.library_paths(device_type="cuda")
     link = ["g++", "-shared", "-o", str(target), *[str(obj) for _, obj in jobs],
             *[f"-L{d}" for d in lib_dirs], f"-L{cuda / 'lib64'}",

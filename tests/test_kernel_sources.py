@@ -1,9 +1,13 @@
-"""Rules of the kernels that reading their source shows (no GPU, no compiler)."""
+"""Rules of the kernels that their source shows, or what the compiler printed when it built them (no GPU)."""
 
 import re
+import shutil
+import subprocess
 from pathlib import Path
 
 import pytest
+
+from lowbit_comm_b200.ops import build
 
 CSRC = Path(__file__).resolve().parents[1] / "lowbit_comm_b200" / "ops" / "csrc"
 CHAINED = sorted(p.name for p in CSRC.glob("*.cu") if "launch_chained(" in p.read_text())
@@ -43,3 +47,26 @@ def test_chained_kernels_wait_before_they_touch_memory(name):
         waits = [i for i, line in enumerate(first) if line == "chain_wait();"]
         assert bool(waits) == (kernel in launched), kernel
         assert all(line.startswith("constexpr") for line in first[:waits[0] if waits else 0]), kernel
+
+
+def _spill_loads(source):
+    """Kernel (with its template arguments) -> bytes of spill loads, from the last build."""
+
+    report = build.ptxas_report(source)
+    if not report.exists() or shutil.which("c++filt") is None:
+        pytest.skip("the extension was not built here")
+    pairs = re.findall(r"Function properties for (\S+)\n.*?(\d+) bytes spill loads", report.read_text())
+    names = subprocess.run(["c++filt"], input="\n".join(name for name, _ in pairs), capture_output=True, text=True,
+                           check=True).stdout.split("\n")
+    return {name.replace("void lbc::", "").split("(LbcReduce")[0]: int(loads) for name, (_, loads) in zip(names, pairs)}
+
+
+def test_decode_kernels_keep_their_registers():
+    """A payload's scale is divided ahead of its sixteen codes: the other way round they live across the division, and these sums
+    were 10872 and 5388 bytes.  The limits are what nvcc 12.9 gives (5840 and 352) and a quarter more."""
+
+    loads = _spill_loads("codec_kernels.cu")
+    one = [v for k, v in loads.items() if k.startswith("decode_kernel<") and re.search(r", \(?(int\))?1>$", k)]
+    ragged = [v for k, v in loads.items() if k.startswith("decode_ragged_kernel<")]
+    assert len(one) == 36 and len(ragged) == 72
+    assert sum(one) <= 7300 and sum(ragged) <= 440
