@@ -38,15 +38,26 @@ struct DeviceStatus {
 // ---------------------------------------------------------------------------
 // kernels in a row
 // ---------------------------------------------------------------------------
-// A kernel launched with launch_chained starts while the last blocks of the one before it in the stream still run, and
-// waits in chain_wait() until that one is through and its stores are visible: its launch and the start of its blocks
-// are off the path (2 to 2.7 us per kernel: 13.1 M bf16 elements through the one-rank pass 10.2 -> 7.8 us, encode of 16 MiB
-// 8.3 -> 6.7, decode 8.0 -> 5.7).  All blocks of the first have started by then, so the early ones take no place
-// from it.  Only for kernels that wait for nobody else.  chain_wait comes before the first access to memory (constants and parameters aside), in every thread;
-// without the attribute it returns at once.
+// A kernel launched with launch_chained may start before the kernel ahead of it in the stream has ended, if that one is such a
+// kernel too (or another that issues launch_dependents): then it starts when all blocks of the first are past their own
+// chain_wait(), and waits in its chain_wait() until the first is through and its stores are visible.  Its launch and the
+// start of its blocks are off the path.  Behind any other kernel, a copy or an event it starts when that has ended.
+// Calls one by one, as Python issues them: 13.1 M bf16 elements through the one-rank pass 10.3 -> 7.9 us, encode of 16 MiB
+// 8.2 -> 6.6, decode 8.2 -> 5.6.  In a CUDA graph, whose plain launches follow one another more closely, 7.80 -> 7.65,
+// 6.90 -> 6.31 and 5.96 -> 5.37, and each behind a kernel of torch 8.67 -> 9.08, 8.14 -> 7.73 and 7.17 -> 6.80.
+// First the wait, then the permission for the next kernel: so all that is ahead of a kernel in the stream has ended before the one
+// behind it starts.  The other way round, three and more were on the GPU at once.  A kernel of another library that reads, ahead of
+// its own wait, what an earlier kernel than the one before it has written would have read too soon; and the blocks
+// of grids below one wave, of which some SMs then held more than others, took longer (1 Mi bf16 elements encoded and
+// decoded in a graph 4.38 -> 3.41 us, a one-rank pass of 1 Mi fp32 elements with a stochastic code-book and one kept value 17.7 ->
+// 11.2).  Grids of several waves pay a little for it: the one-rank pass above 7.81 -> 7.93 us, encode of 16 MiB 6.51 -> 6.56, decode 5.72
+// -> 5.62.  Their last blocks could give the permission at once, since others must have ended for them to start; with a
+// test for that on the grid's size the same three took 8.03, 6.51 and 5.72.
+// Only for kernels that wait for nobody else.  chain_wait comes before the first access to memory (constants and parameters
+// aside), in every thread; without the attribute it returns at once.
 __device__ __forceinline__ void chain_wait() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <typename P>
 static cudaError_t launch_chained(void (*kernel)(const P), unsigned grid, cudaStream_t stream, const P& p) {

@@ -49,6 +49,15 @@ def test_chained_kernels_wait_before_they_touch_memory(name):
         assert all(line.startswith("constexpr") for line in first[:waits[0] if waits else 0]), kernel
 
 
+def test_a_chained_kernel_waits_before_it_lets_the_next_one_start():
+    """Otherwise a kernel two places behind starts beside the first, and what it reads ahead of its own wait may not be written yet."""
+
+    body = _code("common.cuh").split("void chain_wait() {")[1].split("}")[0]
+    assert re.findall(r"griddepcontrol\.(\w+)", body) == ["wait", "launch_dependents"]
+    for path in CSRC.glob("*.cu*"):
+        assert path.name == "common.cuh" or "griddepcontrol" not in _code(path.name)
+
+
 def _spill_loads(source):
     """Kernel (with its template arguments) -> bytes of spill loads, from the last build."""
 
