@@ -1131,10 +1131,9 @@ __device__ __noinline__ void requantize_by_place(uint32_t* words, int lane, int 
 
 // The all-reduce of a group of one rank: encode and decode in registers, no payload (see roundtrip_kernels.cu; here
 // the decoded values are rounded to T before the residual is taken, the rule of these profiles).
-// Blocks per SM, 3 against 4, 16 Mi fp32 elements: one kept value 24.2 / 22.6 us, two 25.1 / 26.3; 16-bit, 4 against 5, 32 Mi bf16: 26.6 / 27.5,
-// 28.2 / 29.1.
-template <typename T, int TOPK, int KIND>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 2 || TOPK == 1 ? 4 : 3) roundtrip_general_kernel(const __grid_constant__ LbcRoundtripGeneral p) {
+// Blocks per SM, 16-bit, 4 against 5, 32 Mi bf16: one kept value 26.6 / 27.5 us, two 28.2 / 29.1; fp32: see its launcher.
+template <typename T, int TOPK, int KIND, int kBlocks>
+__global__ void __launch_bounds__(kThreads, kBlocks) roundtrip_general_kernel(const __grid_constant__ LbcRoundtripGeneral p) {
     constexpr bool by_magnitude = TOPK >= 1 && KIND != kBookNoise;
     chain_wait();
     const GroupShape shape = GroupShape::of<T, TOPK, KIND>(p.group_size);
@@ -1314,7 +1313,23 @@ template <typename T, int TOPK, int KIND>
 struct RoundtripGeneral {
     static constexpr bool noise = true;
     static void run(const LbcRoundtripGeneral& p, int grid, cudaStream_t s) {
-        launch_chained(roundtrip_general_kernel<T, TOPK, KIND>, unsigned(grid), s, p);
+        // fp32, three blocks per SM or four (64 registers, with spills).  Four are faster for one kept value alone (two, 16 Mi elements:
+        // 25.1 / 26.3 us), without a residual, and where three do not hold the whole grid.  Three / four, one kept value, 8 bits: 1 Mi
+        // elements 3.63 / 3.57, 1.75 Mi (the last that three hold) 3.73 / 3.96, 2 Mi 4.53 / 4.35, 4 Mi 7.63 / 7.18, 16 Mi 23.7 / 22.1; with a
+        // residual 3.75 / 5.12, 6.21 / 6.86, 7.01 / 7.12, 11.7 / 12.4, 40.5 / 41.4.  e2m1 4.35 / 5.01, 5.66 / 5.83, 6.30 / 6.01, 10.1 / 9.8,
+        // 30.5 / 29.5; with a residual 5.42 / 6.39, 7.81 / 8.45, 8.56 / 8.61, 13.2 / 14.8, 42.3 / 45.5.  8 bits with noise 4.48 / 5.15,
+        // 5.66 / 6.16, 6.35 / 6.52, 10.3 / 10.2, 32.8 / 31.6; with a residual, the last two, 13.2 / 14.4 and 42.2 / 45.5.  e2m1 with noise,
+        // those two: 30.2 / 34.1 and 107 / 116.
+        if constexpr (sizeof(T) == 2) {
+            launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 4>, unsigned(grid), s, p);
+        } else {
+            if constexpr (TOPK == 1 && KIND != kBookNoise)
+                if (p.residual == nullptr && grid > lbc_default_max_blocks() / 8 * 3) {
+                    launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 4>, unsigned(grid), s, p);
+                    return;
+                }
+            launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 3>, unsigned(grid), s, p);
+        }
     }
 };
 

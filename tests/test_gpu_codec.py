@@ -994,3 +994,24 @@ def test_only_codec_and_one_rank_calls_in_a_row(ext, dtype, kw, n, skew):
         results = [codec.dequantize_tensor(codec.quantize_tensor(g, cfg), (n,), cfg, dtype=dtype) for g in grads * 3]
         assert all(torch.equal(r.cpu(), w) for r, w in zip(results, alone * 3))
     PeerGroup.close_loopback(ranks)
+
+
+@pytest.mark.parametrize("bit,quant_type,group", [(8, "linear", 64), (4, "linear", 16), (4, "e2m1", 32)])
+@pytest.mark.parametrize("past", (0, 1, 4096))
+def test_fp32_one_rank_pass_where_its_blocks_per_sm_change(ext, bit, quant_type, group, past):
+    """One kept value: up to three blocks per SM in all, and above, with and without a residual, against the codec."""
+
+    cfg = _cfg(bit=bit, group_size=group, topk=1, quant_type=quant_type)
+    n = int(ext.default_max_blocks()) // 8 * 3 * 4096 + past
+    x = _repeated(_data(group * 997, torch.float32, seed=5).cuda(), n).clone()
+    for residual in (None, torch.full_like(x, 1e-4)):
+        prepared = torch.empty_like(x)
+        payload = codec.quantize_tensor(x, cfg, residual=residual, prepared_out=prepared)
+        want = codec.dequantize_tensor(payload, (n,), cfg, dtype="fp32")
+        out, rout = torch.empty_like(x), None if residual is None else residual.clone()
+        assert ext.roundtrip_general(x, rout, out, rout, group, bit, 1, codec._QUANT_CODE[quant_type], False, 0, 1)
+        assert torch.equal(out.view(torch.uint8), want.view(torch.uint8))
+        if residual is not None:
+            left = torch.empty_like(x)
+            codec.update_error_feedback_residual(prepared, want, left)
+            assert torch.equal(rout.view(torch.uint8), left.view(torch.uint8))

@@ -67,7 +67,8 @@ def _spill_loads(source):
     pairs = re.findall(r"Function properties for (\S+)\n.*?(\d+) bytes spill loads", report.read_text())
     names = subprocess.run(["c++filt"], input="\n".join(name for name, _ in pairs), capture_output=True, text=True,
                            check=True).stdout.split("\n")
-    return {name.replace("void lbc::", "").split("(LbcReduce")[0]: int(loads) for name, (_, loads) in zip(names, pairs)}
+    plain = [re.sub(r"\((int|bool)\)", "", name.replace("void lbc::", "")).split("(Lbc")[0] for name in names]
+    return {name: int(loads) for name, (_, loads) in zip(plain, pairs)}
 
 
 def test_decode_kernels_keep_their_registers():
@@ -75,7 +76,17 @@ def test_decode_kernels_keep_their_registers():
     were 10872 and 5388 bytes.  The limits are what nvcc 12.9 gives (5840 and 352) and a quarter more."""
 
     loads = _spill_loads("codec_kernels.cu")
-    one = [v for k, v in loads.items() if k.startswith("decode_kernel<") and re.search(r", \(?(int\))?1>$", k)]
+    one = [v for k, v in loads.items() if k.startswith("decode_kernel<") and k.endswith(", 1>")]
     ragged = [v for k, v in loads.items() if k.startswith("decode_ragged_kernel<")]
     assert len(one) == 36 and len(ragged) == 72
     assert sum(one) <= 7300 and sum(ragged) <= 440
+
+
+def test_fp32_one_rank_kernels_with_three_blocks_do_not_spill():
+    """One kept value: the kernels with four blocks per SM do, which passes with a residual and the stochastic code-book pay for
+    (192 bytes of spill loads in that one)."""
+
+    loads = {k: v for k, v in _spill_loads("general_kernels.cu").items() if k.startswith("roundtrip_general_kernel<float, 1, ")}
+    assert sorted(loads) == ["roundtrip_general_kernel<float, 1, %d, %d>" % kind for kind in
+                             ((0, 3), (0, 4), (1, 3), (1, 4), (2, 3), (2, 4), (3, 3))]
+    assert all(v == 0 for k, v in loads.items() if k.endswith(", 3>"))
