@@ -188,8 +188,12 @@ struct EncodeLauncher {
 // decode and reduce
 // ---------------------------------------------------------------------------
 // acc += one payload's 16 values: fma(code, scale / L, acc), one rounding per payload.  kPairs: two of them to an instruction
-// (sm_100+) and the quotient without a branch.  Several payloads draw the card's power limit, so instructions are time; one
-// payload alone is 3 % slower with it (128 Mi bf16 elements 63.6 -> 65.7 us); the mean of eight of 32 Mi 86.5 -> 84.2.
+// (sm_100+) and the quotient without a branch; whole tiles.  Several payloads draw the card's power limit, so instructions are time:
+// mean of eight of 32 Mi bf16 elements 86.5 -> 84.2 us.  One payload (scalar / packed): 128 Mi 62.6 / 61.6, in 4 bits 57.7 / 56.4,
+// records 70.8 / 68.6; 64 Mi fp32 54.2 / 52.9, records 52.0 / 52.1, in 4 bits 50.6 / 49.5, their records 48.8 / 49.3 (with the
+// quotient after the codes packed was behind, 63.6 / 65.7).  Unaligned ones and tensor ends stay scalar: with the quotient without
+// a branch the mean of eight of 16 Mi fp32 elements in records of 16, one payload on 8 bytes, took 64.4 us instead of 61.5, of
+// bf16 ones 56.3 instead of 55.7, of planar bf16 payloads 46.1 instead of 46.9.
 template <typename T, int BIT, bool kPairs>
 __device__ __forceinline__ void add_payload(float (&acc)[16], uint4 codes, float scale) {
     constexpr int lim = BIT == 8 ? 127 : 7;
@@ -214,7 +218,7 @@ __device__ __forceinline__ void add_payload(float (&acc)[16], uint4 codes, float
 
 // Adds payloads r0 .. r0 + K - 1 to a thread's chunk; all K loads are issued before the first is decoded.  Whole warps
 // of whole groups, vector-aligned payloads.  Compact: the warp's span comes in as vectors and turns through `span`.
-template <typename T, int G, int BIT, bool kCompact, int K, bool kPairs>
+template <typename T, int G, int BIT, bool kCompact, int K>
 __device__ __forceinline__ void add_batch(const LbcReduce& p, int r0, int64_t chunk, uint8_t* span, float (&acc)[16]) {
     constexpr int lanes = G / kElemsPerThread;
     constexpr int VB = G * BIT / 8, MB = sizeof(T), CB = kElemsPerThread * BIT / 8;
@@ -236,7 +240,7 @@ __device__ __forceinline__ void add_batch(const LbcReduce& p, int r0, int64_t ch
             scale[j] = load_scale<T>(src + soff);
         }
 #pragma unroll
-        for (int j = 0; j < K; ++j) add_payload<T, BIT, kPairs>(acc, codes[j], scale[j]);
+        for (int j = 0; j < K; ++j) add_payload<T, BIT, true>(acc, codes[j], scale[j]);
     } else {
         constexpr int full = span_bytes(G, VB + MB);            // 17 to 40 vectors
         const int wlane = threadIdx.x & 31;
@@ -258,7 +262,7 @@ __device__ __forceinline__ void add_batch(const LbcReduce& p, int r0, int64_t ch
             span_get_codes<CB>(rec + lane * CB, w);
             const float scale = load_scale<T>(rec + VB);
             __syncwarp();
-            add_payload<T, BIT, kPairs>(acc, make_uint4(w[0], w[1], w[2], w[3]), scale);
+            add_payload<T, BIT, true>(acc, make_uint4(w[0], w[1], w[2], w[3]), scale);
         }
     }
 }
@@ -332,11 +336,11 @@ decode_kernel(const __grid_constant__ LbcReduce p) {
         Raw16<T> held;
         if (B > 1 && rout != nullptr) held = raw16(prep + first);      // on its way while the payloads are summed
         int r = 0;
-        for (; r + B <= R; r += B) add_batch<T, G, BIT, kCompact, B, (B > 1)>(p, r, chunk, span, acc);
+        for (; r + B <= R; r += B) add_batch<T, G, BIT, kCompact, B>(p, r, chunk, span, acc);
         if constexpr (B > 2)
-            for (; r + 2 <= R; r += 2) add_batch<T, G, BIT, kCompact, 2, true>(p, r, chunk, span, acc);
+            for (; r + 2 <= R; r += 2) add_batch<T, G, BIT, kCompact, 2>(p, r, chunk, span, acc);
         if constexpr (B > 1)
-            for (; r < R; ++r) add_batch<T, G, BIT, kCompact, 1, true>(p, r, chunk, span, acc);
+            for (; r < R; ++r) add_batch<T, G, BIT, kCompact, 1>(p, r, chunk, span, acc);
 #pragma unroll
         for (int i = 0; i < 16; ++i) acc[i] *= p.scale;
         if (B > 1 && rout != nullptr) {
