@@ -1275,7 +1275,7 @@ struct QuantGeneral {
     static constexpr bool noise = true;
     static void run(const LbcQuantGeneral& p, int grid, cudaStream_t s) {
         const uintptr_t at = reinterpret_cast<uintptr_t>(p.out);
-        if (p.num_dst > 0)      // for other ranks, who wait for it
+        if (p.num_dst > 0 || p.signal.num_remote > 0)      // for other ranks, who wait for it
             quant_general_kernel<T, TOPK, KIND><<<grid, kThreads, 0, s>>>(p);
         else if (p.compact && (at & 15) == 0)
             launch_chained(encode_general_kernel<T, TOPK, KIND, true>, unsigned(grid), s, p);

@@ -1015,3 +1015,39 @@ def test_fp32_one_rank_pass_where_its_blocks_per_sm_change(ext, bit, quant_type,
             left = torch.empty_like(x)
             codec.update_error_feedback_residual(prepared, want, left)
             assert torch.equal(rout.view(torch.uint8), left.view(torch.uint8))
+
+
+@pytest.mark.parametrize("kw", [{"topk": 1}, {"bit": 4, "quant_type": "e2m1", "compact": True}])
+@pytest.mark.parametrize("where", (0, 4))
+def test_a_general_payload_of_this_gpu_raises_its_signal(ext, kw, where):
+    """The C entry takes a signal without destinations too: raised once the payload is stored, wherever that starts."""
+
+    import ctypes
+
+    from lowbit_comm_b200.ops.build import extension_path
+
+    class Signal(ctypes.Structure):
+        _fields_ = [("remote_flags", ctypes.c_void_p * 16), ("num_remote", ctypes.c_int), ("my_slot", ctypes.c_int),
+                    ("epoch", ctypes.c_uint), ("block_counter", ctypes.c_void_p)]
+
+    class Encode(ctypes.Structure):
+        _fields_ = [*((name, ctypes.c_int) for name in ("dtype", "group_size", "bit", "topk", "quant_type", "stochastic", "compact")),
+                    ("x", ctypes.c_void_p), ("residual", ctypes.c_void_p), ("prepared_out", ctypes.c_void_p),
+                    ("numel", ctypes.c_int64), ("out", ctypes.c_void_p), ("seed", ctypes.c_ulonglong),
+                    ("dst", ctypes.c_void_p * 16), ("num_dst", ctypes.c_int), ("signal", Signal), ("max_blocks", ctypes.c_int),
+                    ("shard_groups", ctypes.c_int64), ("book", ctypes.c_uint32 * 47)]
+
+    cfg, n = _cfg(**kw), 3 * 4096 + 5
+    x = _data(n, torch.bfloat16).cuda()
+    want = oracle.encode(x.cpu(), cfg)
+    raw = torch.zeros(want.numel() + 16, dtype=torch.uint8, device="cuda")
+    flags, counter = torch.zeros(8, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    call = Encode(dtype=1, group_size=cfg.group_size, bit=cfg.bit, topk=cfg.topk, quant_type=codec._QUANT_CODE[cfg.quant_type],
+                  compact=cfg.compact, x=x.data_ptr(), numel=n, out=raw.data_ptr() + where)
+    call.signal = Signal(num_remote=1, my_slot=3, epoch=7, block_counter=counter.data_ptr())
+    call.signal.remote_flags[0] = flags.data_ptr()
+    lib = ctypes.CDLL(str(extension_path()))
+    lib.lbc_quant_general.argtypes = [ctypes.POINTER(Encode), ctypes.c_void_p]
+    assert lib.lbc_quant_general(ctypes.byref(call), torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(raw[where:where + want.numel()].cpu(), want)
+    assert flags.tolist() == [0, 0, 0, 7, 0, 0, 0, 0] and counter.item() == 0
