@@ -47,9 +47,11 @@ def _numel_of(shape) -> int:
 
 
 def _whole(shape) -> bool:
-    """Is it a shape as the native call takes it?  (The general way converts what it is given, iterables and floats too.)"""
+    """Is it a shape as the native call takes it?  (The general way converts what it is given, iterables
+    and floats too, and says what is wrong with dimensions that no tensor has.)"""
 
-    return type(shape) is torch.Size or (type(shape) in (tuple, list) and all(type(dim) is int for dim in shape))
+    return type(shape) is torch.Size or (type(shape) in (tuple, list)
+                                         and all(type(dim) is int and abs(dim) < 1 << 62 for dim in shape))
 
 
 def _dense(tensor: torch.Tensor | None) -> torch.Tensor | None:

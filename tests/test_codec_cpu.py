@@ -205,3 +205,14 @@ def test_codec_corners_on_cpu():
         codec.dequantize_reduce_tensors([], (200,), c, dtype="bf16")
     with pytest.raises(ValueError, match="unsupported reduce"):
         codec.dequantize_reduce_tensors([good], (200,), c, dtype="bf16", reduce="max")
+
+
+def test_shapes_that_the_native_decoder_is_not_given():
+    """Dimensions that a 64-bit integer does not hold would stop at the binding; the general way says what is wrong with them."""
+
+    assert codec._whole((3, 4)) and codec._whole([0, -1]) and codec._whole(torch.Size((2, 3)))
+    for shape in ((1 << 63,), [4, -(1 << 70)], (1 << 70, 0), (True, 2), (4.0,), range(3), None):
+        assert not codec._whole(shape), shape
+    payload = codec.quantize_tensor(torch.ones(64), CompressionConfig())
+    with pytest.raises(ValueError, match="payload has"):
+        codec.dequantize_tensor(payload, (1 << 70,), CompressionConfig(), dtype="fp32")

@@ -856,6 +856,8 @@ def test_native_codec_calls_and_the_general_way(ext, dtype, kw, monkeypatch):
         "an iterator": lambda: codec.dequantize_tensor(whole, np.array([4099]), cfg, dtype=dtype),
         "negative": lambda: codec.dequantize_tensor(whole, (-4099, -1), cfg, dtype=dtype),
         "empty": lambda: codec.dequantize_tensor(bytes_[:0], (0, 3), cfg, dtype=dtype),
+        "beyond 64 bits": lambda: codec.dequantize_tensor(whole, (1 << 70,), cfg, dtype=dtype),
+        "below 64 bits": lambda: codec.dequantize_tensor(whole, [-(1 << 70), 1], cfg, dtype=dtype),
         "output": lambda: codec.dequantize_tensor(whole, (4099,), cfg, dtype=dtype, output=torch.empty_like(x)),
         "output of another shape": lambda: codec.dequantize_tensor(whole, (1, 4099), cfg, dtype=dtype, output=torch.empty_like(x)),
         "output of another type": lambda: codec.dequantize_tensor(whole, (4099,), cfg, dtype=dtype, output=torch.empty_like(x, dtype=DTYPES[other])),
