@@ -455,7 +455,7 @@ class Communicator:
         """Caller-owned output checks (parity: reduce_scatter_transport.py:390-431)."""
 
         if out is None:
-            return tensor.new_empty(shard_numel)
+            return torch.empty(shard_numel, dtype=tensor.dtype, device=tensor.device)
         if hasattr(out, "tensor") and hasattr(out, "mark_submitting"):  # an output lease
             out = out.tensor
         if tuple(out.shape) != (shard_numel,):
@@ -486,7 +486,7 @@ class Communicator:
         if self.peer_usable(tensor, config):
             ws = self.workspace(tensor, config, name)
             if self.world_size == 1:
-                outs = [tensor.new_empty(shape)]
+                outs = [torch.empty(shape, dtype=tensor.dtype, device=tensor.device)]
             else:      # rows of one buffer: the decode of all W payloads is then a single launch
                 outs = list(torch.empty((self.world_size,) + shape, dtype=tensor.dtype, device=tensor.device).unbind(0))
             scope, side = self._stream_scope(tensor, async_op)

@@ -494,3 +494,24 @@ def test_a_stochastic_all_reduce_draws_one_seed(world, fused, serves):
     ws.all_reduce(torch.zeros(640, dtype=torch.bfloat16))
     assert seeds and set(seeds) == {want}
     assert codec._seed() == after
+
+
+@pytest.mark.parametrize("world", (1, 2))
+def test_shards_and_gathered_tensors_are_plain_tensors(monkeypatch, world):
+    """Whatever class of tensor is reduced or gathered, in a group of any size."""
+
+    from lowbit_comm_b200.parallel.communicator import Communicator
+
+    class Marked(torch.Tensor):
+        pass
+
+    x = torch.arange(6, dtype=torch.bfloat16).reshape(2, 3).as_subclass(Marked)
+    comm = Communicator.__new__(Communicator)
+    comm.world_size, comm.stats = world, {"peer_ops": 0}
+    workspace = type("W", (), {"all_gather": staticmethod(lambda t, outs: [o.copy_(t) for o in outs])})
+    monkeypatch.setattr(Communicator, "peer_usable", lambda self, *a: True)
+    monkeypatch.setattr(Communicator, "workspace", lambda self, *a: workspace)
+    outs = comm.all_gather(x, config=CompressionConfig())
+    assert [type(o) for o in outs] == [torch.Tensor] * world and all(torch.equal(o, x.as_subclass(torch.Tensor)) for o in outs)
+    shard = Communicator._validated_out(None, x, 4)
+    assert type(shard) is torch.Tensor and shard.shape == (4,) and shard.dtype == x.dtype
