@@ -79,6 +79,14 @@ def shutdown_communicators() -> None:
         _REGISTRY.clear()
 
 
+def _plain_empty(like: Any, shape: Any) -> Any:
+    """An uninitialized plain tensor of the type and on the device of `like`, whatever class that has."""
+
+    if type(like) is torch.Tensor:
+        return like.new_empty(shape)      # half a microsecond less than naming type and device
+    return torch.empty(shape, dtype=like.dtype, device=like.device)
+
+
 class Communicator:
     def __init__(self, process_group: Any = None, *, arena_bytes: int | None = None, extension_status=None,
                  transport: str = "auto", max_blocks: int = 0) -> None:
@@ -455,7 +463,7 @@ class Communicator:
         """Caller-owned output checks (parity: reduce_scatter_transport.py:390-431)."""
 
         if out is None:
-            return torch.empty(shard_numel, dtype=tensor.dtype, device=tensor.device)
+            return _plain_empty(tensor, shard_numel)
         if hasattr(out, "tensor") and hasattr(out, "mark_submitting"):  # an output lease
             out = out.tensor
         if tuple(out.shape) != (shard_numel,):
@@ -486,7 +494,7 @@ class Communicator:
         if self.peer_usable(tensor, config):
             ws = self.workspace(tensor, config, name)
             if self.world_size == 1:
-                outs = [torch.empty(shape, dtype=tensor.dtype, device=tensor.device)]
+                outs = [_plain_empty(tensor, shape)]
             else:      # rows of one buffer: the decode of all W payloads is then a single launch
                 outs = list(torch.empty((self.world_size,) + shape, dtype=tensor.dtype, device=tensor.device).unbind(0))
             scope, side = self._stream_scope(tensor, async_op)
