@@ -829,6 +829,10 @@ def test_native_codec_calls_and_the_general_way(ext, dtype, kw, monkeypatch):
     bytes_ = torch.zeros(2 * size(4160) + 8, dtype=torch.uint8, device="cuda")
     x, r = base[:4099], base[4160:8259] * 0.01
     whole = codec.quantize_tensor(x, cfg)
+    around = torch.full((4099, 2), 3.0, dtype=torch_dtype, device="cuda")     # every second element belongs to nobody
+    scattered = around[:, 0]
+    outer, square = torch.full((64, 128), 3.0, dtype=torch_dtype, device="cuda"), base[:4096].view(64, 64)
+    inner = outer[:, :64]
     encodes = {
         "plain": lambda: codec.quantize_tensor(x, cfg),
         "shaped": lambda: codec.quantize_tensor(base[:4096].view(16, 256), cfg),
@@ -846,6 +850,8 @@ def test_native_codec_calls_and_the_general_way(ext, dtype, kw, monkeypatch):
         "residual too short": lambda: codec.quantize_tensor(x, cfg, residual=r[:-1]),
         "residual on the host": lambda: codec.quantize_tensor(x, cfg, residual=r.cpu()),
         "whole numbers": lambda: codec.quantize_tensor(torch.ones(64, dtype=torch.int32, device="cuda"), cfg),
+        "strided prepared": lambda: (codec.quantize_tensor(square, cfg, residual=r[:4096], prepared_out=inner), outer.clone())[1],
+        "prepared with one stride": lambda: codec.quantize_tensor(x, cfg, residual=r, prepared_out=scattered),
         "prepared": lambda: torch.cat([codec.quantize_tensor(x, cfg, residual=r, prepared_out=(p := torch.empty_like(x))).float(), p.float()]),
     }
     decodes = {
@@ -861,7 +867,8 @@ def test_native_codec_calls_and_the_general_way(ext, dtype, kw, monkeypatch):
         "output": lambda: codec.dequantize_tensor(whole, (4099,), cfg, dtype=dtype, output=torch.empty_like(x)),
         "output of another shape": lambda: codec.dequantize_tensor(whole, (1, 4099), cfg, dtype=dtype, output=torch.empty_like(x)),
         "output of another type": lambda: codec.dequantize_tensor(whole, (4099,), cfg, dtype=dtype, output=torch.empty_like(x, dtype=DTYPES[other])),
-        "strided output": lambda: codec.dequantize_tensor(whole, (4099,), cfg, dtype=dtype, output=base[:8198:2].clone().as_strided((4099,), (1,))),
+        "strided output": lambda: codec.dequantize_tensor(whole, (4099,), cfg, dtype=dtype, output=scattered),
+        "strided payload": lambda: codec.dequantize_tensor(torch.stack([whole, whole], 1)[:, 0], (4099,), cfg, dtype=dtype),
         "sum": lambda: codec.dequantize_tensor(whole, (4099,), cfg, dtype=dtype, output=r.clone(), reduce_op="sum"),
         "payload too short": lambda: codec.dequantize_tensor(whole[:-2], (4099,), cfg, dtype=dtype),
         "unknown type": lambda: codec.dequantize_tensor(whole, (4099,), cfg, dtype="int8"),
@@ -876,7 +883,18 @@ def test_native_codec_calls_and_the_general_way(ext, dtype, kw, monkeypatch):
             return type(error)
         return result.shape, result.dtype, result.contiguous().view(torch.uint8).cpu().numpy().tobytes()
 
-    native = {name: outcome(call) for calls in (encodes, decodes) for name, call in calls.items()}
+    def every_outcome():
+        around.fill_(3.0)
+        outer.fill_(3.0)
+        got = {("encode", name): outcome(call) for name, call in encodes.items()}
+        got.update({("decode", name): outcome(call) for name, call in decodes.items()})
+        want = oracle.prepare(x[:4096].cpu(), r[:4096].cpu()).view(64, 64)
+        assert torch.equal(inner.cpu(), want) and bool((outer[:, 64:] == 3.0).all())
+        assert bool((around == 3.0).all())                       # strided outputs of one dimension are refused untouched
+        assert got["decode", "strided output"] is ValueError and got["decode", "strided payload"] is ValueError
+        return got
+
+    native = every_outcome()
     taken = {"encode": 0, "decode": 0}
 
     class General:
@@ -891,7 +909,7 @@ def test_native_codec_calls_and_the_general_way(ext, dtype, kw, monkeypatch):
 
     monkeypatch.setattr(codec, "require_extension", lambda status=None: General())
     assert load_cuda_extension().available
-    general = {name: outcome(call) for calls in (encodes, decodes) for name, call in calls.items()}
+    general = every_outcome()
     assert {name for name in native if native[name] != general[name]} == set()
     assert taken["encode"] >= 5 and taken["decode"] >= 4
 
