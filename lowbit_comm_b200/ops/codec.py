@@ -1,12 +1,16 @@
 """Codec facade: the functions transports call to (de)quantize tensors.
 
 Parity: ccdl_comm/quantization/codec.py:104-498 (same public names and
-argument order).  CUDA tensors go to the sm_100a extension — through
-`quant_push` / `reduce` to the kernels of `csrc/codec_kernels.cu` for the
-production profile (linear, top-k 0, deterministic), to the general kernels
-otherwise.  CPU tensors go to the bit-exact
-torch oracle, which makes every transport testable without a GPU.  A CUDA
-tensor without the extension is an error, never a silent fallback.
+argument order).  CUDA tensors go to the sm_100a extension: to the kernels of
+`csrc/codec_kernels.cu` for the production profile (linear, top-k 0,
+deterministic), to the general kernels otherwise.  Dense tensors are encoded and
+decoded by one native call each (`codec_encode`, `codec_decode`), which settles
+sizes, checks and allocation; what it leaves alone (strided tensors, pinned
+payloads, stochastic rounding, sums into an output, every error) goes through
+`quant_push` / `reduce` or `quant_general` / `dequant_general`.  CPU tensors go
+to the bit-exact torch oracle or its C++ twin, which makes every transport
+testable without a GPU.  A CUDA tensor without the extension is an error, never a
+silent fallback.
 """
 
 from __future__ import annotations

@@ -102,6 +102,10 @@ LbcWait make_wait(const WaitArg& arg) {
 }
 
 int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+// Codes, scales and, with kept values, an index word and the values of every group.
+int64_t payload_bytes(int64_t numel, int64_t width, int group_size, int bit, int topk) {
+    return ceil_div(numel, group_size) * (group_size * bit / 8 + (topk == 0 ? 1 : topk + 2) * width);
+}
 
 // ---------------------------------------------------------------------------
 void quant_push(const at::Tensor& x, const std::optional<at::Tensor>& residual,
@@ -221,8 +225,7 @@ void quant_general(const at::Tensor& x, const std::optional<at::Tensor>& residua
     p.residual = opt_ptr(residual, x, "residual");
     p.prepared_out = const_cast<void*>(opt_ptr(prepared_out, x, "prepared_out"));
     p.numel = x.numel();
-    const int64_t meta_words = topk == 0 ? 1 : (topk == 1 ? 3 : 4);
-    const int64_t need = ceil_div(p.numel, group_size) * (group_size * bit / 8 + meta_words * x.element_size());
+    const int64_t need = payload_bytes(p.numel, x.element_size(), group_size, bit, topk);
     TORCH_CHECK(out.numel() == need, "output has an invalid quantized payload size: ", out.numel(), " != ", need);
     p.out = out.data_ptr<uint8_t>();
     check_words(p.out, p.dtype, "payload");
@@ -244,8 +247,7 @@ void dequant_general(const at::Tensor& src, at::Tensor& out, int group_size, int
     p.quant_type = quant_type;
     p.compact = compact ? 1 : 0;
     p.numel = out.numel();
-    const int64_t meta_words = topk == 0 ? 1 : (topk == 1 ? 3 : 4);
-    const int64_t need = ceil_div(p.numel, group_size) * (group_size * bit / 8 + meta_words * out.element_size());
+    const int64_t need = payload_bytes(p.numel, out.element_size(), group_size, bit, topk);
     TORCH_CHECK(src.numel() == need, "payload has an invalid size: ", src.numel(), " != ", need);
     p.src = src.data_ptr<uint8_t>();
     check_words(p.src, p.dtype, "payload");
@@ -352,16 +354,14 @@ void reduce_general(const Ptrs& src, at::Tensor& out, int group_size, int bit, i
 }
 
 // ---- whole codec calls: sizes, checks, allocation and the launch in one crossing --------------------------------
-// The forms that jobs use all the time: dense tensors of one GPU, deterministic rounding.  Anything else (and everything
-// that is an error) gives None and launches nothing; the caller then goes the general way, which says what is wrong.
+// The forms that jobs use all the time: dense tensors of one GPU, deterministic rounding.  Anything else, and sizes, types
+// and addresses that do not fit each other, gives None and launches nothing; the caller then goes the general way, which says what is
+// wrong.  (Allocations and launches that fail raise here as they do there.)
 bool plain(const at::Tensor& t, const at::Device& device) {
     return t.is_cuda() && t.device() == device && t.layout() == at::kStrided && t.is_contiguous();
 }
 bool on_words(const at::Tensor& payload, int dtype) {
     return (reinterpret_cast<uintptr_t>(payload.data_ptr()) & (dtype == LBC_FP32 ? 3 : 1)) == 0;
-}
-int64_t payload_bytes(int64_t numel, int64_t width, int group_size, int bit, int topk) {
-    return ceil_div(numel, group_size) * (group_size * bit / 8 + (topk == 0 ? 1 : topk + 2) * width);
 }
 
 std::optional<at::Tensor> codec_encode(const at::Tensor& x, const std::optional<at::Tensor>& output,

@@ -453,8 +453,9 @@ __device__ __forceinline__ uint32_t quant_bits(float v, float mul) {
     r = fminf(fmaxf(r, kRoundMagic - float(LIM)), kRoundMagic + float(LIM));
     return __float_as_uint(r);
 }
-// s / LIM, correctly rounded (every finite s was tried): the product with 1 / LIM and one Newton correction by its exact
-// remainder, five instructions and no branch.
+// s / LIM, correctly rounded for every finite s (all were tried) but -0, which gives +0 and is no scale: the product with 1 / LIM
+// and one Newton correction by its exact remainder (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000", 1990), five instructions and no branch.
 template <int LIM>
 __device__ __forceinline__ float over_limit(float s) {
     constexpr float inverse = 1.0f / float(LIM);

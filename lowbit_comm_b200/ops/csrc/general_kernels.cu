@@ -20,13 +20,14 @@
 // Measured on a B200: encode + decode of 5 M fp32 elements, e2m1 code-book, 81 -> 27 us (the search in a table in
 // constant memory took one pass per distinct entry in a warp); all-reduce of one rank, 32 Mi bf16 elements, one kept
 // value per group, 107 -> 72 us.  Then, without the clamp and the NaN test where the selection has shown that no value
-// needs them, without a trip through packed bytes, and with a block per tile: 72 -> 36 us (the SM's issue slots are 68-72 %
-// busy, DRAM 41 %), and 81 -> 25 us for the code-book.  Then, with a look-up instead of fourteen thresholds: 24.5 -> 18.4 us for
-// the code-book; encode of 16 MiB, beyond L2, bf16 22.5 -> 14.5 us, fp32 14.0 -> 8.6, one-rank pass bf16 22.7 -> 14.5.
-// The one-rank pass without the places of the kept elements: 35.9 -> 30.8 us (32 Mi bf16 elements, one kept value); of 16 MiB
-// beyond L2, two kept values, bf16 14.4 -> 12.4 us, fp32 12.4 -> 10.3.  Each kernel started before the one ahead of it ends: 29.2 us, and
-// 15.4 us for the code-book; 12.2 us with the encoder for local payloads and native calls around both.  The rare warps of the one-rank pass out of line, its group steps without loops, its sums and products two
-// to an instruction, 32 Mi elements beyond L2: bf16 29.6 -> 26.6 us, two kept values 30.6 -> 28.2, fp16 in 4 bits 29.1 -> 26.4.
+// needs them, without a trip through packed bytes, and with a block per tile: 72 -> 36 us, and 81 -> 25 us for the
+// code-book.  Then, with a look-up instead of fourteen thresholds: 24.5 -> 18.4 us for the code-book; encode of 16 MiB,
+// beyond L2, bf16 22.5 -> 14.5 us, fp32 14.0 -> 8.6, one-rank pass bf16 22.7 -> 14.5.  The one-rank pass without the
+// places of the kept elements: 35.9 -> 30.8 us (32 Mi bf16 elements, one kept value); of 16 MiB beyond L2, two kept
+// values, bf16 14.4 -> 12.4 us, fp32 12.4 -> 10.3.  Each kernel started before the one ahead of it ends: 29.2 us, and
+// 15.4 us for the code-book; 12.3 us with the encoder for local payloads and native calls around both.  The rare warps
+// of the one-rank pass out of line, its group steps without loops, its sums and products two to an instruction, 32 Mi
+// elements beyond L2: bf16 29.6 -> 26.6 us, two kept values 30.6 -> 28.2, fp16 in 4 bits 29.1 -> 26.4.
 
 #include <cmath>
 #include <cstring>
@@ -918,7 +919,7 @@ __global__ void __launch_bounds__(kThreads, 4) quant_general_kernel(const __grid
 // What bounds it: instruction issue.  Before (quant_general_kernel, which asks every chunk where it goes) and here, beyond L2: 64 MiB,
 // bf16, planar, one kept value 34.8 -> 30.6 us, two 42.0 -> 38.5, e2m1 36.8 -> 31.1, with one kept value 46.0 -> 42.1, records of e2m1
 // 38.2 -> 34.2; fp32 25.6 -> 20.7, 31.1 -> 27.5, 22.0 -> 17.4, 28.0 -> 23.2, 22.6 -> 18.0; 1 MiB bf16 3.24 -> 2.54, 3.48 -> 2.87.
-// Blocks per SM, 4 against 5 (no spills at either), 64 MiB: bf16, one kept value 32.1 / 30.6 us, two 39.8 / 40.3, e2m1 31.9 / 33.8, its
+// Blocks per SM, 4 against 5 (no spills at either in these), 64 MiB: bf16, one kept value 32.1 / 30.6 us, two 39.8 / 40.3, e2m1 31.9 / 33.8, its
 // records 34.6 / 36.1; fp32 23.0 / 21.7, 29.3 / 27.5, 19.0 / 18.9, 20.1 / 18.3, e2m1 with one kept value 23.8 / 25.1; 16 MiB bf16, one
 // kept value 10.4 / 9.5, fp32 7.8 / 7.5.
 template <typename T, int TOPK, int KIND>
@@ -1207,11 +1208,14 @@ __global__ void __launch_bounds__(kThreads, kBlocks) roundtrip_general_kernel(co
 }
 
 // A block per 4096 elements up to four times the default grid, a grid that loops above: it pays a block's set-up less
-// often.  One-rank pass, full grid against a looping one: bf16 top-k 1, 8 M elements (1.6 default grids) 12.5 / 12.5 us,
-// 16 M 20.7 / 20.6, 20 M (4.1) 24.8 / 24.2, 24 M 28.9 / 27.5, 32 M 37.1 / 35.0, 64 M 69.8 / 64.0; fp32 top-k 1, 10 M
-// 20.6 / 20.6, 20 M 36.1 / 35.0, 64 M 102.5 / 96.6.  A code-book does not care: fp32, 10 M 28.8 / 28.9, 20 M 49.4 / 49.8, 64 M
-// 146 / 147; bf16, 20 M 48.0 / 49.3, 64 M 143.6 / 144.3.  The default grid also serves blocks that meet at a flag or a
-// counter (`shared`): each costs a system-scope fence or a look at the flags.
+// often.  The line is where a looping grid began to win when a pass took half as long again.  The present one-rank pass, full grid against
+// a looping one (1184 blocks, whole waves of four or eight per SM): bf16 top-k 1, 8 Mi elements (1.7 default grids) 6.79 / 6.31 us, 16 Mi
+// 15.5 / 14.6, 20 Mi (4.3) 19.1 / 17.8, 32 Mi 29.0 / 26.5, 64 Mi 55.1 / 49.8; e2m1 9.93 / 9.33, 19.8 / 17.9, 24.6 / 21.7, 37.8 / 33.1,
+// 71.8 / 61.3; fp32 top-k 1 12.1 / 12.1, 22.1 / 22.8, 27.4 / 28.2, 43.7 / 43.3, 87.6 / 92; top-k 2 15.3 / 13.3, 24.6 / 23.9, 30.1 / 29.3,
+// 47.0 / 45.4, 91.1 / 89.1; e2m1 17.4 / 15.1, 29.0 / 26.7, 34.9 / 32.3, 53.7 / 49.4, 107 / 97.3: looping would serve all but fp32 with one
+// kept value from 8 Mi on.  Grids of other sizes, 64 Mi, 4 / 5 / 8 / 12 / 16 blocks per SM: bf16 top-k 1 49.9 / 62.4 / 49.8 / 50.4 / 50.1,
+// fp32 top-k 2 103 / 92.9 / 89.1 / 87.5 / 89.0.  The default grid also serves blocks that meet at a flag or a counter (`shared`):
+// each costs a system-scope fence or a look at the flags.
 static int general_grid(int64_t groups, int group_size, int max_blocks, bool shared) {
     int64_t want = (groups * (group_size / kElemsPerThread) + kThreads - 1) / kThreads;
     if (want < 1) want = 1;
