@@ -2,7 +2,8 @@
 
     python benchmarks/one_gpu_cases.py               # all listed cases: microseconds per pass, and its bytes at the copy rate
     python benchmarks/one_gpu_cases.py --only "mean of 8, 64 MiB bf16"
-    python benchmarks/one_gpu_cases.py --launch              # 96 Mi bf16 elements through every kernel, for ncu
+    python benchmarks/one_gpu_cases.py --launch              # 96 Mi bf16 elements through the linear kernels, for ncu
+    python benchmarks/one_gpu_cases.py --launch-general      # 32 Mi bf16 elements through the general kernels
 
 A pass is timed with CUDA events over `--passes` passes in a row that go round `--states` states prepared from different
 seeds (so inputs and outputs change from pass to pass), after 2 rounds of warm-up; the median of 7 such runs.
@@ -41,7 +42,7 @@ def microseconds(case: dict, states: int, passes: int, runs: int = 7) -> float:
 
 
 def launch_once(n: int = 96 << 20) -> None:
-    """Encode and the one-rank passes with and without error feedback, decode, and the mean of four payloads."""
+    """Linear profile: encode and the one-rank passes with and without error feedback, decode, and the mean of four payloads."""
 
     from lowbit_comm_b200 import (CompressionConfig, compressed_all_reduce, dequantize_tensor,
                                   inplace_dequantize_reduce_mean_update_error_feedback, quantize_tensor)
@@ -57,10 +58,20 @@ def launch_once(n: int = 96 << 20) -> None:
     inplace_dequantize_reduce_mean_update_error_feedback(payloads, r, out, r, config, reduce="mean")
     compressed_all_reduce(x, config=config, op="mean", strategy="auto")
     get_communicator(None).all_reduce(x, config=config, residual=r)
-    compressed_all_reduce(x, config=CompressionConfig(topk=1, allow_experimental=True), op="mean", strategy="auto")
-    small = torch.randn(n // 4, device="cuda")
-    book = CompressionConfig(bit=4, quant_type="e2m1", allow_experimental=True)
-    dequantize_tensor(quantize_tensor(small, book), (n // 4,), book, dtype="fp32")
+    torch.cuda.synchronize()
+
+
+def launch_general_once(n: int = 32 << 20) -> None:
+    """Encode, decode and the one-rank pass of the 4-bit code-book and of one and two kept values."""
+
+    from lowbit_comm_b200 import CompressionConfig, compressed_all_reduce, dequantize_tensor, quantize_tensor
+
+    cases._join_group()
+    x = torch.randn(n, device="cuda", dtype=torch.bfloat16)
+    for kw in ({"bit": 4, "quant_type": "e2m1"}, {"topk": 1}, {"topk": 2}):
+        config = CompressionConfig(allow_experimental=True, **kw)
+        dequantize_tensor(quantize_tensor(x, config), (n,), config, dtype="bf16")
+        compressed_all_reduce(x.clone(), config=config, op="mean", strategy="auto")
     torch.cuda.synchronize()
 
 
@@ -70,9 +81,12 @@ def main() -> None:
     ap.add_argument("--states", type=int, default=3)
     ap.add_argument("--passes", type=int, default=20)
     ap.add_argument("--launch", action="store_true")
+    ap.add_argument("--launch-general", action="store_true")
     args = ap.parse_args()
     if args.launch:
         launch_once()
+    elif args.launch_general:
+        launch_general_once()
     else:
         peak, kind = peak_gbs()
         for case in cases.listed():
