@@ -11,9 +11,10 @@
 // occupancy); tensors and payloads off those boundaries have kernels of their own.
 // Measured on a B200 through the public calls, int8 groups of 64, before (grid-stride kernels of fast_kernels.cu) and
 // after: encode of 32 Mi bf16 elements with error feedback 47.0 -> 39.2 us, decode of 128 Mi 94 -> 67.6 us, mean of eight payloads
-// of 32 Mi with error feedback 107 -> 89.8 us; then, each kernel started before the one ahead of it ends: 37.6 us (6.3 TB/s),
-// 65.7 us (6.2 TB/s) and 84.2 us (5.7 TB/s).  Those are passes repeated for a second; in bursts of a few milliseconds the mean of
-// eight takes 81 us: it draws the card's 1000 W, and its clock falls to 1.7 GHz.
+// of 32 Mi with error feedback 107 -> 89.8 us; then, each kernel started before the one ahead of it ends, and the scale's quotient
+// without a branch ahead of the codes: 37.5 us (6.3 TB/s), 63.9 us (6.4 TB/s) and 83.7 us (5.7 TB/s).  Those are passes repeated
+// for a second; in bursts of a few milliseconds the mean of eight takes 80.5 us: it draws the card's 1000 W, and its clock falls to
+// 1.7 GHz.
 #include <type_traits>
 
 #include "codec_device.cuh"
@@ -367,8 +368,8 @@ decode_kernel(const __grid_constant__ LbcReduce p) {
 // blocks: one payload 17.6 / 16.5 / 18.5 us, mean of two with error feedback 35.2 / 32.9 / 28.8, of eight 73.8 / 67.8 /
 // 61.6; 8-bit records, mean of eight 82.6 / 76.2 / 84.9.
 // As a branch of decode_kernel this ran out of line, element by element.  16 Mi bf16 elements, buffers in L2 (grid-stride
-// kernel of fast_kernels.cu / that branch / here): a payload on 8 bytes 14.8 / 18.8 / 11.5 us, an output one element in
-// 99.7 / 107.7 / 37.2.
+// kernel of fast_kernels.cu / that branch / here): a payload on 8 bytes 14.8 / 18.8 / 9.6 us, an output one element in
+// 99.7 / 107.7 / 35.8.
 template <typename T, int G, int BIT, bool kCompact, bool kSeveral>
 __global__ void __launch_bounds__(kThreads, kSeveral && !(kCompact && BIT == 8 && sizeof(T) == 2) ? 6 : 5)
 decode_ragged_kernel(const __grid_constant__ LbcReduce p) {

@@ -918,7 +918,7 @@ __global__ void __launch_bounds__(kThreads, 4) quant_general_kernel(const __grid
 // kCompact: records, built in shared memory.
 // What bounds it: instruction issue.  Before (quant_general_kernel, which asks every chunk where it goes) and here, beyond L2: 64 MiB,
 // bf16, planar, one kept value 34.8 -> 30.6 us, two 42.0 -> 38.5, e2m1 36.8 -> 31.1, with one kept value 46.0 -> 42.1, records of e2m1
-// 38.2 -> 34.2; fp32 25.6 -> 20.7, 31.1 -> 27.5, 22.0 -> 17.4, 28.0 -> 23.2, 22.6 -> 18.0; 1 MiB bf16 3.24 -> 2.54, 3.48 -> 2.87.
+// 38.2 -> 34.2; fp32 25.6 -> 20.7, 31.1 -> 27.5, 22.0 -> 17.4, 28.0 -> 23.2, 22.6 -> 18.0; 1 MiB in a graph, bf16, here 2.14, 2.19, 2.10, fp32 2.20, 2.51, 1.97.
 // Blocks per SM, 4 against 5 (no spills at either in these), 64 MiB: bf16, one kept value 32.1 / 30.6 us, two 39.8 / 40.3, e2m1 31.9 / 33.8, its
 // records 34.6 / 36.1; fp32 23.0 / 21.7, 29.3 / 27.5, 19.0 / 18.9, 20.1 / 18.3, e2m1 with one kept value 23.8 / 25.1; 16 MiB bf16, one
 // kept value 10.4 / 9.5, fp32 7.8 / 7.5.
