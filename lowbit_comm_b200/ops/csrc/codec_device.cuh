@@ -5,6 +5,8 @@
 // rounded to the source dtype before use), quantization/dequant_reduce_kernel.cu:38-69 (scale / L decode).
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace lbc {
@@ -15,6 +17,70 @@ __device__ __forceinline__ float group_max(float v) {
 #pragma unroll
     for (int off = lanes / 2; off > 0; off >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off, lanes));
     return v;
+}
+
+// Magnitudes of two 16-bit elements per word (the signs that come out mean nothing; NaN wins).
+template <typename T>
+__device__ __forceinline__ uint32_t abs_max2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    if constexpr (std::is_same<T, __half>::value)
+        asm("max.NaN.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    else
+        asm("max.NaN.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b) {      // NaN wins
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b, float c) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// Calls `step` with the distances of a butterfly over a group's `lanes` threads (no loop, no width: the partner of a thread
+// of an aligned group is in it anyway).
+template <typename Step>
+__device__ __forceinline__ void over_group(int lanes, const Step& step) {
+    if (lanes >= 4) step(2);
+    if (lanes >= 2) step(1);
+}
+
+// The largest magnitude of a group, NaN if one is in it: two 16-bit elements (three fp32 ones) to an instruction.
+template <typename T, int G>
+__device__ __forceinline__ float group_top(const Raw16<T>& p) {
+    constexpr int lanes = G / kElemsPerThread;
+    if constexpr (sizeof(T) == 2) {
+        const uint32_t(&w)[8] = p.part[0].w;
+        const uint32_t best = abs_max2<T>(abs_max2<T>(abs_max2<T>(w[0], w[1]), abs_max2<T>(w[2], w[3])),
+                                          abs_max2<T>(abs_max2<T>(w[4], w[5]), abs_max2<T>(w[6], w[7])));
+        uint32_t top = max(best >> 16 & 0x7fffu, best & 0x7fffu);
+        over_group(lanes, [&](int off) { top = max(top, __shfl_xor_sync(0xffffffffu, top, off)); });
+        return Src<T>::up(uint16_t(top));
+    } else {
+        float v[16];
+        up16<T>(p, v);
+        float top = fabsf(v[0]);
+#pragma unroll
+        for (int i = 1; i + 1 < 16; i += 2) top = max_nan(top, fabsf(v[i]), fabsf(v[i + 1]));
+        top = max_nan(top, fabsf(v[15]));
+        over_group(lanes, [&](int off) { top = max_nan(top, __shfl_xor_sync(0xffffffffu, top, off)); });
+        return top;
+    }
+}
+// Is the scale of every group of the warp one that limit_over takes?  Then no group holds an infinity or a NaN, no value is above
+// its scale, |value * (L / scale)| rounds to L at most, and the codes need no clamp.
+constexpr float kNearScale = 1.0e30f;
+__device__ __forceinline__ bool scales_near(float top) { return __all_sync(0xffffffffu, top < kNearScale); }
+// LIM / s, correctly rounded for every s from 1e-6 to 1e30 (all were tried): the quotient through the reciprocal with one Newton
+// correction by its exact remainder (Markstein, see over_limit), without the branch of the division.
+template <int LIM>
+__device__ __forceinline__ float limit_over(float s) {
+    const float inverse = __frcp_rn(s);
+    const float q = __fmul_rn(float(LIM), inverse);
+    return __fmaf_rn(__fmaf_rn(-q, s, float(LIM)), inverse, q);
 }
 
 // Alignment-agnostic store of `n` bytes (n = 8 or 16) held in `v`.
@@ -147,6 +213,32 @@ __device__ __forceinline__ uint4 encode16(const float (&vals)[16], float stored_
 #pragma unroll
         for (int i = 0; i < 16; ++i) (*decoded)[i] = __fmaf_rn(-float(code_of_bits(b[i])), step, vals[i]);
     }
+    if constexpr (BIT == 8) {
+        return pack16_low_bytes<sizeof(T)>(b);
+    } else {
+        const uint2 h = pack16_low_nibbles<sizeof(T)>(b);
+        return make_uint4(h.x, h.y, 0, 0);
+    }
+}
+
+// The same for a warp of scales_near, half the instructions: no clamp, no branch in the quotient, products and sums two to an
+// instruction (the product as a multiply-add with zero: a packed product before a packed sum is contracted).
+template <typename T, int BIT>
+__device__ __forceinline__ uint4 encode16_near(const float (&vals)[16], float stored_scale, float (*decoded)[16]) {
+    constexpr int lim = BIT == 8 ? 127 : 7;
+    float t[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) t[i] = vals[i];
+    fma16(t, limit_over<lim>(fmaxf(stored_scale, 1.0e-6f)), 0.0f);
+    add16(t, kRoundMagic);
+    if (decoded != nullptr) {
+        const float step = over_limit<lim>(stored_scale);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) (*decoded)[i] = __fmaf_rn(-(t[i] - kRoundMagic), step, vals[i]);
+    }
+    uint32_t b[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) b[i] = __float_as_uint(t[i]);
     if constexpr (BIT == 8) {
         return pack16_low_bytes<sizeof(T)>(b);
     } else {

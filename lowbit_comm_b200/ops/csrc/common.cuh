@@ -252,6 +252,18 @@ __device__ __forceinline__ Raw16<T> raw16(const T* p) {
     return r;
 }
 template <typename T>
+__device__ __forceinline__ Raw16<T> down16(const float (&v)[16]) {
+    Raw16<T> r;
+    if constexpr (sizeof(T) == 2) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) r.part[0].w[i] = Src<T>::down2(v[2 * i], v[2 * i + 1]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) r.part[i / 8].w[i % 8] = __float_as_uint(v[i]);
+    }
+    return r;
+}
+template <typename T>
 __device__ __forceinline__ void up16(const Raw16<T>& r, float (&v)[16]) {
     if constexpr (sizeof(T) == 2) {
 #pragma unroll
@@ -430,12 +442,22 @@ __device__ __forceinline__ void add16(float (&v)[16], float s) {
             : "+f"(v[i]), "+f"(v[i + 1]) : "f"(s));
 }
 
-// prepared = T(x + residual)
+// v = v * s + add, each with one rounding.
+__device__ __forceinline__ void fma16(float (&v)[16], float s, float add) {
+#pragma unroll
+    for (int i = 0; i < 16; i += 2)
+        asm("{.reg .b64 a, b, c; mov.b64 a, {%0, %1}; mov.b64 b, {%2, %2}; mov.b64 c, {%3, %3}; fma.rn.f32x2 a, a, b, c; mov.b64 {%0, %1}, a;}"
+            : "+f"(v[i]), "+f"(v[i + 1]) : "f"(s), "f"(add));
+}
+
+// prepared = T(x + residual), which is also returned in T
 template <typename T>
-__device__ __forceinline__ void compensate16(float (&v)[16], const float (&r)[16]) {
+__device__ __forceinline__ Raw16<T> compensate16(float (&v)[16], const float (&r)[16]) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] += r[i];
-    round16<T>(v);
+    const Raw16<T> held = down16<T>(v);
+    if constexpr (sizeof(T) == 2) up16<T>(held, v);
+    return held;
 }
 
 // ---------------------------------------------------------------------------

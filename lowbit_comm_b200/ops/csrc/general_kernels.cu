@@ -294,14 +294,6 @@ __device__ __forceinline__ constexpr uint32_t inf_bits() {
     return std::is_same<T, __half>::value ? 0x7c00u : 0x7f80u;
 }
 
-// Calls `step` with the distances of a butterfly over a group's `lanes` threads (no loop, no width: the partner of a thread
-// of an aligned group is in it anyway).
-template <typename Step>
-__device__ __forceinline__ void over_group(int lanes, const Step& step) {
-    if (lanes >= 4) step(2);
-    if (lanes >= 2) step(1);
-}
-
 // The k largest magnitudes of a group and the next one, the scale.  `v` are the thread's 16 values, `p` the same in T;
 // the `lanes` threads of a group call this together and all get the answer.  fp32: v of a kept element turns into NaN.
 template <typename T, int TOPK>
@@ -397,16 +389,6 @@ __device__ __forceinline__ GroupMeta select_group(float (&v)[16], const Packed16
 }
 
 // ---- the scale of a group without the places of what it keeps ------------------------------------------------------
-// Magnitudes of two 16-bit elements per word (the signs that come out mean nothing; NaN wins).
-template <typename T>
-__device__ __forceinline__ uint32_t abs_max2(uint32_t a, uint32_t b) {
-    uint32_t r;
-    if constexpr (std::is_same<T, __half>::value)
-        asm("max.NaN.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    else
-        asm("max.NaN.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
 template <typename T>
 __device__ __forceinline__ uint32_t abs_min2(uint32_t a, uint32_t b) {
     uint32_t r;
@@ -424,11 +406,6 @@ __device__ __forceinline__ uint32_t abs_above2(uint32_t a, uint32_t b) {
         asm("{.reg .b32 m; abs.f16x2 m, %1; set.gt.u32.f16x2 %0, m, %2;}" : "=r"(r) : "r"(a), "r"(b));
     else
         asm("{.reg .b32 m; abs.bf16x2 m, %1; set.gt.u32.bf16x2 %0, m, %2;}" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
-__device__ __forceinline__ float max_nan(float a, float b) {      // NaN wins
-    float r;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
     return r;
 }
 __device__ __forceinline__ float max3(float a, float b, float c) {

@@ -15,47 +15,68 @@
 // Measured through the public calls (bf16, int8 groups of 64): 512 Mi elements 919 -> 312 us (6.9 TB/s), 13.1 M elements
 // 41.0 -> 10.2 us, 124 M elements in 7 buckets with error feedback 637 -> 186 us; then, each kernel started before the one ahead
 // of it ends: 7.9 and 174-186 us.
+// What stays in L2 (up to about 13 M elements) is bound by instruction issue instead: 11.5 instructions per element when every value was
+// clamped and its maximum, product and sum took one each.  Now warps of finite groups take no clamp (scales_near), two elements to an
+// instruction and quotients without branches, and two chunks per thread come in above one default grid.  In a CUDA graph, bf16: 1 Mi
+// elements 1.92 -> 1.88 us, 4 Mi 3.18 -> 2.92, 13.1 M 7.77 -> 6.46 (8.1 TB/s), 33 Mi 22.7 -> 22.2; 13.1 M with a residual 17.8 -> 17.3;
+// fp32 and what is beyond L2 stay within 1 %.
 #include "codec_device.cuh"
 #include "common.cuh"
 #include "lbc_api.h"
 
 namespace lbc {
 
-// What a receiver of the codes of 16 rounded values decodes, in fp32 before the rounding to T.  With `own_error` the
-// values are replaced by this rank's quantization error, one rounding: fma(-code, step, value).
+// What a receiver of the codes of 16 rounded values decodes, in fp32 before the rounding to T; `p` are the same values in T.
+// With `own_error` the values are replaced by this rank's quantization error, one rounding: fma(-code, step, value).
 template <typename T, int G, int BIT>
-__device__ __forceinline__ void roundtrip16(float (&v)[16], float (&y)[16], bool own_error) {
+__device__ __forceinline__ void roundtrip16(const Raw16<T>& p, float (&v)[16], float (&y)[16], bool own_error) {
     constexpr int lim = BIT == 8 ? 127 : 7;
+    // the values are exact in T, so their largest magnitude is the stored scale without a rounding
+    const float top = group_top<T, G>(p);
+    if (scales_near(top)) {
+        const float mul = limit_over<lim>(fmaxf(top, 1.0e-6f));
+        const float step = over_limit<lim>(top);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) y[i] = v[i];
+        fma16(y, mul, 0.0f);                                  // (+0 for -0, which the next sum hides anyway)
+        add16(y, kRoundMagic);
+        add16(y, -kRoundMagic);                               // the codes, exactly; +0 for code 0, as the decoder has it
+        if (own_error) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = __fmaf_rn(-y[i], step, v[i]);
+        }
+        fma16(y, step, 0.0f);
+        return;
+    }
     float amax = 0.0f;
 #pragma unroll
     for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
-    // the values are exact in T, so their largest magnitude is the stored scale without a rounding
     const float stored = group_max<G>(amax);
     const float mul = float(lim) / fmaxf(stored, 1.0e-6f);
     const float step = stored / float(lim);
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-        // the clamped sum is kRoundMagic + code exactly, and so is the difference (+0 for code 0, as the decoder has it)
+        // the clamped sum is kRoundMagic + code exactly, and so is the difference
         const float code = __uint_as_float(quant_bits<lim>(v[i], mul)) - kRoundMagic;
         y[i] = __fmaf_rn(code, step, 0.0f);
         if (own_error) v[i] = __fmaf_rn(-code, step, v[i]);
     }
 }
 
-// From the prepared values to the outputs.  Convergent: the group maximum shuffles.
+// From the prepared values (`held`: the same in T) to the outputs.  Convergent: the group maximum shuffles.
 template <typename T, int G, int BIT, bool kResidual, int kFit>
-__device__ __forceinline__ void roundtrip_chunk(const LbcRoundtrip& p, float (&v)[16], int64_t first, bool live) {
+__device__ __forceinline__ void roundtrip_chunk(const LbcRoundtrip& p, const Raw16<T>& held, float (&v)[16], int64_t first,
+                                                bool live) {
     T* out = static_cast<T*>(p.out);
     T* rout = static_cast<T*>(p.residual_out);
     const bool own_error = kResidual && p.own_error != 0;
     float y[16];
-    roundtrip16<T, G, BIT>(v, y, own_error);
+    roundtrip16<T, G, BIT>(held, v, y, own_error);
     if (p.passes == 2) {
+        const Raw16<T> again = down16<T>(y);
         float z[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) z[i] = y[i];
-        round16<T>(z);
-        roundtrip16<T, G, BIT>(z, y, false);
+        up16<T>(again, z);
+        roundtrip16<T, G, BIT>(again, z, y, false);
     }
     if (!live) return;
     if (kResidual && rout != nullptr) {
@@ -79,7 +100,7 @@ __device__ __forceinline__ void roundtrip_edge(const LbcRoundtrip& p, int64_t ch
         load16_fit<T, kFit>(static_cast<const T*>(p.residual), first, p.numel, r);
         compensate16<T>(v, r);
     }
-    roundtrip_chunk<T, G, BIT, kResidual, kFit>(p, v, first, chunk < chunks);
+    roundtrip_chunk<T, G, BIT, kResidual, kFit>(p, down16<T>(v), v, first, chunk < chunks);
 }
 
 // All tensors on 32 bytes.  kResidual: the input is T(x + residual).  U chunks of 16 elements per thread are loaded before
@@ -110,9 +131,9 @@ __global__ void __launch_bounds__(kThreads) roundtrip_kernel(const LbcRoundtrip 
                 if (kResidual) {
                     float r[16];
                     up16<T>(rr[j], r);
-                    compensate16<T>(v, r);
+                    rx[j] = compensate16<T>(v, r);
                 }
-                roundtrip_chunk<T, G, BIT, kResidual, kFitWhole>(p, v, mine + j * (kThreads * kElemsPerThread), true);
+                roundtrip_chunk<T, G, BIT, kResidual, kFitWhole>(p, rx[j], v, mine + j * (kThreads * kElemsPerThread), true);
             }
         } else {
             for (int j = 0; j < U; ++j)
@@ -152,12 +173,14 @@ struct RoundtripLauncher {
             launch_chained(roundtrip_kernel<T, G, BIT, true, 1>, grid(one), stream, *p);
             return cudaGetLastError();
         }
-        // Two chunks per thread (64 bytes in flight) once there are many waves of blocks.  One chunk against two, bf16: 2 M
-        // elements 5.2 / 6.2 us (two leave SMs without a block), 4 M 6.2 / 7.0, 8 M (1.6 default grids) 9.4 / 9.2, 13 M
-        // 12.3 / 12.3, 16 M 14.4 / 13.9, 24 M 18.5 / 18.5, 32 M (6.6) 23.8 / 22.5, 40 M (8.2) 28.6 / 27.5, 64 M 43.1 / 41.6,
-        // 256 M 158 / 152.  fp32 chunks and chunks with a residual have 64 bytes in flight already.
+        // Two chunks per thread (64 bytes in flight) above one default grid.  One chunk against two, bf16, calls in a CUDA graph going round
+        // three tensors: 0.5 Mi elements 1.58 / 1.68 us, 1 Mi 1.79 / 1.68, 2 Mi 2.41 / 1.93, 3 Mi 2.43 / 2.90 (two leave SMs a
+        // block short), 4 Mi 2.94 / 2.92, 5 Mi (1.08 default grids) 3.15 / 3.08, 6 Mi 3.86 / 3.69, 8 Mi 4.45 / 4.17, 13 M 7.02 / 6.54, 16 Mi
+        // 11.3 / 10.5, 24 Mi 16.3 / 16.4, 33 Mi 21.6 / 22.0, 64 Mi 40.3 / 40.8, 256 Mi 165 / 157.  Four chunks: 8 Mi 4.34, 13 M 7.19.  Blocks
+        // of 128 threads, two chunks: 8 Mi 4.10, 13 M 6.40, 33 Mi 22.1; of 512: 4.45, 6.92, 21.6.  fp32 chunks and chunks with a residual
+        // have 64 bytes in flight already.
         if constexpr (sizeof(T) == 2) {
-            if (one > 8 * lbc_default_max_blocks()) {
+            if (one > lbc_default_max_blocks()) {
                 launch_chained(roundtrip_kernel<T, G, BIT, false, 2>, grid((one + 1) / 2), stream, *p);
                 return cudaGetLastError();
             }
