@@ -26,14 +26,15 @@ namespace lbc {
 // ---------------------------------------------------------------------------
 // encode
 // ---------------------------------------------------------------------------
-// Quantizes and stores the thread's 16 values.  Convergent (the group maximum shuffles); `span` is the warp's staging area
-// for compact records.
-template <typename T, int G, int BIT, bool kCompact, int kFit>
-__device__ __forceinline__ void encode_chunk(const LbcQuantPush& p, float (&v)[16], int64_t chunk, uint8_t* span) {
+// Quantizes and stores the thread's 16 values (`held`: the same in T).  Convergent (the group maximum shuffles); `span` is the
+// warp's staging area for compact records.  kPrepared: `held` came out of a sum.  kOwnError: this rank's quantization error may be
+// asked for (local_ef_out).
+template <typename T, int G, int BIT, bool kCompact, bool kPrepared, bool kOwnError, int kFit>
+__device__ __forceinline__ void encode_chunk(const LbcQuantPush& p, const Raw16<T>& held, float (&v)[16], int64_t chunk, uint8_t* span) {
     constexpr int lanes = G / kElemsPerThread;
     constexpr int VB = G * BIT / 8, MB = sizeof(T), CB = kElemsPerThread * BIT / 8;
     T* prep = static_cast<T*>(p.prepared_out);
-    T* lef = static_cast<T*>(p.local_ef_out);
+    T* const lef = kOwnError ? static_cast<T*>(p.local_ef_out) : nullptr;
     uint8_t* dst = p.dst[0];
     const int64_t num_groups = (p.numel + G - 1) / G;
     const int64_t first = chunk * kElemsPerThread;
@@ -41,13 +42,26 @@ __device__ __forceinline__ void encode_chunk(const LbcQuantPush& p, float (&v)[1
     const int64_t g = chunk / lanes;
     const int lane = int(chunk) & (lanes - 1);
     const int wlane = threadIdx.x & 31;
-    float amax = 0.0f;
+    float stored = group_top<T, G>(held);                         // exact in T, like the values
+    if (prep != nullptr && live) {
+        if constexpr (kPrepared && kFit == kFitWhole) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
-    const float stored = group_max<G>(amax);                      // exact in T, like the values
-    if (prep != nullptr && live) store16_fit<T, kFit>(prep, first, p.numel, v);
+            for (int h = 0; h < int(sizeof(T)) / 2; ++h) st32(prep + first + 16 / (sizeof(T) / 2) * h, held.part[h]);
+        } else {
+            store16_fit<T, kFit>(prep, first, p.numel, v);
+        }
+    }
     float err[16];
-    const uint4 codes = encode16<T, BIT>(v, stored, lef != nullptr ? &err : nullptr);
+    uint4 codes;
+    if (scales_near(stored)) {
+        codes = encode16_near<T, BIT>(v, stored, lef != nullptr ? &err : nullptr);
+    } else {
+        float amax = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
+        stored = group_max<G>(amax);
+        codes = encode16<T, BIT>(v, stored, lef != nullptr ? &err : nullptr);
+    }
     if (lef != nullptr && live) store16_fit<T, kFit>(lef, first, p.numel, err);
     if (kCompact && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
         uint8_t* rec = span + (wlane / lanes) * (VB + MB);
@@ -67,7 +81,7 @@ __device__ __forceinline__ void encode_chunk(const LbcQuantPush& p, float (&v)[1
 }
 
 // A tile with the tensor's end in it (kFitTail), or of unaligned tensors.
-template <typename T, int G, int BIT, bool kCompact, int kFit>
+template <typename T, int G, int BIT, bool kCompact, bool kOwnError, int kFit>
 __device__ __forceinline__ void encode_edge(const LbcQuantPush& p, int64_t c0, int chunks_per_thread, uint8_t* span) {
     const T* x = static_cast<const T*>(p.x);
     const T* res = static_cast<const T*>(p.residual);
@@ -80,18 +94,24 @@ __device__ __forceinline__ void encode_edge(const LbcQuantPush& p, int64_t c0, i
             load16_fit<T, kFit>(res, chunk * kElemsPerThread, p.numel, r);
             compensate16<T>(v, r);
         }
-        encode_chunk<T, G, BIT, kCompact, kFit>(p, v, chunk, span);
+        encode_chunk<T, G, BIT, kCompact, false, kOwnError, kFit>(p, down16<T>(v), v, chunk, span);
     }
 }
 
 template <int G, int BIT, typename T>
 constexpr int encode_span(bool compact) { return compact ? span_bytes(G, G * BIT / 8 + int(sizeof(T))) : 16; }
 
-// All tensors on 32 bytes (the payload may start anywhere).
-// Blocks per SM: fp32 values alone take half of the 64 registers that four blocks leave; without a residual and records
-// to turn, three blocks are as fast or faster (4 Mi elements into a payload on 8 bytes 8.3 -> 6.3 us).
+// All tensors on 32 bytes (the payload may start anywhere), no local_ef_out: what that takes in registers made the others spill.
+// Blocks per SM, us, bf16 no residual, one chunk per thread with 4 / 5 / 6, two with 4 / 5: 1 Mi elements 1.44 / 1.47 / 1.48 1.61 / 1.57,
+// 4 Mi 2.67 / 2.57 / 2.56 2.50 / 2.80, 8 Mi 4.88 / 4.69 / 4.47 4.08 / 4.13, 16 Mi 11.5 / 10.6 / 9.81 9.50 / 9.10, 64 Mi 41.0 / 36.8 / 33.8
+// 32.2 / 30.4; records 4 Mi 3.32 / 3.11 / 3.15 3.12 / 3.73, 16 Mi 13.3 / 12.0 / 11.2 11.1 / 10.4.  fp32 2 Mi 1.95 / 2.22 / 2.42 2.01 / 2.02,
+// 4 Mi 2.94 / 3.02 / 3.13 2.84 / 3.28, 8 Mi 7.93 / 7.72 / 7.68 7.70 / 7.75, 32 Mi 26.6 / 25.3 / 25.4 25.6 / 25.8; records 4 Mi 3.35 /
+// 3.39 / 3.49 3.55 / 4.07, 16 Mi 14.8 / 13.8 / 13.7 14.1 / 14.3.  With a residual, 4 / 5 / 6: bf16 4 Mi 4.30 / 4.26 / 4.22, 13 M 15.5 / 15.3 /
+// 15.4, 32 Mi 35.2 / 35.7 / 36.0, records 16 Mi 19.5 / 18.7 / 19.0; fp32 2 Mi 3.77 / 4.38 / 4.89, 16 Mi 33.2 / 33.3 / 33.3.
+template <typename T, bool kCompact, int U>
+constexpr int encode_kernel_blocks() { return (sizeof(T) == 2 && U == 2) || (kCompact && U == 1) ? 5 : 4; }
 template <typename T, int G, int BIT, bool kCompact, bool kResidual, int U>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 && !kCompact && !kResidual ? 3 : 4) encode_kernel(const __grid_constant__ LbcQuantPush p) {
+__global__ void __launch_bounds__(kThreads, encode_kernel_blocks<T, kCompact, U>()) encode_kernel(const __grid_constant__ LbcQuantPush p) {
     chain_wait();
     constexpr int lanes = G / kElemsPerThread;
     constexpr int tile_chunks = kThreads * U;
@@ -102,7 +122,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 && !kCompact && !kRes
     uint8_t* span = spans[threadIdx.x >> 5];
     for (int64_t c0 = int64_t(blockIdx.x) * tile_chunks; c0 < chunks; c0 += int64_t(gridDim.x) * tile_chunks) {
         if ((c0 + tile_chunks) * kElemsPerThread > p.numel) {
-            encode_edge<T, G, BIT, kCompact, kFitTail>(p, c0, U, span);
+            encode_edge<T, G, BIT, kCompact, false, kFitTail>(p, c0, U, span);
             continue;
         }
         const int64_t mine = c0 + threadIdx.x;
@@ -119,9 +139,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 && !kCompact && !kRes
             if (kResidual) {
                 float r[16];
                 up16<T>(rr[j], r);
-                compensate16<T>(v, r);
+                rx[j] = compensate16<T>(v, r);
             }
-            encode_chunk<T, G, BIT, kCompact, kFitWhole>(p, v, mine + j * kThreads, span);
+            encode_chunk<T, G, BIT, kCompact, kResidual, false, kFitWhole>(p, rx[j], v, mine + j * kThreads, span);
         }
     }
 }
@@ -129,14 +149,16 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 && !kCompact && !kRes
 // A tensor on another boundary (a view into a larger one), in a kernel of its own: as a branch of encode_kernel this ran
 // out of line, element by element.  16 Mi elements, the input one element in, with error feedback (grid-stride kernel of
 // fast_kernels.cu / that branch / here): bf16 45.8 / 41.1 / 27.1 us, fp32 45.6 / 61.7 / 43.5.  Blocks per SM, fp32, 4 / 3:
-// 46.3 / 43.1 us.
-template <typename T, int G, int BIT, bool kCompact>
+// 46.3 / 43.1 us.  kOwnError: with local_ef_out, tensors of any boundary; and all of fp32 on another boundary, because without it four
+// blocks fit an SM (4 Mi elements 11.5 -> 12.6 us, 16 Mi 40.9 -> 41.0).  Measured before and with encode16_near: bf16 4 Mi 6.96 -> 6.38, 16 Mi
+// 24.2 -> 22.6; with local_ef_out, aligned, as a branch of encode_kernel and here: bf16 4 Mi 6.5 / 6.0, 16 Mi 21.8 / 23.6, fp32 10.4 / 9.6, 33.8 / 33.0.
+template <typename T, int G, int BIT, bool kCompact, bool kOwnError>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 4) encode_ragged_kernel(const __grid_constant__ LbcQuantPush p) {
     chain_wait();
     const int64_t chunks = (p.numel + G - 1) / G * (G / kElemsPerThread);
     __shared__ __align__(16) uint8_t spans[kThreads / 32][encode_span<G, BIT, T>(kCompact)];
     for (int64_t c0 = int64_t(blockIdx.x) * kThreads; c0 < chunks; c0 += int64_t(gridDim.x) * kThreads)
-        encode_edge<T, G, BIT, kCompact, kFitRagged>(p, c0, 1, spans[threadIdx.x >> 5]);
+        encode_edge<T, G, BIT, kCompact, kOwnError, kFitRagged>(p, c0, 1, spans[threadIdx.x >> 5]);
 }
 
 template <typename T, int G, int BIT>
@@ -151,27 +173,24 @@ struct EncodeLauncher {
         };
         const auto go = [&](auto compact) {
             constexpr bool kCompact = decltype(compact)::value;
-            if (!on_boundary(32, p->x, p->residual, p->prepared_out, p->local_ef_out)) {
-                launch_chained(encode_ragged_kernel<T, G, BIT, kCompact>, grid(one), stream, *p);
+            const bool ragged = !on_boundary(32, p->x, p->residual, p->prepared_out);
+            if (p->local_ef_out != nullptr || (ragged && sizeof(T) == 4)) {
+                launch_chained(encode_ragged_kernel<T, G, BIT, kCompact, true>, grid(one), stream, *p);
+                return;
+            }
+            if (ragged) {
+                if constexpr (sizeof(T) == 2) launch_chained(encode_ragged_kernel<T, G, BIT, kCompact, false>, grid(one), stream, *p);
                 return;
             }
             if (p->residual != nullptr) {
                 launch_chained(encode_kernel<T, G, BIT, kCompact, true, 1>, grid(one), stream, *p);
                 return;
             }
-            // Above one default grid.  Two chunks per thread, but for fp32 records, which gain nothing from them: those
-            // loop over the default grid.  bf16, one chunk against two, planar: 4 M elements (0.8 grids) 6.6 / 7.1 us, 6 M
-            // 8.2 / 8.2, 8 M 10.3 / 8.3, 16 M 14.4 / 12.4, 64 M 47.2 / 36.9; records: 4 M 8.1 / 8.3, 6 M 9.0 / 9.9,
-            // 10 M 12.3 / 12.3, 16 M 16.4 / 14.5, 64 M 53.4 / 45.0.  fp32, planar payload on 16 bytes / on 8, one chunk against two: 16 Mi elements
-            // 18.5 / 18.7 -> 16.5 / 18.0 us, 32 Mi 33.3 / 34.9 -> 29.1 / 30.8; records, full against looping grid: 16 Mi
-            // 18.5 -> 18.3 us, 20 M 20.8 -> 20.6, 32 Mi 34.0 -> 30.9 (all with inputs beyond L2).
-            if (one > lbc_default_max_blocks()) {
-                if constexpr (sizeof(T) == 2 || !kCompact) {
+            // Two chunks per thread above one default grid (4.85 M elements), but for fp32 records, which gain nothing from them: the
+            // figures are at the kernel.
+            if constexpr (sizeof(T) == 2 || !kCompact) {
+                if (one > lbc_default_max_blocks()) {
                     launch_chained(encode_kernel<T, G, BIT, kCompact, false, 2>, grid((one + 1) / 2), stream, *p);
-                    return;
-                }
-                if (p->max_blocks <= 0) {
-                    launch_chained(encode_kernel<T, G, BIT, kCompact, false, 1>, lbc_default_max_blocks(), stream, *p);
                     return;
                 }
             }

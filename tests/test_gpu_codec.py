@@ -1071,3 +1071,39 @@ def test_a_general_payload_of_this_gpu_raises_its_signal(ext, kw, where):
     assert lib.lbc_quant_general(ctypes.byref(call), torch.cuda.current_stream().cuda_stream) == 0
     assert torch.equal(raw[where:where + want.numel()].cpu(), want)
     assert flags.tolist() == [0, 0, 0, 7, 0, 0, 0, 0] and counter.item() == 0
+
+
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("bit,group,compact", [(8, 64, False), (8, 16, True), (4, 32, False)])
+@pytest.mark.parametrize("n", (4096, 4096 * 3 + 513, 5_000_000))
+def test_linear_codes_of_scales_that_need_the_clamp(ext, dtype, bit, group, compact, n):
+    """Groups with an infinity, a NaN or a scale around 1e30 (where the quotient goes another way) between ordinary ones,
+    in the first, a middle and the last tile, one and two chunks per thread: a NaN (an infinity times zero) gets the lowest
+    code, as the clamp gives it.  Every operation is one rounding, so the bytes are the same."""
+
+    cfg = CompressionConfig(bit=bit, group_size=group, compact=compact, allow_experimental=True)
+    T, lim, inf = DTYPES[dtype], 127.0 if bit == 8 else 7.0, float("inf")
+    x = _data(n, T, seed=11)
+    edge = torch.tensor([1e30 if dtype != "fp16" else 6e4], dtype=T).view(torch.int32 if dtype == "fp32" else torch.int16)
+    sizes = [(edge + k).view(T).item() for k in (-1, 0, 1)] + [torch.finfo(T).max, torch.finfo(T).smallest_normal, 1e-6]
+    for at in (0, (n // 2) // 512 * 512 + 64, (n - 1) // 512 * 512 - 1024):
+        for k, size in enumerate(sizes):                # one group of a warp each, its neighbours untouched
+            x[at + 2 * k * group % 512:][:3] = torch.tensor([size, -size, size / 3]).to(T)
+        x[at + 512:][:3] = torch.tensor([inf, 1.0, float("nan")]).to(T)
+        x[at + 512 + group:][:2] = torch.tensor([float("nan"), -2.0]).to(T)
+    values = oracle._grouped(x, group).float()
+    stored = torch.nan_to_num(values.abs(), nan=0.0, posinf=inf).amax(1).to(T)
+    t = values * (torch.tensor(lim) / stored.float().clamp_min(1e-6))[:, None]      # (a number / tensor takes two roundings)
+    codes = torch.where(t.isnan(), -lim, t.round().clamp(-lim, lim)).to(torch.int64) & (255 if bit == 8 else 15)
+    words = oracle._pack_words(codes, bit, x.element_size())
+    scales = stored.view(torch.uint8).reshape(len(stored), -1)
+    want = torch.cat([words, scales], 1).reshape(-1) if compact else torch.cat([words.reshape(-1), scales.reshape(-1)])
+    finite = x.isfinite()
+    assert torch.equal(codec.quantize_tensor(x.cuda(), cfg).cpu(), want)
+    r = torch.zeros_like(x).cuda()
+    prepared = torch.empty_like(r)
+    assert torch.equal(codec.quantize_tensor(x.cuda(), cfg, residual=r, prepared_out=prepared).cpu(), want)
+    assert torch.equal(prepared.cpu()[finite], x[finite]) and bool((prepared.cpu().isnan() == x.isnan()).all())
+    wide = torch.empty(n + 1, dtype=T, device="cuda")    # one element in: the kernel of unaligned tensors
+    wide[1:].copy_(x)
+    assert torch.equal(codec.quantize_tensor(wide[1:], cfg).cpu(), want)
