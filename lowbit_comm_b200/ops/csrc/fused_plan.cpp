@@ -213,23 +213,29 @@ class FusedAllReducePlan {
     }
 
     // Reduce-scatter to a dense shard: rank r receives the reduced elements [r * shard_numel, (r + 1) * shard_numel)
-    // in `out_shard` (shard_numel = shard_groups * group size; the caller has zeroed what lies past the tensor's
-    // end).  With a residual, error feedback uses this rank's own quantization error, written back in place.
+    // in `out_shard` (shard_numel = shard_groups * group size), zeros past the tensor's end.  With a residual, error
+    // feedback uses this rank's own quantization error, written back in place.
     // Three launches (quantize-and-scatter, gate, reduce), one binding crossing.
     int reduce_scatter(uintptr_t x, uintptr_t out_shard, uintptr_t residual, int64_t numel, double scale,
                        bool update_residual, unsigned int epoch, uintptr_t stream_ptr) {
         if (numel < 0 || numel > max_numel_) throw std::invalid_argument("numel exceeds the workspace capacity");
         if (numel == 0) return 0;
         cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_ptr);
-        if (one_pass_ok(world_, x, out_shard, residual, numel * elem_bytes_)) {
-            const LbcRoundtrip p = one_pass(dtype_, group_, bit_, x, out_shard, residual, numel, 1, update_residual,
-                                            true, max_blocks_);
+        const int64_t groups = ceil_div(numel, group_);
+        const int64_t shard_groups = round_up(ceil_div(groups, world_), kAlignGroups);
+        const int64_t shard_numel = shard_groups * group_;
+        const int64_t valid = std::max<int64_t>(0, std::min(numel, (rank_ + 1) * shard_numel) - rank_ * shard_numel);
+        const uintptr_t bytes = numel * elem_bytes_, pad_at = out_shard + valid * elem_bytes_, pad_bytes = (shard_numel - valid) * elem_bytes_;
+        const auto off_pad = [&](uintptr_t in) { return in == 0 || in + bytes <= pad_at || pad_at + pad_bytes <= in; };
+        if (one_pass_ok(world_, x, out_shard, residual, bytes) && off_pad(x) && off_pad(residual)) {
+            LbcRoundtrip p = one_pass(dtype_, group_, bit_, x, out_shard, residual, numel, 1, update_residual, true, max_blocks_);
+            p.pad = static_cast<int>(shard_numel - valid);
             check(lbc_roundtrip(&p, stream), "roundtrip");
             return 1;
         }
+        if (valid < shard_numel)
+            check(cudaMemsetAsync(reinterpret_cast<void*>(pad_at), 0, pad_bytes, stream), "memset(shard's end)");
         const int parity = static_cast<int>(epoch & 1u);
-        const int64_t groups = ceil_div(numel, group_);
-        const int64_t shard_groups = round_up(ceil_div(groups, world_), kAlignGroups);
         Regions r;
         r.channel = channels_[0];
         r.shard_stride = round_up(shard_groups * group_bytes_, 256);
@@ -257,9 +263,6 @@ class FusedAllReducePlan {
         fill_signal(q.signal, r.channel, kPhaseRS, epoch);
         check(lbc_quant_push(&q, stream), "quant_push(scatter)");
 
-        const int64_t shard_numel = shard_groups * group_;
-        const int64_t lo = rank_ * shard_numel;
-        const int64_t valid = std::max<int64_t>(0, std::min(numel, lo + shard_numel) - lo);
         LbcReduce k = base_reduce(valid, scale);
         k.num_src = world_;
         for (int s = 0; s < world_; ++s)

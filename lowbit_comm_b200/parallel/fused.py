@@ -560,10 +560,11 @@ class FusedWorkspace:
         parity = epoch & 1
         valid = geo.shard_valid_numel(self.group.rank)
         flat_out = out_shard if out_shard.dim() == 1 else out_shard.reshape(-1)
-        if valid < geo.shard_numel:
+        native = self._native is not None and self.phase_timer is None
+        if valid < geo.shard_numel and not (native and geo.numel):
             flat_out[valid:].zero_()
-        if self._native is not None and self.phase_timer is None and hasattr(self._native, "reduce_scatter"):
-            # hot path: one binding crossing for the three launches
+        if native:
+            # hot path: one binding crossing for the three launches (one rank: for the one), zeros past the end included
             if geo.numel:
                 self.launches += self._native.reduce_scatter(
                     x.data_ptr(), flat_out.data_ptr(), 0 if res is None else res.data_ptr(), geo.numel, self._scale(op),

@@ -614,3 +614,36 @@ def test_one_rank_pass_matches_the_codec(ext, engine, dtype, bit, group, passes)
     finally:
         groups[0].process_group = None
         PeerGroup.close_loopback(groups)
+
+
+@pytest.mark.parametrize("dtype,bit,group", [("bf16", 8, 64), ("fp16", 4, 32), ("fp32", 8, 16)])
+def test_one_rank_shard_ends_in_zeros(ext, dtype, bit, group):
+    """The one pass writes decode(encode(x)) and zeros up to the shard's end, and nothing behind it: whole and ragged
+    sizes around 8 groups (the shard's unit) and a block's 4096 elements, and tensors off their vectors."""
+
+    cfg = CompressionConfig(bit=bit, group_size=group, allow_experimental=True)
+    groups, wss = _make(1, dtype, cfg, 20_000)
+    try:
+        ws = wss[0]
+        groups[0].process_group = object()          # the native plan serves real process groups only
+        ws._ensure_legacy()
+        ws._build_native()
+        for n in (1, group, 8 * group - 1, 8 * group, 8 * group + 1, 4095, 4096, 4097, 12_288, 19_999):
+            geo = geometry(n, 1, dtype, cfg)
+            x = _inputs(1, n, dtype, seed=n)[0]
+            want = torch.zeros(geo.shard_numel, dtype=DT[dtype])
+            want[:n] = oracle.decode(oracle.encode(x, cfg), n, cfg, dtype)
+            for skew in (0, 1):
+                source = torch.empty(n + skew, dtype=DT[dtype], device="cuda")[skew:]
+                source.copy_(x)
+                base = torch.full((geo.shard_numel + 64 + skew,), 7.0, dtype=DT[dtype], device="cuda")
+                before = ws.launches
+                ws.reduce_scatter(source, base[skew:skew + geo.shard_numel])
+                assert ws.launches == before + 1
+                assert torch.equal(base[skew:skew + geo.shard_numel].cpu().view(torch.uint8), want.view(torch.uint8)), (n, skew)
+                assert bool((base[:skew] == 7).all()) and bool((base[skew + geo.shard_numel:] == 7).all()), (n, skew)
+        torch.cuda.synchronize()
+        groups[0].check_status()
+    finally:
+        groups[0].process_group = None
+        PeerGroup.close_loopback(groups)
