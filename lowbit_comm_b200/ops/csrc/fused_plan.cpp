@@ -27,6 +27,9 @@
 #include "fused_plan.h"
 
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/jit/python/pybind_utils.h>
+#include <torch/extension.h>
 
 #include <algorithm>
 #include <stdexcept>
@@ -80,6 +83,30 @@ LbcRoundtrip one_pass(int dtype, int group, int bit, uintptr_t x, uintptr_t out,
     p.own_error = residual != 0 && update_residual && own_error ? 1 : 0;
     p.max_blocks = max_blocks;
     return p;
+}
+
+// ---- whole calls of a group of one rank: checks, allocation and the launch in one crossing -------------------------
+// They serve dense tensors of one GPU.  Anything else, and a group whose status word is not clear, gives None (false) and launches
+// nothing; the caller then goes the general way, which says what is wrong.
+bool plain(const at::Tensor& t, const at::Device& device) {
+    return t.is_cuda() && t.device() == device && t.layout() == at::kStrided && t.is_contiguous();
+}
+bool of_type(const at::Tensor& t, int dtype) {
+    const at::ScalarType type = t.scalar_type();
+    return type == (dtype == LBC_FP16 ? at::kHalf : dtype == LBC_BF16 ? at::kBFloat16 : at::kFloat);
+}
+bool like(const std::optional<at::Tensor>& t, const at::Tensor& x) {
+    return !t.has_value() || (plain(*t, x.device()) && t->scalar_type() == x.scalar_type() && t->numel() == x.numel());
+}
+bool status_clear_at(uintptr_t host) { return host != 0 && *reinterpret_cast<const volatile unsigned int*>(host) == 0u; }
+uintptr_t address(const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()); }
+uintptr_t address(const std::optional<at::Tensor>& t) { return t.has_value() ? address(*t) : 0; }
+
+// Completes `future` with `value` (a tensor, as Python holds it) on the current stream of its device.  `set_result` finds the storages
+// of a value by pickling it; here they are given.
+void complete(torch::jit::PythonFutureWrapper& future, const py::object& value, const at::Tensor& tensor) {
+    std::vector<c10::weak_intrusive_ptr<c10::StorageImpl>> storages{tensor.storage().getWeakStorageImpl()};
+    future.fut->markCompleted(torch::jit::toIValue(value, c10::PyObjectType::get()), std::move(storages));
 }
 
 struct Regions {        // byte offsets inside every rank's arena, for one chunk
@@ -212,6 +239,29 @@ class FusedAllReducePlan {
         return true;
     }
 
+    // All-gather and reduce-scatter to a dense shard of one rank, into tensors of their own (see `plain`).
+    std::optional<at::Tensor> one_rank_gather(const at::Tensor& x, uintptr_t status_host) const {
+        const int64_t n = x.numel();
+        if (world_ != 1 || n == 0 || n > max_numel_ || !plain(x, x.device()) || !of_type(x, dtype_) || !status_clear_at(status_host))
+            return std::nullopt;
+        c10::cuda::CUDAGuard guard(x.device());
+        at::Tensor out = at::empty(x.sizes(), x.options());
+        launch(one_pass(dtype_, group_, bit_, address(x), address(out), 0, n, 1, false, false, max_blocks_));
+        return out;
+    }
+    std::optional<at::Tensor> one_rank_shard(const at::Tensor& x, uintptr_t status_host) const {
+        const int64_t n = x.numel();
+        if (world_ != 1 || n == 0 || n > max_numel_ || !plain(x, x.device()) || !of_type(x, dtype_) || !status_clear_at(status_host))
+            return std::nullopt;
+        c10::cuda::CUDAGuard guard(x.device());
+        const int64_t shard_numel = round_up(ceil_div(n, group_), kAlignGroups) * group_;
+        at::Tensor out = at::empty({shard_numel}, x.options());
+        LbcRoundtrip p = one_pass(dtype_, group_, bit_, address(x), address(out), 0, n, 1, false, true, max_blocks_);
+        p.pad = static_cast<int>(shard_numel - n);
+        launch(p);
+        return out;
+    }
+
     // Reduce-scatter to a dense shard: rank r receives the reduced elements [r * shard_numel, (r + 1) * shard_numel)
     // in `out_shard` (shard_numel = shard_groups * group size), zeros past the tensor's end.  With a residual, error
     // feedback uses this rank's own quantization error, written back in place.
@@ -276,6 +326,8 @@ class FusedAllReducePlan {
     }
 
   private:
+    static void launch(const LbcRoundtrip& p) { check(lbc_roundtrip(&p, at::cuda::getCurrentCUDAStream()), "roundtrip"); }
+
     struct Side {
         cudaStream_t stream = nullptr;
         cudaEvent_t done = nullptr;
@@ -537,7 +589,51 @@ class PipeAllReducePlan {
         return launches + 1;
     }
 
+    // The all-reduce of one rank, in place or into `out`, on the current stream.
+    std::optional<at::Tensor> one_rank(const at::Tensor& x, const std::optional<at::Tensor>& out,
+                                       const std::optional<at::Tensor>& residual, int passes, bool update_residual, bool ef_local,
+                                       uintptr_t status_host) const {
+        if (!one_rank_serves(x, out, residual, passes, status_host)) return std::nullopt;
+        c10::cuda::CUDAGuard guard(x.device());
+        const at::Tensor& target = out.has_value() ? *out : x;
+        launch(x, target, residual, passes, update_residual, ef_local, at::cuda::getCurrentCUDAStream());
+        return target;
+    }
+
+    // A bucket of one rank, in place on the stream with the id `side` behind what the current one holds; `future` is completed there.
+    bool one_rank_bucket(const py::object& bucket, const std::optional<at::Tensor>& residual, int passes, bool update_residual,
+                         bool ef_local, int64_t side, torch::jit::PythonFutureWrapper& future, uintptr_t status_host) const {
+        const at::Tensor x = bucket.cast<at::Tensor>();
+        if (!one_rank_serves(x, std::nullopt, residual, passes, status_host)) return false;
+        c10::cuda::CUDAGuard guard(x.device());
+        const auto stream = at::cuda::CUDAStream::unpack3(side, x.device().index(), c10::DeviceType::CUDA);
+        cudaEvent_t event = nullptr;
+        check(cudaEventCreateWithFlags(&event, cudaEventDisableTiming), "cudaEventCreateWithFlags");
+        cudaError_t err = cudaEventRecord(event, at::cuda::getCurrentCUDAStream());
+        if (err == cudaSuccess) err = cudaStreamWaitEvent(stream, event, 0);
+        cudaEventDestroy(event);      // released when the device is through with it
+        check(err, "order streams");
+        c10::cuda::CUDAStreamGuard on_side(stream);
+        launch(x, x, residual, passes, update_residual, ef_local, stream);
+        complete(future, bucket, x);
+        return true;
+    }
+
   private:
+    bool one_rank_serves(const at::Tensor& x, const std::optional<at::Tensor>& out, const std::optional<at::Tensor>& residual,
+                         int passes, uintptr_t status_host) const {
+        const int64_t n = x.numel();
+        return world_ == 1 && profile_ == 0 && n > 0 && n <= max_numel_ && (passes == 1 || passes == 2) && plain(x, x.device()) &&
+               of_type(x, dtype_) && like(out, x) && like(residual, x) && status_clear_at(status_host) &&
+               one_pass_ok(1, address(x), out.has_value() ? address(*out) : address(x), address(residual), x.nbytes());
+    }
+    void launch(const at::Tensor& x, const at::Tensor& out, const std::optional<at::Tensor>& residual, int passes,
+                bool update_residual, bool ef_local, cudaStream_t stream) const {
+        const LbcRoundtrip p = one_pass(dtype_, group_, bit_, address(x), address(out), address(residual), x.numel(), passes,
+                                        update_residual, ef_local, max_blocks_);
+        check(lbc_roundtrip(&p, stream), "roundtrip");
+    }
+
     int dtype_, group_, bit_, rank_, world_ = 1;
     std::vector<uintptr_t> peers_;
     int64_t q_off_, q_bytes_, ag_off_, ag_bytes_, ctl_off_;
@@ -567,6 +663,8 @@ void bind_fused_plan(py::module_& m) {
         .def("all_reduce", &FusedAllReducePlan::all_reduce, py::arg("x"), py::arg("out"), py::arg("residual"),
              py::arg("numel"), py::arg("stages"), py::arg("scale"), py::arg("update_residual"), py::arg("ef_local"),
              py::arg("epoch"), py::arg("stream"))
+        .def("one_rank_gather", &FusedAllReducePlan::one_rank_gather)
+        .def("one_rank_shard", &FusedAllReducePlan::one_rank_shard)
         .def("gather_own", &FusedAllReducePlan::gather_own, py::arg("x"), py::arg("out"), py::arg("numel"),
              py::arg("stream"))
         .def("reduce_scatter", &FusedAllReducePlan::reduce_scatter, py::arg("x"), py::arg("out_shard"),
@@ -581,10 +679,40 @@ void bind_fused_plan(py::module_& m) {
         .def("set_ring_depth", &PipeAllReducePlan::set_ring_depth, py::arg("depth"))
         .def("set_max_blocks", &PipeAllReducePlan::set_max_blocks, py::arg("blocks"))
         .def("set_profile_buffer", &PipeAllReducePlan::set_profile_buffer, py::arg("ptr"))
+        .def("one_rank", &PipeAllReducePlan::one_rank)
+        .def("one_rank_bucket", &PipeAllReducePlan::one_rank_bucket)
         .def("all_reduce", &PipeAllReducePlan::all_reduce, py::arg("x"), py::arg("out"), py::arg("residual"),
              py::arg("numel"), py::arg("stages"), py::arg("scale"), py::arg("update_residual"), py::arg("ef_local"),
              py::arg("epoch"), py::arg("stream"), py::arg("phase_mask") = static_cast<int>(LBC_PIPE_ALL),
              py::arg("gate") = false);
+    // The all-reduce of one rank through the general kernels (deterministic rounding), as PipeAllReducePlan::one_rank.
+    m.def("one_rank_general", [](int group_size, int bit, int topk, int quant_type, int dtype, int max_blocks, int64_t max_numel,
+                                 const at::Tensor& x, const std::optional<at::Tensor>& out,
+                                 const std::optional<at::Tensor>& residual, int passes, bool update_residual, bool,
+                                 uintptr_t status_host) -> std::optional<at::Tensor> {
+        const int64_t n = x.numel();
+        if (n == 0 || n > max_numel || !plain(x, x.device()) || !of_type(x, dtype) || !like(out, x) || !like(residual, x) ||
+            !status_clear_at(status_host))
+            return std::nullopt;
+        const at::Tensor& target = out.has_value() ? *out : x;
+        if (!one_pass_ok(1, address(x), address(target), address(residual), x.nbytes())) return std::nullopt;
+        c10::cuda::CUDAGuard guard(x.device());
+        LbcRoundtripGeneral p{};
+        p.dtype = dtype;
+        p.group_size = group_size;
+        p.bit = bit;
+        p.topk = topk;
+        p.quant_type = quant_type;
+        p.x = x.data_ptr();
+        p.residual = reinterpret_cast<const void*>(address(residual));
+        p.out = target.data_ptr();
+        p.residual_out = update_residual ? reinterpret_cast<void*>(address(residual)) : nullptr;
+        p.numel = n;
+        p.passes = passes;
+        p.max_blocks = max_blocks;
+        check(lbc_roundtrip_general(&p, at::cuda::getCurrentCUDAStream()), "roundtrip_general");
+        return target;
+    });
     // free-function form, so that callers that record and replay launches can treat it like the other launchers
     m.def("pipe_all_reduce",
           [](PipeAllReducePlan& plan, uintptr_t x, uintptr_t out, uintptr_t residual, int64_t numel, int stages,

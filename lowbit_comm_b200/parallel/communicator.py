@@ -45,6 +45,8 @@ from .torch_transport import make_torch_all_gather, make_torch_all_to_all, make_
 TWO_STAGE = frozenset({"reduce_scatter", "topology", "ring", "tree", "p2p", "overlap-gather", "overlap-p2p",
                        "overlap-tree", "overlap-scale", "compressed"})
 ONE_STAGE = frozenset({"all_gather"})
+# encodings an all-reduce of one rank makes of a value: one for every stage of the strategy
+_ONE_RANK_PASSES = {"auto": 1, "all_reduce": 1, **dict.fromkeys(ONE_STAGE, 1), **dict.fromkeys(TWO_STAGE, 2)}
 
 _REGISTRY: dict[int, "Communicator"] = {}
 _REGISTRY_LOCK = threading.Lock()
@@ -102,6 +104,7 @@ class Communicator:
         self.mailbox = None   # PeerMailbox after enable_peer_mailbox()
         self._peer_failed: str | None = None
         self._workspaces: dict[tuple, Any] = {}
+        self._one_rank: dict[tuple, Any] = {}      # a group of one rank: the workspaces by what a call shows at once
         self._subcomms: dict[tuple, Any] = {}
         self.closed = False
         self.stats = {"peer_ops": 0, "torch_ops": 0}
@@ -192,6 +195,7 @@ class Communicator:
         old.close()
         self.peer_group = None
         self._workspaces.clear()
+        self._one_rank.clear()
         self.stats["arena_rebuilds"] = self.stats.get("arena_rebuilds", 0) + 1
         dist = _dist()
         pg = self.process_group if self.process_group is not None else dist.group.WORLD
@@ -243,6 +247,19 @@ class Communicator:
         self._workspaces[key] = ws
         return ws
 
+    # -- whole calls of one rank ------------------------------------------------
+    # With one rank a collective is one launch, and settling profile, workspace and geometry cost more than it.  Blocking calls of
+    # plain tensors whose workspace is there go to the native plan, which checks the tensors, reads the status word, allocates and
+    # launches in one crossing, or declines; then they go the way of all others.
+    def _one_rank_workspace(self, tensor: Any, config: CompressionConfig) -> Any:
+        if tracing.ENABLED or self.transport == "torch" or self._peer_failed is not None:
+            return None
+        return self._one_rank.get((tensor.dtype, config.bit, config.group_size, config.topk, config.quant_type, config.stochastic))
+
+    def _settle_one_rank(self, ws: Any, tensor: Any, config: CompressionConfig) -> None:
+        if self.world_size == 1 and hasattr(ws, "one_rank_plans"):
+            self._one_rank[(tensor.dtype, config.bit, config.group_size, config.topk, config.quant_type, config.stochastic)] = ws
+
     def _stream_scope(self, tensor: Any, async_op: bool):
         """(context manager, completion factory) for running on the side stream when async."""
 
@@ -274,6 +291,16 @@ class Communicator:
                    update_residual: bool = True, ef_mode: str = "reference") -> Any:
         if op not in ("sum", "mean"):
             raise UnsupportedCollective(f"all_reduce:{op}", reason="only op='sum' and op='mean' are implemented")
+        if self.world_size == 1 and not async_op and dtype == "auto" and type(tensor) is torch.Tensor:
+            ws, passes = self._one_rank_workspace(tensor, config), _ONE_RANK_PASSES.get(strategy)
+            if ws is not None and passes is not None and ef_mode in ("reference", "local"):
+                plan = ws.one_rank_plans()[0]
+                result = None if plan is None else plan.one_rank(tensor, out, residual, passes, bool(update_residual),
+                                                                 ef_mode == "local", ws.group.status_host)
+                if result is not None:
+                    ws.launches += 1
+                    self.stats["peer_ops"] += 1
+                    return result
         name = codec.resolve_dtype(dtype, tensor)
         if strategy == "native_nccl":
             result = make_torch_tensor_all_reduce(group=self.process_group)(tensor if out is None else out.copy_(tensor), op)
@@ -289,6 +316,7 @@ class Communicator:
                     raise
                 ws = None
             if ws is not None:
+                self._settle_one_rank(ws, tensor, config)
                 if out is not None or residual is not None:
                     self._check_alike(ws.ext, tensor, out, residual)
                 if not async_op and not tracing.ENABLED:
@@ -310,6 +338,7 @@ class Communicator:
                     raise
                 gws = None
             if gws is not None:
+                self._settle_one_rank(gws, tensor, config)
                 # a strided residual goes in as a copy, which is written back
                 dense = residual if residual is None or residual.is_contiguous() else residual.contiguous()
                 if out is not None or residual is not None:
@@ -425,6 +454,20 @@ class Communicator:
 
         if op not in ("sum", "mean"):
             raise UnsupportedCollective(f"reduce_scatter:{op}", reason="only op='sum' and op='mean' are implemented")
+        if self.world_size == 1 and not async_op and dtype == "auto" and out is None and residual is None \
+                and type(tensor) is torch.Tensor:
+            ws = self._one_rank_workspace(tensor, config)
+            plan = None if ws is None else ws.one_rank_plans()[1]
+            shard = None if plan is None else plan.one_rank_shard(tensor, ws.group.status_host)
+            if shard is not None:
+                ws.launches += 1
+                self.stats["peer_ops"] += 1
+                n = tensor.numel()
+                est = estimate_quantized_size(n, dtype=ws.dtype, config=config)
+                return ReducedShard.whole(shard, shape=tuple(tensor.shape), numel=n, shard_numel=shard.numel(), reduce=op,
+                                          dtype=ws.dtype, transport="fused_peer_scatter",
+                                          metadata={"fused": True, "caller_owned_output": False,
+                                                    "payload_bytes": est.quantized_bytes, "group_aligned": True})
         name = codec.resolve_dtype(dtype, tensor)
         shape = tuple(tensor.shape)
         n = tensor.numel()
@@ -435,6 +478,7 @@ class Communicator:
             geo = geometry(n, self.world_size, name, config)
             shard = self._validated_out(out, tensor, geo.shard_numel)
             ws = self.workspace(tensor, config, name)
+            self._settle_one_rank(ws, tensor, config)
             scope, side = self._stream_scope(tensor, async_op)
             with scope:
                 ws.reduce_scatter(tensor if tensor.is_contiguous() else tensor.reshape(-1), shard, residual=residual, op=op)
@@ -489,10 +533,19 @@ class Communicator:
     # -- all-gather -------------------------------------------------------------
     def all_gather(self, tensor: Any, *, config: CompressionConfig, async_op: bool = False,
                    dtype: str = "auto") -> Any:
+        if self.world_size == 1 and not async_op and dtype == "auto" and type(tensor) is torch.Tensor:
+            ws = self._one_rank_workspace(tensor, config)
+            plan = None if ws is None else ws.one_rank_plans()[1]
+            result = None if plan is None else plan.one_rank_gather(tensor, ws.group.status_host)
+            if result is not None:
+                ws.launches += 1
+                self.stats["peer_ops"] += 1
+                return [result]
         name = codec.resolve_dtype(dtype, tensor)
         shape = tuple(tensor.shape)
         if self.peer_usable(tensor, config):
             ws = self.workspace(tensor, config, name)
+            self._settle_one_rank(ws, tensor, config)
             if self.world_size == 1:
                 outs = [_plain_empty(tensor, shape)]
             else:      # rows of one buffer: the decode of all W payloads is then a single launch
@@ -616,3 +669,4 @@ class Communicator:
             self.peer_group.close()
             self.peer_group = None
         self._workspaces.clear()
+        self._one_rank.clear()

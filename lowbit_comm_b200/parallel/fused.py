@@ -372,6 +372,15 @@ class FusedWorkspace:
             self.launches += 1 if done is None else done      # None: a recorder deferred the launch
         return target
 
+    def one_rank_plans(self) -> tuple:
+        """(plan of whole one-rank all-reduces and buckets, plan of whole one-rank shards and all-gathers), None where the
+        calls have to go through this workspace: more ranks, the kernel sequence, phases that are being timed, a closed
+        arena.  The plans read the status word themselves, and decline what is not a dense tensor that they hold."""
+
+        if self.group.world_size != 1 or self.phase_timer is not None or self.group._closed:
+            return None, None
+        return (self._pipe if self.engine != "legacy" else None), self._native
+
     # -- helpers ---------------------------------------------------------------
     def _geom(self, x: torch.Tensor) -> FusedGeometry:
         if x.numel() > self.max_numel:

@@ -38,6 +38,9 @@ launches (quantize, copy-and-signal, wait, W decodes, scale, residual update) fo
 
 from __future__ import annotations
 
+from functools import partial
+from types import SimpleNamespace
+
 import torch
 
 from ..config import CompressionConfig
@@ -69,6 +72,9 @@ class GeneralPeerWorkspace:
         self.launches = 0
         self.gather_off: list[int] | None = None          # two-stage only: reserved on first use
         self._shard: torch.Tensor | None = None           # two-stage only: this rank's dense reduced shard
+        self._one_rank = None if not hasattr(self.ext, "one_rank_general") else SimpleNamespace(one_rank=partial(
+            self.ext.one_rank_general, config.group_size, config.bit, config.topk, _QUANT_CODE[config.quant_type],
+            _DTYPE_CODE[dtype], self.max_blocks, self.max_numel))
 
     @staticmethod
     def payload_bytes(dtype: str, config: CompressionConfig, numel: int) -> int:
@@ -88,6 +94,13 @@ class GeneralPeerWorkspace:
 
         groups = -(-max(1, numel) // config.group_size)
         return _round_up(-(-groups // world_size), 8) * config.group_size
+
+    def one_rank_plans(self) -> tuple:
+        """As `FusedWorkspace.one_rank_plans`: whole one-rank all-reduces, where rounding is deterministic."""
+
+        if self.group.world_size != 1 or not self.fused or self.config.stochastic or self.group._closed:
+            return None, None
+        return self._one_rank, None
 
     def all_reduce(self, x: torch.Tensor, out: torch.Tensor | None = None, *, residual: torch.Tensor | None = None,
                    update_residual: bool = True, op: str = "mean", stages: int = 1) -> torch.Tensor:
