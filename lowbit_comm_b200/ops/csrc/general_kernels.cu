@@ -27,7 +27,9 @@
 // values, bf16 14.4 -> 12.4 us, fp32 12.4 -> 10.3.  Each kernel started before the one ahead of it ends: 29.2 us, and
 // 15.4 us for the code-book; 12.3 us with the encoder for local payloads and native calls around both.  The rare warps
 // of the one-rank pass out of line, its group steps without loops, its sums and products two to an instruction, 32 Mi
-// elements beyond L2: bf16 29.6 -> 26.6 us, two kept values 30.6 -> 28.2, fp16 in 4 bits 29.1 -> 26.4.
+// elements beyond L2: bf16 29.6 -> 26.6 us, two kept values 30.6 -> 28.2, fp16 in 4 bits 29.1 -> 26.4.  Without a residual, in
+// kernels that know it, with the next tile under way, no clamp for fp32 and quotients without branches: 22.9 us, 24.5 and 22.9; 16 Mi
+// bf16 elements 15.0 -> 12.1, fp32 with two kept values 24.2 -> 21.2; encode of 4 Mi fp32 elements in records, one kept value, 6.46 -> 5.43.
 
 #include <cmath>
 #include <cstring>
@@ -285,8 +287,10 @@ struct GroupMeta {
     float stored;             // the scale, exact in T
     int idx[2];               // positions of the kept elements inside the group
     uint32_t kept[2];         // their bits
-    bool tame;                // 16-bit sources: no infinity and no NaN in the group
+    bool tame;                // no infinity and no NaN in the group (fp32: false where it is not asked for)
 };
+
+__device__ __forceinline__ bool all_near(const GroupMeta& m) { return __all_sync(0xffffffffu, m.tame && m.stored < kNearScale); }
 
 // Magnitude bits of infinity.
 template <typename T>
@@ -296,7 +300,7 @@ __device__ __forceinline__ constexpr uint32_t inf_bits() {
 
 // The k largest magnitudes of a group and the next one, the scale.  `v` are the thread's 16 values, `p` the same in T;
 // the `lanes` threads of a group call this together and all get the answer.  fp32: v of a kept element turns into NaN.
-template <typename T, int TOPK>
+template <typename T, int TOPK, int KIND>
 __device__ __forceinline__ GroupMeta select_group(float (&v)[16], const Packed16<T>& p, int lane, int lanes) {
     GroupMeta m;
     m.idx[0] = m.idx[1] = 0;
@@ -364,7 +368,18 @@ __device__ __forceinline__ GroupMeta select_group(float (&v)[16], const Packed16
             for (int off = lanes / 2; off > 0; off >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, off, lanes));
             return a;
         };
-        m.stored = largest();
+        if constexpr (!Kind<KIND>::book) {      // (linear codes without a clamp: the first maximum looks for a NaN, which is passed over else)
+            float top = fabsf(v[0]);
+#pragma unroll
+            for (int i = 1; i + 1 < 16; i += 2) top = max_nan(top, fabsf(v[i]), fabsf(v[i + 1]));
+            top = max_nan(top, fabsf(v[15]));
+            over_group(lanes, [&](int off) { top = max_nan(top, __shfl_xor_sync(0xffffffffu, top, off)); });
+            m.tame = top < INFINITY;
+            m.stored = top;
+            if (!__all_sync(0xffffffffu, m.tame)) m.stored = largest();
+        } else {
+            m.stored = largest();
+        }
 #pragma unroll
         for (int j = 0; j < TOPK; ++j) {
             int at = -1;
@@ -478,7 +493,7 @@ __device__ __forceinline__ GroupTop top_of_group(const Packed16<T>& p, int lanes
 // Then the places need not be found, which took a key with index and sign through every comparison.
 template <typename T, int TOPK>
 __device__ __forceinline__ bool kept_by_magnitude(const GroupTop& g, const Packed16<T>& p, bool noise) {
-    bool ok = g.finite && (g.last_kept > g.stored || (sizeof(T) == 2 && !noise && g.stored >= 1.0e-6f));
+    bool ok = g.finite && g.stored < kNearScale && (g.last_kept > g.stored || (sizeof(T) == 2 && !noise && g.stored >= 1.0e-6f));
     if (__all_sync(0xffffffffu, ok)) return true;
     if (!ok && g.finite && !noise && g.stored == 0.0f) {
         bool minus = false;
@@ -595,11 +610,13 @@ __device__ __noinline__ void book_codes_far(const float* v, float safe, const fl
 // its scale, which bounds no value: the test is on the scale as stored, false for NaN.)
 __device__ __forceinline__ bool book_near(float stored) { return __all_sync(0xffffffffu, stored < 1.0e30f); }
 
-// Codes of 16 values against the group's scale, as bit patterns whose low byte (nibble) is the code.  With `tame` (no
-// infinity and no NaN in any group of the warp) no value that is not kept verbatim is larger than the scale, so
-// |value * mul| rounds to at most the limit and neither the clamp nor the test for NaN has anything to do.
-template <int KIND>
-__device__ __forceinline__ void encode_general(const float (&v)[16], float stored, bool tame, const CodeRule& rule,
+// Codes of 16 values against the group's scale, as bit patterns whose low byte (nibble) is the code.  With `near` (no infinity, no
+// NaN and no scale above kNearScale in any group of the warp) no value that is not kept verbatim is larger than the scale, so
+// |value * mul| rounds to at most the limit, neither the clamp nor the test for NaN has anything to do, and the quotient
+// needs no branch.  kPacked: products two to an instruction and that quotient; without, the 16-bit encoders are a little faster (4 Mi bf16
+// elements in records, one kept value, 5.11 / 5.04 us; fp32 ones 5.43 / 6.46).
+template <int KIND, bool kPacked>
+__device__ __forceinline__ void encode_general(const float (&v)[16], float stored, bool near, const CodeRule& rule,
                                                int64_t first, uint32_t (&b)[16]) {
     static_assert(KIND != kBook, "book_code");
     constexpr int lim = Kind<KIND>::lim;
@@ -607,11 +624,20 @@ __device__ __forceinline__ void encode_general(const float (&v)[16], float store
     for (int i = 0; i < 16; ++i) b[i] = 0u;
     const float safe = fmaxf(stored, 1.0e-6f);
     if constexpr (!Kind<KIND>::book) {
-        const float mul = float(lim) / safe;
         float t[16];
+        if (kPacked && near && !rule.stochastic) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) t[i] = v[i];
+            fma16(t, limit_over<lim>(safe), 0.0f);             // (see encode16_near)
+            add16(t, kRoundMagic);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) b[i] = __float_as_uint(t[i]);
+            return;
+        }
+        const float mul = float(lim) / safe;
 #pragma unroll
         for (int i = 0; i < 16; ++i) t[i] = __fmul_rn(v[i], mul);
-        if (tame && !rule.stochastic) {
+        if (!kPacked && near && !rule.stochastic) {
             add16(t, kRoundMagic);
 #pragma unroll
             for (int i = 0; i < 16; ++i) b[i] = __float_as_uint(t[i]);
@@ -663,7 +689,7 @@ __device__ __forceinline__ void pack_codes(const uint32_t (&b)[16], uint32_t (&w
 
 // Values to packed codes.  Convergent.
 template <typename T, int KIND>
-__device__ __forceinline__ void encode_words(const float (&v)[16], float stored, bool tame, const CodeRule& rule,
+__device__ __forceinline__ void encode_words(const float (&v)[16], float stored, bool near, const CodeRule& rule,
                                              int64_t first, uint32_t (&w)[4]) {
     uint32_t b[16];
     if constexpr (KIND == kBook) {
@@ -685,7 +711,7 @@ __device__ __forceinline__ void encode_words(const float (&v)[16], float stored,
         for (int i = 0; i < 16; ++i) far[i] = v[i];
         book_codes_far(far, safe, rule.thresholds, b);
     } else {
-        encode_general<KIND>(v, stored, tame, rule, first, b);
+        encode_general<KIND, sizeof(T) == 4>(v, stored, near, rule, first, b);
     }
     pack_codes<T, KIND>(b, w);
 }
@@ -737,7 +763,7 @@ __device__ __forceinline__ Packed16<T> decode_bits(const uint32_t (&b)[16], floa
 
 // Values -> T(decode(encode(value))).  Convergent.
 template <typename T, int KIND>
-__device__ __forceinline__ Packed16<T> requantize(const float (&v)[16], float stored, bool tame, const CodeRule& rule,
+__device__ __forceinline__ Packed16<T> requantize(const float (&v)[16], float stored, bool near, const CodeRule& rule,
                                                   int64_t first, const float* lut) {
     uint32_t b[16];
     if constexpr (KIND == kBook) {
@@ -760,7 +786,7 @@ __device__ __forceinline__ Packed16<T> requantize(const float (&v)[16], float st
         for (int i = 0; i < 16; ++i) far[i] = v[i];
         book_codes_far(far, safe, rule.thresholds, b);
     } else {
-        encode_general<KIND>(v, stored, tame, rule, first, b);
+        encode_general<KIND, true>(v, stored, near, rule, first, b);
     }
     return decode_bits<T, KIND>(b, stored, lut);
 }
@@ -859,9 +885,9 @@ __global__ void __launch_bounds__(kThreads, 4) quant_general_kernel(const __grid
             if constexpr (sizeof(T) == 2) unpack_elems<T>(elems, v);
         }
         if (prep != nullptr && live) store_elems<T>(prep, first, n, p_vec, res != nullptr ? elems : pack_elems<T>(v));
-        const GroupMeta m = select_group<T, TOPK>(v, elems, lane, lanes);
+        const GroupMeta m = select_group<T, TOPK, KIND>(v, elems, lane, lanes);
         uint32_t w[4];
-        encode_words<T, KIND>(v, m.stored, __all_sync(0xffffffffu, m.tame), rule, first, w);
+        encode_words<T, KIND>(v, m.stored, all_near(m), rule, first, w);
 #pragma unroll
         for (int j = 0; j < TOPK; ++j) patch_code<T, KIND>(w, m.idx[j] - lane * 16);
         if (!live) continue;
@@ -941,9 +967,9 @@ __global__ void __launch_bounds__(kThreads, encode_blocks<T, TOPK, KIND>()) enco
             if constexpr (sizeof(T) == 2) unpack_elems<T>(elems, v);
         }
         if (prep != nullptr && live) store_elems<T>(prep, first, end, whole || p_vec, res != nullptr ? elems : pack_elems<T>(v));
-        const GroupMeta m = select_group<T, TOPK>(v, elems, lane, lanes);
+        const GroupMeta m = select_group<T, TOPK, KIND>(v, elems, lane, lanes);
         uint32_t w[4];
-        encode_words<T, KIND>(v, m.stored, __all_sync(0xffffffffu, m.tame), rule, first, w);
+        encode_words<T, KIND>(v, m.stored, all_near(m), rule, first, w);
 #pragma unroll
         for (int j = 0; j < TOPK; ++j) patch_code<T, KIND>(w, m.idx[j] - lane * 16);
         if constexpr (kCompact) {
@@ -1085,11 +1111,10 @@ __device__ __forceinline__ Packed16<T> place_and_requantize(Packed16<T> y, int l
                                                             int64_t first, const float* lut) {
     float v[16];
     unpack_elems<T>(y, v);
-    const GroupMeta m = select_group<T, TOPK>(v, y, lane, lanes);
-    const bool tame = __all_sync(0xffffffffu, m.tame);
-    if (sizeof(T) == 2 && !tame) y = pack_elems<T>(v);          // a NaN that is kept has one pattern
+    const GroupMeta m = select_group<T, TOPK, KIND>(v, y, lane, lanes);
+    if (sizeof(T) == 2 && !__all_sync(0xffffffffu, m.tame)) y = pack_elems<T>(v);          // a NaN that is kept has one pattern
     const Packed16<T> from = y;
-    y = requantize<T, KIND>(v, m.stored, tame, rule, first, lut);
+    y = requantize<T, KIND>(v, m.stored, all_near(m), rule, first, lut);
 #pragma unroll
     for (int j = 0; j < TOPK; ++j) copy_elem<T>(y, from, int(uint32_t(m.idx[j]) & 0xffu) - lane * 16);
     return y;
@@ -1109,8 +1134,11 @@ __device__ __noinline__ void requantize_by_place(uint32_t* words, int lane, int 
 
 // The all-reduce of a group of one rank: encode and decode in registers, no payload (see roundtrip_kernels.cu; here
 // the decoded values are rounded to T before the residual is taken, the rule of these profiles).
-// Blocks per SM, 16-bit, 4 against 5, 32 Mi bf16: one kept value 26.6 / 27.5 us, two 28.2 / 29.1; fp32: see its launcher.
-template <typename T, int TOPK, int KIND, int kBlocks>
+// Blocks per SM, 16-bit, with a residual 4 against 5, 32 Mi bf16: one kept value 26.6 / 27.5 us, two 28.2 / 29.1; others: see the launcher.
+// kFull: with a residual or two passes.  kPlain: neither.  kPlainAhead: neither, and the loads of a block's next tile are issued ahead of the
+// work on the present one (which waits for its loads at four blocks per SM otherwise: ncu, long scoreboard 3.6 per issue).
+enum : int { kFull = 0, kPlain = 1, kPlainAhead = 2 };
+template <typename T, int TOPK, int KIND, int kBlocks, int kForm>
 __global__ void __launch_bounds__(kThreads, kBlocks) roundtrip_general_kernel(const __grid_constant__ LbcRoundtripGeneral p) {
     constexpr bool by_magnitude = TOPK >= 1 && KIND != kBookNoise;
     chain_wait();
@@ -1119,9 +1147,10 @@ __global__ void __launch_bounds__(kThreads, kBlocks) roundtrip_general_kernel(co
     __shared__ float lut[16];
     load_lut<KIND>(lut, p.quant_type);
     const T* x = static_cast<const T*>(p.x);
-    const T* res = static_cast<const T*>(p.residual);
+    const T* res = kForm == kFull ? static_cast<const T*>(p.residual) : nullptr;
     T* out = static_cast<T*>(p.out);
-    T* rout = static_cast<T*>(p.residual_out);
+    T* rout = kForm == kFull ? static_cast<T*>(p.residual_out) : nullptr;
+    const int passes = kForm == kFull ? p.passes : 1;
     const int64_t n = p.numel;
     const int64_t num_chunks = (n + p.group_size - 1) >> (shape.shift + 4) << shape.shift;
     const int64_t chunk_span = (num_chunks + 31) / 32 * 32;
@@ -1131,14 +1160,24 @@ __global__ void __launch_bounds__(kThreads, kBlocks) roundtrip_general_kernel(co
     // 16-bit tensors: tile by tile, whole ones without a test per chunk (32 Mi bf16 elements, e2m1 40.7 -> 38.0 us; 8 Mi, one kept value
     // 9.6 -> 9.3).  fp32: chunk by chunk (by tiles it spills: 16 Mi elements, one kept value, 22.6 -> 30.4 us).
     constexpr bool tiles = sizeof(T) == 2;
+    const auto whole_at = [&](int64_t at) { return tiles && vec && (at + kThreads) * kElemsPerThread <= n; };
+    Packed16<T> next;
+    if (kForm == kPlainAhead && whole_at(int64_t(blockIdx.x) * kThreads))
+        next = load_elems<T>(x, (int64_t(blockIdx.x) * kThreads + threadIdx.x) * kElemsPerThread, n, true);
     for (int64_t at = int64_t(blockIdx.x) * kThreads + (tiles ? 0 : threadIdx.x); at < (tiles ? num_chunks : chunk_span);
          at += int64_t(gridDim.x) * kThreads) {
         const int64_t chunk = tiles ? at + threadIdx.x : at;
-        const bool whole = tiles && vec && (at + kThreads) * kElemsPerThread <= n;
+        const bool whole = whole_at(at);
         const bool live = whole || chunk < num_chunks;
         const int64_t first = chunk * kElemsPerThread, end = whole ? first + 16 : n;
         const int lane = tiles ? int(threadIdx.x) & (lanes - 1) : int(chunk) & (lanes - 1);
-        Packed16<T> elems = load_elems<T>(x, first, end, vec);          // zeros past the end
+        Packed16<T> elems;
+        if (kForm == kPlainAhead && whole) elems = next;
+        else elems = load_elems<T>(x, first, end, vec);                 // zeros past the end
+        if (kForm == kPlainAhead) {
+            const int64_t then = at + int64_t(gridDim.x) * kThreads;
+            if (whole_at(then)) next = load_elems<T>(x, (then + threadIdx.x) * kElemsPerThread, (then + threadIdx.x) * kElemsPerThread + 16, true);
+        }
         if (res != nullptr) {
             float v[16], r[16];
             unpack_elems<T>(elems, v);
@@ -1148,7 +1187,7 @@ __global__ void __launch_bounds__(kThreads, kBlocks) roundtrip_general_kernel(co
             elems = pack_elems<T>(v);
         }
         Packed16<T> y = elems;
-        for (int pass = 0; pass < p.passes; ++pass) {
+        for (int pass = 0; pass < passes; ++pass) {
             if constexpr (by_magnitude) {
                 const GroupTop top = top_of_group<T, TOPK>(y, lanes);
                 if (kept_by_magnitude<T, TOPK>(top, y, p.stochastic)) {
@@ -1185,13 +1224,8 @@ __global__ void __launch_bounds__(kThreads, kBlocks) roundtrip_general_kernel(co
 }
 
 // A block per 4096 elements up to four times the default grid, a grid that loops above: it pays a block's set-up less
-// often.  The line is where a looping grid began to win when a pass took half as long again.  The present one-rank pass, full grid against
-// a looping one (1184 blocks, whole waves of four or eight per SM): bf16 top-k 1, 8 Mi elements (1.7 default grids) 6.79 / 6.31 us, 16 Mi
-// 15.5 / 14.6, 20 Mi (4.3) 19.1 / 17.8, 32 Mi 29.0 / 26.5, 64 Mi 55.1 / 49.8; e2m1 9.93 / 9.33, 19.8 / 17.9, 24.6 / 21.7, 37.8 / 33.1,
-// 71.8 / 61.3; fp32 top-k 1 12.1 / 12.1, 22.1 / 22.8, 27.4 / 28.2, 43.7 / 43.3, 87.6 / 92; top-k 2 15.3 / 13.3, 24.6 / 23.9, 30.1 / 29.3,
-// 47.0 / 45.4, 91.1 / 89.1; e2m1 17.4 / 15.1, 29.0 / 26.7, 34.9 / 32.3, 53.7 / 49.4, 107 / 97.3: looping would serve all but fp32 with one
-// kept value from 8 Mi on.  Grids of other sizes, 64 Mi, 4 / 5 / 8 / 12 / 16 blocks per SM: bf16 top-k 1 49.9 / 62.4 / 49.8 / 50.4 / 50.1,
-// fp32 top-k 2 103 / 92.9 / 89.1 / 87.5 / 89.0.  The default grid also serves blocks that meet at a flag or a counter (`shared`):
+// often.  The line is where a looping grid began to win when a pass took half as long again.  (One-rank passes without a residual
+// have a rule of their own, RoundtripGeneral.)  The default grid also serves blocks that meet at a flag or a counter (`shared`):
 // each costs a system-scope fence or a look at the flags.
 static int general_grid(int64_t groups, int group_size, int max_blocks, bool shared) {
     int64_t want = (groups * (group_size / kElemsPerThread) + kThreads - 1) / kThreads;
@@ -1294,22 +1328,48 @@ template <typename T, int TOPK, int KIND>
 struct RoundtripGeneral {
     static constexpr bool noise = true;
     static void run(const LbcRoundtripGeneral& p, int grid, cudaStream_t s) {
-        // fp32, three blocks per SM or four (64 registers, with spills).  Four are faster for one kept value alone (two, 16 Mi elements:
-        // 25.1 / 26.3 us), without a residual, and where three do not hold the whole grid.  Three / four, one kept value, 8 bits: 1 Mi
-        // elements 3.63 / 3.57, 1.75 Mi (the last that three hold) 3.73 / 3.96, 2 Mi 4.53 / 4.35, 4 Mi 7.63 / 7.18, 16 Mi 23.7 / 22.1; with a
-        // residual 3.75 / 5.12, 6.21 / 6.86, 7.01 / 7.12, 11.7 / 12.4, 40.5 / 41.4.  e2m1 4.35 / 5.01, 5.66 / 5.83, 6.30 / 6.01, 10.1 / 9.8,
-        // 30.5 / 29.5; with a residual 5.42 / 6.39, 7.81 / 8.45, 8.56 / 8.61, 13.2 / 14.8, 42.3 / 45.5.  8 bits with noise 4.48 / 5.15,
-        // 5.66 / 6.16, 6.35 / 6.52, 10.3 / 10.2, 32.8 / 31.6; with a residual, the last two, 13.2 / 14.4 and 42.2 / 45.5.  e2m1 with noise,
-        // those two: 30.2 / 34.1 and 107 / 116.
+        // No residual and one pass: kernels that know it (what the others hold for both costs registers).  Above one default grid (books
+        // without kept values, which pay for it alone up to there: half of one) 16-bit tensors take as many blocks as are resident, each with its next tile under way.  Before / one tile a
+        // block / resident blocks (4 per SM), bf16: one kept value 4 Mi elements 3.80 / 3.62 / 3.83 us, 6 Mi 5.1 / 5.08 / 4.59, 8 Mi 6.60 /
+        // 6.40 / 5.82, 16 Mi 15.0 / 14.5 / 12.0, 32 Mi 26.2 / 28.2 / 22.8; two 4 Mi 4.07 / 3.96 / 4.21, 8 Mi 7.08 / 6.96 / 6.42, 16 Mi 15.7 / 15.2 /
+        // 13.2, 32 Mi 27.9 / 29.7 / 24.4; e2m1 4 Mi - / 6.23 / 5.70, 8 Mi 9.3 / 10.3 / 8.96, 16 Mi 17.9 / 19.8 / 16.2, 32 Mi 33.1 / 37.1 / 30.0.  Without
+        // the next tile under way 8 Mi with one kept value took 5.89, 32 Mi 25.4; twice the blocks 6.02 and 23.1; three per SM 5.67
+        // and 24.3; five spill; copies into shared memory (cp.async, two tiles ahead) 7.38 and 30.6.
+        // fp32, full grids, before / 4 blocks per SM / 5: one kept value 1 Mi 2.87 / 2.21 / 2.17, 4 Mi 5.59 / 4.81 / 4.69, 16 Mi 22.0 / 20.9 / 21.0;
+        // two 2.88 / 2.22 / 2.43, 5.47 / 4.94 / 5.33, 24.2 / 21.2 / 21.2; e2m1 - / 3.15 / 3.11, - / 7.28 / 6.70, 26.7 / 24.6 / 23.1.  Grids that loop
+        // from one default grid on: 8 Mi with one kept value 10.7 / 10.7 / 10.7, 16 Mi 22.0 / 22.3 / 22.1.
+        const int64_t tiles = (p.numel + kThreads * kElemsPerThread - 1) / (kThreads * kElemsPerThread);
+        const auto capped = [&](int64_t blocks) { return unsigned(p.max_blocks > 0 && p.max_blocks < blocks ? p.max_blocks : blocks); };
+        if constexpr (KIND != kBookNoise) {
+            // (tensors off 32 bytes keep the others: going round took 98 us instead of 86 for 16 Mi bf16 elements, one element in)
+            if (p.residual == nullptr && p.passes == 1 && on_boundary(32, p.x, p.out)) {
+                if constexpr (sizeof(T) == 2) {
+                    constexpr bool book = KIND == kBook && TOPK == 0;
+                    const int64_t resident = lbc_default_max_blocks() / 2;
+                    if (tiles > (book ? resident : 2 * resident) || capped(tiles) < tiles)
+                        launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 4, kPlainAhead>, capped(tiles < resident ? tiles : resident), s, p);
+                    else
+                        launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 4, book ? kFull : kPlain>, unsigned(tiles), s, p);
+                } else {
+                    launch_chained(roundtrip_general_kernel<T, TOPK, KIND, KIND == kBook && TOPK == 0 ? 5 : 4, kPlain>, capped(tiles), s, p);
+                }
+                return;
+            }
+        }
+        // fp32, three blocks per SM or four (64 registers, with spills).  Four are faster for two passes of one kept value without a residual
+        // alone (two, 16 Mi elements: 25.1 / 26.3 us), where three do not hold the whole grid.  Three / four with a residual, one kept value, 8 bits:
+        // 1 Mi elements 3.75 / 5.12, 1.75 Mi 6.21 / 6.86, 2 Mi 7.01 / 7.12, 4 Mi 11.7 / 12.4, 16 Mi 40.5 / 41.4; e2m1 5.42 / 6.39, 7.81 / 8.45,
+        // 8.56 / 8.61, 13.2 / 14.8, 42.3 / 45.5; 8 bits with noise, the last two, 13.2 / 14.4 and 42.2 / 45.5; e2m1 with noise 30.2 / 34.1 and
+        // 107 / 116.
         if constexpr (sizeof(T) == 2) {
-            launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 4>, unsigned(grid), s, p);
+            launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 4, kFull>, unsigned(grid), s, p);
         } else {
             if constexpr (TOPK == 1 && KIND != kBookNoise)
                 if (p.residual == nullptr && grid > lbc_default_max_blocks() / 8 * 3) {
-                    launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 4>, unsigned(grid), s, p);
+                    launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 4, kFull>, unsigned(grid), s, p);
                     return;
                 }
-            launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 3>, unsigned(grid), s, p);
+            launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 3, kFull>, unsigned(grid), s, p);
         }
     }
 };

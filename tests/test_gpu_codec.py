@@ -1107,3 +1107,32 @@ def test_linear_codes_of_scales_that_need_the_clamp(ext, dtype, bit, group, comp
     wide = torch.empty(n + 1, dtype=T, device="cuda")    # one element in: the kernel of unaligned tensors
     wide[1:].copy_(x)
     assert torch.equal(codec.quantize_tensor(wide[1:], cfg).cpu(), want)
+
+
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("bit,quant_type,topk,group", [(8, "linear", 1, 64), (4, "linear", 2, 16), (4, "e2m1", 0, 32), (4, "normal", 1, 64)])
+def test_one_rank_pass_without_a_residual(ext, dtype, bit, quant_type, topk, group):
+    """The forms of the pass that only encode and decode: a tile per block, and blocks that go round with their next tile under way,
+    which a cap on the blocks and the sizes where they begin bring in; whole and ragged ends, tensors off their vectors, in
+    place.  Beside them infinities, NaN and a scale above 1e30 (fp16: the largest), whose warps take the clamp: in finite groups the
+    bytes are the oracle's."""
+
+    cfg, code = _cfg(bit=bit, group_size=group, topk=topk, quant_type=quant_type), codec._QUANT_CODE[quant_type]
+    edge = int(ext.default_max_blocks()) * 4096 // (2 if quant_type != "linear" and topk == 0 else 1)
+    large = () if dtype == "fp16" else ((edge, 0, 0), (edge + 4099, 0, 0))
+    for n, blocks, skew in ((1, 0, 0), (4096, 0, 0), (8191, 1, 0), (4096 * 3 + 17, 2, 0), (4096 * 7, 2, 0), (4096 * 5 + 1, 3, 1)) + large:
+        x = _data(n, DTYPES[dtype], seed=n % 97)
+        finite = torch.ones(n, dtype=torch.bool)
+        if n > 2000:
+            x[group:group + 3] = torch.tensor([torch.finfo(x.dtype).max, -torch.finfo(x.dtype).max / 2, 1.0]).to(x)
+            x[20 * group:20 * group + 2] = torch.tensor([float("inf"), float("nan")]).to(x)
+            x[n - 1] = float("nan")
+            finite[20 * group:21 * group] = False
+            finite[(n - 1) // group * group:] = False
+        want = oracle.decode(oracle.encode(torch.where(finite, x, torch.zeros_like(x)), cfg), n, cfg, dtype)
+        for in_place in (False, True):
+            source = torch.empty(n + skew, dtype=x.dtype, device="cuda")[skew:]
+            source.copy_(x)
+            out = source if in_place else torch.empty_like(source)
+            assert ext.roundtrip_general(source, None, out, None, group, bit, topk, code, False, 0, 1, blocks)
+            assert torch.equal(out.cpu()[finite].view(torch.uint8), want[finite].view(torch.uint8)), (n, blocks, skew, in_place)
