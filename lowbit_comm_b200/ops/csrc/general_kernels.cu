@@ -930,15 +930,23 @@ constexpr int encode_blocks() {
     if (KIND == kBook) return sizeof(T) == 4 && TOPK == 0 ? 5 : 4;
     return KIND != kBookNoise && (TOPK == 1 || (TOPK == 2 && sizeof(T) == 4)) ? 5 : 4;
 }
-template <typename T, int TOPK, int KIND, bool kCompact>
-__global__ void __launch_bounds__(kThreads, encode_blocks<T, TOPK, KIND>()) encode_general_kernel(const __grid_constant__ LbcQuantGeneral p) {
+// kPrepare: with a residual or prepared_out.  Without, in kernels that know it, and their blocks per SM (us, beyond L2 from 8 Mi bf16 elements on;
+// with both / without, 3 / 4 / 5 / 6): bf16, one kept value 2 Mi 3.38 / 2.98 / 2.74 / 3.37 / 3.81, 4 Mi 4.59 / 4.48 / 4.28 / 4.52 / 4.56, 8 Mi 8.07 /
+// 8.63 / 8.10 / 8.28 / 8.29; two 4 Mi 5.70 / 5.46 / 5.26 / 5.64 / 5.89, 8 Mi 10.9 / 10.3 / 9.97 / 10.5 / 10.9; e2m1 2 Mi 3.04 / 3.40 / 3.42 / 3.52 / 4.00,
+// 4 Mi 5.16 / 4.93 / 5.21 / 5.02 / 5.61, 8 Mi 8.97 / 8.51 / 8.67 / 8.16 / 8.43; fp32, one kept value 2 Mi 4.23 / 3.25 / 3.04 / 3.83 / 4.44, 4 Mi 5.53 /
+// 4.97 / 4.60 / 5.20 / 5.31; two 5.27 / 4.45 / 4.27 / 5.17 / 6.01, 6.97 / 6.87 / 6.65 / 6.87 / 7.14; e2m1 3.87 / 3.72 / 3.45 / 3.62 / 4.06, 5.41 / 5.56 /
+// 5.09 / 5.40 / 5.69.
+template <typename T, int KIND>
+constexpr int encode_plain_blocks() { return KIND == kBook && sizeof(T) == 2 ? 5 : 4; }
+template <typename T, int TOPK, int KIND, bool kCompact, bool kPrepare>
+__global__ void __launch_bounds__(kThreads, kPrepare ? encode_blocks<T, TOPK, KIND>() : encode_plain_blocks<T, KIND>()) encode_general_kernel(const __grid_constant__ LbcQuantGeneral p) {
     chain_wait();
     const GroupShape shape = GroupShape::of<T, TOPK, KIND>(p.group_size);
     const int lanes = shape.lanes, VB = shape.VB, MB = shape.MB;
     constexpr int CB = Kind<KIND>::CB;
     const T* x = static_cast<const T*>(p.x);
-    const T* res = static_cast<const T*>(p.residual);
-    T* prep = static_cast<T*>(p.prepared_out);
+    const T* res = kPrepare ? static_cast<const T*>(p.residual) : nullptr;
+    T* prep = kPrepare ? static_cast<T*>(p.prepared_out) : nullptr;
     const int64_t n = p.numel;
     const int64_t num_groups = (n + p.group_size - 1) >> (shape.shift + 4);
     const int64_t num_chunks = num_groups << shape.shift;
@@ -1292,10 +1300,28 @@ struct QuantGeneral {
         const uintptr_t at = reinterpret_cast<uintptr_t>(p.out);
         if (p.num_dst > 0 || p.signal.num_remote > 0)      // for other ranks, who wait for it
             quant_general_kernel<T, TOPK, KIND><<<grid, kThreads, 0, s>>>(p);
-        else if (p.compact && (at & 15) == 0)
-            launch_chained(encode_general_kernel<T, TOPK, KIND, true>, unsigned(grid), s, p);
-        else if (!p.compact && (at & (Kind<KIND>::CB - 1)) == 0)
-            launch_chained(encode_general_kernel<T, TOPK, KIND, false>, unsigned(grid), s, p);
+        else if (p.compact ? (at & 15) == 0 : (at & (Kind<KIND>::CB - 1)) == 0) {
+            // Without a residual, but where that is slower: 16-bit code-books up to half a default grid; fp32 code-books that keep nothing
+            // above one (8 Mi elements 9.28 / 10.2 us, 16 Mi 16.7 / 17.8); 16-bit planar payloads with linear codes and one kept value between
+            // one and a half and four (8 Mi 7.99 / 8.04, 16 Mi 16.4 / 16.8, 32 Mi 30.0 / 28.7).
+            const int64_t halves = p.numel / (lbc_default_max_blocks() / 2 * int64_t(kThreads * kElemsPerThread));
+            bool plain = KIND != kBookNoise && p.residual == nullptr && p.prepared_out == nullptr;
+            if (KIND == kBook && sizeof(T) == 2) plain = plain && halves >= 1;
+            if (KIND == kBook && sizeof(T) == 4 && TOPK == 0) plain = plain && halves < 2;
+            if (KIND != kBook && sizeof(T) == 2 && TOPK == 1) plain = plain && (p.compact || halves < 3 || halves >= 8);
+            const auto go = [&](auto prepare) {
+                constexpr bool kPrepare = decltype(prepare)::value;
+                if (p.compact) launch_chained(encode_general_kernel<T, TOPK, KIND, true, kPrepare>, unsigned(grid), s, p);
+                else launch_chained(encode_general_kernel<T, TOPK, KIND, false, kPrepare>, unsigned(grid), s, p);
+            };
+            if constexpr (KIND != kBookNoise) {
+                if (plain) {
+                    go(std::false_type{});
+                    return;
+                }
+            }
+            go(std::true_type{});
+        }
         else                    // a payload off its vectors
             launch_chained(quant_general_kernel<T, TOPK, KIND>, unsigned(grid), s, p);
     }
@@ -1310,8 +1336,17 @@ struct DequantGeneral {
         // against 8 (fp32: 6): bf16, one kept value 21.9 / 20.1, two 23.1 / 22.4, e2m1 19.4 / 17.1, its records 20.6 / 17.8; fp32 16.6 / 15.2,
         // 18.1 / 16.4, 16.6 / 14.7, 17.1 / 15.2; 16 MiB bf16 7.94 / 7.01, 8.45 / 7.73, 7.63 / 6.42, 8.14 / 6.50.
         const int64_t tiles = (p.numel + kThreads * kElemsPerThread - 1) / (kThreads * kElemsPerThread);
-        const bool many = sizeof(T) == 2 ? !(p.compact && TOPK >= 1) : tiles > 2 * lbc_default_max_blocks();
-        if (many && !p.accumulate)
+        // Five, above half a default grid and up to two (us, four / five / six / eight): fp32, e2m1 4 Mi 4.41 / 4.11 / 4.12 / 4.27, 5 M 5.11 /
+        // 4.74 / 4.79 / 4.72, one kept value 4.44 / 4.05 / 4.07 / 4.68, 5.58 / 5.11 / 5.07 / 5.29, below, 2 Mi, 2.94 / 3.18 / 3.45 / 3.01; planar
+        // 16-bit payloads with kept values and linear codes, bf16, one 4 Mi 3.39 / 3.35 / 3.42 / 3.67, 8 Mi 6.10 / 5.97 / 5.88 / 6.14, two 3.72 / 3.57 /
+        // 3.59 / 4.03, 6.80 / 6.58 / 6.43 / 6.90, below, 2 Mi, 2.60 / 2.57 / 2.79 / 2.50, above, 16 Mi, - / 11.8 / - / 11.3.
+        const int64_t grid_tiles = lbc_default_max_blocks();
+        const bool five = 2 * tiles > grid_tiles && tiles <= 2 * grid_tiles &&
+                          (sizeof(T) == 4 || (!p.compact && TOPK >= 1 && !Kind<KIND>::book));
+        const bool many = sizeof(T) == 2 ? !(p.compact && TOPK >= 1) : tiles > 2 * grid_tiles;
+        if (five && !p.accumulate)
+            launch_chained(dequant_general_kernel<T, TOPK, KIND, false, 5>, unsigned(grid), s, p);
+        else if (many && !p.accumulate)
             launch_chained(dequant_general_kernel<T, TOPK, KIND, false, sizeof(T) == 2 ? 8 : 6>, unsigned(grid), s, p);
         else
             launch_chained(dequant_general_kernel<T, TOPK, KIND, true, 4>, unsigned(grid), s, p);
