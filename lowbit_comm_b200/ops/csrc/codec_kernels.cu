@@ -12,7 +12,8 @@
 // Measured on a B200 through the public calls, int8 groups of 64, before (grid-stride kernels of fast_kernels.cu) and
 // after: encode of 32 Mi bf16 elements with error feedback 47.0 -> 39.2 us, decode of 128 Mi 94 -> 67.6 us, mean of eight payloads
 // of 32 Mi with error feedback 107 -> 89.8 us; then, each kernel started before the one ahead of it ends, and the scale's quotient
-// without a branch ahead of the codes: 37.5 us (6.3 TB/s), 63.9 us (6.4 TB/s) and 83.7 us (5.7 TB/s).  Those are passes repeated
+// without a branch ahead of the codes: 37.5 us (6.3 TB/s), 63.9 us (6.4 TB/s) and 83.7 us (5.7 TB/s); the encode without a clamp and the decode
+// of one payload in a kernel of its own: 35.9 us (6.6 TB/s) and 61.5 us (6.6 TB/s).  Those are passes repeated
 // for a second; in bursts of a few milliseconds the mean of eight takes 80.5 us: it draws the card's 1000 W, and its clock falls to
 // 1.7 GHz.
 #include <type_traits>
@@ -325,7 +326,8 @@ __device__ __forceinline__ void decode_edge(const LbcReduce& p, int64_t chunk) {
     store16_fit<T, kFit>(out, first, p.numel, acc);             // rounds to T
 }
 
-// Tensors on 32 bytes, payloads on their vectors.  B payloads are in flight per thread.  B == 1: one payload, no error feedback (the launcher's rule).
+// Tensors on 32 bytes, payloads on their vectors.  B payloads are in flight per thread.  B == 1: one payload, no error feedback, that is
+// scaled or added to the output (the launcher's rule; decode_one_kernel has the others).
 // Blocks per SM, measured at 128 Mi bf16 elements (decode) and 32 Mi (mean of 8, with error feedback): decode with 8 / 6 /
 // 5 / 4 blocks 66 / 71 / 76 / 84 us; mean with four payloads in flight and 5 / 4 / 3 / 2 blocks 82 / 81 / 89 / 90 us (of two
 // payloads 49 / 50 / 56 / 56), eight in flight 107 / 82 / 91 / 100.  Compact, two in flight: 105 / 101 / 113 / 144.
@@ -381,6 +383,67 @@ decode_kernel(const __grid_constant__ LbcReduce p) {
     }
 }
 
+// One payload, written as it is (no scale, nothing added to): what a decode mostly is, without the registers of the rest.  U chunks per
+// thread are loaded before the first is decoded.
+// Microseconds in a CUDA graph, decode_kernel (8 blocks per SM, fp32: 6) / one chunk per thread at 8, 6 and 5 blocks / two at 8, 6, 5 and 4: bf16 2 Mi
+// elements 2.33 / 2.06 2.20 1.96 / 2.05 2.05 2.15 2.21, 4 Mi 2.70 / 2.56 2.53 2.53 / 3.10 3.06 2.72 2.43, 8 Mi 4.12 / 3.93 4.05 4.22 / 3.88 3.82 3.79 3.83, 16 Mi
+// 9.13 / 9.07 9.64 10.3 / 8.90 9.00 9.11 9.57, 128 Mi 61.5 / 60.9 66.1 70.8 / 61.2 61.0 60.7 63.1; in 4 bits 16 Mi 8.41 / 8.20 8.73 9.52 / 7.71 7.92 8.00
+// 8.79, 128 Mi 55.8 / 54.2 60.0 65.2 / 52.1 51.8 53.6 57.9; records 8 Mi 4.99 / 4.88 4.96 4.71 / 5.25 5.18 5.11 4.76, 32 Mi 18.4 / 18.1 19.4 19.5 / 18.5 19.1
+// 20.0 20.3; fp32 4 Mi 3.84 / 3.79 3.65 3.65 / 3.76 4.80 4.37 3.79, 8 Mi 8.11 / 7.27 7.78 7.79 / 6.99 7.64 7.49 7.43, 16 Mi 14.7 / 13.7 14.0 14.4 / 12.8 13.6
+// 13.2 13.9; 2 Mi 3.09 / 3.23 3.04 2.64 / 2.38 2.37 2.43 2.85; 4-bit records 1 Mi 1.94 / 2.19 2.18 2.18 / 1.92 1.92 1.89 1.88, 2 Mi 3.04 / 2.96 2.99 2.70 /
+// 2.60 2.63 2.46 2.46, 8 Mi 7.58 / 6.93 7.46 7.39 / 8.44 8.54 7.83 7.82.
+template <typename T, int G, int BIT, bool kCompact, int U, int kBlocks>
+__global__ void __launch_bounds__(kThreads, kBlocks) decode_one_kernel(const __grid_constant__ LbcReduce p) {
+    chain_wait();
+    constexpr int lanes = G / kElemsPerThread, lim = BIT == 8 ? 127 : 7;
+    constexpr int VB = G * BIT / 8, MB = sizeof(T), CB = kElemsPerThread * BIT / 8;
+    constexpr int tile_chunks = kThreads * U;
+    T* out = static_cast<T*>(p.out);
+    const uint8_t* src = p.src[0];
+    const int64_t chunks = (p.numel + G - 1) / G * lanes;
+    __shared__ __align__(16) uint8_t spans[kThreads / 32][kCompact ? span_bytes(G, VB + MB) : 16];
+    uint8_t* span = spans[threadIdx.x >> 5];
+    for (int64_t c0 = int64_t(blockIdx.x) * tile_chunks; c0 < chunks; c0 += int64_t(gridDim.x) * tile_chunks) {
+        const int64_t mine = c0 + threadIdx.x;
+        if ((c0 + tile_chunks) * kElemsPerThread > p.numel) {
+            for (int j = 0; j < U; ++j) decode_edge<T, G, BIT, kCompact, kFitTail>(p, mine + j * kThreads);
+            continue;
+        }
+        if constexpr (kCompact) {
+#pragma unroll
+            for (int j = 0; j < U; ++j) {
+                float d[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) d[i] = 0.0f;
+                add_batch<T, G, BIT, kCompact, 1>(p, 0, mine + j * kThreads, span, d);
+                store16<T>(out + (mine + j * kThreads) * kElemsPerThread, 0, 16, true, d);
+            }
+        } else {
+            uint4 codes[U];
+            float scale[U];
+#pragma unroll
+            for (int j = 0; j < U; ++j) {
+                const int64_t chunk = mine + j * kThreads;
+                if constexpr (CB == 16) {
+                    codes[j] = ld16_once(src + chunk * CB);
+                } else {
+                    const uint2 c = *reinterpret_cast<const uint2*>(src + chunk * CB);
+                    codes[j] = make_uint4(c.x, c.y, 0u, 0u);
+                }
+                scale[j] = load_scale<T>(src + p.layout_groups * VB + chunk / lanes * MB);
+            }
+#pragma unroll
+            for (int j = 0; j < U; ++j) {
+                const float step = over_limit<lim>(scale[j]);      // ahead of the codes, as in add_payload
+                float d[16];
+                codes16<T, BIT>(codes[j], d);
+                fma16(d, step, 0.0f);
+                store16<T>(out + (mine + j * kThreads) * kElemsPerThread, 0, 16, true, d);
+            }
+        }
+    }
+}
+
 // A tensor or a payload on another boundary (a view into a larger one; a row of a gather buffer whose payloads are no
 // multiple of 16 bytes).  kSeveral: more than one payload, or error feedback.
 // Blocks per SM, 16 Mi bf16 elements, planar 8-bit payloads of which one starts on 4 bytes, inputs beyond L2, 4 / 5 / 6
@@ -415,6 +478,22 @@ struct DecodeLauncher {
                     launch_chained(decode_ragged_kernel<T, G, BIT, kCompact, false>, grid, stream, *p);
                 else
                     launch_chained(decode_ragged_kernel<T, G, BIT, kCompact, true>, grid, stream, *p);
+                return;
+            }
+            if (p->num_src == 1 && p->residual_out == nullptr && p->scale == 1.0f && !p->accumulate) {
+                // Up to one default grid one chunk per thread, five blocks per SM; above, eight, and planar payloads two chunks (figures
+                // at the kernel).
+                if (blocks <= lbc_default_max_blocks()) {
+                    launch_chained(decode_one_kernel<T, G, BIT, kCompact, 1, 5>, grid, stream, *p);
+                    return;
+                }
+                if constexpr (!kCompact) {
+                    const int64_t pairs = (blocks + 1) / 2;
+                    launch_chained(decode_one_kernel<T, G, BIT, kCompact, 2, 8>, unsigned(p->max_blocks > 0 && pairs > p->max_blocks ? p->max_blocks : pairs),
+                                   stream, *p);
+                } else {
+                    launch_chained(decode_one_kernel<T, G, BIT, kCompact, 1, 8>, grid, stream, *p);
+                }
                 return;
             }
             // a compact payload takes two vectors per lane, so half as many are in flight
