@@ -13,7 +13,7 @@
 // after: encode of 32 Mi bf16 elements with error feedback 47.0 -> 39.2 us, decode of 128 Mi 94 -> 67.6 us, mean of eight payloads
 // of 32 Mi with error feedback 107 -> 89.8 us; then, each kernel started before the one ahead of it ends, and the scale's quotient
 // without a branch ahead of the codes: 37.5 us (6.3 TB/s), 63.9 us (6.4 TB/s) and 83.7 us (5.7 TB/s); the encode without a clamp and the decode
-// of one payload in a kernel of its own: 35.9 us (6.6 TB/s) and 61.5 us (6.6 TB/s).  Those are passes repeated
+// of one payload and the reduction of several in kernels of their own: 35.9 us (6.6 TB/s), 61.5 us (6.6 TB/s) and 76.7 us (6.2 TB/s).  Those are passes repeated
 // for a second; in bursts of a few milliseconds the mean of eight takes 80.5 us: it draws the card's 1000 W, and its clock falls to
 // 1.7 GHz.
 #include <type_traits>
@@ -326,11 +326,11 @@ __device__ __forceinline__ void decode_edge(const LbcReduce& p, int64_t chunk) {
     store16_fit<T, kFit>(out, first, p.numel, acc);             // rounds to T
 }
 
-// Tensors on 32 bytes, payloads on their vectors.  B payloads are in flight per thread.  B == 1: one payload, no error feedback, that is
-// scaled or added to the output (the launcher's rule; decode_one_kernel has the others).
-// Blocks per SM, measured at 128 Mi bf16 elements (decode) and 32 Mi (mean of 8, with error feedback): decode with 8 / 6 /
-// 5 / 4 blocks 66 / 71 / 76 / 84 us; mean with four payloads in flight and 5 / 4 / 3 / 2 blocks 82 / 81 / 89 / 90 us (of two
-// payloads 49 / 50 / 56 / 56), eight in flight 107 / 82 / 91 / 100.  Compact, two in flight: 105 / 101 / 113 / 144.
+// Tensors on 32 bytes, payloads on their vectors, decoded sums that are added to the output (`accumulate`), and fp32 records with error
+// feedback; decode_one_kernel and decode_several_kernel have the others.  B payloads are in flight per thread.  B == 1: one payload, no error feedback (the launcher's rule).
+// Blocks per SM, measured at 128 Mi bf16 elements (decode, while this kernel did all of them) and 32 Mi (mean of 8, with error feedback): decode
+// with 8 / 6 / 5 / 4 blocks 66 / 71 / 76 / 84 us; mean with four payloads in flight and 5 / 4 / 3 / 2 blocks 82 / 81 / 89 / 90 us (of two payloads 49 / 50
+// / 56 / 56), eight in flight 107 / 82 / 91 / 100.  Compact, two in flight: 105 / 101 / 113 / 144.
 template <typename T, int G, int BIT, bool kCompact, int B>
 __global__ void __launch_bounds__(kThreads, B == 1 ? (sizeof(T) == 2 ? 8 : 6) : (kCompact || sizeof(T) == 4 ? 4 : 5))
 decode_kernel(const __grid_constant__ LbcReduce p) {
@@ -378,6 +378,55 @@ decode_kernel(const __grid_constant__ LbcReduce p) {
             round16<T>(acc);
 #pragma unroll
             for (int i = 0; i < 16; ++i) acc[i] += prev[i];
+        }
+        store16<T>(out + first, 0, 16, true, acc);                     // rounds to T
+    }
+}
+
+// Several payloads, or one with error feedback, not added to the output: the reduction of gathered payloads, without the registers of the rest, which
+// made it spill at five blocks per SM.  B payloads are in flight per thread.
+// Microseconds in a CUDA graph with error feedback, decode_kernel (four in flight, five blocks per SM, fp32: four) / four in flight and 5 / 4 / 6
+// blocks / two and 5 / eight and 4: bf16, two payloads of 4 Mi elements 6.03 / 5.09 5.20 7.17 / 5.66 / 5.18, of 32 Mi 43.9 / 41.2 41.3 45.9 / 43.0 / 41.2; three 53.5
+// / 48.0 51.0 53.6 / 52.1 / 51.0; four 8.04 / 7.08 6.85 8.41 / 8.42 / 7.45, 56.3 / 52.5 51.1 53.7 / 60.2 / 55.1; eight 11.4 / 10.6 9.59 11.9 / 13.2 / 9.56, 79.7 /
+// 76.1 72.8 76.2 / 89.9 / 72.8; fp32, four of 2 Mi 5.67 / 6.98 5.53 9.09 / 6.97 / 5.78, eight 7.36 / 9.66 7.25 11.0 / 9.66 / 7.19, of 16 Mi 55.8 / 61.6 55.7 58.0 /
+// 61.6 / 54.2; eight of 16 Mi bf16 elements in 4 bits 32.9 / 32.8 32.5 33.4 / 34.0 / 31.9.
+// Without error feedback, four / five blocks, two bf16 payloads of 16 Mi 11.1 / 10.6.
+template <typename T, int G, int BIT, bool kCompact, int B, bool kFeedback>
+__global__ void __launch_bounds__(kThreads, kFeedback || kCompact || sizeof(T) == 4 ? 4 : 5) decode_several_kernel(const __grid_constant__ LbcReduce p) {
+    chain_wait();
+    constexpr int lanes = G / kElemsPerThread;
+    constexpr int VB = G * BIT / 8, MB = sizeof(T);
+    T* out = static_cast<T*>(p.out);
+    const T* prep = static_cast<const T*>(p.prepared);
+    T* rout = static_cast<T*>(p.residual_out);
+    const int64_t chunks = (p.numel + G - 1) / G * lanes;
+    const int R = p.num_src;
+    __shared__ __align__(16) uint8_t spans[kThreads / 32][kCompact ? span_bytes(G, VB + MB) : 16];
+    uint8_t* span = spans[threadIdx.x >> 5];
+    for (int64_t c0 = int64_t(blockIdx.x) * kThreads; c0 < chunks; c0 += int64_t(gridDim.x) * kThreads) {
+        const int64_t chunk = c0 + threadIdx.x;
+        if ((c0 + kThreads) * kElemsPerThread > p.numel) {
+            decode_edge<T, G, BIT, kCompact, kFitTail>(p, chunk);
+            continue;
+        }
+        const int64_t first = chunk * kElemsPerThread;
+        float acc[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[i] = 0.0f;
+        Raw16<T> held;
+        if (kFeedback) held = raw16(prep + first);                     // on its way while the payloads are summed
+        int r = 0;
+        for (; r + B <= R; r += B) add_batch<T, G, BIT, kCompact, B>(p, r, chunk, span, acc);
+        if constexpr (B > 2)
+            for (; r + 2 <= R; r += 2) add_batch<T, G, BIT, kCompact, 2>(p, r, chunk, span, acc);
+        for (; r < R; ++r) add_batch<T, G, BIT, kCompact, 1>(p, r, chunk, span, acc);
+        fma16(acc, p.scale, -0.0f);                                    // the product, with its sign where it is zero
+        if (kFeedback) {
+            float e[16];
+            up16<T>(held, e);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) e[i] -= acc[i];
+            store16<T>(rout + first, 0, 16, true, e);
         }
         store16<T>(out + first, 0, 16, true, acc);                     // rounds to T
     }
@@ -497,7 +546,12 @@ struct DecodeLauncher {
                 return;
             }
             // a compact payload takes two vectors per lane, so half as many are in flight
-            if (p->num_src == 1 && p->residual_out == nullptr)
+            // (fp32 records with error feedback are faster in decode_kernel: mean of two of 16 Mi elements 38.5 / 40.5 us, of eight 61.6 / 69.7)
+            if (!p->accumulate && p->residual_out != nullptr && !(kCompact && sizeof(T) == 4))
+                launch_chained(decode_several_kernel<T, G, BIT, kCompact, kCompact ? 2 : 4, true>, grid, stream, *p);
+            else if (!p->accumulate && p->residual_out == nullptr)
+                launch_chained(decode_several_kernel<T, G, BIT, kCompact, kCompact ? 2 : 4, false>, grid, stream, *p);
+            else if (p->num_src == 1 && p->residual_out == nullptr)
                 launch_chained(decode_kernel<T, G, BIT, kCompact, 1>, grid, stream, *p);
             else
                 launch_chained(decode_kernel<T, G, BIT, kCompact, kCompact ? 2 : 4>, grid, stream, *p);
