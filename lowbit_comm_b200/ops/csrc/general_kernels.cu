@@ -1146,10 +1146,9 @@ __device__ __noinline__ void requantize_by_place(uint32_t* words, int lane, int 
 // kFull: with a residual or two passes.  kPlain: neither.  kPlainAhead: neither, and the loads of a block's next tile are issued ahead of the
 // work on the present one (which waits for its loads at four blocks per SM otherwise: ncu, long scoreboard 3.6 per issue).
 enum : int { kFull = 0, kPlain = 1, kPlainAhead = 2 };
-template <typename T, int TOPK, int KIND, int kBlocks, int kForm>
-__global__ void __launch_bounds__(kThreads, kBlocks) roundtrip_general_kernel(const __grid_constant__ LbcRoundtripGeneral p) {
+template <typename T, int TOPK, int KIND, int kForm>
+__device__ __forceinline__ void roundtrip_general(const LbcRoundtripGeneral& p) {
     constexpr bool by_magnitude = TOPK >= 1 && KIND != kBookNoise;
-    chain_wait();
     const GroupShape shape = GroupShape::of<T, TOPK, KIND>(p.group_size);
     const int lanes = shape.lanes;
     __shared__ float lut[16];
@@ -1229,6 +1228,17 @@ __global__ void __launch_bounds__(kThreads, kBlocks) roundtrip_general_kernel(co
         }
         store_elems<T>(out, first, end, vec, y);
     }
+}
+
+template <typename T, int TOPK, int KIND, int kBlocks>
+__global__ void __launch_bounds__(kThreads, kBlocks) roundtrip_general_kernel(const __grid_constant__ LbcRoundtripGeneral p) {
+    chain_wait();
+    roundtrip_general<T, TOPK, KIND, kFull>(p);
+}
+template <typename T, int TOPK, int KIND, int kBlocks, bool kAhead>
+__global__ void __launch_bounds__(kThreads, kBlocks) roundtrip_plain_kernel(const __grid_constant__ LbcRoundtripGeneral p) {
+    chain_wait();
+    roundtrip_general<T, TOPK, KIND, kAhead ? kPlainAhead : kPlain>(p);
 }
 
 // A block per 4096 elements up to four times the default grid, a grid that loops above: it pays a block's set-up less
@@ -1382,11 +1392,13 @@ struct RoundtripGeneral {
                     constexpr bool book = KIND == kBook && TOPK == 0;
                     const int64_t resident = lbc_default_max_blocks() / 2;
                     if (tiles > (book ? resident : 2 * resident) || capped(tiles) < tiles)
-                        launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 4, kPlainAhead>, capped(tiles < resident ? tiles : resident), s, p);
+                        launch_chained(roundtrip_plain_kernel<T, TOPK, KIND, 4, true>, capped(tiles < resident ? tiles : resident), s, p);
+                    else if constexpr (book)
+                        launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 4>, unsigned(tiles), s, p);
                     else
-                        launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 4, book ? kFull : kPlain>, unsigned(tiles), s, p);
+                        launch_chained(roundtrip_plain_kernel<T, TOPK, KIND, 4, false>, unsigned(tiles), s, p);
                 } else {
-                    launch_chained(roundtrip_general_kernel<T, TOPK, KIND, KIND == kBook && TOPK == 0 ? 5 : 4, kPlain>, capped(tiles), s, p);
+                    launch_chained(roundtrip_plain_kernel<T, TOPK, KIND, KIND == kBook && TOPK == 0 ? 5 : 4, false>, capped(tiles), s, p);
                 }
                 return;
             }
@@ -1397,14 +1409,14 @@ struct RoundtripGeneral {
         // 8.56 / 8.61, 13.2 / 14.8, 42.3 / 45.5; 8 bits with noise, the last two, 13.2 / 14.4 and 42.2 / 45.5; e2m1 with noise 30.2 / 34.1 and
         // 107 / 116.
         if constexpr (sizeof(T) == 2) {
-            launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 4, kFull>, unsigned(grid), s, p);
+            launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 4>, unsigned(grid), s, p);
         } else {
             if constexpr (TOPK == 1 && KIND != kBookNoise)
                 if (p.residual == nullptr && grid > lbc_default_max_blocks() / 8 * 3) {
-                    launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 4, kFull>, unsigned(grid), s, p);
+                    launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 4>, unsigned(grid), s, p);
                     return;
                 }
-            launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 3, kFull>, unsigned(grid), s, p);
+            launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 3>, unsigned(grid), s, p);
         }
     }
 };
