@@ -169,8 +169,8 @@ typedef struct {
     int passes;                // 2: T(y) is encoded and decoded once more (the two-stage all-reduce)
     int own_error;             // residual_out = T(prepared - code * step) of the first encoding, one rounding
     int max_blocks;            // 0 = one block per tile
-    int pad;                   // out[numel .. numel + pad) becomes zero (a shard's elements past the tensor's end); with a
-                               // pad, numel is no multiple of 8 groups
+    int pad;                   // out[numel .. numel + pad) becomes zero (a shard's elements past the tensor's end); a
+                               // pad behind a multiple of 8 groups is refused
 } LbcRoundtrip;
 
 cudaError_t lbc_roundtrip(const LbcRoundtrip* p, cudaStream_t stream);

@@ -207,7 +207,8 @@ extern "C" {
 cudaError_t lbc_roundtrip(const LbcRoundtrip* p, cudaStream_t stream) {
     if (p == nullptr || p->numel < 0 || (p->passes != 1 && p->passes != 2)) return cudaErrorInvalidValue;
     if (p->residual == nullptr && (p->residual_out != nullptr || p->own_error)) return cudaErrorInvalidValue;
-    if (p->pad < 0) return cudaErrorInvalidValue;
+    // the pad is written with the tile that holds the tensor's end: a tensor that fills its tiles has none (see lbc_api.h)
+    if (p->pad < 0 || (p->pad > 0 && p->group_size > 0 && p->numel % (8 * int64_t(p->group_size)) == 0)) return cudaErrorInvalidValue;
     if (p->numel == 0) return cudaSuccess;
     if (p->x == nullptr || p->out == nullptr) return cudaErrorInvalidValue;
     return lbc::dispatch_profile<lbc::RoundtripLauncher>(p, stream);

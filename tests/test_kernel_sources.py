@@ -58,6 +58,33 @@ def test_a_chained_kernel_waits_before_it_lets_the_next_one_start():
         assert path.name == "common.cuh" or "griddepcontrol" not in _code(path.name)
 
 
+def test_a_pad_that_no_tile_would_write_is_refused():
+    """The one-rank pass clears a shard's pad with the tile that the tensor ends in, so behind whole tiles (and with nothing to
+    encode) no block would.  Refused before anything is launched: the addresses here belong to nobody."""
+
+    import ctypes
+
+    torch = pytest.importorskip("torch")      # (the extension links against its libraries)
+    assert torch is not None
+    if not build.extension_path().exists():
+        pytest.skip("the extension was not built here")
+
+    class Roundtrip(ctypes.Structure):
+        _fields_ = [*((name, ctypes.c_int) for name in ("dtype", "group_size", "bit")),
+                    *((name, ctypes.c_void_p) for name in ("x", "residual", "out", "residual_out")), ("numel", ctypes.c_int64),
+                    *((name, ctypes.c_int) for name in ("passes", "own_error", "max_blocks", "pad"))]
+
+    lib = ctypes.CDLL(str(build.extension_path()))
+    lib.lbc_roundtrip.argtypes = [ctypes.POINTER(Roundtrip), ctypes.c_void_p]
+    invalid = 1
+    for group in (16, 32, 64):
+        for numel, pad in ((0, 64), (8 * group, 8), (4096, 512), (3 * 8192, 1), (8 * group, -1)):
+            call = Roundtrip(dtype=1, group_size=group, bit=8, x=1 << 20, out=1 << 24, numel=numel, passes=1, pad=pad)
+            assert lib.lbc_roundtrip(ctypes.byref(call), None) == invalid, (group, numel, pad)
+    empty = Roundtrip(dtype=1, group_size=64, bit=8, x=1 << 20, out=1 << 24, numel=0, passes=1)
+    assert lib.lbc_roundtrip(ctypes.byref(empty), None) == 0
+
+
 def _spill_loads(source):
     """Kernel (with its template arguments) -> bytes of spill loads, from the last build."""
 
