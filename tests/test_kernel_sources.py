@@ -58,6 +58,16 @@ def test_a_chained_kernel_waits_before_it_lets_the_next_one_start():
         assert path.name == "common.cuh" or "griddepcontrol" not in _code(path.name)
 
 
+def test_code_books_take_no_vote_for_linear_codes():
+    """Whether linear codes may go without a clamp is one vote per chunk, and it waits for the group's scale.  The compiler keeps a vote whose
+    result nobody reads, so the code-book kernels must not ask."""
+
+    code = _code("general_kernels.cu")
+    body = code.split("bool all_near(", 1)[1].split("\n}\n")[0]
+    assert re.search(r"return !Kind<KIND>::book && __all_sync\(", body)
+    assert len(re.findall(r"all_near<KIND>\(", code)) == 3 and "all_near(m)" not in code
+
+
 def test_a_pad_that_no_tile_would_write_is_refused():
     """The one-rank pass clears a shard's pad with the tile that the tensor ends in, so behind whole tiles (and with nothing to
     encode) no block would.  Refused before anything is launched: the addresses here belong to nobody."""
