@@ -1139,14 +1139,14 @@ def test_one_rank_pass_without_a_residual(ext, dtype, bit, quant_type, topk, gro
 
 
 @pytest.mark.parametrize("dtype", ("bf16", "fp32"))
-@pytest.mark.parametrize("bit,quant_type,topk,compact", [(8, "linear", 1, False), (8, "linear", 2, True), (4, "e2m1", 0, False), (4, "normal", 1, True)])
+@pytest.mark.parametrize("bit,quant_type,topk,compact", [(8, "linear", 1, False), (8, "linear", 2, True), (4, "e2m1", 0, False), (4, "e2m1", 0, True), (4, "normal", 1, True)])
 def test_general_codec_where_its_kernels_change(ext, dtype, bit, quant_type, topk, compact):
     """Encode without a residual, and decode, on both sides of the sizes from which other kernels serve them (halves of the default
     grid), whole and ragged."""
 
     cfg = _cfg(bit=bit, quant_type=quant_type, topk=topk, compact=compact)
     half = int(ext.default_max_blocks()) // 2 * 4096
-    for n in (half - 1, half + 4096, 2 * half + 7, 3 * half, 4 * half + 1):
+    for n in (half // 2 - 7, half // 2 + 4096, half - 1, half + 4096, 2 * half, 2 * half + 7, 3 * half, 4 * half + 1):
         x = _data(n, DTYPES[dtype], seed=n % 89)
         want = oracle.encode(x, cfg)
         assert torch.equal(codec.quantize_tensor(x.cuda(), cfg).cpu(), want), n
