@@ -109,10 +109,15 @@ constexpr int encode_span(bool compact) { return compact ? span_bytes(G, G * BIT
 // 4 Mi 2.94 / 3.02 / 3.13 2.84 / 3.28, 8 Mi 7.93 / 7.72 / 7.68 7.70 / 7.75, 32 Mi 26.6 / 25.3 / 25.4 25.6 / 25.8; records 4 Mi 3.35 /
 // 3.39 / 3.49 3.55 / 4.07, 16 Mi 14.8 / 13.8 / 13.7 14.1 / 14.3.  With a residual, 4 / 5 / 6: bf16 4 Mi 4.30 / 4.26 / 4.22, 13 M 15.5 / 15.3 /
 // 15.4, 32 Mi 35.2 / 35.7 / 36.0, records 16 Mi 19.5 / 18.7 / 19.0; fp32 2 Mi 3.77 / 4.38 / 4.89, 16 Mi 33.2 / 33.3 / 33.3.
-template <typename T, bool kCompact, int U>
-constexpr int encode_kernel_blocks() { return (sizeof(T) == 2 && U == 2) || (kCompact && U == 1) ? 5 : 4; }
+// fp32 records with a residual, which hold 16 values, 16 residuals and the codes, 4 / 5: 1 Mi 2.39 / 2.50, 1.5 Mi 3.64 / 4.42, 2 Mi 3.87 / 4.61, 16 Mi
+// 33.2 / 33.4.
+template <typename T, bool kCompact, bool kResidual, int U>
+constexpr int encode_kernel_blocks() {
+    if (sizeof(T) == 4 && kResidual) return 4;
+    return (sizeof(T) == 2 && U == 2) || (kCompact && U == 1) ? 5 : 4;
+}
 template <typename T, int G, int BIT, bool kCompact, bool kResidual, int U>
-__global__ void __launch_bounds__(kThreads, encode_kernel_blocks<T, kCompact, U>()) encode_kernel(const __grid_constant__ LbcQuantPush p) {
+__global__ void __launch_bounds__(kThreads, encode_kernel_blocks<T, kCompact, kResidual, U>()) encode_kernel(const __grid_constant__ LbcQuantPush p) {
     chain_wait();
     constexpr int lanes = G / kElemsPerThread;
     constexpr int tile_chunks = kThreads * U;

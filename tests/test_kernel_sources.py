@@ -95,6 +95,11 @@ def test_a_pad_that_no_tile_would_write_is_refused():
     assert lib.lbc_roundtrip(ctypes.byref(empty), None) == 0
 
 
+def _plain_names(mangled):
+    names = subprocess.run(["c++filt"], input="\n".join(mangled), capture_output=True, text=True, check=True).stdout.split("\n")
+    return [re.sub(r"\((int|bool)\)", "", name.replace("void lbc::", "")).split("(Lbc")[0] for name in names]
+
+
 def _spill_loads(source):
     """Kernel (with its template arguments) -> bytes of spill loads, from the last build."""
 
@@ -102,10 +107,7 @@ def _spill_loads(source):
     if not report.exists() or shutil.which("c++filt") is None:
         pytest.skip("the extension was not built here")
     pairs = re.findall(r"Function properties for (\S+)\n.*?(\d+) bytes spill loads", report.read_text())
-    names = subprocess.run(["c++filt"], input="\n".join(name for name, _ in pairs), capture_output=True, text=True,
-                           check=True).stdout.split("\n")
-    plain = [re.sub(r"\((int|bool)\)", "", name.replace("void lbc::", "")).split("(Lbc")[0] for name in names]
-    return {name: int(loads) for name, (_, loads) in zip(plain, pairs)}
+    return {name: int(loads) for name, (_, loads) in zip(_plain_names([name for name, _ in pairs]), pairs)}
 
 
 def test_decode_kernels_keep_their_registers():
@@ -117,6 +119,21 @@ def test_decode_kernels_keep_their_registers():
     ragged = [v for k, v in loads.items() if k.startswith("decode_ragged_kernel<")]
     assert len(one) == 36 and len(ragged) == 72
     assert sum(one) <= 7300 and sum(ragged) <= 440
+
+
+def _registers(source):
+    report = build.ptxas_report(source)
+    if not report.exists() or shutil.which("c++filt") is None:
+        pytest.skip("the extension was not built here")
+    pairs = re.findall(r"Function properties for (\S+)\n.*\n.*?Used (\d+) registers", report.read_text())
+    return dict(zip(_plain_names([name for name, _ in pairs]), (int(n) for _, n in pairs)))
+
+
+def test_fp32_encoders_with_a_residual_have_room_for_both_tensors():
+    """Sixteen values and sixteen residuals per thread: with five blocks per SM (48 registers) records took a tenth longer."""
+
+    with_residual = [v for k, v in _registers("codec_kernels.cu").items() if re.match(r"encode_kernel<float, \d+, \d, \w+, true, 1", k)]
+    assert len(with_residual) == 12 and min(with_residual) > 48
 
 
 def test_fp32_one_rank_kernels_with_three_blocks_do_not_spill():
