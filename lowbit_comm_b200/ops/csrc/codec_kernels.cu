@@ -102,7 +102,7 @@ __device__ __forceinline__ void encode_edge(const LbcQuantPush& p, int64_t c0, i
 template <int G, int BIT, typename T>
 constexpr int encode_span(bool compact) { return compact ? span_bytes(G, G * BIT / 8 + int(sizeof(T))) : 16; }
 
-// All tensors on 32 bytes (the payload may start anywhere), no local_ef_out: what that takes in registers made the others spill.
+// All tensors on 32 bytes (the payload may start anywhere).  kOwnError: with local_ef_out, whose registers made the others spill.
 // Blocks per SM, us, bf16 no residual, one chunk per thread with 4 / 5 / 6, two with 4 / 5: 1 Mi elements 1.44 / 1.47 / 1.48 1.61 / 1.57,
 // 4 Mi 2.67 / 2.57 / 2.56 2.50 / 2.80, 8 Mi 4.88 / 4.69 / 4.47 4.08 / 4.13, 16 Mi 11.5 / 10.6 / 9.81 9.50 / 9.10, 64 Mi 41.0 / 36.8 / 33.8
 // 32.2 / 30.4; records 4 Mi 3.32 / 3.11 / 3.15 3.12 / 3.73, 16 Mi 13.3 / 12.0 / 11.2 11.1 / 10.4.  fp32 2 Mi 1.95 / 2.22 / 2.42 2.01 / 2.02,
@@ -116,8 +116,8 @@ constexpr int encode_kernel_blocks() {
     if (sizeof(T) == 4 && kResidual) return 4;
     return (sizeof(T) == 2 && U == 2) || (kCompact && U == 1) ? 5 : 4;
 }
-template <typename T, int G, int BIT, bool kCompact, bool kResidual, int U>
-__global__ void __launch_bounds__(kThreads, encode_kernel_blocks<T, kCompact, kResidual, U>()) encode_kernel(const __grid_constant__ LbcQuantPush p) {
+template <typename T, int G, int BIT, bool kCompact, bool kResidual, bool kOwnError, int U>
+__global__ void __launch_bounds__(kThreads, kOwnError ? 4 : encode_kernel_blocks<T, kCompact, kResidual, U>()) encode_kernel(const __grid_constant__ LbcQuantPush p) {
     chain_wait();
     constexpr int lanes = G / kElemsPerThread;
     constexpr int tile_chunks = kThreads * U;
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kThreads, encode_kernel_blocks<T, kCompact, kR
     uint8_t* span = spans[threadIdx.x >> 5];
     for (int64_t c0 = int64_t(blockIdx.x) * tile_chunks; c0 < chunks; c0 += int64_t(gridDim.x) * tile_chunks) {
         if ((c0 + tile_chunks) * kElemsPerThread > p.numel) {
-            encode_edge<T, G, BIT, kCompact, false, kFitTail>(p, c0, U, span);
+            encode_edge<T, G, BIT, kCompact, kOwnError, kFitTail>(p, c0, U, span);
             continue;
         }
         const int64_t mine = c0 + threadIdx.x;
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kThreads, encode_kernel_blocks<T, kCompact, kR
                 up16<T>(rr[j], r);
                 rx[j] = compensate16<T>(v, r);
             }
-            encode_chunk<T, G, BIT, kCompact, kResidual, false, kFitWhole>(p, rx[j], v, mine + j * kThreads, span);
+            encode_chunk<T, G, BIT, kCompact, kResidual, kOwnError, kFitWhole>(p, rx[j], v, mine + j * kThreads, span);
         }
     }
 }
@@ -155,9 +155,9 @@ __global__ void __launch_bounds__(kThreads, encode_kernel_blocks<T, kCompact, kR
 // A tensor on another boundary (a view into a larger one), in a kernel of its own: as a branch of encode_kernel this ran
 // out of line, element by element.  16 Mi elements, the input one element in, with error feedback (grid-stride kernel of
 // fast_kernels.cu / that branch / here): bf16 45.8 / 41.1 / 27.1 us, fp32 45.6 / 61.7 / 43.5.  Blocks per SM, fp32, 4 / 3:
-// 46.3 / 43.1 us.  kOwnError: with local_ef_out, tensors of any boundary; and all of fp32 on another boundary, because without it four
-// blocks fit an SM (4 Mi elements 11.5 -> 12.6 us, 16 Mi 40.9 -> 41.0).  Measured before and with encode16_near: bf16 4 Mi 6.96 -> 6.38, 16 Mi
-// 24.2 -> 22.6; with local_ef_out, aligned, as a branch of encode_kernel and here: bf16 4 Mi 6.5 / 6.0, 16 Mi 21.8 / 23.6, fp32 10.4 / 9.6, 33.8 / 33.0.
+// 46.3 / 43.1 us.  kOwnError: with local_ef_out, where the launcher finds this kernel faster for aligned tensors too; and all of fp32
+// on another boundary, because without it four blocks fit an SM (4 Mi elements 11.5 -> 12.6 us, 16 Mi 40.9 -> 41.0).  Measured before and
+// with encode16_near: bf16 4 Mi 6.96 -> 6.38, 16 Mi 24.2 -> 22.6.
 template <typename T, int G, int BIT, bool kCompact, bool kOwnError>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 4) encode_ragged_kernel(const __grid_constant__ LbcQuantPush p) {
     chain_wait();
@@ -180,6 +180,15 @@ struct EncodeLauncher {
         const auto go = [&](auto compact) {
             constexpr bool kCompact = decltype(compact)::value;
             const bool ragged = !on_boundary(32, p->x, p->residual, p->prepared_out);
+            // Aligned tensors with local_ef_out, encode_kernel / encode_ragged_kernel, us, bf16: 3 Mi elements 4.95 / 4.35, 4 Mi 6.54 / 5.80, 5 Mi
+            // (above one default grid) 8.08 / 8.96, 16 Mi 21.5 / 23.5, records 4 Mi 6.38 / 6.05, 5 Mi 8.41 / 9.46; fp32 1 Mi 2.92 / 3.10 (groups
+            // of 16: 3.25 / 2.99), 4 Mi 9.54 / 9.60, 32 Mi 64.0 / 64.0: always the second.
+            if constexpr (sizeof(T) == 2) {
+                if (p->local_ef_out != nullptr && p->residual != nullptr && !ragged && on_boundary(32, p->local_ef_out) && one > lbc_default_max_blocks()) {
+                    launch_chained(encode_kernel<T, G, BIT, kCompact, true, true, 1>, grid(one), stream, *p);
+                    return;
+                }
+            }
             if (p->local_ef_out != nullptr || (ragged && sizeof(T) == 4)) {
                 launch_chained(encode_ragged_kernel<T, G, BIT, kCompact, true>, grid(one), stream, *p);
                 return;
@@ -189,18 +198,18 @@ struct EncodeLauncher {
                 return;
             }
             if (p->residual != nullptr) {
-                launch_chained(encode_kernel<T, G, BIT, kCompact, true, 1>, grid(one), stream, *p);
+                launch_chained(encode_kernel<T, G, BIT, kCompact, true, false, 1>, grid(one), stream, *p);
                 return;
             }
             // Two chunks per thread above one default grid (4.85 M elements), but for fp32 records, which gain nothing from them: the
             // figures are at the kernel.
             if constexpr (sizeof(T) == 2 || !kCompact) {
                 if (one > lbc_default_max_blocks()) {
-                    launch_chained(encode_kernel<T, G, BIT, kCompact, false, 2>, grid((one + 1) / 2), stream, *p);
+                    launch_chained(encode_kernel<T, G, BIT, kCompact, false, false, 2>, grid((one + 1) / 2), stream, *p);
                     return;
                 }
             }
-            launch_chained(encode_kernel<T, G, BIT, kCompact, false, 1>, grid(one), stream, *p);
+            launch_chained(encode_kernel<T, G, BIT, kCompact, false, false, 1>, grid(one), stream, *p);
         };
         if (p->mode == LBC_PUSH_COMPACT_LOCAL)
             go(std::true_type{});

@@ -1152,3 +1152,39 @@ def test_general_codec_where_its_kernels_change(ext, dtype, bit, quant_type, top
         assert torch.equal(codec.quantize_tensor(x.cuda(), cfg).cpu(), want), n
         got = codec.dequantize_tensor(want.cuda(), (n,), cfg, dtype=dtype)
         assert torch.equal(got.cpu().view(torch.uint8), oracle.decode(want, n, cfg, dtype).view(torch.uint8)), n
+
+
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("bit,group,compact", [(8, 64, False), (8, 16, True), (4, 32, False)])
+def test_own_error_on_both_sides_of_one_grid(ext, dtype, bit, group, compact):
+    """Encode with this rank's own quantization error (one rounding, then the rounding to the type): the kernel of small and unaligned
+    tensors, and the one that takes aligned 16-bit ones above one default grid, whole, ragged and on a capped grid; the error in place of
+    the residual, and an infinity whose warp takes the clamp."""
+
+    cfg, T, lim = _cfg(bit=bit, group_size=group, compact=compact), DTYPES[dtype], 127.0 if bit == 8 else 7.0
+    edge = int(ext.default_max_blocks()) * 4096
+    for n, blocks in ((edge, 0), (edge + 4096, 0), (edge + 4099, 0), (edge + 8192 + 5, 700)):
+        x = _data(n, T, seed=n % 83)
+        r = (_data(n, T, seed=n % 79, outliers=False) * 1e-3).to(T)
+        x[n // 3] = float("inf")
+        prepared = oracle.prepare(x, r)
+        values = oracle._grouped(prepared, group).float()
+        scale = values.abs().amax(1).to(T).float()
+        t = values * (torch.tensor(lim) / scale.clamp_min(1e-6))[:, None]
+        codes = torch.where(t.isnan(), -lim, t.round().clamp(-lim, lim))       # (infinity times zero: the clamp's lowest code)
+        words = oracle._pack_words(codes.to(torch.int64) & (255 if bit == 8 else 15), bit, x.element_size())
+        scales = scale.to(T).view(torch.uint8).reshape(len(scale), -1)
+        want = torch.cat([words, scales], 1).reshape(-1) if compact else torch.cat([words.reshape(-1), scales.reshape(-1)])
+        left = (values.double() - codes.double() * (scale / torch.tensor(lim))[:, None].double()).float().to(T).reshape(-1)[:n]
+        finite = torch.ones(n, dtype=torch.bool)
+        finite[n // 3 // group * group:(n // 3 // group + 1) * group] = False
+        for skew in (0, 1):
+            source = torch.empty(n + skew, dtype=T, device="cuda")[skew:]
+            source.copy_(x)
+            residual, payload = r.cuda(), torch.zeros(want.numel(), dtype=torch.uint8, device="cuda")
+            ext.quant_push(source, residual, None, residual, [payload.data_ptr()],
+                           ext.PUSH_COMPACT_LOCAL if compact else ext.PUSH_BROADCAST, 0, -(-n // group), 0, group, bit, None, blocks)
+            assert torch.equal(payload.cpu(), want), (n, skew)
+            got = residual.cpu()
+            assert torch.equal(got[finite].view(torch.uint8), left[finite].view(torch.uint8)), (n, skew)
+            assert bool(got[~finite].float().isnan().any()) or bool((~got[~finite].float().isfinite()).any())
