@@ -1354,9 +1354,10 @@ struct DequantGeneral {
         // Five, above half a default grid and up to two (us, four / five / six / eight): fp32, e2m1 4 Mi 4.41 / 4.11 / 4.12 / 4.27, 5 M 5.11 /
         // 4.74 / 4.79 / 4.72, one kept value 4.44 / 4.05 / 4.07 / 4.68, 5.58 / 5.11 / 5.07 / 5.29, below, 2 Mi, 2.94 / 3.18 / 3.45 / 3.01; planar
         // 16-bit payloads with kept values and linear codes, bf16, one 4 Mi 3.39 / 3.35 / 3.42 / 3.67, 8 Mi 6.10 / 5.97 / 5.88 / 6.14, two 3.72 / 3.57 /
-        // 3.59 / 4.03, 6.80 / 6.58 / 6.43 / 6.90, below, 2 Mi, 2.60 / 2.57 / 2.79 / 2.50, above, 16 Mi, - / 11.8 / - / 11.3.
+        // 3.59 / 4.03, 6.80 / 6.58 / 6.43 / 6.90, below, 2 Mi, 2.60 / 2.57 / 2.79 / 2.50, above, 16 Mi, - / 11.8 / - / 11.3.  16-bit ones in 4 bits up to
+        // one default grid, five / eight, bf16, two kept values: 3 Mi 3.22 / 3.89, 4 Mi 3.86 / 3.96, 5 Mi 4.61 / 4.45, 8 Mi 6.84 / 6.43.
         const int64_t grid_tiles = lbc_default_max_blocks();
-        const bool five = 2 * tiles > grid_tiles && tiles <= 2 * grid_tiles &&
+        const bool five = 2 * tiles > grid_tiles && tiles <= (sizeof(T) == 2 && Kind<KIND>::bit == 4 ? grid_tiles : 2 * grid_tiles) &&
                           (sizeof(T) == 4 || (!p.compact && TOPK >= 1 && !Kind<KIND>::book));
         const bool many = sizeof(T) == 2 ? !(p.compact && TOPK >= 1) : tiles > 2 * grid_tiles;
         if (five && !p.accumulate)

@@ -1139,7 +1139,8 @@ def test_one_rank_pass_without_a_residual(ext, dtype, bit, quant_type, topk, gro
 
 
 @pytest.mark.parametrize("dtype", ("bf16", "fp32"))
-@pytest.mark.parametrize("bit,quant_type,topk,compact", [(8, "linear", 1, False), (8, "linear", 2, True), (4, "e2m1", 0, False), (4, "e2m1", 0, True), (4, "normal", 1, True)])
+@pytest.mark.parametrize("bit,quant_type,topk,compact", [(8, "linear", 1, False), (8, "linear", 2, True), (4, "linear", 2, False), (4, "e2m1", 0, False),
+                                                        (4, "e2m1", 0, True), (4, "normal", 1, True)])
 def test_general_codec_where_its_kernels_change(ext, dtype, bit, quant_type, topk, compact):
     """Encode without a residual, and decode, on both sides of the sizes from which other kernels serve them (halves of the default
     grid), whole and ragged."""
