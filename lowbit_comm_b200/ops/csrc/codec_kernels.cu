@@ -340,8 +340,8 @@ __device__ __forceinline__ void decode_edge(const LbcReduce& p, int64_t chunk) {
     store16_fit<T, kFit>(out, first, p.numel, acc);             // rounds to T
 }
 
-// Tensors on 32 bytes, payloads on their vectors, decoded sums that are added to the output (`accumulate`), and fp32 records with error
-// feedback; decode_one_kernel and decode_several_kernel have the others.  B payloads are in flight per thread.  B == 1: one payload, no error feedback (the launcher's rule).
+// Tensors on 32 bytes, payloads on their vectors, decoded sums that are added to the output (`accumulate`), fp32 records with error
+// feedback, and some in 4 bits; decode_one_kernel and decode_several_kernel have the others.  B payloads are in flight per thread.  B == 1: one payload, no error feedback (the launcher's rule).
 // Blocks per SM, measured at 128 Mi bf16 elements (decode, while this kernel did all of them) and 32 Mi (mean of 8, with error feedback): decode
 // with 8 / 6 / 5 / 4 blocks 66 / 71 / 76 / 84 us; mean with four payloads in flight and 5 / 4 / 3 / 2 blocks 82 / 81 / 89 / 90 us (of two payloads 49 / 50
 // / 56 / 56), eight in flight 107 / 82 / 91 / 100.  Compact, two in flight: 105 / 101 / 113 / 144.
@@ -544,6 +544,16 @@ struct DecodeLauncher {
                 return;
             }
             if (p->num_src == 1 && p->residual_out == nullptr && p->scale == 1.0f && !p->accumulate) {
+                // fp32 records in 4 bits from a block for every other SM up to three per SM, decode_kernel / decode_one_kernel, us: 0.25 Mi elements 1.57 /
+                // 1.53, 0.5 Mi 1.69 / 1.78, 1 Mi 1.91 / 2.14, 1.5 Mi 2.17 / 2.56, 2 Mi 3.05 / 2.69; groups of 16, 1 Mi, 2.07 / 2.04.  (Six blocks per SM in
+                // decode_one_kernel, or its product with the scale, do not bring them there; what does was not found.)
+                if constexpr (kCompact && BIT == 4 && sizeof(T) == 4 && G > 16) {
+                    const int64_t full = lbc_default_max_blocks();
+                    if (blocks > full / 16 && blocks <= full / 8 * 3) {
+                        launch_chained(decode_kernel<T, G, BIT, kCompact, 1>, grid, stream, *p);
+                        return;
+                    }
+                }
                 // Up to one default grid one chunk per thread, five blocks per SM; above, eight, and planar payloads two chunks (figures
                 // at the kernel).
                 if (blocks <= lbc_default_max_blocks()) {

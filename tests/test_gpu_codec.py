@@ -1189,3 +1189,15 @@ def test_own_error_on_both_sides_of_one_grid(ext, dtype, bit, group, compact):
             got = residual.cpu()
             assert torch.equal(got[finite].view(torch.uint8), left[finite].view(torch.uint8)), (n, skew)
             assert bool(got[~finite].float().isnan().any()) or bool((~got[~finite].float().isfinite()).any())
+
+
+@pytest.mark.parametrize("group", (16, 32, 64))
+def test_fp32_records_in_four_bits_where_their_kernels_change(ext, group):
+    """Decode on both sides of a sixteenth, three eighths and the whole of a default grid, whole and ragged."""
+
+    cfg, full = _cfg(bit=4, group_size=group, compact=True), int(ext.default_max_blocks()) * 4096
+    for n in (full // 16, full // 16 + 5, full // 8 * 3 - 4096, full // 8 * 3, full // 8 * 3 + 1, full, full + 9):
+        x = _data(n, torch.float32, seed=n % 73)
+        payload = oracle.encode(x, cfg)
+        got = codec.dequantize_tensor(payload.cuda(), (n,), cfg, dtype="fp32")
+        assert torch.equal(got.cpu().view(torch.uint8), oracle.decode(payload, n, cfg, "fp32").view(torch.uint8)), n
