@@ -340,8 +340,9 @@ __device__ __forceinline__ void decode_edge(const LbcReduce& p, int64_t chunk) {
     store16_fit<T, kFit>(out, first, p.numel, acc);             // rounds to T
 }
 
-// Tensors on 32 bytes, payloads on their vectors, decoded sums that are added to the output (`accumulate`), fp32 records with error
-// feedback, and some in 4 bits; decode_one_kernel and decode_several_kernel have the others.  B payloads are in flight per thread.  B == 1: one payload, no error feedback (the launcher's rule).
+// Tensors on 32 bytes, payloads on their vectors.  B == 1: one payload without error feedback that is added to the output (`accumulate`), and
+// some fp32 records in 4 bits.  B == 2: fp32 records with error feedback, two payloads in flight per thread.  decode_one_kernel and decode_several_kernel have
+// the others.
 // Blocks per SM, measured at 128 Mi bf16 elements (decode, while this kernel did all of them) and 32 Mi (mean of 8, with error feedback): decode
 // with 8 / 6 / 5 / 4 blocks 66 / 71 / 76 / 84 us; mean with four payloads in flight and 5 / 4 / 3 / 2 blocks 82 / 81 / 89 / 90 us (of two payloads 49 / 50
 // / 56 / 56), eight in flight 107 / 82 / 91 / 100.  Compact, two in flight: 105 / 101 / 113 / 144.
@@ -536,14 +537,16 @@ struct DecodeLauncher {
             bool vectors = on_boundary(32, p->out, p->prepared, p->residual_out);
             for (int r = 0; r < p->num_src; ++r)
                 vectors = vectors && on_boundary(kCompact ? 16 : kElemsPerThread * BIT / 8, p->src[r]);
-            if (!vectors) {
-                if (p->num_src == 1 && p->residual_out == nullptr)
+            const bool alone = p->num_src == 1 && p->residual_out == nullptr;
+            // (a sum of several, or one with error feedback, that is added to the output: no call of the library asks for it)
+            if (!vectors || (p->accumulate && !alone)) {
+                if (alone)
                     launch_chained(decode_ragged_kernel<T, G, BIT, kCompact, false>, grid, stream, *p);
                 else
                     launch_chained(decode_ragged_kernel<T, G, BIT, kCompact, true>, grid, stream, *p);
                 return;
             }
-            if (p->num_src == 1 && p->residual_out == nullptr && p->scale == 1.0f && !p->accumulate) {
+            if (alone && p->scale == 1.0f && !p->accumulate) {
                 // fp32 records in 4 bits from a block for every other SM up to three per SM, decode_kernel / decode_one_kernel, us: 0.25 Mi elements 1.57 /
                 // 1.53, 0.5 Mi 1.69 / 1.78, 1 Mi 1.91 / 2.14, 1.5 Mi 2.17 / 2.56, 2 Mi 3.05 / 2.69; groups of 16, 1 Mi, 2.07 / 2.04.  (Six blocks per SM in
                 // decode_one_kernel, or its product with the scale, do not bring them there; what does was not found.)
@@ -570,15 +573,14 @@ struct DecodeLauncher {
                 return;
             }
             // a compact payload takes two vectors per lane, so half as many are in flight
-            // (fp32 records with error feedback are faster in decode_kernel: mean of two of 16 Mi elements 38.5 / 40.5 us, of eight 61.6 / 69.7)
-            if (!p->accumulate && p->residual_out != nullptr && !(kCompact && sizeof(T) == 4))
-                launch_chained(decode_several_kernel<T, G, BIT, kCompact, kCompact ? 2 : 4, true>, grid, stream, *p);
-            else if (!p->accumulate && p->residual_out == nullptr)
-                launch_chained(decode_several_kernel<T, G, BIT, kCompact, kCompact ? 2 : 4, false>, grid, stream, *p);
-            else if (p->num_src == 1 && p->residual_out == nullptr)
+            if (p->accumulate)
                 launch_chained(decode_kernel<T, G, BIT, kCompact, 1>, grid, stream, *p);
+            else if (p->residual_out == nullptr)
+                launch_chained(decode_several_kernel<T, G, BIT, kCompact, kCompact ? 2 : 4, false>, grid, stream, *p);
+            else if constexpr (kCompact && sizeof(T) == 4)      // (mean of two of 16 Mi elements, decode_kernel / decode_several_kernel, 38.5 / 40.5 us, of eight 61.6 / 69.7)
+                launch_chained(decode_kernel<T, G, BIT, kCompact, 2>, grid, stream, *p);
             else
-                launch_chained(decode_kernel<T, G, BIT, kCompact, kCompact ? 2 : 4>, grid, stream, *p);
+                launch_chained(decode_several_kernel<T, G, BIT, kCompact, kCompact ? 2 : 4, true>, grid, stream, *p);
         };
         if (p->compact)
             go(std::true_type{});

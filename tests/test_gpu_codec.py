@@ -1201,3 +1201,27 @@ def test_fp32_records_in_four_bits_where_their_kernels_change(ext, group):
         payload = oracle.encode(x, cfg)
         got = codec.dequantize_tensor(payload.cuda(), (n,), cfg, dtype="fp32")
         assert torch.equal(got.cpu().view(torch.uint8), oracle.decode(payload, n, cfg, "fp32").view(torch.uint8)), n
+
+
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("bit,group,compact", [(8, 64, False), (8, 16, True), (4, 32, True)])
+def test_sums_that_are_added_to_the_output(ext, dtype, bit, group, compact):
+    """One payload and several, with and without error feedback, whole and ragged ends, aligned tensors and views: T(sum) is added to what the
+    output holds, one rounding; the residual is that of the sum alone."""
+
+    cfg, T = _cfg(bit=bit, group_size=group, compact=compact), DTYPES[dtype]
+    for n in (group, 4096 * 2, 4096 * 3 + group + 5):
+        payloads = [oracle.encode(_data(n, T, seed=k), cfg) for k in range(5)]
+        held, prepared = _data(n, T, seed=11), _data(n, T, seed=12)
+        for count in (1, 2, 5):
+            y, y32 = oracle.reduce_mean(payloads[:count], n, cfg, dtype)
+            want = (held.float() + y.float()).to(T)
+            for feedback in (False, True):
+                for skew in (0, 1):
+                    out = torch.empty(n + skew, dtype=T, device="cuda")[skew:]
+                    out.copy_(held)
+                    dev, res = [p.cuda() for p in payloads[:count]], torch.empty(n, dtype=T, device="cuda")
+                    ext.reduce([d.data_ptr() for d in dev], -(-n // group), 0, compact, n, codec._DTYPE_CODE[dtype], group, bit, 1.0 / count, out, True,
+                               prepared.cuda() if feedback else None, res if feedback else None, [], 0, 0, None, None, 0)
+                    assert torch.equal(out.cpu(), want), (n, count, feedback, skew)
+                    assert not feedback or torch.equal(res.cpu(), oracle.residual_update(prepared, y32)), (n, count, skew)

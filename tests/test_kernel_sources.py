@@ -129,6 +129,15 @@ def _registers(source):
     return dict(zip(_plain_names([name for name, _ in pairs]), (int(n) for _, n in pairs)))
 
 
+def test_no_decode_kernel_that_nothing_reaches():
+    """The general form of the decoder serves one payload that is added to the output, and fp32 records with error feedback."""
+
+    names = [k for k in _spill_loads("codec_kernels.cu") if k.startswith("decode_kernel<")]
+    assert len([k for k in names if k.endswith(", 1>")]) == 36
+    assert sorted(k for k in names if not k.endswith(", 1>")) == sorted(
+        "decode_kernel<float, %d, %d, true, 2>" % (group, bit) for group in (16, 32, 64) for bit in (4, 8))
+
+
 def test_fp32_encoders_with_a_residual_have_room_for_both_tensors():
     """Sixteen values and sixteen residuals per thread: with five blocks per SM (48 registers) records took a tenth longer."""
 
