@@ -62,8 +62,9 @@ class GeneralPeerWorkspace:
         if is_fast_profile(config):
             raise ValueError("linear / top-k 0 / deterministic profiles are served by FusedWorkspace")
         self.group, self.dtype, self.config = group, dtype, config
-        self.max_numel, self.max_blocks, self.fused = int(max_numel), int(max_blocks), bool(fused)
+        self.max_numel, self.fused = int(max_numel), bool(fused)
         self.ext = group._ext
+        self.max_blocks = int(max_blocks)
         self._torch_dtype = oracle.TORCH_DTYPES[dtype]
         self.slot_bytes = self.payload_bytes(dtype, config, self.max_numel)
         self.stage_off = group.alloc(self.slot_bytes)
@@ -72,9 +73,19 @@ class GeneralPeerWorkspace:
         self.launches = 0
         self.gather_off: list[int] | None = None          # two-stage only: reserved on first use
         self._shard: torch.Tensor | None = None           # two-stage only: this rank's dense reduced shard
+
+    @property
+    def max_blocks(self) -> int:
+        """Most blocks of a launch (0: as many as the kernel's own rule has)."""
+
+        return self._max_blocks
+
+    @max_blocks.setter
+    def max_blocks(self, blocks: int) -> None:
+        cfg, self._max_blocks = self.config, blocks
         self._one_rank = None if not hasattr(self.ext, "one_rank_general") else SimpleNamespace(one_rank=partial(
-            self.ext.one_rank_general, config.group_size, config.bit, config.topk, _QUANT_CODE[config.quant_type],
-            _DTYPE_CODE[dtype], self.max_blocks, self.max_numel))
+            self.ext.one_rank_general, cfg.group_size, cfg.bit, cfg.topk, _QUANT_CODE[cfg.quant_type],
+            _DTYPE_CODE[self.dtype], blocks, self.max_numel))
 
     @staticmethod
     def payload_bytes(dtype: str, config: CompressionConfig, numel: int) -> int:

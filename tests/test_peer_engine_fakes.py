@@ -515,3 +515,20 @@ def test_shards_and_gathered_tensors_are_plain_tensors(monkeypatch, world):
     assert [type(o) for o in outs] == [torch.Tensor] * world and all(torch.equal(o, x.as_subclass(torch.Tensor)) for o in outs)
     shard = Communicator._validated_out(None, x, 4)
     assert type(shard) is torch.Tensor and shard.shape == (4,) and shard.dtype == x.dtype
+
+
+def test_whole_one_rank_calls_of_a_general_workspace_follow_its_block_limit():
+    """`max_blocks` may be set on a workspace at any time: the native call has the one that `all_reduce` reads."""
+
+    from types import SimpleNamespace
+
+    from lowbit_comm_b200.parallel.fused_general import GeneralPeerWorkspace
+
+    calls = []
+    ext = SimpleNamespace(one_rank_general=lambda *args: calls.append(args))
+    group = SimpleNamespace(_ext=ext, world_size=1, rank=0, _closed=False, alloc=lambda nbytes: 0, new_channel=lambda: 0)
+    ws = GeneralPeerWorkspace(group, dtype="bf16", config=CompressionConfig(topk=1), max_numel=4096, max_blocks=3)
+    for limit in (3, 7, 0):
+        ws.max_blocks = limit
+        ws.one_rank_plans()[0].one_rank("x", None, None, 1, True, False, 99)
+        assert ws.max_blocks == limit and calls[-1][5] == limit and calls[-1][-1] == 99
