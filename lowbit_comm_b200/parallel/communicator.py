@@ -39,14 +39,29 @@ from ..ops import codec
 from ..ops.loader import load_cuda_extension
 from ..ops.sizing import estimate_quantized_size
 from ..utils import tracing
+from .fused import default_stages
 from .payload import payload_buffer
 from .torch_transport import make_torch_all_gather, make_torch_all_to_all, make_torch_tensor_all_reduce
 
 TWO_STAGE = frozenset({"reduce_scatter", "topology", "ring", "tree", "p2p", "overlap-gather", "overlap-p2p",
                        "overlap-tree", "overlap-scale", "compressed"})
 ONE_STAGE = frozenset({"all_gather"})
+
+
+def _stages(strategy: str) -> int | None:
+    """Stages that a strategy names; None: as many as are faster (`default_stages`)."""
+
+    if strategy in ("auto", "all_reduce"):
+        return None
+    if strategy in ONE_STAGE:
+        return 1
+    if strategy in TWO_STAGE:
+        return 2
+    raise UnsupportedCollective(f"all_reduce:{strategy}", reason="unknown strategy")
+
+
 # encodings an all-reduce of one rank makes of a value: one for every stage of the strategy
-_ONE_RANK_PASSES = {"auto": 1, "all_reduce": 1, **dict.fromkeys(ONE_STAGE, 1), **dict.fromkeys(TWO_STAGE, 2)}
+_ONE_RANK_PASSES = {name: _stages(name) or default_stages(1, 0) for name in ("auto", "all_reduce", *ONE_STAGE, *TWO_STAGE)}
 
 _REGISTRY: dict[int, "Communicator"] = {}
 _REGISTRY_LOCK = threading.Lock()
@@ -307,7 +322,7 @@ class Communicator:
             return ImmediateWork(result) if async_op else result
         if strategy == "hierarchical":
             return self.hierarchical_all_reduce(tensor, config=config, op=op, async_op=async_op, dtype=dtype, out=out)
-        stages = self._stages(strategy)
+        stages = _stages(strategy)
         if self.peer_usable(tensor, config):
             try:
                 ws = self.workspace(tensor, config, name)
@@ -376,7 +391,7 @@ class Communicator:
         if op not in ("sum", "mean"):
             raise UnsupportedCollective(f"all_reduce:{op}", reason="only op='sum' and op='mean' are implemented")
         general = strategy in ("native_nccl", "hierarchical")
-        stages = None if general else self._stages(strategy)
+        stages = None if general else _stages(strategy)
         held: list[Any] = [None]
 
         def call(tensor: Any) -> Any:
@@ -400,19 +415,8 @@ class Communicator:
 
         return call
 
-    def _stages(self, strategy: str) -> int | None:
-        if strategy in ("auto", "all_reduce"):
-            return None
-        if strategy in ONE_STAGE:
-            return 1
-        if strategy in TWO_STAGE:
-            return 2
-        raise UnsupportedCollective(f"all_reduce:{strategy}", reason="unknown strategy")
-
     def _torch_all_reduce(self, tensor, config, op, stages, name, out, residual, update_residual):
         prepared = tensor if residual is None else (tensor.float() + residual.float()).to(tensor.dtype)
-        from .fused import default_stages
-
         stages = stages or default_stages(self.world_size, tensor.numel() * tensor.element_size())
         shape = tuple(tensor.shape)
         gather = make_torch_all_gather(group=self.process_group)
