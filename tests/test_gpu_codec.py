@@ -1225,3 +1225,29 @@ def test_sums_that_are_added_to_the_output(ext, dtype, bit, group, compact):
                                prepared.cuda() if feedback else None, res if feedback else None, [], 0, 0, None, None, 0)
                     assert torch.equal(out.cpu(), want), (n, count, feedback, skew)
                     assert not feedback or torch.equal(res.cpu(), oracle.residual_update(prepared, y32)), (n, count, skew)
+
+
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("bit", (8, 4))
+def test_quotients_over_the_range_of_scales(ext, dtype, bit):
+    """The encoder multiplies by L / scale and the decoder by scale / L, both rounded correctly without a division: every scale of the
+    16-bit types from 1e-6 to 1e30 and one in 1021 of fp32, each with values whose products lie beside the halves between two codes, where a
+    quotient one step off gives another code."""
+
+    cfg, T, lim, group = _cfg(bit=bit, group_size=16), DTYPES[dtype], 127.0 if bit == 8 else 7.0, 16
+    if dtype == "fp32":
+        ends = torch.tensor([1e-6, 1e30]).view(torch.int32).tolist()
+        scale = torch.arange(ends[0], ends[1] + 1021, 1021, dtype=torch.int32).view(T)
+    else:
+        scale = torch.arange(1 << 15, dtype=torch.int32).to(torch.int16).view(T)
+        scale = scale[(scale.float() >= 1e-6) & (scale.float() <= 1e30)]
+    mul = torch.tensor(lim) / scale.float()
+    at = torch.linspace(0.0, lim - 1, 15).round() + 0.5
+    values = (at * torch.tensor([1.0, -1.0]).repeat(8)[:15] / mul.double()[:, None]).float().to(T)
+    x = torch.cat([scale[:, None], torch.minimum(torch.maximum(values, -scale[:, None]), scale[:, None])], 1)
+    codes = (x.float() * mul[:, None]).round().clamp(-lim, lim)
+    want = (codes * (scale.float() / torch.tensor(lim))[:, None]).to(T)
+    payload = codec.quantize_tensor(x.reshape(-1).cuda(), cfg)
+    got = codec.dequantize_tensor(payload, (x.numel(),), cfg, dtype=dtype).cpu().reshape(x.shape)
+    wrong = (got + 0.0 != want + 0.0).any(1)                       # (a code 0 is +0)
+    assert not bool(wrong.any()), (int(wrong.sum()), scale[wrong][:4], x[wrong][:1], got[wrong][:1], want[wrong][:1])

@@ -647,3 +647,65 @@ def test_one_rank_shard_ends_in_zeros(ext, dtype, bit, group):
     finally:
         groups[0].process_group = None
         PeerGroup.close_loopback(groups)
+
+
+@pytest.mark.parametrize("blocks", (0, 7))
+@pytest.mark.parametrize("dtype", ("bf16", "fp32"))
+def test_one_rank_shard_of_many_tiles_ends_in_zeros(ext, dtype, blocks):
+    """As above where a thread takes two chunks (16 bits, above one default grid): an end in the first and in the second half of a
+    tile of 8192 elements, whole tiles beside it; and on a capped grid, whose blocks go round."""
+
+    cfg, edge = CompressionConfig(allow_experimental=True), int(ext.default_max_blocks()) * 4096
+    groups, wss = _make(1, dtype, cfg, edge + 40_000, max_blocks=blocks)
+    try:
+        ws = wss[0]
+        groups[0].process_group = object()          # the native plan serves real process groups only
+        ws._ensure_legacy()
+        ws._build_native()
+        for n in (8192 * 20, 8192 * 20 + 4096 + 63, edge + 1, edge + 4096 + 65, edge + 8192, edge + 3 * 8192 + 511):
+            shard_numel = geometry(n, 1, dtype, cfg).shard_numel
+            x = torch.empty(n, dtype=DT[dtype], device="cuda").normal_(std=1e-2)
+            want = codec.dequantize_tensor(codec.quantize_tensor(x, cfg), (n,), cfg, dtype=dtype)
+            base = torch.full((shard_numel + 64,), 7.0, dtype=DT[dtype], device="cuda")
+            before = ws.launches
+            ws.reduce_scatter(x, base[:shard_numel])
+            assert ws.launches == before + 1
+            assert torch.equal(base[:n], want), n
+            assert bool((base[n:shard_numel] == 0).all()) and bool((base[shard_numel:] == 7).all()), n
+        torch.cuda.synchronize()
+        groups[0].check_status()
+    finally:
+        groups[0].process_group = None
+        PeerGroup.close_loopback(groups)
+
+
+@pytest.mark.parametrize("over", ("input", "residual"))
+def test_a_shard_whose_pad_lies_over_its_input_is_cleared_first(ext, over):
+    """The one pass would write zeros that other blocks still read: such a call goes the way of the phases, which clear the pad, then read."""
+
+    cfg, n = CompressionConfig(), 4096 * 3 + 100
+    groups, wss = _make(1, "bf16", cfg, 20_000)
+    try:
+        ws = wss[0]
+        groups[0].process_group = object()          # the native plan serves real process groups only
+        ws._ensure_legacy()
+        ws._build_native()
+        shard_numel = geometry(n, 1, "bf16", cfg).shard_numel
+        pad = shard_numel - n
+        x, r = (torch.empty(n, dtype=torch.bfloat16, device="cuda").normal_(std=1e-2) for _ in range(2))
+        apart = {"input": x.clone(), "residual": r.clone()}
+        apart[over][:pad] = 0
+        want = torch.empty(shard_numel, dtype=torch.bfloat16, device="cuda")
+        ws.reduce_scatter(apart["input"], want, residual=apart["residual"])
+        base = torch.zeros(2 * n, dtype=torch.bfloat16, device="cuda")
+        base[n:] = x if over == "input" else r
+        given = {"input": x, "residual": r, over: base[n:]}
+        before = ws.launches
+        ws.reduce_scatter(given["input"], base[:shard_numel], residual=given["residual"])
+        assert ws.launches > before + 1
+        assert torch.equal(base[:n], want[:n]) and torch.equal(given["residual"], apart["residual"])
+        torch.cuda.synchronize()
+        groups[0].check_status()
+    finally:
+        groups[0].process_group = None
+        PeerGroup.close_loopback(groups)
