@@ -1316,14 +1316,18 @@ struct QuantGeneral {
         if (p.num_dst > 0 || p.signal.num_remote > 0)      // for other ranks, who wait for it
             quant_general_kernel<T, TOPK, KIND><<<grid, kThreads, 0, s>>>(p);
         else if (p.compact ? (at & 15) == 0 : (at & (Kind<KIND>::CB - 1)) == 0) {
-            // Without a residual, in the kernels that know it, but for code-books where those are slower.  us with / without, encodes in a CUDA
-            // graph, spread 0.2 %.  16 bits: up to half a default grid (bf16 e2m1 2 Mi elements 3.07 / 3.54, 3 Mi 4.61 / 4.37), records that keep
-            // nothing up to a whole one (4 Mi 5.26 / 5.45, 5 Mi 6.54 / 5.98).  fp32 that keeps nothing: outside a quarter of one (1 Mi 2.34 / 2.53,
-            // 1.5 Mi 3.80 / 3.45) to a whole one (4 Mi 5.46 / 5.11, 5 Mi 5.88 / 6.04, 8 Mi 9.2 / 10.0).
+            // Without a residual, in the kernels that know it, but where those are slower.  us with / without, encodes in a CUDA graph,
+            // spread 0.2 %.  Code-books, 16 bits: up to half a default grid (bf16 e2m1 2 Mi elements 3.07 / 3.54, 3 Mi 4.61 / 4.37),
+            // records that keep nothing up to a whole one (4 Mi 5.26 / 5.45, 5 Mi 6.54 / 5.98).  fp32 ones that keep nothing: outside a
+            // quarter of one (1 Mi 2.34 / 2.53, 1.5 Mi 3.80 / 3.45) to a whole one (4 Mi 5.46 / 5.11, 5 Mi 5.88 / 6.04, 8 Mi 9.2 / 10.0).
+            // Linear codes, 16 bits, planar, one kept value: many waves of full grids, where five blocks per SM hide more than the
+            // residual's registers cost (bf16 8 Mi 7.95 / 8.00, fp16 7.80 / 7.62, bf16 12 Mi 12.7 / 13.0, 16 Mi 16.4 / 16.8); looping grids
+            // have no waves (32 Mi 30.2 / 28.7).
             const int64_t tiles = (p.numel + kThreads * kElemsPerThread - 1) / (kThreads * kElemsPerThread), full = lbc_default_max_blocks();
             bool plain = KIND != kBookNoise && p.residual == nullptr && p.prepared_out == nullptr;
             if (KIND == kBook && sizeof(T) == 2) plain = plain && tiles > (p.compact && TOPK == 0 ? full : full / 2);
             if (KIND == kBook && sizeof(T) == 4 && TOPK == 0) plain = plain && tiles > full / 4 && tiles <= full;
+            if (KIND != kBook && sizeof(T) == 2 && TOPK == 1 && !p.compact) plain = plain && (tiles <= 2 * full || tiles > grid);
             const auto go = [&](auto prepare) {
                 constexpr bool kPrepare = decltype(prepare)::value;
                 if (p.compact) launch_chained(encode_general_kernel<T, TOPK, KIND, true, kPrepare>, unsigned(grid), s, p);

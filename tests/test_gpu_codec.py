@@ -1147,7 +1147,7 @@ def test_general_codec_where_its_kernels_change(ext, dtype, bit, quant_type, top
 
     cfg = _cfg(bit=bit, quant_type=quant_type, topk=topk, compact=compact)
     half = int(ext.default_max_blocks()) // 2 * 4096
-    for n in (half // 2 - 7, half // 2 + 4096, half - 1, half + 4096, 2 * half, 2 * half + 7, 3 * half, 4 * half + 1):
+    for n in (half // 2 - 7, half // 2 + 4096, half - 1, half + 4096, 2 * half, 2 * half + 7, 3 * half, 4 * half + 1, 5 * half + 3):
         x = _data(n, DTYPES[dtype], seed=n % 89)
         want = oracle.encode(x, cfg)
         assert torch.equal(codec.quantize_tensor(x.cuda(), cfg).cpu(), want), n
