@@ -6,16 +6,13 @@
 // Reference: quantization/quant_pack_kernel.cu:84-163, quantization/dequant_reduce_kernel.cu:38-69, 150-221.
 //
 // What bounds these kernels: memory.  A block per tile (a persistent grid moved 10-15 % less; the loops over tiles serve
-// grids that a caller caps, and fp32 records), 32 bytes of input per thread in one load, payloads read and written as
-// 16-byte vectors in both layouts, the whole-tile path free of bounds and alignment tests (their registers cost
-// occupancy); tensors and payloads off those boundaries have kernels of their own.
-// Measured on a B200 through the public calls, int8 groups of 64, before (grid-stride kernels of fast_kernels.cu) and
-// after: encode of 32 Mi bf16 elements with error feedback 47.0 -> 39.2 us, decode of 128 Mi 94 -> 67.6 us, mean of eight payloads
-// of 32 Mi with error feedback 107 -> 89.8 us; then, each kernel started before the one ahead of it ends, and the scale's quotient
-// without a branch ahead of the codes: 37.5 us (6.3 TB/s), 63.9 us (6.4 TB/s) and 83.7 us (5.7 TB/s); the encode without a clamp and the decode
-// of one payload and the reduction of several in kernels of their own: 35.9 us (6.6 TB/s), 61.5 us (6.6 TB/s) and 76.7 us (6.2 TB/s).  Those are passes repeated
-// for a second; in bursts of a few milliseconds the mean of eight takes 80.5 us: it draws the card's 1000 W, and its clock falls to
-// 1.7 GHz.
+// grids that a caller caps), 32 bytes of input per thread in one load, payloads read and written as 16-byte vectors in
+// both layouts, the whole-tile path free of bounds and alignment tests (their registers cost occupancy); tensors and
+// payloads off those boundaries have kernels of their own.
+// Measured on a B200 through the public calls, passes repeated for a second, int8 groups of 64, the grid-stride kernels
+// of fast_kernels.cu and now: encode of 32 Mi bf16 elements with error feedback 47.0 -> 36.0 us (6.6 TB/s), decode of
+// 128 Mi 94 -> 61.5 (6.6 TB/s), mean of eight payloads of 32 Mi with error feedback 107 -> 76.4 (6.3 TB/s): that one
+// draws the card's 1000 W, and its clock falls to 1.7 GHz.  Below, us in CUDA graphs.
 #include <type_traits>
 
 #include "codec_device.cuh"
@@ -31,7 +28,8 @@ namespace lbc {
 // warp's staging area for compact records.  kPrepared: `held` came out of a sum.  kOwnError: this rank's quantization error may be
 // asked for (local_ef_out).
 template <typename T, int G, int BIT, bool kCompact, bool kPrepared, bool kOwnError, int kFit>
-__device__ __forceinline__ void encode_chunk(const LbcQuantPush& p, const Raw16<T>& held, float (&v)[16], int64_t chunk, uint8_t* span) {
+__device__ __forceinline__ void encode_chunk(const LbcQuantPush& p, const Raw16<T>& held, float (&v)[16], int64_t chunk,
+                                             uint8_t* span) {
     constexpr int lanes = G / kElemsPerThread;
     constexpr int VB = G * BIT / 8, MB = sizeof(T), CB = kElemsPerThread * BIT / 8;
     T* prep = static_cast<T*>(p.prepared_out);
@@ -102,22 +100,21 @@ __device__ __forceinline__ void encode_edge(const LbcQuantPush& p, int64_t c0, i
 template <int G, int BIT, typename T>
 constexpr int encode_span(bool compact) { return compact ? span_bytes(G, G * BIT / 8 + int(sizeof(T))) : 16; }
 
-// All tensors on 32 bytes (the payload may start anywhere).  kOwnError: with local_ef_out, whose registers made the others spill.
-// Blocks per SM, us, bf16 no residual, one chunk per thread with 4 / 5 / 6, two with 4 / 5: 1 Mi elements 1.44 / 1.47 / 1.48 1.61 / 1.57,
-// 4 Mi 2.67 / 2.57 / 2.56 2.50 / 2.80, 8 Mi 4.88 / 4.69 / 4.47 4.08 / 4.13, 16 Mi 11.5 / 10.6 / 9.81 9.50 / 9.10, 64 Mi 41.0 / 36.8 / 33.8
-// 32.2 / 30.4; records 4 Mi 3.32 / 3.11 / 3.15 3.12 / 3.73, 16 Mi 13.3 / 12.0 / 11.2 11.1 / 10.4.  fp32 2 Mi 1.95 / 2.22 / 2.42 2.01 / 2.02,
-// 4 Mi 2.94 / 3.02 / 3.13 2.84 / 3.28, 8 Mi 7.93 / 7.72 / 7.68 7.70 / 7.75, 32 Mi 26.6 / 25.3 / 25.4 25.6 / 25.8; records 4 Mi 3.35 /
-// 3.39 / 3.49 3.55 / 4.07, 16 Mi 14.8 / 13.8 / 13.7 14.1 / 14.3.  With a residual, 4 / 5 / 6: bf16 4 Mi 4.30 / 4.26 / 4.22, 13 M 15.5 / 15.3 /
-// 15.4, 32 Mi 35.2 / 35.7 / 36.0, records 16 Mi 19.5 / 18.7 / 19.0; fp32 2 Mi 3.77 / 4.38 / 4.89, 16 Mi 33.2 / 33.3 / 33.3.
-// fp32 records with a residual, which hold 16 values, 16 residuals and the codes, 4 / 5: 1 Mi 2.39 / 2.50, 1.5 Mi 3.64 / 4.42, 2 Mi 3.87 / 4.61, 16 Mi
-// 33.2 / 33.4.
+// All tensors on 32 bytes (the payload may start anywhere).  kOwnError: with local_ef_out, whose registers made the
+// others spill.
+// Blocks per SM: four leave a thread 64 registers, five 48.  Five where two 16-bit chunks are in flight (bf16, 4 / 5:
+// 8 Mi elements 4.08 / 4.13, 16 Mi 9.50 / 9.10, 64 Mi 32.2 / 30.4) and for records, but for fp32 ones with a residual, whose
+// 16 values and 16 residuals do not fit (without: bf16 16 Mi 13.3 / 12.0, fp32 14.8 / 13.8; bf16 with one, 19.5 / 18.6; fp32
+// with one, 1.5 Mi 3.66 / 4.42, 16 Mi 33.3 / 33.4).  Four for the others (bf16, 1 Mi 1.44 / 1.47, with a residual
+// 32 Mi 35.2 / 35.7; fp32, 2 Mi 1.95 / 2.22, with a residual 3.77 / 4.38).
 template <typename T, bool kCompact, bool kResidual, int U>
 constexpr int encode_kernel_blocks() {
     if (sizeof(T) == 4 && kResidual) return 4;
     return (sizeof(T) == 2 && U == 2) || (kCompact && U == 1) ? 5 : 4;
 }
 template <typename T, int G, int BIT, bool kCompact, bool kResidual, bool kOwnError, int U>
-__global__ void __launch_bounds__(kThreads, kOwnError ? 4 : encode_kernel_blocks<T, kCompact, kResidual, U>()) encode_kernel(const __grid_constant__ LbcQuantPush p) {
+__global__ void __launch_bounds__(kThreads, kOwnError ? 4 : encode_kernel_blocks<T, kCompact, kResidual, U>())
+encode_kernel(const __grid_constant__ LbcQuantPush p) {
     chain_wait();
     constexpr int lanes = G / kElemsPerThread;
     constexpr int tile_chunks = kThreads * U;
@@ -180,11 +177,12 @@ struct EncodeLauncher {
         const auto go = [&](auto compact) {
             constexpr bool kCompact = decltype(compact)::value;
             const bool ragged = !on_boundary(32, p->x, p->residual, p->prepared_out);
-            // Aligned tensors with local_ef_out, encode_kernel / encode_ragged_kernel, us, bf16: 3 Mi elements 4.95 / 4.35, 4 Mi 6.54 / 5.80, 5 Mi
-            // (above one default grid) 8.08 / 8.96, 16 Mi 21.5 / 23.5, records 4 Mi 6.38 / 6.05, 5 Mi 8.41 / 9.46; fp32 1 Mi 2.92 / 3.10 (groups
-            // of 16: 3.25 / 2.99), 4 Mi 9.54 / 9.60, 32 Mi 64.0 / 64.0: always the second.
+            // Aligned tensors with local_ef_out, encode_kernel / encode_ragged_kernel: bf16, 3 Mi elements 4.95 / 4.35, 4 Mi
+            // 6.54 / 5.80, 5 Mi (above one default grid) 8.08 / 8.96, 16 Mi 21.5 / 23.5, records 4 Mi 6.38 / 6.05, 5 Mi 8.41 / 9.46;
+            // fp32 always the second: 1 Mi 2.92 / 3.10 (groups of 16: 3.25 / 2.99), 4 Mi 9.54 / 9.60, 32 Mi 64.0 / 64.0.
             if constexpr (sizeof(T) == 2) {
-                if (p->local_ef_out != nullptr && p->residual != nullptr && !ragged && on_boundary(32, p->local_ef_out) && one > lbc_default_max_blocks()) {
+                if (p->local_ef_out != nullptr && p->residual != nullptr && !ragged && on_boundary(32, p->local_ef_out) &&
+                    one > lbc_default_max_blocks()) {
                     launch_chained(encode_kernel<T, G, BIT, kCompact, true, true, 1>, grid(one), stream, *p);
                     return;
                 }
@@ -194,15 +192,16 @@ struct EncodeLauncher {
                 return;
             }
             if (ragged) {
-                if constexpr (sizeof(T) == 2) launch_chained(encode_ragged_kernel<T, G, BIT, kCompact, false>, grid(one), stream, *p);
+                if constexpr (sizeof(T) == 2)
+                    launch_chained(encode_ragged_kernel<T, G, BIT, kCompact, false>, grid(one), stream, *p);
                 return;
             }
             if (p->residual != nullptr) {
                 launch_chained(encode_kernel<T, G, BIT, kCompact, true, false, 1>, grid(one), stream, *p);
                 return;
             }
-            // Two chunks per thread above one default grid (4.85 M elements), but for fp32 records, which gain nothing from them: the
-            // figures are at the kernel.
+            // Two chunks per thread above one default grid (one / two: bf16 4 Mi elements 2.57 / 2.50, 8 Mi 4.88 / 4.08, 64 Mi 41.0 /
+            // 30.4; fp32 4 Mi 2.94 / 2.84, 32 Mi 26.6 / 25.6), but for fp32 records, which gain nothing (16 Mi 13.8 / 14.1).
             if constexpr (sizeof(T) == 2 || !kCompact) {
                 if (one > lbc_default_max_blocks()) {
                     launch_chained(encode_kernel<T, G, BIT, kCompact, false, false, 2>, grid((one + 1) / 2), stream, *p);
@@ -223,12 +222,10 @@ struct EncodeLauncher {
 // decode and reduce
 // ---------------------------------------------------------------------------
 // acc += one payload's 16 values: fma(code, scale / L, acc), one rounding per payload.  kPairs: two of them to an instruction
-// (sm_100+) and the quotient without a branch; whole tiles.  Several payloads draw the card's power limit, so instructions are time:
-// mean of eight of 32 Mi bf16 elements 86.5 -> 84.2 us.  One payload (scalar / packed): 128 Mi 62.6 / 61.6, in 4 bits 57.7 / 56.4,
-// records 70.8 / 68.6; 64 Mi fp32 54.2 / 52.9, records 52.0 / 52.1, in 4 bits 50.6 / 49.5, their records 48.8 / 49.3 (with the
-// quotient after the codes packed was behind, 63.6 / 65.7).  Unaligned ones and tensor ends stay scalar: with the quotient without
-// a branch the mean of eight of 16 Mi fp32 elements in records of 16, one payload on 8 bytes, took 64.4 us instead of 61.5, of
-// bf16 ones 56.3 instead of 55.7, of planar bf16 payloads 46.1 instead of 46.9.
+// (sm_100+) and the quotient without a branch; whole tiles.  Several payloads draw the card's power limit, so instructions
+// are time: mean of eight of 32 Mi bf16 elements 86.5 -> 84.2 us, decode of 128 Mi 62.6 -> 61.6.  Unaligned tensors and
+// tensor ends stay scalar: packed, the mean of eight of 16 Mi fp32 elements in records of 16, one payload on 8 bytes, took
+// 64.4 us instead of 61.5.
 template <typename T, int BIT, bool kPairs>
 __device__ __forceinline__ void add_payload(float (&acc)[16], uint4 codes, float scale) {
     constexpr int lim = BIT == 8 ? 127 : 7;
@@ -243,7 +240,8 @@ __device__ __forceinline__ void add_payload(float (&acc)[16], uint4 codes, float
     if constexpr (kPairs) {
 #pragma unroll
         for (int i = 0; i < 16; i += 2)
-            asm("{.reg .b64 a, b, c; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %4}; mov.b64 c, {%0, %1}; fma.rn.f32x2 c, a, b, c; mov.b64 {%0, %1}, c;}"
+            asm("{.reg .b64 a, b, c; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %4}; mov.b64 c, {%0, %1}; "
+                "fma.rn.f32x2 c, a, b, c; mov.b64 {%0, %1}, c;}"
                 : "+f"(acc[i]), "+f"(acc[i + 1]) : "f"(d[i]), "f"(d[i + 1]), "f"(step));
     } else {
 #pragma unroll
@@ -340,12 +338,11 @@ __device__ __forceinline__ void decode_edge(const LbcReduce& p, int64_t chunk) {
     store16_fit<T, kFit>(out, first, p.numel, acc);             // rounds to T
 }
 
-// Tensors on 32 bytes, payloads on their vectors.  B == 1: one payload without error feedback that is added to the output (`accumulate`), and
-// some fp32 records in 4 bits.  B == 2: fp32 records with error feedback, two payloads in flight per thread.  decode_one_kernel and decode_several_kernel have
-// the others.
-// Blocks per SM, measured at 128 Mi bf16 elements (decode, while this kernel did all of them) and 32 Mi (mean of 8, with error feedback): decode
-// with 8 / 6 / 5 / 4 blocks 66 / 71 / 76 / 84 us; mean with four payloads in flight and 5 / 4 / 3 / 2 blocks 82 / 81 / 89 / 90 us (of two payloads 49 / 50
-// / 56 / 56), eight in flight 107 / 82 / 91 / 100.  Compact, two in flight: 105 / 101 / 113 / 144.
+// Tensors on 32 bytes, payloads on their vectors.  B == 1: one payload without error feedback that is added to the
+// output (`accumulate`), and some fp32 records in 4 bits.  B == 2: fp32 records with error feedback, two payloads in
+// flight per thread.  decode_one_kernel and decode_several_kernel have the others.
+// Blocks per SM as where this kernel did all of them: a decode of 128 Mi bf16 elements with 8 / 6 / 5 / 4 blocks 66 / 71 /
+// 76 / 84; records, mean of eight, two in flight, with 5 / 4 / 3 blocks 105 / 101 / 113.
 template <typename T, int G, int BIT, bool kCompact, int B>
 __global__ void __launch_bounds__(kThreads, B == 1 ? (sizeof(T) == 2 ? 8 : 6) : (kCompact || sizeof(T) == 4 ? 4 : 5))
 decode_kernel(const __grid_constant__ LbcReduce p) {
@@ -398,16 +395,14 @@ decode_kernel(const __grid_constant__ LbcReduce p) {
     }
 }
 
-// Several payloads, or one with error feedback, not added to the output: the reduction of gathered payloads, without the registers of the rest, which
-// made it spill at five blocks per SM.  B payloads are in flight per thread.
-// Microseconds in a CUDA graph with error feedback, decode_kernel (four in flight, five blocks per SM, fp32: four) / four in flight and 5 / 4 / 6
-// blocks / two and 5 / eight and 4: bf16, two payloads of 4 Mi elements 6.03 / 5.09 5.20 7.17 / 5.66 / 5.18, of 32 Mi 43.9 / 41.2 41.3 45.9 / 43.0 / 41.2; three 53.5
-// / 48.0 51.0 53.6 / 52.1 / 51.0; four 8.04 / 7.08 6.85 8.41 / 8.42 / 7.45, 56.3 / 52.5 51.1 53.7 / 60.2 / 55.1; eight 11.4 / 10.6 9.59 11.9 / 13.2 / 9.56, 79.7 /
-// 76.1 72.8 76.2 / 89.9 / 72.8; fp32, four of 2 Mi 5.67 / 6.98 5.53 9.09 / 6.97 / 5.78, eight 7.36 / 9.66 7.25 11.0 / 9.66 / 7.19, of 16 Mi 55.8 / 61.6 55.7 58.0 /
-// 61.6 / 54.2; eight of 16 Mi bf16 elements in 4 bits 32.9 / 32.8 32.5 33.4 / 34.0 / 31.9.
-// Without error feedback, four / five blocks, two bf16 payloads of 16 Mi 11.1 / 10.6.
+// Several payloads, or one with error feedback, not added to the output: the reduction of gathered payloads, without the
+// registers of the rest, which made it spill at five blocks per SM.  B payloads are in flight per thread.
+// With error feedback four blocks per SM (mean of eight of 32 Mi bf16 elements, decode_kernel / five / four / six 79.7 /
+// 76.1 / 72.8 / 76.2; eight of 2 Mi fp32 7.36 / 9.66 / 7.25 / 11.0), four in flight (two of 32 Mi bf16, two / four / eight
+// 43.0 / 41.3 / 41.2; four of 4 Mi 8.42 / 6.85 / 7.45).  Without, five for 16 bits: two of 16 Mi 11.1 / 10.6.
 template <typename T, int G, int BIT, bool kCompact, int B, bool kFeedback>
-__global__ void __launch_bounds__(kThreads, kFeedback || kCompact || sizeof(T) == 4 ? 4 : 5) decode_several_kernel(const __grid_constant__ LbcReduce p) {
+__global__ void __launch_bounds__(kThreads, kFeedback || kCompact || sizeof(T) == 4 ? 4 : 5)
+decode_several_kernel(const __grid_constant__ LbcReduce p) {
     chain_wait();
     constexpr int lanes = G / kElemsPerThread;
     constexpr int VB = G * BIT / 8, MB = sizeof(T);
@@ -447,15 +442,12 @@ __global__ void __launch_bounds__(kThreads, kFeedback || kCompact || sizeof(T) =
     }
 }
 
-// One payload, written as it is (no scale, nothing added to): what a decode mostly is, without the registers of the rest.  U chunks per
-// thread are loaded before the first is decoded.
-// Microseconds in a CUDA graph, decode_kernel (8 blocks per SM, fp32: 6) / one chunk per thread at 8, 6 and 5 blocks / two at 8, 6, 5 and 4: bf16 2 Mi
-// elements 2.33 / 2.06 2.20 1.96 / 2.05 2.05 2.15 2.21, 4 Mi 2.70 / 2.56 2.53 2.53 / 3.10 3.06 2.72 2.43, 8 Mi 4.12 / 3.93 4.05 4.22 / 3.88 3.82 3.79 3.83, 16 Mi
-// 9.13 / 9.07 9.64 10.3 / 8.90 9.00 9.11 9.57, 128 Mi 61.5 / 60.9 66.1 70.8 / 61.2 61.0 60.7 63.1; in 4 bits 16 Mi 8.41 / 8.20 8.73 9.52 / 7.71 7.92 8.00
-// 8.79, 128 Mi 55.8 / 54.2 60.0 65.2 / 52.1 51.8 53.6 57.9; records 8 Mi 4.99 / 4.88 4.96 4.71 / 5.25 5.18 5.11 4.76, 32 Mi 18.4 / 18.1 19.4 19.5 / 18.5 19.1
-// 20.0 20.3; fp32 4 Mi 3.84 / 3.79 3.65 3.65 / 3.76 4.80 4.37 3.79, 8 Mi 8.11 / 7.27 7.78 7.79 / 6.99 7.64 7.49 7.43, 16 Mi 14.7 / 13.7 14.0 14.4 / 12.8 13.6
-// 13.2 13.9; 2 Mi 3.09 / 3.23 3.04 2.64 / 2.38 2.37 2.43 2.85; 4-bit records 1 Mi 1.94 / 2.19 2.18 2.18 / 1.92 1.92 1.89 1.88, 2 Mi 3.04 / 2.96 2.99 2.70 /
-// 2.60 2.63 2.46 2.46, 8 Mi 7.58 / 6.93 7.46 7.39 / 8.44 8.54 7.83 7.82.
+// One payload, written as it is (no scale, nothing added to): what a decode mostly is, without the registers of the rest.
+// U chunks per thread are loaded before the first is decoded.
+// Small grids want five blocks per SM (48 registers), large ones eight, and planar payloads two chunks: one chunk with
+// 5 / 8 blocks / two with 8, bf16 2 Mi elements 1.96 / 2.06 / 2.05, 4 Mi 2.53 / 2.56 / 3.10, 8 Mi 4.22 / 3.93 / 3.88,
+// 128 Mi 70.8 / 60.9 / 61.2, in 4 bits 65.2 / 54.2 / 52.1; records 32 Mi 19.5 / 18.1 / 18.5; fp32 4 Mi 3.65 / 3.79 / 3.76,
+// 16 Mi 14.4 / 13.7 / 12.8.
 template <typename T, int G, int BIT, bool kCompact, int U, int kBlocks>
 __global__ void __launch_bounds__(kThreads, kBlocks) decode_one_kernel(const __grid_constant__ LbcReduce p) {
     chain_wait();
@@ -538,7 +530,8 @@ struct DecodeLauncher {
             for (int r = 0; r < p->num_src; ++r)
                 vectors = vectors && on_boundary(kCompact ? 16 : kElemsPerThread * BIT / 8, p->src[r]);
             const bool alone = p->num_src == 1 && p->residual_out == nullptr;
-            // (a sum of several, or one with error feedback, that is added to the output: no call of the library asks for it)
+            // (A sum of several, or one with error feedback, that is added to the output: no call of the library asks for it.
+            // Eight of 16 Mi bf16 elements take 42.9 us there, 35.6 in a kernel of their own.)
             if (!vectors || (p->accumulate && !alone)) {
                 if (alone)
                     launch_chained(decode_ragged_kernel<T, G, BIT, kCompact, false>, grid, stream, *p);
@@ -547,9 +540,10 @@ struct DecodeLauncher {
                 return;
             }
             if (alone && p->scale == 1.0f && !p->accumulate) {
-                // fp32 records in 4 bits from a block for every other SM up to three per SM, decode_kernel / decode_one_kernel, us: 0.25 Mi elements 1.57 /
-                // 1.53, 0.5 Mi 1.69 / 1.78, 1 Mi 1.91 / 2.14, 1.5 Mi 2.17 / 2.56, 2 Mi 3.05 / 2.69; groups of 16, 1 Mi, 2.07 / 2.04.  (Six blocks per SM in
-                // decode_one_kernel, or its product with the scale, do not bring them there; what does was not found.)
+                // fp32 records in 4 bits from a block for every other SM up to three per SM, decode_kernel / decode_one_kernel:
+                // 0.25 Mi elements 1.57 / 1.53, 0.5 Mi 1.69 / 1.78, 1 Mi 1.91 / 2.14, 1.5 Mi 2.17 / 2.56, 2 Mi 3.05 / 2.69; groups of
+                // 16, 1 Mi, 2.07 / 2.04.  (Neither six blocks per SM nor the product with the scale bring decode_one_kernel
+                // there; what does was not found.)
                 if constexpr (kCompact && BIT == 4 && sizeof(T) == 4 && G > 16) {
                     const int64_t full = lbc_default_max_blocks();
                     if (blocks > full / 16 && blocks <= full / 8 * 3) {
@@ -557,16 +551,14 @@ struct DecodeLauncher {
                         return;
                     }
                 }
-                // Up to one default grid one chunk per thread, five blocks per SM; above, eight, and planar payloads two chunks (figures
-                // at the kernel).
+                // Up to one default grid (bf16: 4 Mi small, 8 Mi large in the figures at the kernel)
                 if (blocks <= lbc_default_max_blocks()) {
                     launch_chained(decode_one_kernel<T, G, BIT, kCompact, 1, 5>, grid, stream, *p);
                     return;
                 }
                 if constexpr (!kCompact) {
-                    const int64_t pairs = (blocks + 1) / 2;
-                    launch_chained(decode_one_kernel<T, G, BIT, kCompact, 2, 8>, unsigned(p->max_blocks > 0 && pairs > p->max_blocks ? p->max_blocks : pairs),
-                                   stream, *p);
+                    const int64_t pairs = (blocks + 1) / 2, cap = p->max_blocks > 0 ? p->max_blocks : pairs;
+                    launch_chained(decode_one_kernel<T, G, BIT, kCompact, 2, 8>, unsigned(pairs < cap ? pairs : cap), stream, *p);
                 } else {
                     launch_chained(decode_one_kernel<T, G, BIT, kCompact, 1, 8>, grid, stream, *p);
                 }
@@ -577,7 +569,7 @@ struct DecodeLauncher {
                 launch_chained(decode_kernel<T, G, BIT, kCompact, 1>, grid, stream, *p);
             else if (p->residual_out == nullptr)
                 launch_chained(decode_several_kernel<T, G, BIT, kCompact, kCompact ? 2 : 4, false>, grid, stream, *p);
-            else if constexpr (kCompact && sizeof(T) == 4)      // (mean of two of 16 Mi elements, decode_kernel / decode_several_kernel, 38.5 / 40.5 us, of eight 61.6 / 69.7)
+            else if constexpr (kCompact && sizeof(T) == 4)      // (16 Mi, this / the other, two 38.5 / 40.5, eight 61.6 / 69.7)
                 launch_chained(decode_kernel<T, G, BIT, kCompact, 2>, grid, stream, *p);
             else
                 launch_chained(decode_several_kernel<T, G, BIT, kCompact, kCompact ? 2 : 4, true>, grid, stream, *p);

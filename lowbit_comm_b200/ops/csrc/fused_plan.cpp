@@ -685,10 +685,11 @@ void bind_fused_plan(py::module_& m) {
              py::arg("numel"), py::arg("stages"), py::arg("scale"), py::arg("update_residual"), py::arg("ef_local"),
              py::arg("epoch"), py::arg("stream"), py::arg("phase_mask") = static_cast<int>(LBC_PIPE_ALL),
              py::arg("gate") = false);
-    // The all-reduce of one rank through the general kernels (deterministic rounding), as PipeAllReducePlan::one_rank.
+    // The all-reduce of one rank through the general kernels (deterministic rounding), as PipeAllReducePlan::one_rank.  (Their
+    // residual follows one rule, T(prepared - result), whatever `ef_local` says.)
     m.def("one_rank_general", [](int group_size, int bit, int topk, int quant_type, int dtype, int max_blocks, int64_t max_numel,
                                  const at::Tensor& x, const std::optional<at::Tensor>& out,
-                                 const std::optional<at::Tensor>& residual, int passes, bool update_residual, bool,
+                                 const std::optional<at::Tensor>& residual, int passes, bool update_residual, bool /*ef_local*/,
                                  uintptr_t status_host) -> std::optional<at::Tensor> {
         const int64_t n = x.numel();
         if (n == 0 || n > max_numel || !plain(x, x.device()) || !of_type(x, dtype) || !like(out, x) || !like(residual, x) ||

@@ -17,19 +17,12 @@
 // selected that the profile does not keep); kept elements are patched into the packed words (8 predicated permutes
 // instead of 32 selects on the values); a code of a code-book is one look-up and one addition; payload
 // words move as vectors; records of the compact layout, which break the alignment, are built in shared memory.
-// Measured on a B200: encode + decode of 5 M fp32 elements, e2m1 code-book, 81 -> 27 us (the search in a table in
-// constant memory took one pass per distinct entry in a warp); all-reduce of one rank, 32 Mi bf16 elements, one kept
-// value per group, 107 -> 72 us.  Then, without the clamp and the NaN test where the selection has shown that no value
-// needs them, without a trip through packed bytes, and with a block per tile: 72 -> 36 us, and 81 -> 25 us for the
-// code-book.  Then, with a look-up instead of fourteen thresholds: 24.5 -> 18.4 us for the code-book; encode of 16 MiB,
-// beyond L2, bf16 22.5 -> 14.5 us, fp32 14.0 -> 8.6, one-rank pass bf16 22.7 -> 14.5.  The one-rank pass without the
-// places of the kept elements: 35.9 -> 30.8 us (32 Mi bf16 elements, one kept value); of 16 MiB beyond L2, two kept
-// values, bf16 14.4 -> 12.4 us, fp32 12.4 -> 10.3.  Each kernel started before the one ahead of it ends: 29.2 us, and
-// 15.4 us for the code-book; 12.3 us with the encoder for local payloads and native calls around both.  The rare warps
-// of the one-rank pass out of line, its group steps without loops, its sums and products two to an instruction, 32 Mi
-// elements beyond L2: bf16 29.6 -> 26.6 us, two kept values 30.6 -> 28.2, fp16 in 4 bits 29.1 -> 26.4.  Without a residual, in
-// kernels that know it, with the next tile under way, no clamp for fp32 and quotients without branches: 22.9 us, 24.5 and 22.9; 16 Mi
-// bf16 elements 15.0 -> 12.1, fp32 with two kept values 24.2 -> 21.2; encode of 4 Mi fp32 elements in records, one kept value, 6.46 -> 5.43.
+// Measured on a B200, first form / now: encode + decode of 5 M fp32 elements, e2m1 code-book, 81 -> 11.9 us (the search in a
+// table in constant memory took one pass per distinct entry in a warp; now kernels and host calls are level); all-reduce
+// of one rank, 32 Mi bf16 elements, one kept value per group, 107 -> 22.9 us, two 24.5, fp16 in 4 bits 22.9; 16 Mi 12.1,
+// fp32 with two kept values 21.2.  What gave most: no clamp and no NaN test where the selection has shown that no value
+// needs them, no trip through packed bytes and a block per tile (72 -> 36 us), no places of the kept elements where
+// magnitudes decide (35.9 -> 30.8), the next tile under way without a residual (26.2 -> 22.9).
 
 #include <cmath>
 #include <cstring>
@@ -373,7 +366,7 @@ __device__ __forceinline__ GroupMeta select_group(float (&v)[16], const Packed16
             for (int off = lanes / 2; off > 0; off >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, off, lanes));
             return a;
         };
-        if constexpr (!Kind<KIND>::book) {      // (linear codes without a clamp: the first maximum looks for a NaN, which is passed over else)
+        if constexpr (!Kind<KIND>::book) {      // (linear codes without a clamp: the first maximum looks for a NaN)
             float top = fabsf(v[0]);
 #pragma unroll
             for (int i = 1; i + 1 < 16; i += 2) top = max_nan(top, fabsf(v[i]), fabsf(v[i + 1]));
@@ -613,7 +606,7 @@ __device__ __noinline__ void book_codes_far(const float* v, float safe, const fl
 }
 // Is the scale of every group of the warp one that book_code takes?  (A 16-bit group with more NaN than it keeps has NaN for
 // its scale, which bounds no value: the test is on the scale as stored, false for NaN.)
-__device__ __forceinline__ bool book_near(float stored) { return __all_sync(0xffffffffu, stored < 1.0e30f); }
+__device__ __forceinline__ bool book_near(float stored) { return __all_sync(0xffffffffu, stored < kNearScale); }
 
 // Codes of 16 values against the group's scale, as bit patterns whose low byte (nibble) is the code.  With `near` (no infinity, no
 // NaN and no scale above kNearScale in any group of the warp) no value that is not kept verbatim is larger than the scale, so
@@ -922,29 +915,25 @@ __global__ void __launch_bounds__(kThreads, 4) quant_general_kernel(const __grid
     grid_signal(p.signal);      // no-op without destinations to notify
 }
 
-// Encode of a payload of this GPU alone, on its vectors: no destinations, shards or signal, whole tiles without a test per chunk.
-// kCompact: records, built in shared memory.
-// What bounds it: instruction issue.  Before (quant_general_kernel, which asks every chunk where it goes) and here, beyond L2: 64 MiB,
-// bf16, planar, one kept value 34.8 -> 30.6 us, two 42.0 -> 38.5, e2m1 36.8 -> 31.1, with one kept value 46.0 -> 42.1, records of e2m1
-// 38.2 -> 34.2; fp32 25.6 -> 20.7, 31.1 -> 27.5, 22.0 -> 17.4, 28.0 -> 23.2, 22.6 -> 18.0; 1 MiB in a graph, bf16, here 2.14, 2.19, 2.10, fp32 2.20, 2.51, 1.97.
-// Blocks per SM, 4 against 5 (no spills at either in these), 64 MiB: bf16, one kept value 32.1 / 30.6 us, two 39.8 / 40.3, e2m1 31.9 / 33.8, its
-// records 34.6 / 36.1; fp32 23.0 / 21.7, 29.3 / 27.5, 19.0 / 18.9, 20.1 / 18.3, e2m1 with one kept value 23.8 / 25.1; 16 MiB bf16, one
-// kept value 10.4 / 9.5, fp32 7.8 / 7.5.
+// Encode of a payload of this GPU alone, on its vectors: no destinations, shards or signal, whole tiles without a test per
+// chunk.  kCompact: records, built in shared memory.
+// What bounds it: instruction issue.  quant_general_kernel, which asks every chunk where it goes, and here, 64 MiB beyond L2:
+// bf16, one kept value 34.8 -> 30.6 us, e2m1 36.8 -> 31.1, fp32 25.6 -> 20.7 and 22.0 -> 17.4.
+// Blocks per SM with a residual, 4 / 5 (no spills at either in these), 64 MiB: bf16, one kept value 32.1 / 30.6, two 39.8 /
+// 40.3, e2m1 31.9 / 33.8; fp32 23.0 / 21.7, 29.3 / 27.5, 19.0 / 18.9, e2m1 with one kept value 23.8 / 25.1.
 template <typename T, int TOPK, int KIND>
 constexpr int encode_blocks() {
     if (KIND == kBook) return sizeof(T) == 4 && TOPK == 0 ? 5 : 4;
     return KIND != kBookNoise && (TOPK == 1 || (TOPK == 2 && sizeof(T) == 4)) ? 5 : 4;
 }
-// kPrepare: with a residual or prepared_out.  Without, in kernels that know it, and their blocks per SM (us, beyond L2 from 8 Mi bf16 elements on;
-// with both / without, 3 / 4 / 5 / 6): bf16, one kept value 2 Mi 3.38 / 2.98 / 2.74 / 3.37 / 3.81, 4 Mi 4.59 / 4.48 / 4.28 / 4.52 / 4.56, 8 Mi 8.07 /
-// 8.63 / 8.10 / 8.28 / 8.29; two 4 Mi 5.70 / 5.46 / 5.26 / 5.64 / 5.89, 8 Mi 10.9 / 10.3 / 9.97 / 10.5 / 10.9; e2m1 2 Mi 3.04 / 3.40 / 3.42 / 3.52 / 4.00,
-// 4 Mi 5.16 / 4.93 / 5.21 / 5.02 / 5.61, 8 Mi 8.97 / 8.51 / 8.67 / 8.16 / 8.43; fp32, one kept value 2 Mi 4.23 / 3.25 / 3.04 / 3.83 / 4.44, 4 Mi 5.53 /
-// 4.97 / 4.60 / 5.20 / 5.31; two 5.27 / 4.45 / 4.27 / 5.17 / 6.01, 6.97 / 6.87 / 6.65 / 6.87 / 7.14; e2m1 3.87 / 3.72 / 3.45 / 3.62 / 4.06, 5.41 / 5.56 /
-// 5.09 / 5.40 / 5.69.
+// kPrepare: with a residual or prepared_out.  Without, in kernels that know it, four blocks per SM, 16-bit code-books five:
+// 4 / 5, bf16, one kept value 2 Mi elements 2.74 / 3.37, 8 Mi 8.10 / 8.28, two 9.97 / 10.5, e2m1 8.67 / 8.16; fp32, one kept
+// value 4 Mi 4.60 / 5.20, e2m1 5.09 / 5.40.
 template <typename T, int KIND>
 constexpr int encode_plain_blocks() { return KIND == kBook && sizeof(T) == 2 ? 5 : 4; }
 template <typename T, int TOPK, int KIND, bool kCompact, bool kPrepare>
-__global__ void __launch_bounds__(kThreads, kPrepare ? encode_blocks<T, TOPK, KIND>() : encode_plain_blocks<T, KIND>()) encode_general_kernel(const __grid_constant__ LbcQuantGeneral p) {
+__global__ void __launch_bounds__(kThreads, kPrepare ? encode_blocks<T, TOPK, KIND>() : encode_plain_blocks<T, KIND>())
+encode_general_kernel(const __grid_constant__ LbcQuantGeneral p) {
     chain_wait();
     const GroupShape shape = GroupShape::of<T, TOPK, KIND>(p.group_size);
     const int lanes = shape.lanes, VB = shape.VB, MB = shape.MB;
@@ -1148,8 +1137,9 @@ __device__ __noinline__ void requantize_by_place(uint32_t* words, int lane, int 
 // The all-reduce of a group of one rank: encode and decode in registers, no payload (see roundtrip_kernels.cu; here
 // the decoded values are rounded to T before the residual is taken, the rule of these profiles).
 // Blocks per SM, 16-bit, with a residual 4 against 5, 32 Mi bf16: one kept value 26.6 / 27.5 us, two 28.2 / 29.1; others: see the launcher.
-// kFull: with a residual or two passes.  kPlain: neither.  kPlainAhead: neither, and the loads of a block's next tile are issued ahead of the
-// work on the present one (which waits for its loads at four blocks per SM otherwise: ncu, long scoreboard 3.6 per issue).
+// kFull: with a residual or two passes.  kPlain: neither.  kPlainAhead: neither, and the loads of a block's next tile are issued
+// ahead of the work on the present one (which waits for its loads at four blocks per SM otherwise: ncu, long scoreboard 3.6
+// per issue).
 enum : int { kFull = 0, kPlain = 1, kPlainAhead = 2 };
 template <typename T, int TOPK, int KIND, int kForm>
 __device__ __forceinline__ void roundtrip_general(const LbcRoundtripGeneral& p) {
@@ -1188,7 +1178,8 @@ __device__ __forceinline__ void roundtrip_general(const LbcRoundtripGeneral& p) 
         else elems = load_elems<T>(x, first, end, vec);                 // zeros past the end
         if (kForm == kPlainAhead) {
             const int64_t then = at + int64_t(gridDim.x) * kThreads;
-            if (whole_at(then)) next = load_elems<T>(x, (then + threadIdx.x) * kElemsPerThread, (then + threadIdx.x) * kElemsPerThread + 16, true);
+            const int64_t from = (then + threadIdx.x) * kElemsPerThread;
+            if (whole_at(then)) next = load_elems<T>(x, from, from + 16, true);
         }
         if (res != nullptr) {
             float v[16], r[16];
@@ -1323,7 +1314,8 @@ struct QuantGeneral {
             // Linear codes, 16 bits, planar, one kept value: many waves of full grids, where five blocks per SM hide more than the
             // residual's registers cost (bf16 8 Mi 7.95 / 8.00, fp16 7.80 / 7.62, bf16 12 Mi 12.7 / 13.0, 16 Mi 16.4 / 16.8); looping grids
             // have no waves (32 Mi 30.2 / 28.7).
-            const int64_t tiles = (p.numel + kThreads * kElemsPerThread - 1) / (kThreads * kElemsPerThread), full = lbc_default_max_blocks();
+            const int64_t tiles = (p.numel + kThreads * kElemsPerThread - 1) / (kThreads * kElemsPerThread);
+            const int64_t full = lbc_default_max_blocks();
             bool plain = KIND != kBookNoise && p.residual == nullptr && p.prepared_out == nullptr;
             if (KIND == kBook && sizeof(T) == 2) plain = plain && tiles > (p.compact && TOPK == 0 ? full : full / 2);
             if (KIND == kBook && sizeof(T) == 4 && TOPK == 0) plain = plain && tiles > full / 4 && tiles <= full;
@@ -1349,19 +1341,18 @@ template <typename T, int TOPK, int KIND>
 struct DequantGeneral {
     static constexpr bool noise = false;
     static void run(const LbcDequantGeneral& p, int grid, cudaStream_t s) {
-        // Blocks per SM.  A decode waits for its loads: as many as the registers leave without the sum into `out`, but for 16-bit
-        // records with kept values, whose words are read one by one (64 MiB beyond L2 24.5 us with four, 25.2 with eight), and
-        // for fp32 up to two default grids, where six blocks per SM leave a short last wave (16 MiB, e2m1, 5.58 / 5.89 us).  64 MiB, 4 blocks
-        // against 8 (fp32: 6): bf16, one kept value 21.9 / 20.1, two 23.1 / 22.4, e2m1 19.4 / 17.1, its records 20.6 / 17.8; fp32 16.6 / 15.2,
-        // 18.1 / 16.4, 16.6 / 14.7, 17.1 / 15.2; 16 MiB bf16 7.94 / 7.01, 8.45 / 7.73, 7.63 / 6.42, 8.14 / 6.50.
+        // Blocks per SM.  A decode waits for its loads: as many as the registers leave without the sum into `out` (64 MiB, 4 / 8,
+        // bf16, one kept value 21.9 / 20.1, e2m1 19.4 / 17.1; fp32, 4 / 6, 16.6 / 15.2), but for 16-bit records with kept
+        // values, whose words are read one by one (24.5 / 25.2), and fp32 up to two default grids, where six leave a short last
+        // wave (16 MiB, e2m1, 5.58 / 5.89).
         const int64_t tiles = (p.numel + kThreads * kElemsPerThread - 1) / (kThreads * kElemsPerThread);
-        // Five, above half a default grid and up to two (us, four / five / six / eight): fp32, e2m1 4 Mi 4.41 / 4.11 / 4.12 / 4.27, 5 M 5.11 /
-        // 4.74 / 4.79 / 4.72, one kept value 4.44 / 4.05 / 4.07 / 4.68, 5.58 / 5.11 / 5.07 / 5.29, below, 2 Mi, 2.94 / 3.18 / 3.45 / 3.01; planar
-        // 16-bit payloads with kept values and linear codes, bf16, one 4 Mi 3.39 / 3.35 / 3.42 / 3.67, 8 Mi 6.10 / 5.97 / 5.88 / 6.14, two 3.72 / 3.57 /
-        // 3.59 / 4.03, 6.80 / 6.58 / 6.43 / 6.90, below, 2 Mi, 2.60 / 2.57 / 2.79 / 2.50, above, 16 Mi, - / 11.8 / - / 11.3.  16-bit ones in 4 bits up to
-        // one default grid, five / eight, bf16, two kept values: 3 Mi 3.22 / 3.89, 4 Mi 3.86 / 3.96, 5 Mi 4.61 / 4.45, 8 Mi 6.84 / 6.43.
+        // Five, above half a default grid and up to two: fp32 (four / five / six, e2m1, 2 Mi elements 2.94 / 3.18 / 3.45, 4 Mi
+        // 4.41 / 4.11 / 4.12, 5 M 5.11 / 4.74 / 4.79), planar 16-bit payloads with kept values and linear codes (five / eight, bf16, one:
+        // 2 Mi 2.57 / 2.50, 4 Mi 3.35 / 3.67, 8 Mi 5.97 / 6.14, 16 Mi 11.8 / 11.3), those in 4 bits up to one default grid (two:
+        // 3 Mi 3.22 / 3.89, 4 Mi 3.86 / 3.96, 5 Mi 4.61 / 4.45, 8 Mi 6.84 / 6.43).
         const int64_t grid_tiles = lbc_default_max_blocks();
-        const bool five = 2 * tiles > grid_tiles && tiles <= (sizeof(T) == 2 && Kind<KIND>::bit == 4 ? grid_tiles : 2 * grid_tiles) &&
+        const int64_t most = sizeof(T) == 2 && Kind<KIND>::bit == 4 ? grid_tiles : 2 * grid_tiles;
+        const bool five = 2 * tiles > grid_tiles && tiles <= most &&
                           (sizeof(T) == 4 || (!p.compact && TOPK >= 1 && !Kind<KIND>::book));
         const bool many = sizeof(T) == 2 ? !(p.compact && TOPK >= 1) : tiles > 2 * grid_tiles;
         if (five && !p.accumulate)
@@ -1383,16 +1374,13 @@ template <typename T, int TOPK, int KIND>
 struct RoundtripGeneral {
     static constexpr bool noise = true;
     static void run(const LbcRoundtripGeneral& p, int grid, cudaStream_t s) {
-        // No residual and one pass: kernels that know it (what the others hold for both costs registers).  Above one default grid (books
-        // without kept values, which pay for it alone up to there: half of one) 16-bit tensors take as many blocks as are resident, each with its next tile under way.  Before / one tile a
-        // block / resident blocks (4 per SM), bf16: one kept value 4 Mi elements 3.80 / 3.62 / 3.83 us, 6 Mi 5.1 / 5.08 / 4.59, 8 Mi 6.60 /
-        // 6.40 / 5.82, 16 Mi 15.0 / 14.5 / 12.0, 32 Mi 26.2 / 28.2 / 22.8; two 4 Mi 4.07 / 3.96 / 4.21, 8 Mi 7.08 / 6.96 / 6.42, 16 Mi 15.7 / 15.2 /
-        // 13.2, 32 Mi 27.9 / 29.7 / 24.4; e2m1 4 Mi - / 6.23 / 5.70, 8 Mi 9.3 / 10.3 / 8.96, 16 Mi 17.9 / 19.8 / 16.2, 32 Mi 33.1 / 37.1 / 30.0.  Without
-        // the next tile under way 8 Mi with one kept value took 5.89, 32 Mi 25.4; twice the blocks 6.02 and 23.1; three per SM 5.67
-        // and 24.3; five spill; copies into shared memory (cp.async, two tiles ahead) 7.38 and 30.6.
-        // fp32, full grids, before / 4 blocks per SM / 5: one kept value 1 Mi 2.87 / 2.21 / 2.17, 4 Mi 5.59 / 4.81 / 4.69, 16 Mi 22.0 / 20.9 / 21.0;
-        // two 2.88 / 2.22 / 2.43, 5.47 / 4.94 / 5.33, 24.2 / 21.2 / 21.2; e2m1 - / 3.15 / 3.11, - / 7.28 / 6.70, 26.7 / 24.6 / 23.1.  Grids that loop
-        // from one default grid on: 8 Mi with one kept value 10.7 / 10.7 / 10.7, 16 Mi 22.0 / 22.3 / 22.1.
+        // No residual and one pass: kernels that know it (what the others hold for both costs registers).  Above one default
+        // grid 16-bit tensors take as many blocks as are resident, each with its next tile under way: a tile per block /
+        // resident blocks, bf16, one kept value, 4 Mi elements 3.62 / 3.83, 6 Mi 5.08 / 4.59, 16 Mi 14.5 / 12.0, 32 Mi 28.2 / 22.8
+        // (without the next tile under way 25.4, with twice the blocks 23.1).  Books without kept values from half a grid on
+        // (e2m1, 4 Mi 6.23 / 5.70, 32 Mi 37.1 / 30.0); below, the form without a residual does not pay for them.  fp32, full grids:
+        // with a residual's registers / without, one kept value, 4 Mi 5.59 / 4.81, two, 16 Mi 24.2 / 21.2, e2m1 (five blocks per
+        // SM) 26.7 / 23.1; looping gains nothing (16 Mi 20.9 / 22.3).
         const int64_t tiles = (p.numel + kThreads * kElemsPerThread - 1) / (kThreads * kElemsPerThread);
         const auto capped = [&](int64_t blocks) { return unsigned(p.max_blocks > 0 && p.max_blocks < blocks ? p.max_blocks : blocks); };
         if constexpr (KIND != kBookNoise) {
@@ -1413,11 +1401,10 @@ struct RoundtripGeneral {
                 return;
             }
         }
-        // fp32, three blocks per SM or four (64 registers, with spills).  Four are faster for two passes of one kept value without a residual
-        // alone (two, 16 Mi elements: 25.1 / 26.3 us), where three do not hold the whole grid.  Three / four with a residual, one kept value, 8 bits:
-        // 1 Mi elements 3.75 / 5.12, 1.75 Mi 6.21 / 6.86, 2 Mi 7.01 / 7.12, 4 Mi 11.7 / 12.4, 16 Mi 40.5 / 41.4; e2m1 5.42 / 6.39, 7.81 / 8.45,
-        // 8.56 / 8.61, 13.2 / 14.8, 42.3 / 45.5; 8 bits with noise, the last two, 13.2 / 14.4 and 42.2 / 45.5; e2m1 with noise 30.2 / 34.1 and
-        // 107 / 116.
+        // fp32, three blocks per SM or four (64 registers, with spills).  Four are faster for two passes of one kept value without
+        // a residual alone (two kept values, 16 Mi elements: 25.1 / 26.3), where three do not hold the whole grid.  Three / four
+        // with a residual, one kept value, 8 bits: 1 Mi 3.75 / 5.12, 2 Mi 7.01 / 7.12, 16 Mi 40.5 / 41.4; e2m1 42.3 / 45.5, with
+        // noise 107 / 116.
         if constexpr (sizeof(T) == 2) {
             launch_chained(roundtrip_general_kernel<T, TOPK, KIND, 4>, unsigned(grid), s, p);
         } else {

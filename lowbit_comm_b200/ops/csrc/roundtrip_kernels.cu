@@ -183,12 +183,10 @@ struct RoundtripLauncher {
             launch_chained(roundtrip_kernel<T, G, BIT, true, 1>, grid(one), stream, *p);
             return cudaGetLastError();
         }
-        // Two chunks per thread (64 bytes in flight) above one default grid.  One chunk against two, bf16, calls in a CUDA graph going round
-        // three tensors: 0.5 Mi elements 1.58 / 1.68 us, 1 Mi 1.79 / 1.68, 2 Mi 2.41 / 1.93, 3 Mi 2.43 / 2.90 (two leave SMs a
-        // block short), 4 Mi 2.94 / 2.92, 5 Mi (1.08 default grids) 3.15 / 3.08, 6 Mi 3.86 / 3.69, 8 Mi 4.45 / 4.17, 13 M 7.02 / 6.54, 16 Mi
-        // 11.3 / 10.5, 24 Mi 16.3 / 16.4, 33 Mi 21.6 / 22.0, 64 Mi 40.3 / 40.8, 256 Mi 165 / 157.  Four chunks: 8 Mi 4.34, 13 M 7.19.  Blocks
-        // of 128 threads, two chunks: 8 Mi 4.10, 13 M 6.40, 33 Mi 22.1; of 512: 4.45, 6.92, 21.6.  fp32 chunks and chunks with a residual
-        // have 64 bytes in flight already.
+        // Two chunks per thread (64 bytes in flight) above one default grid.  One chunk / two, in a CUDA graph, bf16: 2 Mi
+        // elements 1.91 / 1.93 us, 2.5 Mi 2.44 / 2.69, 4.5 Mi 3.18 / 2.67, 5 Mi (above) 3.62 / 3.42, 8 Mi 4.86 / 4.13, 13.1 M 7.52 / 6.60,
+        // 33 Mi 24.9 / 21.7, 128 Mi 91.1 / 78.9; fp16 3 Mi 2.63 / 3.00, 4.5 Mi 3.09 / 3.08, which is why the line is not lower, where
+        // bf16 would gain (4 Mi 2.91 / 2.68).  fp32 chunks and chunks with a residual have 64 bytes in flight already.
         if constexpr (sizeof(T) == 2) {
             if (one > lbc_default_max_blocks()) {
                 launch_chained(roundtrip_kernel<T, G, BIT, false, 2>, grid((one + 1) / 2), stream, *p);
@@ -208,7 +206,8 @@ cudaError_t lbc_roundtrip(const LbcRoundtrip* p, cudaStream_t stream) {
     if (p == nullptr || p->numel < 0 || (p->passes != 1 && p->passes != 2)) return cudaErrorInvalidValue;
     if (p->residual == nullptr && (p->residual_out != nullptr || p->own_error)) return cudaErrorInvalidValue;
     // the pad is written with the tile that holds the tensor's end: a tensor that fills its tiles has none (see lbc_api.h)
-    if (p->pad < 0 || (p->pad > 0 && p->group_size > 0 && p->numel % (8 * int64_t(p->group_size)) == 0)) return cudaErrorInvalidValue;
+    if (p->pad < 0 || (p->pad > 0 && p->group_size > 0 && p->numel % (8 * int64_t(p->group_size)) == 0))
+        return cudaErrorInvalidValue;
     if (p->numel == 0) return cudaSuccess;
     if (p->x == nullptr || p->out == nullptr) return cudaErrorInvalidValue;
     return lbc::dispatch_profile<lbc::RoundtripLauncher>(p, stream);
